@@ -334,10 +334,14 @@ struct AttnArgs {
   // row_pos / row_seq are given (prefill chunks); lets the tensor-core prefill kernel take them
   int64_t uniform_base = -1, uniform_seq = 0;
   int64_t ldq = 0;  // floats between consecutive rows of q (0: dense, nh*d)
+  // f32 caches: where the tensor-core prefill kernel may keep the cache's f16 pairs (else it allocates)
+  void* pair_ws = nullptr;
+  size_t pair_ws_bytes = 0;
 };
 int launch_attention(const AttnArgs& a, cudaStream_t s);
 size_t attention_split_scratch_bytes(int64_t rows, int64_t nh, int64_t d, int nsplit);
 int launch_attention_split(const AttnArgs& a, float* part, int nsplit, cudaStream_t s, bool* handled);
+size_t attention_prefill_scratch_bytes(const AttnArgs& a);
 int launch_attention_prefill(const AttnArgs& a, int64_t base_pos, int64_t seq, cudaStream_t s, bool* handled);
 
 size_t argmax_scratch_bytes(int64_t n);

@@ -74,6 +74,8 @@ struct dyninfer_cuda_session_t {
   uint8_t* kcache = nullptr;  // [layer][seq][nkv][cap][d]
   uint8_t* vcache = nullptr;
   size_t kv_bytes_each = 0;
+  void* pair_ws = nullptr;  // f32 cache: one sequence's keys and values as f16 pairs (prefill attention)
+  size_t pair_ws_bytes = 0;
   // scratch
   int64_t max_rows = 0;
   float *hidden = nullptr, *xn = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *ctx = nullptr,
@@ -434,6 +436,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       aa.rows = rows, aa.nh = c.heads, aa.nkv = c.kv_heads, aa.d = c.head_dim, aa.cap = cap;
       aa.kv_type = s->kv_type;
       aa.ldq = ldq;
+      aa.pair_ws = s->pair_ws, aa.pair_ws_bytes = s->pair_ws_bytes;
       aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;
       if (launch_attention(aa, st)) return 1;
       // o: hidden += W ctx, then the FFN norm straight into the GEMM's operand
@@ -522,6 +525,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
     aa.rows = rows, aa.nh = c.heads, aa.nkv = c.kv_heads, aa.d = c.head_dim, aa.cap = cap;
     aa.kv_type = s->kv_type;
     aa.ldq = ldq;
+    aa.pair_ws = s->pair_ws, aa.pair_ws_bytes = s->pair_ws_bytes;
     aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;  // a prefill chunk: consecutive positions
     if (launch_attention(aa, st)) return 1;
     bool ffn_normed = false;
@@ -1215,7 +1219,7 @@ void dyninfer_cuda_session_destroy(dyninfer_cuda_session_t* s) {
                  s->logits, s->tokens_dev, s->row_pos_dev, s->row_seq_dev, s->out_token_dev,
                  s->hist_dev, s->hist_count_dev, s->argmax_scratch, s->mega_layers, s->io_dev,
                  s->prof_dev, s->trace_dev, s->prog_dev, s->ll_dev, s->batch_logits, s->batch_tokens_dev, s->tp_part, s->tp_logits,
-                 s->tp_gather, s->scratch, s->qkv1, s->gu1, s->xh, s->xinv, s->gpart};
+                 s->tp_gather, s->scratch, s->pair_ws, s->qkv1, s->gu1, s->xh, s->xinv, s->gpart};
   for (void* p : dev)
     if (p) cudaFree(p);
   if (s->logits_host) cudaFreeHost(s->logits_host);
@@ -1373,6 +1377,15 @@ int dyninfer_cuda_session_ensure_kv_pages(dyninfer_cuda_session_t* s, size_t pag
   s->vcache = nv;
   s->kv_bytes_each = bytes;
   s->pages = page_count;
+  AttnArgs aa{};
+  aa.kv_type = s->kv_type, aa.nkv = c.kv_heads, aa.cap = (int64_t)(page_count * s->page_size);
+  const size_t pair_bytes = c.head_dim == 128 ? attention_prefill_scratch_bytes(aa) : 0;
+  if (pair_bytes > s->pair_ws_bytes) {
+    dev_free(s, s->pair_ws, s->pair_ws_bytes);
+    s->pair_ws = nullptr, s->pair_ws_bytes = 0;
+    if (dev_alloc(s, &s->pair_ws, pair_bytes)) return 1;
+    s->pair_ws_bytes = pair_bytes;
+  }
   destroy_graphs(s);
   return 0;
 }
