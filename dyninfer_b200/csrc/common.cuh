@@ -288,6 +288,7 @@ int launch_norm_prepare(const float* x, const float* partial, int splits, const 
                         const void* w, int w_type, int64_t rows, int64_t width, float eps, __half* xh, float* inv_s,
                         cudaStream_t s);
 // The same for the SwiGLU: rows of [gate | up] -> silu(gate) * up as the GEMM's activation operand.
+bool silu_prepare_takes(int64_t inter);
 int launch_silu_prepare(const float* gate_up, int64_t rows, int64_t inter, __half* xh, float* inv_s, cudaStream_t s);
 // One row of [gate | up] (2 * inter values, deferred or in `gate_up`): y = silu(gate) * up
 int launch_silu_mul_deferred(const Deferred& d, const float* gate_up, int64_t inter, float* y, cudaStream_t s);

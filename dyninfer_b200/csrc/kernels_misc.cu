@@ -1,6 +1,8 @@
 // RMSNorm, RoPE, QK-norm + RoPE + KV write, GQA attention, SiLU*up, argmax.
 #include <math.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace dyn {
@@ -146,19 +148,34 @@ norm_prepare_kernel(const float* __restrict__ x, const float* __restrict__ parti
                     float eps, __half* __restrict__ xh, float* __restrict__ inv_s) {
   __shared__ float red[32];
   const int64_t row = blockIdx.x;
+  pdl_trigger();
   float v[PER], wv[PER];
 #pragma unroll
   for (int k = 0; k < PER; k++) {
     const int64_t i = threadIdx.x + (int64_t)k * blockDim.x;
-    float t = 0.f;
-    if (i < width) {
-      if (S) {
-        for (int z = 0; z < S; z++) t += partial[((int64_t)z * rows + row) * width + i];
-      } else {
-        t = x[row * width + i];
+    wv[k] = i < width ? aux_load(reinterpret_cast<const uint8_t*>(w), w_type, i) : 0.f;
+  }
+  pdl_wait();  // everything but the norm weights comes from the kernels before
+  // the slices outermost: all of a slice's loads are in flight together (one element's slices after the
+  // other waited for an L2 round trip each: 512 x 4096 with two slices 33 us, now 9)
+  if (S) {
+#pragma unroll
+    for (int k = 0; k < PER; k++) v[k] = 0.f;
+#pragma unroll 2
+    for (int z = 0; z < S; z++) {
+      const float* p = partial + ((int64_t)z * rows + row) * width;
+#pragma unroll
+      for (int k = 0; k < PER; k++) {
+        const int64_t i = threadIdx.x + (int64_t)k * blockDim.x;
+        if (i < width) v[k] += p[i];
       }
     }
-    v[k] = t;
+  } else {
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const int64_t i = threadIdx.x + (int64_t)k * blockDim.x;
+      v[k] = i < width ? x[row * width + i] : 0.f;
+    }
   }
   if (residual) {
 #pragma unroll
@@ -170,7 +187,6 @@ norm_prepare_kernel(const float* __restrict__ x, const float* __restrict__ parti
 #pragma unroll
   for (int k = 0; k < PER; k++) {
     const int64_t i = threadIdx.x + (int64_t)k * blockDim.x;
-    wv[k] = i < width ? aux_load(reinterpret_cast<const uint8_t*>(w), w_type, i) : 0.f;
     if (hidden && i < width) hidden[row * width + i] = v[k];
   }
   float ss = 0.f;
@@ -201,37 +217,78 @@ int launch_norm_prepare(const float* x, const float* partial, int splits, const 
   const int threads = width >= 1024 ? 256 : (width >= 256 ? 128 : 32);  // rms_norm_kernel's: same summation order
   DYN_CHECK(width <= 32 * threads, "row of %lld elements is too wide for the fused RMSNorm", (long long)width);
   const int S = splits > 1 ? splits : 0;
+  cudaError_t e;
   if (width <= 8 * threads)
-    norm_prepare_kernel<8><<<(unsigned)rows, threads, 0, s>>>(x, partial, S, rows, residual, hidden, w, w_type, width, eps, xh, inv_s);
+    e = launch_pdl(norm_prepare_kernel<8>, dim3((unsigned)rows), dim3(threads), 0, s, x, partial, S, rows, residual, hidden, w, w_type, width, eps, xh, inv_s);
   else if (width <= 16 * threads)
-    norm_prepare_kernel<16><<<(unsigned)rows, threads, 0, s>>>(x, partial, S, rows, residual, hidden, w, w_type, width, eps, xh, inv_s);
+    e = launch_pdl(norm_prepare_kernel<16>, dim3((unsigned)rows), dim3(threads), 0, s, x, partial, S, rows, residual, hidden, w, w_type, width, eps, xh, inv_s);
   else
-    norm_prepare_kernel<32><<<(unsigned)rows, threads, 0, s>>>(x, partial, S, rows, residual, hidden, w, w_type, width, eps, xh, inv_s);
+    e = launch_pdl(norm_prepare_kernel<32>, dim3((unsigned)rows), dim3(threads), 0, s, x, partial, S, rows, residual, hidden, w, w_type, width, eps, xh, inv_s);
+  DYN_CUDA(e);
   count_launch();
   DYN_CUDA(cudaGetLastError());
   return 0;
 }
 
-__global__ void __launch_bounds__(256)
+// One block per row of [gate | up]; PER4 groups of four values per thread are evaluated once and stay in
+// registers between the row's maximum and the conversion, four pairs of loads in flight (two passes
+// over the row, each waiting for its loads, took 50 us on 512 x 12288; now 13).
+template <int PER4>
+__global__ void __launch_bounds__(1024)
 silu_prepare_kernel(const float* __restrict__ gu, int64_t I, __half* __restrict__ xh, float* __restrict__ inv_s) {
   __shared__ float red[32];
+  pdl_trigger();
   const int64_t row = blockIdx.x;
-  const float* g = gu + row * 2 * I;
-  auto val = [&](int64_t i) {
-    const float gv = g[i];
-    return (gv / (1.0f + expf(-gv))) * g[I + i];
-  };
+  const float4* g = reinterpret_cast<const float4*>(gu + row * 2 * I);
+  const float4* u = reinterpret_cast<const float4*>(gu + row * 2 * I + I);
+  const int n4 = (int)(I >> 2);
+  auto val = [](float gv, float uv) { return (gv / (1.0f + expf(-gv))) * uv; };
+  float4 v[PER4];
   float mx = 0.f;
-  for (int64_t i = threadIdx.x; i < I; i += blockDim.x) mx = fmaxf(mx, fabsf(val(i)));
+  pdl_wait();
+#pragma unroll
+  for (int k0 = 0; k0 < PER4; k0 += 4) {  // at most four pairs in flight: 1024 threads leave 64 registers each
+    float4 w[4];
+#pragma unroll
+    for (int j = 0; j < 4 && k0 + j < PER4; j++) {
+      const int i = threadIdx.x + (k0 + j) * blockDim.x;
+      v[k0 + j] = i < n4 ? g[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      w[j] = i < n4 ? u[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int j = 0; j < 4 && k0 + j < PER4; j++) {
+      float4& q = v[k0 + j];
+      q = make_float4(val(q.x, w[j].x), val(q.y, w[j].y), val(q.z, w[j].z), val(q.w, w[j].w));
+      mx = fmaxf(mx, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
+    }
+  }
   float sc, is;
   f16_row_scale(mx, red, &sc, &is);
   if (threadIdx.x == 0) inv_s[row] = is;
-  for (int64_t i = threadIdx.x; i < I; i += blockDim.x) xh[row * I + i] = __float2half_rn(val(i) * sc);
+#pragma unroll
+  for (int k = 0; k < PER4; k++) {
+    const int i = threadIdx.x + k * blockDim.x;
+    if (i >= n4) continue;
+    __half2 h[2] = {__floats2half2_rn(v[k].x * sc, v[k].y * sc), __floats2half2_rn(v[k].z * sc, v[k].w * sc)};
+    *reinterpret_cast<uint2*>(xh + row * I + 4 * i) = *reinterpret_cast<const uint2*>(h);
+  }
 }
+
+// Rows as wide as a block's registers hold (1024 threads x 28 values); multiples of four.
+bool silu_prepare_takes(int64_t inter) { return inter % 4 == 0 && inter <= 28 * 1024; }
 
 int launch_silu_prepare(const float* gate_up, int64_t rows, int64_t inter, __half* xh, float* inv_s, cudaStream_t s) {
   if (rows == 0 || inter == 0) return 0;
-  silu_prepare_kernel<<<(unsigned)rows, 256, 0, s>>>(gate_up, inter, xh, inv_s);
+  DYN_CHECK(silu_prepare_takes(inter), "row of %lld elements is too wide for the fused SwiGLU", (long long)inter);
+  // few groups per thread (4) as long as the block does not grow past 1024 threads
+  const int64_t n4 = inter / 4;
+  const int threads = (int)std::min<int64_t>(1024, std::max<int64_t>(32, ((n4 + 3) / 4 + 31) / 32 * 32));
+  const dim3 grid((unsigned)rows), block(threads);
+  const int per = (int)((n4 + threads - 1) / threads);
+  cudaError_t e;
+  if (per <= 4) e = launch_pdl(silu_prepare_kernel<4>, grid, block, 0, s, gate_up, inter, xh, inv_s);
+  else e = launch_pdl(silu_prepare_kernel<7>, grid, block, 0, s, gate_up, inter, xh, inv_s);
+  DYN_CUDA(e);
   count_launch();
   DYN_CUDA(cudaGetLastError());
   return 0;
@@ -443,21 +500,145 @@ __global__ void __launch_bounds__(128) qkv_prepare_kernel(QkvPrepArgs a, FreqTab
   }
 }
 
+// Head dims 64 and 128: a warp per (row, head), so that a head's values never leave the warp (the form above
+// takes a block of two warps and three block barriers per head: 512 rows of 48 heads 30 us, now 9). A lane
+// holds the E = D / 64 rotated pairs (i, i + D / 2), i = E * lane ...; the K-slice sums are added in
+// ascending order, four slices' loads in flight.
+template <int KV, int D>
+__global__ void __launch_bounds__(256) qkv_prepare_warp_kernel(const QkvPrepArgs a, const __grid_constant__ FreqTable ft) {
+  using T = typename KvT<KV>::T;
+  constexpr int E = D / 64, HALF = D / 2;
+  const int lane = threadIdx.x & 31;
+  const int64_t r = blockIdx.x, hh = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
+  pdl_trigger();
+  if (hh >= a.nh + 2 * a.nkv) return;
+  const int kind = hh < a.nh ? 0 : (hh < a.nh + a.nkv ? 1 : 2);
+  const int64_t head = kind == 0 ? hh : (kind == 1 ? hh - a.nh : hh - a.nh - a.nkv);
+  const int i0 = E * lane;
+  float w[2 * E];  // norm weights: not produced by the kernels before
+  if (kind < 2 && a.has_norm) {
+    const uint8_t* nwb = reinterpret_cast<const uint8_t*>(kind == 0 ? a.q_norm_w : a.k_norm_w);
+#pragma unroll
+    for (int e = 0; e < E; e++) w[e] = aux_load(nwb, a.norm_w_type, i0 + e), w[E + e] = aux_load(nwb, a.norm_w_type, HALF + i0 + e);
+  }
+  pdl_wait();
+  const int64_t pos = a.row_pos ? a.row_pos[r] : a.base_pos + r;
+  const int64_t seq = a.row_seq ? a.row_seq[r] : 0;
+  struct __align__(4 * E) Vec { float v[E]; };
+  float x[2 * E];  // values i0 .. then HALF + i0 ..
+  float* qv = a.q + r * (a.ldq ? a.ldq : a.nh * D) + head * D;
+  const DeferredCols& dc = kind == 0 ? a.dq : (kind == 1 ? a.dk : a.dv);
+  if (dc.S) {
+    const float* p = dc.partial + r * dc.N + dc.col + head * D + i0;
+    const int64_t step = dc.rows * dc.N;
+#pragma unroll
+    for (int e = 0; e < 2 * E; e++) x[e] = 0.f;
+    for (int j0 = 0; j0 < dc.S; j0 += 4) {
+      Vec lo[4], hi[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (j0 + u < dc.S) {
+          lo[u] = *reinterpret_cast<const Vec*>(p + (j0 + u) * step);
+          hi[u] = *reinterpret_cast<const Vec*>(p + (j0 + u) * step + HALF);
+        }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (j0 + u < dc.S) {
+#pragma unroll
+          for (int e = 0; e < E; e++) x[e] += lo[u].v[e], x[E + e] += hi[u].v[e];
+        }
+    }
+    const float sc = dc.scale ? dc.scale[0] : 1.0f;
+#pragma unroll
+    for (int e = 0; e < 2 * E; e++) x[e] *= sc;
+  } else {
+    const float* in = kind == 0 ? qv
+                                : (kind == 1 ? a.k + r * (a.ldk ? a.ldk : a.nkv * D) + head * D
+                                             : a.v + r * (a.ldv ? a.ldv : a.nkv * D) + head * D);
+    const Vec lo = *reinterpret_cast<const Vec*>(in + i0), hi = *reinterpret_cast<const Vec*>(in + HALF + i0);
+#pragma unroll
+    for (int e = 0; e < E; e++) x[e] = lo.v[e], x[E + e] = hi.v[e];
+  }
+  struct __align__(sizeof(T) * E) Out { T v[E]; };
+  Out olo, ohi;
+  if (kind == 2) {
+    T* dst = reinterpret_cast<T*>(a.vcache) + ((seq * a.nkv + head) * a.cap + pos) * D;
+#pragma unroll
+    for (int e = 0; e < E; e++) olo.v[e] = KvT<KV>::enc(x[e]), ohi.v[e] = KvT<KV>::enc(x[E + e]);
+    *reinterpret_cast<Out*>(dst + i0) = olo;
+    *reinterpret_cast<Out*>(dst + HALF + i0) = ohi;
+    return;
+  }
+  if (a.has_norm) {
+    // the order of the block form's sum (thread i held elements i and i + D/2 of its head): same bits
+    float ss[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) ss[e] = fmaf(x[E + e], x[E + e], x[e] * x[e]);
+#pragma unroll
+    for (int o = E == 2 ? 8 : 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int e = 0; e < E; e++) ss[e] += __shfl_xor_sync(0xffffffffu, ss[e], o);
+    }
+    if (E == 2) {
+      ss[0] += ss[E - 1];
+      ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 16);
+    }
+    const float inv = 1.0f / sqrtf(ss[0] / (float)D + a.eps);
+#pragma unroll
+    for (int e = 0; e < 2 * E; e++) x[e] = __fmul_rn(__fmul_rn(x[e], inv), w[e]);
+  }
+  if (a.has_rope) {
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      float lo, hi;
+      rope_pair(x[e], x[E + e], (float)pos, ft.f[i0 + e], &lo, &hi);
+      x[e] = lo, x[E + e] = hi;
+    }
+  }
+  if (kind == 0) {
+    Vec lo, hi;
+#pragma unroll
+    for (int e = 0; e < E; e++) lo.v[e] = x[e], hi.v[e] = x[E + e];
+    *reinterpret_cast<Vec*>(qv + i0) = lo;
+    *reinterpret_cast<Vec*>(qv + HALF + i0) = hi;
+  } else {
+    T* dst = reinterpret_cast<T*>(a.kcache) + ((seq * a.nkv + head) * a.cap + pos) * D;
+#pragma unroll
+    for (int e = 0; e < E; e++) olo.v[e] = KvT<KV>::enc(x[e]), ohi.v[e] = KvT<KV>::enc(x[E + e]);
+    *reinterpret_cast<Out*>(dst + i0) = olo;
+    *reinterpret_cast<Out*>(dst + HALF + i0) = ohi;
+  }
+}
+
+template <int KV>
+static int run_qkv_prepare(const QkvPrepArgs& a, const FreqTable& ft, cudaStream_t s) {
+  const unsigned heads = (unsigned)(a.nh + 2 * a.nkv);
+  // the warp form loads pairs of floats: rows and deferred columns have to start on 8-byte boundaries
+  const bool pairs = !((a.ldq | a.ldk | a.ldv | a.dq.N | a.dk.N | a.dv.N | a.dq.col | a.dk.col | a.dv.col) & 1) &&
+                     !((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v) |
+                        reinterpret_cast<uintptr_t>(a.dq.partial) | reinterpret_cast<uintptr_t>(a.dk.partial) |
+                        reinterpret_cast<uintptr_t>(a.dv.partial)) & 7);
+  const dim3 warps((unsigned)a.rows, (heads + 7) / 8);
+  if (a.d == 128 && pairs)
+    DYN_CUDA(launch_pdl(qkv_prepare_warp_kernel<KV, 128>, warps, dim3(256), 0, s, a, ft));
+  else if (a.d == 64)
+    DYN_CUDA(launch_pdl(qkv_prepare_warp_kernel<KV, 64>, warps, dim3(256), 0, s, a, ft));
+  else
+    qkv_prepare_kernel<KV><<<dim3((unsigned)a.rows, heads), a.d >= 128 ? 64 : 32, 0, s>>>(a, ft);
+  count_launch();
+  DYN_CUDA(cudaGetLastError());
+  return 0;
+}
+
 int launch_qkv_prepare(const QkvPrepArgs& a, const FreqTable& ft, cudaStream_t s) {
   if (a.rows == 0) return 0;
   DYN_CHECK(a.d % 2 == 0 && a.d <= 256, "head_dim %lld unsupported (even, <= 256)", (long long)a.d);
-  dim3 grid((unsigned)a.rows, (unsigned)(a.nh + 2 * a.nkv));
-  const int threads = a.d >= 128 ? 64 : 32;
-  if (a.kv_type == E_F32) {
-    qkv_prepare_kernel<E_F32><<<grid, threads, 0, s>>>(a, ft);
-  } else if (a.kv_type == E_F16) {
-    qkv_prepare_kernel<E_F16><<<grid, threads, 0, s>>>(a, ft);
-  } else if (a.kv_type == E_BF16) {
-    qkv_prepare_kernel<E_BF16><<<grid, threads, 0, s>>>(a, ft);
-  } else
-    DYN_CHECK(false, "kv_type %d unsupported", a.kv_type);
-  count_launch();
-  DYN_CUDA(cudaGetLastError());
+  switch (a.kv_type) {
+    case E_F32: return run_qkv_prepare<E_F32>(a, ft, s);
+    case E_F16: return run_qkv_prepare<E_F16>(a, ft, s);
+    case E_BF16: return run_qkv_prepare<E_BF16>(a, ft, s);
+    default: DYN_CHECK(false, "kv_type %d unsupported", a.kv_type);
+  }
   return 0;
 }
 

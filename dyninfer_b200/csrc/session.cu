@@ -372,7 +372,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   // per layer and five passes over the activations fewer, with the same bits as the separate kernels.
   // (one block per row: with few rows -- batched decode steps -- the separate multi-block kernels are faster:
   // 32 rows of the 32B shape 13.5 against 14.4 ms per step)
-  bool fuse_n = rows >= 64 && !tp && s->xh && H <= 8192;
+  bool fuse_n = rows >= 64 && !tp && s->xh && H <= 8192 && silu_prepare_takes(c.inter);
   for (int l = 0; l < c.layers && fuse_n; l++) {
     const LayerW& L = s->layers[l];
     const WRef* ws[8] = {L.qkv_parts >= 2 ? &L.qkv : &L.q, L.qkv_parts >= 2 ? nullptr : &L.k, L.qkv_parts == 3 ? nullptr : &L.v,
