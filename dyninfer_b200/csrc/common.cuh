@@ -198,6 +198,42 @@ struct WRef {
   }
 };
 
+#ifdef __CUDACC__
+// Where the four elements k .. k + 3 (k a multiple of 4) of a row sit in fragment order (in halfs; for MLX-U4
+// the eight elements of an aligned run share 16 bytes and k is a multiple of 8).
+__device__ __forceinline__ int sk_frag_off(int enc, int k) {
+  const int r = k & 255, unit = (k >> 8) * 256;
+  int c, t, b = 0;
+  if (enc == E_Q4_K) {
+    t = r >> 6, b = (r >> 5) & 1, c = (r & 31) >> 2;
+  } else if (enc == E_Q6_K) {
+    c = (r >> 7) * 4 + ((r & 15) >> 2), b = (r >> 6) & 1, t = (r & 63) >> 4;
+  } else {
+    t = r >> 6;
+    c = ((r >> 5) & 1) * 4;
+    if (enc == E_Q4_0 || enc == E_Q4_1) c += (r & 15) >> 2, b = (r >> 4) & 1;
+    else c += (r & 31) >> 3, b = (r >> 2) & 1;
+  }
+  return unit + (c * 4 + t) * 8 + b * 4;
+}
+// Eight elements k .. k + 7 (k a multiple of 8) times `sc` into a row in fragment order.
+__device__ __forceinline__ void sk_store_frag8(__half* row, int enc, int k, const float (&v)[8], float sc) {
+  auto pk = [&](int i, int j) {
+    const __half2 h = __floats2half2_rn(v[i] * sc, v[j] * sc);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  };
+  if (enc == E_MLX_U4) {
+    *reinterpret_cast<uint4*>(row + sk_frag_off(enc, k)) = make_uint4(pk(0, 4), pk(1, 5), pk(2, 6), pk(3, 7));
+  } else if (enc == E_Q4_0 || enc == E_Q4_1 || enc == E_Q4_K) {
+    *reinterpret_cast<uint2*>(row + sk_frag_off(enc, k)) = make_uint2(pk(0, 2), pk(1, 3));
+    *reinterpret_cast<uint2*>(row + sk_frag_off(enc, k + 4)) = make_uint2(pk(4, 6), pk(5, 7));
+  } else {
+    *reinterpret_cast<uint2*>(row + sk_frag_off(enc, k)) = make_uint2(pk(0, 1), pk(2, 3));
+    *reinterpret_cast<uint2*>(row + sk_frag_off(enc, k + 4)) = make_uint2(pk(4, 5), pk(6, 7));
+  }
+}
+#endif
+
 int wref_from_api(const dyninfer_cuda_weight_t* w, WRef* out);
 
 // ---- small device helpers -------------------------------------------------------
@@ -225,6 +261,15 @@ __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
+}
+
+// Power of two that puts a row's largest magnitude into [2^12, 2^13) -- no f16 overflow, ordinary entries stay out
+// of the subnormals -- and its inverse.
+__device__ __forceinline__ void f16_scale_for(float mx, float* s, float* inv_s) {
+  int e = 0;
+  if (mx > 0.f && mx < 3.0e38f) frexpf(mx, &e);
+  *s = ldexpf(1.0f, 13 - e);
+  *inv_s = ldexpf(1.0f, e - 13);
 }
 
 struct FreqTable {  // inverse RoPE frequencies, one per rotated pair (head_dim <= 256)
@@ -258,6 +303,16 @@ int launch_dqgemm_tc(const WRef& w, const void* x, int x_type, int64_t M, float*
 // Whether launch_dqgemm_tc takes the product, and the activation rows its tiling pads M to.
 bool dqgemm_tc_takes(const WRef& w, int64_t M);
 int64_t dqgemm_tc_padded_rows(const WRef& w, int64_t M);
+// The fused dequant GEMM for 1..64 activation rows (gemm_skinny.cu).
+// Activations: f16 rows in the fragment order of the weight's encoding (sk_frag_off), gemm_skinny_terms planes of
+// [M, K], scaled by a power of two per row, with the inverse scales beside them.
+bool gemm_skinny_takes(const WRef& w, int64_t M);
+int gemm_skinny_terms(const WRef& w, int64_t M);
+int launch_gemm_skinny(const WRef& w, const __half* x, const float* x_inv, int64_t M, float* y, const float* residual,
+                       bool swiglu, cudaStream_t s, bool* handled);
+int launch_skinny_prepare(const WRef& w, const void* x, int x_type, int64_t M, __half* out, float* inv_s, cudaStream_t s);
+int launch_linear_skinny(const WRef& w, const void* x, int x_type, int64_t M, float* y, const float* residual, cudaStream_t s,
+                         bool* handled);
 bool gemv_cs_q8_0_shape_ok(const WRef& w, int M);
 size_t gemv_cs_q8_0_workspace_bytes(const WRef& w, int M);
 int launch_gemv_cs_q8_0(const WRef& w, const void* x, int x_type, float* y, const float* residual, uint8_t* ws,
@@ -287,6 +342,9 @@ int launch_rms_norm(const float* x, const void* w, int w_type, int64_t rows, int
 int launch_norm_prepare(const float* x, const float* partial, int splits, const float* residual, float* hidden,
                         const void* w, int w_type, int64_t rows, int64_t width, float eps, __half* xh, float* inv_s,
                         cudaStream_t s);
+// RMSNorm(x) * w of every row as the skinny GEMM's operand: f16 in the fragment order of encoding `enc`.
+int launch_norm_frag(const float* x, const void* w, int w_type, int64_t rows, int64_t width, float eps, int enc, __half* xh,
+                     float* inv_s, cudaStream_t s);
 // The same for the SwiGLU: rows of [gate | up] -> silu(gate) * up as the GEMM's activation operand.
 bool silu_prepare_takes(int64_t inter);
 int launch_silu_prepare(const float* gate_up, int64_t rows, int64_t inter, __half* xh, float* inv_s, cudaStream_t s);
@@ -340,6 +398,11 @@ struct AttnArgs {
   size_t pair_ws_bytes = 0;
 };
 int launch_attention(const AttnArgs& a, cudaStream_t s);
+// Decode attention on 2-byte caches (attention_decode.cu): `part` holds rows * nh * nsplit * (d + 2) floats. The
+// context goes to a.ctx, or with `frag` straight into the f16 operand of a product with weights of encoding `enc`.
+bool attention_decode_takes(const AttnArgs& a);
+int attention_decode_splits(const AttnArgs& a);
+int launch_attention_decode(const AttnArgs& a, float* part, int nsplit, __half* frag, float* inv_s, int enc, cudaStream_t s);
 size_t attention_split_scratch_bytes(int64_t rows, int64_t nh, int64_t d, int nsplit);
 int launch_attention_split(const AttnArgs& a, float* part, int nsplit, cudaStream_t s, bool* handled);
 size_t attention_prefill_scratch_bytes(const AttnArgs& a);

@@ -79,12 +79,7 @@ __host__ __device__ inline size_t xstage_sx_bytes(int K, int rows) { return (siz
 
 // Power-of-two scale for one activation row whose largest magnitude is `mx`:
 // mx * s lies in [2^12, 2^13).
-__device__ __forceinline__ void scale_for(float mx, float* s, float* inv_s) {
-  int e = 0;
-  if (mx > 0.f && mx < 3.0e38f) frexpf(mx, &e);
-  *s = ldexpf(1.0f, 13 - e);
-  *inv_s = ldexpf(1.0f, e - 13);
-}
+__device__ __forceinline__ void scale_for(float mx, float* s, float* inv_s) { f16_scale_for(mx, s, inv_s); }
 
 // Writes the fragments of one (block, lane-quarter) of one activation row.
 //   HILO: two columns (2*m, 2*m+1) hold hi and lo; else one column m holds the f16 value.

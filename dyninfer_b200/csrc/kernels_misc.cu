@@ -230,6 +230,72 @@ int launch_norm_prepare(const float* x, const float* partial, int splits, const 
   return 0;
 }
 
+// RMSNorm of a row straight into the skinny GEMM's operand (f16, fragment order, power-of-two scale). One block
+// per row, a thread takes R runs of eight elements and keeps them in registers.
+template <int R>
+__global__ void __launch_bounds__(256)
+norm_frag_kernel(const float* __restrict__ x, const void* __restrict__ w, int w_type, int width, float eps, int enc,
+                 __half* __restrict__ xh, float* __restrict__ inv_s) {
+  __shared__ float red[32];
+  pdl_trigger();
+  const int64_t row = blockIdx.x;
+  float v[R][8], wv[R][8];
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int k = (threadIdx.x + i * blockDim.x) * 8;
+#pragma unroll
+    for (int e = 0; e < 8; e++) wv[i][e] = k < width ? aux_load(reinterpret_cast<const uint8_t*>(w), w_type, k + e) : 0.f;
+  }
+  pdl_wait();
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int k = (threadIdx.x + i * blockDim.x) * 8;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (k < width) {
+      a = __ldcg(reinterpret_cast<const float4*>(x + row * width + k));
+      b = __ldcg(reinterpret_cast<const float4*>(x + row * width + k) + 1);
+    }
+    v[i][0] = a.x, v[i][1] = a.y, v[i][2] = a.z, v[i][3] = a.w, v[i][4] = b.x, v[i][5] = b.y, v[i][6] = b.z, v[i][7] = b.w;
+  }
+#pragma unroll
+  for (int i = 0; i < R; i++)
+#pragma unroll
+    for (int e = 0; e < 8; e++) ss = fmaf(v[i][e], v[i][e], ss);
+  ss = block_sum(ss, red);
+  const float inv = 1.0f / sqrtf(ss / (float)width + eps);
+  float mx = 0.f;
+#pragma unroll
+  for (int i = 0; i < R; i++)
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      v[i][e] = __fmul_rn(__fmul_rn(v[i][e], inv), wv[i][e]);
+      mx = fmaxf(mx, fabsf(v[i][e]));
+    }
+  float sc, is;
+  f16_row_scale(mx, red, &sc, &is);
+  if (threadIdx.x == 0) inv_s[row] = is;
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int k = (threadIdx.x + i * blockDim.x) * 8;
+    if (k < width) sk_store_frag8(xh + row * width, enc, k, v[i], sc);
+  }
+}
+
+int launch_norm_frag(const float* x, const void* w, int w_type, int64_t rows, int64_t width, float eps, int enc, __half* xh,
+                     float* inv_s, cudaStream_t s) {
+  DYN_CHECK(width % 256 == 0 && width <= 8192, "row of %lld elements does not fit the fused RMSNorm", (long long)width);
+  const int runs = (int)(width / 8), threads = std::min(256, runs);
+  cudaError_t e;
+  if (runs <= 256) e = launch_pdl(norm_frag_kernel<1>, dim3((unsigned)rows), dim3(threads), 0, s, x, w, w_type, (int)width, eps, enc, xh, inv_s);
+  else if (runs <= 512) e = launch_pdl(norm_frag_kernel<2>, dim3((unsigned)rows), dim3(threads), 0, s, x, w, w_type, (int)width, eps, enc, xh, inv_s);
+  else e = launch_pdl(norm_frag_kernel<4>, dim3((unsigned)rows), dim3(threads), 0, s, x, w, w_type, (int)width, eps, enc, xh, inv_s);
+  DYN_CUDA(e);
+  count_launch();
+  DYN_CUDA(cudaGetLastError());
+  return 0;
+}
+
 // One block per row of [gate | up]; PER4 groups of four values per thread are evaluated once and stay in
 // registers between the row's maximum and the conversion, four pairs of loads in flight (two passes
 // over the row, each waiting for its loads, took 50 us on 512 x 12288; now 13).
@@ -876,8 +942,23 @@ int launch_attention(const AttnArgs& a, cudaStream_t s) {
       return 1;
     if (handled) return 0;
   }
+  if (attention_decode_takes(a)) {
+    const int nsplit = attention_decode_splits(a);
+    const size_t bytes = attention_split_scratch_bytes(a.rows, a.nh, a.d, nsplit);
+    float* part = reinterpret_cast<float*>(thread_scratch(bytes));
+    const bool pooled = part == nullptr;
+    if (pooled) {
+      if (keep_scratch_pool_cached()) return 1;
+      DYN_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&part), bytes, s));
+    }
+    const int rc = launch_attention_decode(a, part, nsplit, nullptr, nullptr, 0, s);
+    const cudaError_t fe = pooled ? cudaFreeAsync(part, s) : cudaSuccess;
+    if (rc) return rc;
+    if (fe != cudaSuccess) return cuda_fail(fe, "cudaFreeAsync", __FILE__, __LINE__);
+    return 0;
+  }
   if (a.d == 64 || a.d == 128 || a.d == 256) {
-    // decode / batched decode: slice every row's keys over enough CTAs to fill the GPU. The slice
+    // f32 caches, decode / batched decode: slice every row's keys over enough CTAs to fill the GPU. The slice
     // count depends only on shapes and capacity, so a captured graph stays valid as positions grow.
     int nsplit = (int)(592 / (a.rows * a.nh));
     const int by_cap = (int)(a.cap / 128);
@@ -975,45 +1056,71 @@ argmax_final_kernel(const ArgPair* part, int count, int64_t* out) {
   if (threadIdx.x == 0) out[0] = si[0] == 0x7fffffffffffffffLL ? 0 : si[0];
 }
 
-// One block per row of v [rows, n]: first strict maximum of every row (batched decode).
-__global__ void __launch_bounds__(1024)
+// First strict maximum of every row of v [rows, n] (batched decode). A cluster of AR_CL blocks takes a row (one
+// block per row left most SMs idle: 8 rows of 151936 logits 30 us, now 6); candidates meet in rank 0's shared memory.
+constexpr int AR_CL = 8, AR_T = 512;
+__global__ void __cluster_dims__(AR_CL, 1, 1) __launch_bounds__(AR_T)
 argmax_rows_kernel(const float* __restrict__ v, int64_t n, int shards, int64_t* out) {
-  __shared__ float sv[32];
-  __shared__ long long si[32];
+  __shared__ float sv[AR_T / 32], cv[AR_CL];
+  __shared__ long long si[AR_T / 32], ci[AR_CL];
+  const int rank = blockIdx.x % AR_CL;
+  const int64_t r = blockIdx.x / AR_CL, rows = gridDim.x / AR_CL;
   float bv = -INFINITY;
   long long bi = 0x7fffffffffffffffLL;
+  pdl_trigger();
+  pdl_wait();
   // slice w of this row sits at [w][row][n]; its elements are indices w * n + j
   for (int w = 0; w < shards; w++) {
-    const float* row = v + ((int64_t)w * gridDim.x + blockIdx.x) * n;
-    for (int64_t i = threadIdx.x; i < n; i += 1024) {
-      const float x = row[i];
-      if (x > -INFINITY && arg_better(x, (int64_t)w * n + i, bv, bi)) bv = x, bi = (int64_t)w * n + i;
+    const float* row = v + ((int64_t)w * rows + r) * n;
+    for (int64_t i0 = (int64_t)rank * AR_T + threadIdx.x; i0 < n; i0 += 8 * AR_CL * AR_T) {
+      float x[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int64_t i = i0 + (int64_t)u * AR_CL * AR_T;
+        x[u] = i < n ? row[i] : -INFINITY;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int64_t i = (int64_t)w * n + i0 + (int64_t)u * AR_CL * AR_T;
+        if (x[u] > -INFINITY && arg_better(x[u], i, bv, bi)) bv = x[u], bi = i;
+      }
     }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-    const long long oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (arg_better(ov, oi, bv, bi)) bv = ov, bi = oi;
-  }
-  if (lane == 0) sv[warp] = bv, si[warp] = bi;
-  __syncthreads();
-  if (warp == 0) {
-    bv = sv[lane], bi = si[lane];
+  auto warp_best = [&]() {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
       const long long oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (arg_better(ov, oi, bv, bi)) bv = ov, bi = oi;
     }
-    if (lane == 0) out[blockIdx.x] = bi == 0x7fffffffffffffffLL ? 0 : bi;
+  };
+  warp_best();
+  if (lane == 0) sv[warp] = bv, si[warp] = bi;
+  __syncthreads();
+  if (warp == 0) {
+    bv = lane < AR_T / 32 ? sv[lane] : -INFINITY, bi = lane < AR_T / 32 ? si[lane] : 0x7fffffffffffffffLL;
+    warp_best();
+    if (lane == 0) {
+      uint32_t av, ai;
+      asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(av) : "r"((uint32_t)__cvta_generic_to_shared(&cv[rank])));
+      asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(ai) : "r"((uint32_t)__cvta_generic_to_shared(&ci[rank])));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(av), "f"(bv) : "memory");
+      asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(ai), "l"(bi) : "memory");
+    }
+    __syncwarp();
+  }
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+  if (rank == 0 && threadIdx.x == 0) {
+    for (int k = 0; k < AR_CL; k++)
+      if (k == 0 || arg_better(cv[k], ci[k], bv, bi)) bv = cv[k], bi = ci[k];
+    out[r] = bi == 0x7fffffffffffffffLL ? 0 : bi;
   }
 }
 
 int launch_argmax_rows(const float* v, int64_t rows, int64_t n, int64_t* out, cudaStream_t s) {
   DYN_CHECK(rows >= 1 && n >= 1, "argmax_rows: rows and n must be >= 1");
-  argmax_rows_kernel<<<(unsigned)rows, 1024, 0, s>>>(v, n, 1, out);
+  DYN_CUDA(launch_pdl(argmax_rows_kernel, dim3((unsigned)(rows * AR_CL)), dim3(AR_T), 0, s, v, n, 1, out));
   count_launch();
   DYN_CUDA(cudaGetLastError());
   return 0;
@@ -1022,7 +1129,7 @@ int launch_argmax_rows(const float* v, int64_t rows, int64_t n, int64_t* out, cu
 int launch_argmax_rows_sharded(const float* v, int64_t rows, int64_t n_local, int shards, int64_t* out,
                                cudaStream_t s) {
   DYN_CHECK(rows >= 1 && n_local >= 1 && shards >= 1, "argmax_rows: rows, n and shards must be >= 1");
-  argmax_rows_kernel<<<(unsigned)rows, 1024, 0, s>>>(v, n_local, shards, out);
+  DYN_CUDA(launch_pdl(argmax_rows_kernel, dim3((unsigned)(rows * AR_CL)), dim3(AR_T), 0, s, v, n_local, shards, out));
   count_launch();
   DYN_CUDA(cudaGetLastError());
   return 0;

@@ -86,6 +86,8 @@ struct dyninfer_cuda_session_t {
   float *xinv = nullptr, *gpart = nullptr;
   int64_t xh_rows = 0, xh_cols = 0;
   size_t gpart_bytes = 0;
+  __half* sk_x = nullptr;   // few-row steps: one product's activations in fragment order, and their inverse scales
+  float* sk_inv = nullptr;
   float *qkv1 = nullptr, *gu1 = nullptr;  // rows of [q | k | v] and of [gate | up] for the fused products
   int64_t *tokens_dev = nullptr, *row_pos_dev = nullptr, *row_seq_dev = nullptr,
           *out_token_dev = nullptr, *hist_dev = nullptr, *hist_count_dev = nullptr;
@@ -365,6 +367,25 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
     if (d->S) thread_scratch_hold(d->ws_bytes);
     return 0;
   };
+  // 5 to 64 rows on one GPU (batched decode steps, short prompts): the skinny GEMM, its operands written by the
+  // kernels in front of it (norm, attention merge), the residuals and the SwiGLU applied behind it: ten launches
+  // per layer, each a programmatic dependent of the one before, so that weights stream while it drains. (0.6B
+  // MLX-U4, 8 sequences at context 512: 3.2 ms per step on the tcgen05 GEMM with its activation passes and
+  // K-split reductions.) Four rows and fewer stay on the kernels that carry 22 bits of an activation.
+  auto frag_class = [](int enc) { return enc == E_Q4_1 ? (int)E_Q4_0 : enc; };
+  bool skinny = rows > 4 && rows <= 64 && !tp && s->sk_x && H % 256 == 0 && H <= 8192 && c.inter % 32 == 0;
+  for (int l = 0; l < c.layers && skinny; l++) {
+    const LayerW& L = s->layers[l];
+    for (const WRef* w : {&L.q, &L.k, &L.v, &L.o, &L.gate, &L.up, &L.down})
+      skinny = skinny && gemm_skinny_takes(*w, rows) && gemm_skinny_terms(*w, rows) == 1;
+    skinny = skinny && frag_class(L.q.enc) == frag_class(L.k.enc) && frag_class(L.q.enc) == frag_class(L.v.enc) && L.gate_up.data;
+  }
+  auto few = [&](const WRef& w, float* y, const float* residual, bool swiglu) -> int {
+    bool handled = false;
+    if (launch_gemm_skinny(w, s->sk_x, s->sk_inv, rows, y, residual, swiglu, st, &handled)) return 1;
+    DYN_CHECK(handled, "skinny GEMM refused a product it had accepted");
+    return 0;
+  };
   // Many rows on one GPU (prefill chunks), every product on the dequant GEMM: RMSNorm
   // and SwiGLU write the GEMM's activation operand themselves (f16 rows + inverse scales) and the K-split
   // sums of o / down are added inside the following residual + RMSNorm kernel, those of a single [q; k; v]
@@ -372,7 +393,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   // per layer and five passes over the activations fewer, with the same bits as the separate kernels.
   // (one block per row: with few rows -- batched decode steps -- the separate multi-block kernels are faster:
   // 32 rows of the 32B shape 13.5 against 14.4 ms per step)
-  bool fuse_n = rows >= 64 && !tp && s->xh && H <= 8192 && silu_prepare_takes(c.inter);
+  bool fuse_n = !skinny && rows >= 64 && !tp && s->xh && H <= 8192 && silu_prepare_takes(c.inter);
   for (int l = 0; l < c.layers && fuse_n; l++) {
     const LayerW& L = s->layers[l];
     const WRef* ws[8] = {L.qkv_parts >= 2 ? &L.qkv : &L.q, L.qkv_parts >= 2 ? nullptr : &L.k, L.qkv_parts == 3 ? nullptr : &L.v,
@@ -393,6 +414,52 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   };
   for (int l = 0; l < c.layers; l++) {
     const LayerW& L = s->layers[l];
+    if (skinny) {
+      if (launch_norm_frag(s->hidden, L.attn_norm.ptr, L.attn_norm.type, rows, H, c.eps, L.q.enc, s->sk_x, s->sk_inv, st)) return 1;
+      float *qp = s->q, *kp = s->k, *vp = s->v;
+      int64_t ldq = 0, ldk = 0, ldv = 0;
+      if (L.qkv_parts >= 2) {
+        qp = s->qkv1, kp = qp + qd;
+        ldq = ldk = L.qkv_parts == 3 ? qd + 2 * kvd : qd + kvd;
+        if (few(L.qkv, qp, nullptr, false)) return 1;
+        if (L.qkv_parts == 3) vp = kp + kvd, ldv = ldq;
+        else if (few(L.v, vp, nullptr, false)) return 1;
+      } else if (few(L.q, qp, nullptr, false) || few(L.k, kp, nullptr, false) || few(L.v, vp, nullptr, false)) {
+        return 1;
+      }
+      QkvPrepArgs pa{};
+      pa.q = qp, pa.k = kp, pa.v = vp;
+      pa.kcache = s->kcache + (size_t)l * layer_stride, pa.vcache = s->vcache + (size_t)l * layer_stride;
+      pa.q_norm_w = L.q_norm.ptr, pa.k_norm_w = L.k_norm.ptr, pa.norm_w_type = L.q_norm.type;
+      pa.row_pos = s->row_pos_dev, pa.row_seq = s->row_seq_dev, pa.base_pos = 0;
+      pa.rows = rows, pa.nh = c.heads, pa.nkv = c.kv_heads, pa.d = c.head_dim, pa.cap = cap;
+      pa.kv_type = s->kv_type, pa.has_norm = c.qk_norm ? 1 : 0, pa.has_rope = c.rope ? 1 : 0;
+      pa.eps = c.eps;
+      pa.ldq = ldq, pa.ldk = ldk, pa.ldv = ldv;
+      if (launch_qkv_prepare(pa, s->freq, st)) return 1;
+      AttnArgs aa{};
+      aa.q = qp, aa.kcache = pa.kcache, aa.vcache = pa.vcache;
+      aa.row_pos = s->row_pos_dev, aa.row_seq = s->row_seq_dev, aa.base_pos = 0;
+      aa.ctx = s->ctx;
+      aa.rows = rows, aa.nh = c.heads, aa.nkv = c.kv_heads, aa.d = c.head_dim, aa.cap = cap;
+      aa.kv_type = s->kv_type;
+      aa.ldq = ldq;
+      aa.pair_ws = s->pair_ws, aa.pair_ws_bytes = s->pair_ws_bytes;
+      aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;
+      const int nsplit = attention_decode_splits(aa);
+      void* part = thread_scratch(attention_split_scratch_bytes(rows, c.heads, c.head_dim, nsplit));
+      if (attention_decode_takes(aa) && part && !(chunk_start >= 0 && rows >= 32)) {
+        if (launch_attention_decode(aa, reinterpret_cast<float*>(part), nsplit, s->sk_x, s->sk_inv, L.o.enc, st)) return 1;
+      } else if (launch_attention(aa, st) || launch_skinny_prepare(L.o, s->ctx, E_F32, rows, s->sk_x, s->sk_inv, st)) {
+        return 1;
+      }
+      if (few(L.o, s->hidden, s->hidden, false) ||
+          launch_norm_frag(s->hidden, L.ffn_norm.ptr, L.ffn_norm.type, rows, H, c.eps, L.gate.enc, s->sk_x, s->sk_inv, st) ||
+          few(L.gate_up, s->act, nullptr, true) || launch_skinny_prepare(L.down, s->act, E_F32, rows, s->sk_x, s->sk_inv, st) ||
+          few(L.down, s->hidden, s->hidden, false))
+        return 1;
+      continue;
+    }
     if (fuse_n) {
       if (!xh_ready && launch_norm_prepare(s->hidden, nullptr, 0, nullptr, nullptr, L.attn_norm.ptr, L.attn_norm.type, rows, H,
                                            c.eps, s->xh, s->xinv, st))
@@ -566,6 +633,13 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   }
   if (all_rows) {
     // batched decode: every row is the last token of its own sequence
+    if (rows > 4 && rows <= 64 && !tp && s->sk_x && H % 256 == 0 && H <= 8192 && gemm_skinny_takes(s->lm_head, rows) &&
+        gemm_skinny_terms(s->lm_head, rows) == 1) {
+      if (launch_norm_frag(s->hidden, s->out_norm.ptr, s->out_norm.type, rows, H, c.eps, s->lm_head.enc, s->sk_x, s->sk_inv, st) ||
+          few(s->lm_head, s->batch_logits, nullptr, false))
+        return 1;
+      return launch_argmax_rows(s->batch_logits, rows, c.vocab, s->batch_tokens_dev, st);
+    }
     if (launch_rms_norm(s->hidden, s->out_norm.ptr, s->out_norm.type, rows, H, c.eps, s->xn, st)) return 1;
     if (tp) {
       // every rank scores its rows of the vocabulary; the slices are gathered as
@@ -1002,10 +1076,34 @@ int dyninfer_cuda_session_create_with_file_params(
         placed.insert(run[i]);
       }
     };
+    // MLX-U4: the words, the scales and the biases of a run lie back to back, each in a range of their own
+    auto place_mlx = [&](const std::vector<std::string>& names) {
+      static const char* const comps[3] = {"packed", "scales", "biases"};
+      size_t n = 0;
+      for (; n < names.size(); n++) {
+        auto it = pd.find(names[n]);
+        if (it == pd.end() || it->second.enc != E_MLX_U4 || it->second.shape.size() != 2 || it->second.comps.size() != 3) break;
+        const ParamDesc &p = it->second, &p0 = pd[names[0]];
+        if (p.shape[1] != p0.shape[1] || p.group != p0.group || p.aux != p0.aux) break;
+        bool whole = true;
+        for (const char* c : comps) whole = whole && p.comps.count(c) && p.comps.at(c).length % 16 == 0;
+        if (!whole) break;
+      }
+      if (n < 2) return;
+      for (const char* c : comps)
+        for (size_t i = 0; i < n; i++) {
+          Upload* u = &pd[names[i]].comps[c];
+          u->arena_off = cursor;
+          cursor += i + 1 < n ? u->length : (u->length + 64 + 255) / 256 * 256;
+          placed.insert(u);
+        }
+    };
     for (int l = 0; l < cfg.layers; l++) {
       const std::string b = "blk." + std::to_string(l) + ".";
-      place_run({b + "attn_q.weight", b + "attn_k.weight", b + "attn_v.weight"});
-      place_run({b + "ffn_gate.weight", b + "ffn_up.weight"});
+      const std::vector<std::string> qkv = {b + "attn_q.weight", b + "attn_k.weight", b + "attn_v.weight"};
+      const std::vector<std::string> gu = {b + "ffn_gate.weight", b + "ffn_up.weight"};
+      place_run(qkv), place_mlx(qkv);
+      place_run(gu), place_mlx(gu);
     }
     for (auto& p : pd)
       for (auto& c : p.second.comps) {
@@ -1106,8 +1204,10 @@ int dyninfer_cuda_session_create_with_file_params(
       return fail();
     {
       auto follows = [](const WRef& a, const WRef& b) {
-        return a.enc == b.enc && a.enc != E_MLX_U4 && a.cols == b.cols &&
-               reinterpret_cast<const uint8_t*>(b.data) == reinterpret_cast<const uint8_t*>(a.data) + a.total_bytes();
+        if (a.enc != b.enc || a.cols != b.cols || b.data != a.data + a.rows * a.row_bytes()) return false;
+        if (a.enc != E_MLX_U4) return true;
+        const int64_t aux = a.rows * (a.cols / a.group) * aux_elem_bytes(a.aux);
+        return a.group == b.group && a.aux == b.aux && b.scales == a.scales + aux && b.biases == a.biases + aux;
       };
       if (follows(L.q, L.k)) {
         L.qkv = L.q;
@@ -1147,6 +1247,11 @@ int dyninfer_cuda_session_create_with_file_params(
         const int64_t per = std::max<int64_t>(1, std::min<int64_t>(32, 592 / (r * cfg.heads)));
         need = std::max(need, attention_split_scratch_bytes(r, cfg.heads, cfg.head_dim, (int)per));
       }
+      for (int64_t r = 1; r <= std::max<int64_t>(64, cfg.batch); r++) {  // ... and those of the tensor-core form
+        const int64_t per = std::max<int64_t>(1, std::min<int64_t>(32, 3 * std::max(1, sm_count()) / (r * cfg.kv_heads)));
+        need = std::max(need, attention_split_scratch_bytes(r, cfg.heads, cfg.head_dim, (int)per));
+      }
+      need = std::max(need, (size_t)3 * 64 * std::max(cfg.hidden, cfg.inter) * 2 + 4096);  // activations of a few-row product
       if (dev_alloc(s, &s->scratch, need)) return fail();
       s->scratch_bytes = need;
       set_thread_scratch(s->scratch, s->scratch_bytes);  // `scope` was entered before the region existed
@@ -1219,7 +1324,7 @@ void dyninfer_cuda_session_destroy(dyninfer_cuda_session_t* s) {
                  s->logits, s->tokens_dev, s->row_pos_dev, s->row_seq_dev, s->out_token_dev,
                  s->hist_dev, s->hist_count_dev, s->argmax_scratch, s->mega_layers, s->io_dev,
                  s->prof_dev, s->trace_dev, s->prog_dev, s->ll_dev, s->batch_logits, s->batch_tokens_dev, s->tp_part, s->tp_logits,
-                 s->tp_gather, s->scratch, s->pair_ws, s->qkv1, s->gu1, s->xh, s->xinv, s->gpart};
+                 s->tp_gather, s->scratch, s->pair_ws, s->sk_x, s->sk_inv, s->qkv1, s->gu1, s->xh, s->xinv, s->gpart};
   for (void* p : dev)
     if (p) cudaFree(p);
   if (s->logits_host) cudaFreeHost(s->logits_host);
@@ -1276,6 +1381,8 @@ int dyninfer_cuda_session_configure_paged_kv(dyninfer_cuda_session_t* s, size_t 
          (dev_alloc(s, (void**)&s->xh, (size_t)(rows + rows / 2 + 64) * std::max(c.hidden, c.inter) * 2) ||
           dev_alloc(s, (void**)&s->xinv, (size_t)(rows + rows / 2 + 64) * 4) ||
           dev_alloc(s, (void**)&s->gpart, (size_t)8 * rows * std::max<int64_t>(c.hidden, qd + 2 * kvd) * 4))) ||
+        (c.tp_world == 1 && (dev_alloc(s, (void**)&s->sk_x, (size_t)64 * std::max({(int64_t)c.hidden, (int64_t)c.inter, qd}) * 2) ||
+                             dev_alloc(s, (void**)&s->sk_inv, 64 * 4))) ||
         dev_alloc(s, (void**)&s->qkv1, (size_t)rows * (qd + 2 * kvd) * 4) ||
         dev_alloc(s, (void**)&s->gu1, (size_t)rows * 2 * c.inter * 4) ||
         (c.tp_world > 1 && dev_alloc(s, (void**)&s->tp_part, (size_t)rows * c.hidden * 4)) ||

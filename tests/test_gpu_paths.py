@@ -25,3 +25,32 @@ def test_attention_prefill_f32_cache(native_lib, oracle, s, start, nh, nkv, mag)
     want = oracle.attention(q, np.nan_to_num(kc), np.nan_to_num(vc), start, s)
     assert np.isfinite(got).all()
     assert helpers.rel_err(got, want) < 2e-5
+
+
+SKINNY = ["gguf.q4_0", "gguf.q4_1", "gguf.q8_0", "gguf.q6_k", "gguf.q4_k", "mlx.affine.u4", "plain.bf16", "plain.f16"]
+
+
+@pytest.mark.parametrize("enc", SKINNY)
+@pytest.mark.parametrize("m,n,k", [(5, 40, 512), (8, 1000, 3072), (9, 33, 5120), (16, 130, 1024), (17, 1024, 2048),
+                                   (33, 513, 1536), (64, 4096, 1024), (64, 48, 12800)])
+def test_linear_few_rows(native_lib, oracle, enc, m, n, k):
+    """5 to 64 activation rows: ragged rows and tiles, row groups of 8 that are not full, K split over warps and
+    over the CTAs of a cluster; a row of zeros and one far outside the f16 range."""
+    from dyninfer_b200 import ops
+    from test_gpu_ops import make_pair
+    dw, ow = make_pair(oracle, enc, n, k, seed=n + m)
+    x = np.random.default_rng(m).normal(size=(m, k)).astype(np.float32)
+    x[1] = 0.0
+    x[2] *= 1e7
+    got = ops.linear(dw, torch.from_numpy(x).cuda()).cpu().numpy()
+    want = oracle.linear(ow, x, fast=True)
+    assert np.isfinite(got).all()
+    for r in (0, 2, m - 1):
+        assert helpers.rel_err(got[r], want[r]) < 1e-3
+    assert not got[1].any()
+    others = np.delete(np.arange(m), 2)
+    assert helpers.rel_err(got[others], want[others]) < (1e-5 if enc.startswith("plain") and m <= 16 else 1e-3)
+    if m > 8:
+        xb = torch.from_numpy(x).to(torch.bfloat16)
+        got = ops.linear(dw, xb.cuda()).cpu().numpy()
+        assert helpers.rel_err(got[others], oracle.linear(ow, xb.float().numpy(), fast=True)[others]) < 1e-3
