@@ -313,6 +313,11 @@ int launch_gemm_skinny(const WRef& w, const __half* x, const float* x_inv, int64
 int launch_skinny_prepare(const WRef& w, const void* x, int x_type, int64_t M, __half* out, float* inv_s, cudaStream_t s);
 int launch_linear_skinny(const WRef& w, const void* x, int x_type, int64_t M, float* y, const float* residual, cudaStream_t s,
                          bool* handled);
+// The exact few-row product (gemv_rows.cu): 1 to 8 rows, optionally RMSNorm in front, residual or SwiGLU behind.
+bool gemv_rows_takes(const WRef& w, int64_t M);
+bool gemv_rows_prefers(const WRef& w, int64_t M);
+int launch_gemv_rows(const WRef& w, const void* x, int x_type, int64_t M, const void* norm_w, int norm_type, float eps, float* y,
+                     const float* residual, bool swiglu, cudaStream_t s, bool* handled);
 bool gemv_cs_q8_0_shape_ok(const WRef& w, int M);
 size_t gemv_cs_q8_0_workspace_bytes(const WRef& w, int M);
 int launch_gemv_cs_q8_0(const WRef& w, const void* x, int x_type, float* y, const float* residual, uint8_t* ws,

@@ -407,7 +407,7 @@ gemm_skinny_kernel(const SkArgs a, const __grid_constant__ CUtensorMap wmap, con
   unsigned parity = 0;
   const uint8_t* xu = xs + kw * KU * 512 + t * 16 + g * pitch;  // activations of the current stage
   for (int i = 0; i < my; i++) {
-    if (!mbar_wait_bounded_sleepy(bars + slot, parity, SK_SPINS, &s_abort, 1000u)) {
+    if (!mbar_try_wait(bars + slot, parity) && !mbar_wait_bounded_sleepy(bars + slot, parity, SK_SPINS, &s_abort, 1000u)) {
       give_up();
       break;  // warp-uniform; the barriers below are still joined
     }

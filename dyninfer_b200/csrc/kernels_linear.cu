@@ -127,6 +127,12 @@ int launch_linear(const WRef& w, const void* x, int x_type, int64_t m, float* y,
   // dequant-in-shared-memory tensor-core GEMM, one pass over the weights for all rows
   // (below 17 rows only for the encodings with a word-fetching GEMM producer, which beats repeated GEMV
   // passes: the GEMM's dequantisation cost does not shrink with the row count)
+  // few rows, exact weights and 22-bit activations: f32 rows up to 4, bf16 rows up to 8
+  if (m <= (x_type == E_BF16 ? 8 : 4) && gemv_rows_prefers(w, m)) {
+    bool handled = false;
+    if (launch_gemv_rows(w, x, x_type, m, nullptr, 0, 0.f, y, residual, false, s, &handled)) return 1;
+    if (handled) return 0;
+  }
   // up to 64 rows beyond what the exact few-row kernels take: one launch, weights streamed once
   if (m <= 64 && m > (x_type == E_BF16 ? 8 : 4)) {
     bool handled = false;

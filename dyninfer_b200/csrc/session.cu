@@ -89,6 +89,7 @@ struct dyninfer_cuda_session_t {
   __half* sk_x = nullptr;   // few-row steps: one product's activations in fragment order, and their inverse scales
   float* sk_inv = nullptr;
   float *qkv1 = nullptr, *gu1 = nullptr;  // rows of [q | k | v] and of [gate | up] for the fused products
+  // a step's tokens, positions and slots: one block of 3 x rows values, filled by one copy (set_step_rows)
   int64_t *tokens_dev = nullptr, *row_pos_dev = nullptr, *row_seq_dev = nullptr,
           *out_token_dev = nullptr, *hist_dev = nullptr, *hist_count_dev = nullptr;
   size_t hist_cap = 0;
@@ -301,6 +302,12 @@ void destroy_graphs(Session* s) {
   s->batch_graphs.clear();
 }
 
+// Where the steps of `rows` rows keep positions and slots: behind the tokens.
+void set_step_rows(Session* s, int64_t rows) {
+  s->row_pos_dev = s->tokens_dev + rows;
+  s->row_seq_dev = s->tokens_dev + 2 * rows;
+}
+
 // Device-side greedy feedback: the produced token becomes the next input, the
 // position advances, and the token is appended to the history buffer.
 __global__ void advance_kernel(int64_t* tokens, int64_t* row_pos, const int64_t* out_token,
@@ -402,6 +409,22 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       if (w && !(dqgemm_tc_takes(*w, rows) && dqgemm_tc_padded_rows(*w, rows) <= s->xh_rows)) fuse_n = false;
     if (H > s->xh_cols || c.inter > s->xh_cols) fuse_n = false;
   }
+  // Up to four rows on one GPU: products with the norm in front and the residual or the SwiGLU behind them, seven
+  // launches per layer (thirteen when norm, activation and K-split sums were launches of their own). A product the
+  // other kernels are better at gets its norm and its activation as separate launches.
+  const bool exact = rows <= 4 && !tp;
+  const NormW* normed_by = nullptr;  // which norm of `hidden` xn holds
+  auto norm_product = [&](const WRef& w, const NormW& nw, float* y, bool swiglu) -> int {
+    bool handled = false;
+    if (gemv_rows_prefers(w, rows) &&
+        launch_gemv_rows(w, s->hidden, E_F32, rows, nw.ptr, nw.type, c.eps, y, nullptr, swiglu, st, &handled))
+      return 1;
+    if (handled) return 0;
+    if (normed_by != &nw && launch_rms_norm(s->hidden, nw.ptr, nw.type, rows, H, c.eps, s->xn, st)) return 1;
+    normed_by = &nw;
+    if (!swiglu) return launch_linear(w, s->xn, E_F32, rows, y, nullptr, st);
+    return launch_linear(w, s->xn, E_F32, rows, s->gu1, nullptr, st) || launch_silu_mul_rows(s->gu1, rows, c.inter, y, st);
+  };
   bool xh_ready = false;  // xh already holds this layer's normalised rows (written by the layer before)
   auto gemm = [&](const WRef& w, const float* x, bool prepared, float* y, const float* residual, TgIo* io) -> int {
     TgIo local;
@@ -539,6 +562,49 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       }
       continue;
     }
+    if (exact) {
+      float *qp = s->q, *kp = s->k, *vp = s->v;
+      int64_t ldq = 0, ldk = 0, ldv = 0;
+      if (L.qkv_parts >= 2) {
+        qp = s->qkv1, kp = qp + qd;
+        ldq = ldk = L.qkv_parts == 3 ? qd + 2 * kvd : qd + kvd;
+        if (norm_product(L.qkv, L.attn_norm, qp, false)) return 1;
+        if (L.qkv_parts == 3) vp = kp + kvd, ldv = ldq;
+        else if (norm_product(L.v, L.attn_norm, vp, false)) return 1;
+      } else if (norm_product(L.q, L.attn_norm, qp, false) || norm_product(L.k, L.attn_norm, kp, false) ||
+                 norm_product(L.v, L.attn_norm, vp, false)) {
+        return 1;
+      }
+      QkvPrepArgs pa{};
+      pa.q = qp, pa.k = kp, pa.v = vp;
+      pa.kcache = s->kcache + (size_t)l * layer_stride, pa.vcache = s->vcache + (size_t)l * layer_stride;
+      pa.q_norm_w = L.q_norm.ptr, pa.k_norm_w = L.k_norm.ptr, pa.norm_w_type = L.q_norm.type;
+      pa.row_pos = s->row_pos_dev, pa.row_seq = s->row_seq_dev, pa.base_pos = 0;
+      pa.rows = rows, pa.nh = c.heads, pa.nkv = c.kv_heads, pa.d = c.head_dim, pa.cap = cap;
+      pa.kv_type = s->kv_type, pa.has_norm = c.qk_norm ? 1 : 0, pa.has_rope = c.rope ? 1 : 0;
+      pa.eps = c.eps;
+      pa.ldq = ldq, pa.ldk = ldk, pa.ldv = ldv;
+      if (launch_qkv_prepare(pa, s->freq, st)) return 1;
+      AttnArgs aa{};
+      aa.q = qp, aa.kcache = pa.kcache, aa.vcache = pa.vcache;
+      aa.row_pos = s->row_pos_dev, aa.row_seq = s->row_seq_dev, aa.base_pos = 0;
+      aa.ctx = s->ctx;
+      aa.rows = rows, aa.nh = c.heads, aa.nkv = c.kv_heads, aa.d = c.head_dim, aa.cap = cap;
+      aa.kv_type = s->kv_type;
+      aa.ldq = ldq;
+      aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;
+      if (launch_attention(aa, st) || launch_linear(L.o, s->ctx, E_F32, rows, s->hidden, s->hidden, st)) return 1;
+      normed_by = nullptr;
+      if (L.gate_up.data && c.inter % 32 == 0) {
+        if (norm_product(L.gate_up, L.ffn_norm, s->act, true)) return 1;
+      } else if (norm_product(L.gate, L.ffn_norm, s->act, false) || norm_product(L.up, L.ffn_norm, s->up, false) ||
+                 launch_silu_mul(s->act, s->up, rows * c.inter, s->act, st)) {
+        return 1;
+      }
+      if (launch_linear(L.down, s->act, E_F32, rows, s->hidden, s->hidden, st)) return 1;
+      normed_by = nullptr;
+      continue;
+    }
     if (!normed &&
         launch_rms_norm(s->hidden, L.attn_norm.ptr, L.attn_norm.type, rows, H, c.eps, s->xn, st))
       return 1;
@@ -663,8 +729,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   } else if (launch_linear(s->lm_head, s->xn, E_F32, 1, s->logits, nullptr, st)) {
     return 1;
   }
-  if (launch_argmax(s->logits, c.vocab, s->out_token_dev, s->argmax_scratch, st)) return 1;
-  (void)kvd;
+  if (launch_argmax_rows(s->logits, 1, c.vocab, s->out_token_dev, st)) return 1;
   return 0;
 }
 
@@ -689,16 +754,11 @@ int capture(Session* s, bool loop, cudaGraphExec_t* out, uint64_t* nodes) {
   cudaGraph_t g = nullptr;
   uint64_t before = s->launches;
   if (tp_warm_collectives(s, 1, false)) return 1;
+  set_step_rows(s, 1);
   DYN_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   int rc = 0;
   if (!loop) {
-    if (cudaMemcpyAsync(s->tokens_dev, s->stage_host, 8, cudaMemcpyHostToDevice, s->stream) !=
-            cudaSuccess ||
-        cudaMemcpyAsync(s->row_pos_dev, s->stage_host + 1, 8, cudaMemcpyHostToDevice, s->stream) !=
-            cudaSuccess ||
-        cudaMemcpyAsync(s->row_seq_dev, s->stage_host + 2, 8, cudaMemcpyHostToDevice, s->stream) !=
-            cudaSuccess)
-      rc = 1;
+    if (cudaMemcpyAsync(s->tokens_dev, s->stage_host, 24, cudaMemcpyHostToDevice, s->stream) != cudaSuccess) rc = 1;
   }
   if (!rc) rc = enqueue_forward(s, 1, 0);
   if (!rc) {
@@ -733,6 +793,7 @@ int capture_batch(Session* s, int64_t rows, cudaGraphExec_t* out, uint64_t* node
   cudaGraph_t g = nullptr;
   const uint64_t before = s->launches;
   if (tp_warm_collectives(s, rows, true)) return 1;
+  set_step_rows(s, rows);
   DYN_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
   const int rc = enqueue_forward(s, rows, 0, true);
   cudaError_t e = cudaStreamEndCapture(s->stream, &g);
@@ -1321,7 +1382,7 @@ void dyninfer_cuda_session_destroy(dyninfer_cuda_session_t* s) {
   if (s->stream) cudaStreamSynchronize(s->stream);
   destroy_graphs(s);
   void* dev[] = {s->arena, s->kcache, s->vcache, s->hidden, s->xn, s->ctx, s->act,
-                 s->logits, s->tokens_dev, s->row_pos_dev, s->row_seq_dev, s->out_token_dev,
+                 s->logits, s->tokens_dev, s->out_token_dev,
                  s->hist_dev, s->hist_count_dev, s->argmax_scratch, s->mega_layers, s->io_dev,
                  s->prof_dev, s->trace_dev, s->prog_dev, s->ll_dev, s->batch_logits, s->batch_tokens_dev, s->tp_part, s->tp_logits,
                  s->tp_gather, s->scratch, s->pair_ws, s->sk_x, s->sk_inv, s->qkv1, s->gu1, s->xh, s->xinv, s->gpart};
@@ -1386,9 +1447,7 @@ int dyninfer_cuda_session_configure_paged_kv(dyninfer_cuda_session_t* s, size_t 
         dev_alloc(s, (void**)&s->qkv1, (size_t)rows * (qd + 2 * kvd) * 4) ||
         dev_alloc(s, (void**)&s->gu1, (size_t)rows * 2 * c.inter * 4) ||
         (c.tp_world > 1 && dev_alloc(s, (void**)&s->tp_part, (size_t)rows * c.hidden * 4)) ||
-        dev_alloc(s, (void**)&s->tokens_dev, (size_t)rows * 8) ||
-        dev_alloc(s, (void**)&s->row_pos_dev, (size_t)rows * 8) ||
-        dev_alloc(s, (void**)&s->row_seq_dev, (size_t)rows * 8) ||
+        dev_alloc(s, (void**)&s->tokens_dev, (size_t)3 * rows * 8) ||
         host_alloc(s, (void**)&s->stage_host, (size_t)(8 + 3 * rows) * 8))
       return 1;
     if (s->xh) s->xh_rows = rows + rows / 2 + 64, s->xh_cols = std::max(c.hidden, c.inter), s->gpart_bytes = (size_t)8 * rows * std::max<int64_t>(c.hidden, qd + 2 * kvd) * 4;
@@ -1637,10 +1696,8 @@ int dyninfer_cuda_session_invoke_paged_chunk_slot(dyninfer_cuda_session_t* s, co
       st[rows + i] = start_pos + i;
       st[2 * rows + i] = slot;
     }
-    DYN_CUDA(cudaMemcpyAsync(s->tokens_dev, st, rows * 8, cudaMemcpyHostToDevice, s->stream));
-    DYN_CUDA(cudaMemcpyAsync(s->row_pos_dev, st + rows, rows * 8, cudaMemcpyHostToDevice, s->stream));
-    DYN_CUDA(cudaMemcpyAsync(s->row_seq_dev, st + 2 * rows, rows * 8, cudaMemcpyHostToDevice,
-                             s->stream));
+    set_step_rows(s, rows);
+    DYN_CUDA(cudaMemcpyAsync(s->tokens_dev, st, 3 * rows * 8, cudaMemcpyHostToDevice, s->stream));
     if (enqueue_forward(s, rows, last, false, start_pos, slot)) return 1;
     DYN_CUDA(cudaMemcpyAsync(s->stage_host + 3, s->out_token_dev, 8, cudaMemcpyDeviceToHost,
                              s->stream));
@@ -1706,9 +1763,7 @@ int dyninfer_cuda_session_decode_batch(dyninfer_cuda_session_t* s, const int64_t
     st[rows + i] = positions[i];
     st[2 * rows + i] = slots[i];
   }
-  DYN_CUDA(cudaMemcpyAsync(s->tokens_dev, st, rows * 8, cudaMemcpyHostToDevice, s->stream));
-  DYN_CUDA(cudaMemcpyAsync(s->row_pos_dev, st + rows, rows * 8, cudaMemcpyHostToDevice, s->stream));
-  DYN_CUDA(cudaMemcpyAsync(s->row_seq_dev, st + 2 * rows, rows * 8, cudaMemcpyHostToDevice, s->stream));
+  DYN_CUDA(cudaMemcpyAsync(s->tokens_dev, st, 3 * rows * 8, cudaMemcpyHostToDevice, s->stream));
   auto it = s->batch_graphs.find(rows);
   if (it == s->batch_graphs.end()) {
     cudaGraphExec_t exec = nullptr;
@@ -1855,9 +1910,7 @@ int dyninfer_cuda_session_decode_loop(dyninfer_cuda_session_t* s, int64_t first_
   s->stage_host[0] = first_token;
   s->stage_host[1] = start_pos;
   s->stage_host[2] = 0;
-  DYN_CUDA(cudaMemcpyAsync(s->tokens_dev, s->stage_host, 8, cudaMemcpyHostToDevice, s->stream));
-  DYN_CUDA(cudaMemcpyAsync(s->row_pos_dev, s->stage_host + 1, 8, cudaMemcpyHostToDevice, s->stream));
-  DYN_CUDA(cudaMemcpyAsync(s->row_seq_dev, s->stage_host + 2, 8, cudaMemcpyHostToDevice, s->stream));
+  DYN_CUDA(cudaMemcpyAsync(s->tokens_dev, s->stage_host, 24, cudaMemcpyHostToDevice, s->stream));
   DYN_CUDA(cudaMemsetAsync(s->hist_count_dev, 0, 8, s->stream));
   DYN_CUDA(cudaEventRecord(s->ev0, s->stream));
   for (size_t i = 0; i < steps; i++) DYN_CUDA(cudaGraphLaunch(s->loop_graph, s->stream));

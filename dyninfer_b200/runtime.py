@@ -95,6 +95,7 @@ class CudaSession:
         self.history: list[int] = []
         self.pad_token_id = int(model.metadata.get("pad_token_id", model.metadata.get("bos_token_id", 0)) or 0)
         self._h = C.c_void_p()
+        self._view = None
         cfg = model.catalog.config
         self.kv_dtype = model.kv_dtype
         self.kv_elem = 4 if self.kv_dtype == "f32" else 2
@@ -197,8 +198,16 @@ class CudaSession:
         logits = None
         if want_logits:
             # session-owned scratch, valid until the next invoke: copy immediately
-            logits = np.ctypeslib.as_array(ptr, shape=(count.value,)).copy()
+            logits = self._logits_view(ptr, count.value).copy()
         return logits, int(tok.value)
+
+    def _logits_view(self, ptr, count: int):
+        """`count` floats at `ptr` as an array; the session hands out the same scratch every time, and building
+        the view anew costs as much as copying it."""
+        address = C.addressof(ptr.contents)
+        if self._view is None or self._view[0] != (address, count):
+            self._view = ((address, count), np.ctypeslib.as_array(ptr, shape=(count,)))
+        return self._view[1]
 
     def _prefill(self, tokens, want_logits: bool):
         self._require_batch_1()

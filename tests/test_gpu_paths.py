@@ -54,3 +54,26 @@ def test_linear_few_rows(native_lib, oracle, enc, m, n, k):
         xb = torch.from_numpy(x).to(torch.bfloat16)
         got = ops.linear(dw, xb.cuda()).cpu().numpy()
         assert helpers.rel_err(got[others], oracle.linear(ow, xb.float().numpy(), fast=True)[others]) < 1e-3
+
+
+@pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q4_1", "gguf.q8_0", "gguf.q6_k", "gguf.q4_k", "mlx.affine.u4"])
+@pytest.mark.parametrize("m,n,k", [(1, 17, 512), (2, 100, 1024), (3, 1000, 3072), (4, 40, 25600), (7, 513, 2048),
+                                   (8, 33, 12800)])
+def test_linear_exact_rows(native_lib, oracle, enc, m, n, k):
+    """1 to 4 f32 rows and 1 to 8 bf16 rows keep the weights exact: f32 accuracy, ragged tiles, K split over warps and
+    clusters, rows of zeros, of huge and of mixed magnitude."""
+    from dyninfer_b200 import ops
+    from test_gpu_ops import make_pair
+    dw, ow = make_pair(oracle, enc, n, k, seed=n + m)
+    x = np.random.default_rng(m).normal(size=(m, k)).astype(np.float32)
+    x[0, ::5] *= 1e-4
+    if m > 1:
+        x[1] = 0.0
+    if m > 2:
+        x[2] *= 1e9
+    xb = torch.from_numpy(x).to(torch.bfloat16)
+    for t in ([torch.from_numpy(x), xb] if m <= 4 else [xb]):
+        got = ops.linear(dw, t.cuda()).cpu().numpy()
+        want = oracle.linear(ow, t.float().numpy(), fast=True)
+        for r in range(m):
+            assert helpers.rel_err(got[r], want[r]) < 2e-5 if r != 1 else not got[r].any()
