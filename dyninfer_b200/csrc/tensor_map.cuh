@@ -36,6 +36,23 @@ inline int make_row_box_map(const uint8_t* data, size_t row_bytes, int64_t rows,
     DYN_CHECK(fn != nullptr && q == cudaDriverEntryPointSuccess, "cuTensorMapEncodeTiled is not available");
     encode = reinterpret_cast<EncodeTiledFn>(fn);
   }
+  // A map depends on its arguments only; the maps of recent products are kept (a fixed number per thread), because
+  // encoding one costs the host more than the rest of a small product's preparation.
+  struct Kept {
+    const uint8_t* data;
+    size_t row_bytes;
+    int64_t rows;
+    int shape;
+    CUtensorMap map;
+  };
+  static thread_local Kept kept[256];
+  const int shape = (box_words << 9) | (box_rows << 1) | (swizzle128 ? 1 : 0);
+  const uint64_t h = ((uint64_t)reinterpret_cast<uintptr_t>(data) >> 8) * 0x9E3779B97F4A7C15ull + (uint64_t)rows * 31 + shape;
+  Kept& k = kept[(h >> 32) & 255];
+  if (k.data == data && k.row_bytes == row_bytes && k.rows == rows && k.shape == shape && data) {
+    *out = k.map;
+    return 0;
+  }
   DYN_CHECK(row_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(data) & 15) == 0 && box_words % 4 == 0 && box_words <= 256,
             "tensor map: rows of %zu bytes / boxes of %d words do not meet the 16-byte rules", row_bytes, box_words);
   const cuuint64_t dims[2] = {(cuuint64_t)(row_bytes / 4), (cuuint64_t)rows};
@@ -47,6 +64,7 @@ inline int make_row_box_map(const uint8_t* data, size_t row_bytes, int64_t rows,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   DYN_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with %d", (int)r);
+  k.data = data, k.row_bytes = row_bytes, k.rows = rows, k.shape = shape, k.map = *out;
   return 0;
 }
 

@@ -16,11 +16,11 @@ from ._lib import ENC, check, lib
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _p(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _dev(a, device="cuda"):
@@ -46,12 +46,20 @@ class DeviceWeight:
         self.data = buf
         self.scales = _dev(np.ascontiguousarray(scales).view(np.uint8).reshape(-1), device) if scales is not None else None
         self.biases = _dev(np.ascontiguousarray(biases).view(np.uint8).reshape(-1), device) if biases is not None else None
+        self._ref = None
         self.nbytes = raw.size + (self.scales.numel() if self.scales is not None else 0) + \
             (self.biases.numel() if self.biases is not None else 0)
 
     def c(self) -> _lib.Weight:
         return _lib.Weight(ENC[self.encoding], ENC.get(self.aux, 2), self.group, 0, self.rows,
                            self.cols, _p(self.data), _p(self.scales), _p(self.biases))
+
+    def ref(self):
+        """The descriptor by reference, built once: a small product's time is mostly the host's."""
+        key = (self.data.data_ptr(), self.scales.data_ptr() if self.scales is not None else 0)
+        if self._ref is None or self._ref[0] != key:
+            self._ref = (key, C.byref(self.c()))
+        return self._ref[1]
 
 
 def dequant(w: DeviceWeight) -> torch.Tensor:
@@ -69,16 +77,24 @@ def embedding_gather(w: DeviceWeight, tokens: torch.Tensor) -> torch.Tensor:
     return out
 
 
+_XT = {torch.float32: ENC["plain.f32"], torch.bfloat16: ENC["plain.bf16"]}
+_linear_fn = None
+
+
 def linear(w: DeviceWeight, x: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    if x.dtype not in (torch.float32, torch.bfloat16):
+    global _linear_fn
+    xt = _XT.get(x.dtype)
+    if xt is None:
         raise TypeError("x must be float32 or bfloat16")
-    x = x.contiguous().view(-1, w.cols)
+    if x.dim() != 2 or x.shape[1] != w.cols or not x.is_contiguous():
+        x = x.contiguous().view(-1, w.cols)
     m = x.shape[0]
     if out is None:
         out = torch.empty((m, w.rows), dtype=torch.float32, device=x.device)
-    cw = w.c()
-    xt = ENC["plain.f32"] if x.dtype == torch.float32 else ENC["plain.bf16"]
-    check(lib().dyninfer_cuda_linear(C.byref(cw), _p(x), xt, m, _p(out), _stream()))
+    if _linear_fn is None:
+        _linear_fn = lib().dyninfer_cuda_linear
+    if _linear_fn(w.ref(), x.data_ptr(), xt, m, out.data_ptr(), _stream()):
+        check(1)
     return out
 
 
