@@ -403,11 +403,13 @@ struct AttnArgs {
   size_t pair_ws_bytes = 0;
 };
 int launch_attention(const AttnArgs& a, cudaStream_t s);
-// Decode attention on 2-byte caches (attention_decode.cu): `part` holds rows * nh * nsplit * (d + 2) floats. The
-// context goes to a.ctx, or with `frag` straight into the f16 operand of a product with weights of encoding `enc`.
+// Decode attention on 2-byte caches (attention_decode.cu), with `prep` the QKV preparation in it. The context goes to
+// a.ctx, or with `frag` (and `part`: rows * nh * splits * (d + 2) floats) straight into the f16 operand of a product
+// with weights of encoding `enc`.
 bool attention_decode_takes(const AttnArgs& a);
 int attention_decode_splits(const AttnArgs& a);
-int launch_attention_decode(const AttnArgs& a, float* part, int nsplit, __half* frag, float* inv_s, int enc, cudaStream_t s);
+int launch_attention_decode(const AttnArgs& a, const QkvPrepArgs* prep, const FreqTable* ft, float* part, __half* frag, float* inv_s,
+                            int enc, cudaStream_t s);
 size_t attention_split_scratch_bytes(int64_t rows, int64_t nh, int64_t d, int nsplit);
 int launch_attention_split(const AttnArgs& a, float* part, int nsplit, cudaStream_t s, bool* handled);
 size_t attention_prefill_scratch_bytes(const AttnArgs& a);

@@ -942,21 +942,7 @@ int launch_attention(const AttnArgs& a, cudaStream_t s) {
       return 1;
     if (handled) return 0;
   }
-  if (attention_decode_takes(a)) {
-    const int nsplit = attention_decode_splits(a);
-    const size_t bytes = attention_split_scratch_bytes(a.rows, a.nh, a.d, nsplit);
-    float* part = reinterpret_cast<float*>(thread_scratch(bytes));
-    const bool pooled = part == nullptr;
-    if (pooled) {
-      if (keep_scratch_pool_cached()) return 1;
-      DYN_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&part), bytes, s));
-    }
-    const int rc = launch_attention_decode(a, part, nsplit, nullptr, nullptr, 0, s);
-    const cudaError_t fe = pooled ? cudaFreeAsync(part, s) : cudaSuccess;
-    if (rc) return rc;
-    if (fe != cudaSuccess) return cuda_fail(fe, "cudaFreeAsync", __FILE__, __LINE__);
-    return 0;
-  }
+  if (attention_decode_takes(a)) return launch_attention_decode(a, nullptr, nullptr, nullptr, nullptr, nullptr, 0, s);
   if (a.d == 64 || a.d == 128 || a.d == 256) {
     // f32 caches, decode / batched decode: slice every row's keys over enough CTAs to fill the GPU. The slice
     // count depends only on shapes and capacity, so a captured graph stays valid as positions grow.

@@ -459,7 +459,6 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       pa.kv_type = s->kv_type, pa.has_norm = c.qk_norm ? 1 : 0, pa.has_rope = c.rope ? 1 : 0;
       pa.eps = c.eps;
       pa.ldq = ldq, pa.ldk = ldk, pa.ldv = ldv;
-      if (launch_qkv_prepare(pa, s->freq, st)) return 1;
       AttnArgs aa{};
       aa.q = qp, aa.kcache = pa.kcache, aa.vcache = pa.vcache;
       aa.row_pos = s->row_pos_dev, aa.row_seq = s->row_seq_dev, aa.base_pos = 0;
@@ -469,10 +468,13 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       aa.ldq = ldq;
       aa.pair_ws = s->pair_ws, aa.pair_ws_bytes = s->pair_ws_bytes;
       aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;
-      const int nsplit = attention_decode_splits(aa);
-      void* part = thread_scratch(attention_split_scratch_bytes(rows, c.heads, c.head_dim, nsplit));
-      if (attention_decode_takes(aa) && part && !(chunk_start >= 0 && rows >= 32)) {
-        if (launch_attention_decode(aa, reinterpret_cast<float*>(part), nsplit, s->sk_x, s->sk_inv, L.o.enc, st)) return 1;
+      void* part = thread_scratch(attention_split_scratch_bytes(rows, c.heads, c.head_dim, attention_decode_splits(aa)));
+      // (the rows of a chunk see one another's keys: their preparation is a launch of its own)
+      const bool decode = chunk_start < 0;
+      if (!(decode && attention_decode_takes(aa) && part) && launch_qkv_prepare(pa, s->freq, st)) return 1;
+      if (attention_decode_takes(aa) && part && (decode || rows < 32)) {
+        if (launch_attention_decode(aa, decode ? &pa : nullptr, &s->freq, reinterpret_cast<float*>(part), s->sk_x, s->sk_inv, L.o.enc, st))
+          return 1;
       } else if (launch_attention(aa, st) || launch_skinny_prepare(L.o, s->ctx, E_F32, rows, s->sk_x, s->sk_inv, st)) {
         return 1;
       }
@@ -584,7 +586,6 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       pa.kv_type = s->kv_type, pa.has_norm = c.qk_norm ? 1 : 0, pa.has_rope = c.rope ? 1 : 0;
       pa.eps = c.eps;
       pa.ldq = ldq, pa.ldk = ldk, pa.ldv = ldv;
-      if (launch_qkv_prepare(pa, s->freq, st)) return 1;
       AttnArgs aa{};
       aa.q = qp, aa.kcache = pa.kcache, aa.vcache = pa.vcache;
       aa.row_pos = s->row_pos_dev, aa.row_seq = s->row_seq_dev, aa.base_pos = 0;
@@ -593,7 +594,12 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       aa.kv_type = s->kv_type;
       aa.ldq = ldq;
       aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;
-      if (launch_attention(aa, st) || launch_linear(L.o, s->ctx, E_F32, rows, s->hidden, s->hidden, st)) return 1;
+      if (attention_decode_takes(aa) && (rows == 1 || chunk_start < 0)) {
+        if (launch_attention_decode(aa, &pa, &s->freq, nullptr, nullptr, nullptr, 0, st)) return 1;
+      } else if (launch_qkv_prepare(pa, s->freq, st) || launch_attention(aa, st)) {
+        return 1;
+      }
+      if (launch_linear(L.o, s->ctx, E_F32, rows, s->hidden, s->hidden, st)) return 1;
       normed_by = nullptr;
       if (L.gate_up.data && c.inter % 32 == 0) {
         if (norm_product(L.gate_up, L.ffn_norm, s->act, true)) return 1;
