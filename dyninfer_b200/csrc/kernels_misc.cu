@@ -141,53 +141,51 @@ __device__ __forceinline__ void f16_row_scale(float mx, float* red, float* sc, f
   *inv = ldexpf(1.0f, e - 13);
 }
 
-template <int PER>
-__global__ void __launch_bounds__(256)
+// FULL: the row is exactly PER x 256 elements, so that every access is a constant offset from a thread's own pointers
+// (with bounds and 64-bit indices per element the kernel took 130 registers and one block per SM: 512 rows x 4096
+// with two slices 36 us).
+template <int PER, bool FULL>
+__global__ void __launch_bounds__(256, PER <= 8 ? 6 : PER <= 16 ? 4 : 2)
 norm_prepare_kernel(const float* __restrict__ x, const float* __restrict__ partial, int S, int64_t rows,
-                    const float* residual, float* hidden, const void* __restrict__ w, int w_type, int64_t width,
+                    const float* residual, float* hidden, const void* __restrict__ w, int w_type, int width,
                     float eps, __half* __restrict__ xh, float* __restrict__ inv_s) {
   __shared__ float red[32];
-  const int64_t row = blockIdx.x;
+  const int T = FULL ? 256 : (int)blockDim.x, tid = threadIdx.x;
+  const int64_t at = (int64_t)blockIdx.x * width + tid;
+  auto in = [&](int k) { return FULL || tid + k * T < width; };
   pdl_trigger();
-  float v[PER], wv[PER];
-#pragma unroll
-  for (int k = 0; k < PER; k++) {
-    const int64_t i = threadIdx.x + (int64_t)k * blockDim.x;
-    wv[k] = i < width ? aux_load(reinterpret_cast<const uint8_t*>(w), w_type, i) : 0.f;
-  }
-  pdl_wait();  // everything but the norm weights comes from the kernels before
-  // the slices outermost: all of a slice's loads are in flight together (one element's slices after the
-  // other waited for an L2 round trip each: 512 x 4096 with two slices 33 us, now 9)
+  float v[PER];
+  pdl_wait();
+  // the slices outermost: all of a slice's loads are in flight together
   if (S) {
+    const float* p = partial + at;
 #pragma unroll
-    for (int k = 0; k < PER; k++) v[k] = 0.f;
-#pragma unroll 2
-    for (int z = 0; z < S; z++) {
-      const float* p = partial + ((int64_t)z * rows + row) * width;
+    for (int k = 0; k < PER; k++) v[k] = in(k) ? p[k * T] : 0.f;
+    for (int z = 1; z < S; z++) {
+      p += rows * width;
+      float u[PER];
 #pragma unroll
-      for (int k = 0; k < PER; k++) {
-        const int64_t i = threadIdx.x + (int64_t)k * blockDim.x;
-        if (i < width) v[k] += p[i];
-      }
+      for (int k = 0; k < PER; k++) u[k] = in(k) ? p[k * T] : 0.f;
+#pragma unroll
+      for (int k = 0; k < PER; k++) v[k] += u[k];
     }
   } else {
 #pragma unroll
-    for (int k = 0; k < PER; k++) {
-      const int64_t i = threadIdx.x + (int64_t)k * blockDim.x;
-      v[k] = i < width ? x[row * width + i] : 0.f;
-    }
+    for (int k = 0; k < PER; k++) v[k] = in(k) ? x[at + k * T] : 0.f;
   }
   if (residual) {
+    const float* p = residual + at;
+    float u[PER];
 #pragma unroll
-    for (int k = 0; k < PER; k++) {
-      const int64_t i = threadIdx.x + (int64_t)k * blockDim.x;
-      if (i < width) v[k] += residual[row * width + i];
-    }
+    for (int k = 0; k < PER; k++) u[k] = in(k) ? p[k * T] : 0.f;
+#pragma unroll
+    for (int k = 0; k < PER; k++) v[k] += u[k];
   }
+  if (hidden) {
+    float* p = hidden + at;
 #pragma unroll
-  for (int k = 0; k < PER; k++) {
-    const int64_t i = threadIdx.x + (int64_t)k * blockDim.x;
-    if (hidden && i < width) hidden[row * width + i] = v[k];
+    for (int k = 0; k < PER; k++)
+      if (in(k)) p[k * T] = v[k];
   }
   float ss = 0.f;
 #pragma unroll
@@ -195,19 +193,22 @@ norm_prepare_kernel(const float* __restrict__ x, const float* __restrict__ parti
   ss = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(ss / (float)width + eps);
   float mx = 0.f;
+  auto weigh = [&](auto weight) {
 #pragma unroll
-  for (int k = 0; k < PER; k++) {
-    v[k] = __fmul_rn(__fmul_rn(v[k], inv), wv[k]);
-    mx = fmaxf(mx, fabsf(v[k]));
-  }
+    for (int k = 0; k < PER; k++) {
+      v[k] = __fmul_rn(__fmul_rn(v[k], inv), in(k) ? weight(tid + k * T) : 0.f);
+      mx = fmaxf(mx, fabsf(v[k]));
+    }
+  };
+  if (w_type == E_F32) weigh([&](int i) { return reinterpret_cast<const float*>(w)[i]; });
+  else weigh([&](int i) { return aux_load(reinterpret_cast<const uint8_t*>(w), w_type, i); });
   float sc, is;
   f16_row_scale(mx, red, &sc, &is);
-  if (threadIdx.x == 0) inv_s[row] = is;
+  if (tid == 0) inv_s[blockIdx.x] = is;
+  __half* out = xh + at;
 #pragma unroll
-  for (int k = 0; k < PER; k++) {
-    const int64_t i = threadIdx.x + (int64_t)k * blockDim.x;
-    if (i < width) xh[row * width + i] = __float2half_rn(v[k] * sc);
-  }
+  for (int k = 0; k < PER; k++)
+    if (in(k)) out[k * T] = __float2half_rn(v[k] * sc);
 }
 
 int launch_norm_prepare(const float* x, const float* partial, int splits, const float* residual, float* hidden,
@@ -217,13 +218,18 @@ int launch_norm_prepare(const float* x, const float* partial, int splits, const 
   const int threads = width >= 1024 ? 256 : (width >= 256 ? 128 : 32);  // rms_norm_kernel's: same summation order
   DYN_CHECK(width <= 32 * threads, "row of %lld elements is too wide for the fused RMSNorm", (long long)width);
   const int S = splits > 1 ? splits : 0;
+  auto run = [&](auto kernel) {
+    return launch_pdl(kernel, dim3((unsigned)rows), dim3(threads), 0, s, x, partial, S, rows, residual, hidden, w, w_type, (int)width,
+                      eps, xh, inv_s);
+  };
   cudaError_t e;
-  if (width <= 8 * threads)
-    e = launch_pdl(norm_prepare_kernel<8>, dim3((unsigned)rows), dim3(threads), 0, s, x, partial, S, rows, residual, hidden, w, w_type, width, eps, xh, inv_s);
-  else if (width <= 16 * threads)
-    e = launch_pdl(norm_prepare_kernel<16>, dim3((unsigned)rows), dim3(threads), 0, s, x, partial, S, rows, residual, hidden, w, w_type, width, eps, xh, inv_s);
-  else
-    e = launch_pdl(norm_prepare_kernel<32>, dim3((unsigned)rows), dim3(threads), 0, s, x, partial, S, rows, residual, hidden, w, w_type, width, eps, xh, inv_s);
+  if (width == 1024) e = run(norm_prepare_kernel<4, true>);
+  else if (width == 2048) e = run(norm_prepare_kernel<8, true>);
+  else if (width == 4096) e = run(norm_prepare_kernel<16, true>);
+  else if (width == 5120) e = run(norm_prepare_kernel<20, true>);
+  else if (width <= 8 * threads) e = run(norm_prepare_kernel<8, false>);
+  else if (width <= 16 * threads) e = run(norm_prepare_kernel<16, false>);
+  else e = run(norm_prepare_kernel<32, false>);
   DYN_CUDA(e);
   count_launch();
   DYN_CUDA(cudaGetLastError());
@@ -571,25 +577,31 @@ __global__ void __launch_bounds__(128) qkv_prepare_kernel(QkvPrepArgs a, FreqTab
 // holds the E = D / 64 rotated pairs (i, i + D / 2), i = E * lane ...; the K-slice sums are added in
 // ascending order, four slices' loads in flight.
 template <int KV, int D>
-__global__ void __launch_bounds__(256) qkv_prepare_warp_kernel(const QkvPrepArgs a, const __grid_constant__ FreqTable ft) {
+__global__ void __launch_bounds__(256, 4) qkv_prepare_warp_kernel(const QkvPrepArgs a, const __grid_constant__ FreqTable ft) {
   using T = typename KvT<KV>::T;
   constexpr int E = D / 64, HALF = D / 2;
   const int lane = threadIdx.x & 31;
-  const int64_t r = blockIdx.x, hh = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
+  const int64_t r = blockIdx.x;
+  const int i0 = E * lane;
   pdl_trigger();
-  if (hh >= a.nh + 2 * a.nkv) return;
+  pdl_wait();
+  const int64_t pos = a.row_pos ? a.row_pos[r] : a.base_pos + r;
+  const int64_t seq = a.row_seq ? a.row_seq[r] : 0;
+  // the rotation is the row's: a warp that takes several heads evaluates it once
+  float sn[E], cs[E];
+  if (a.has_rope) {
+#pragma unroll
+    for (int e = 0; e < E; e++) sincosf(__fmul_rn((float)pos, ft.f[i0 + e]), &sn[e], &cs[e]);
+  }
+  for (int64_t hh = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5); hh < a.nh + 2 * a.nkv; hh += (int64_t)gridDim.y * 8) {
   const int kind = hh < a.nh ? 0 : (hh < a.nh + a.nkv ? 1 : 2);
   const int64_t head = kind == 0 ? hh : (kind == 1 ? hh - a.nh : hh - a.nh - a.nkv);
-  const int i0 = E * lane;
-  float w[2 * E];  // norm weights: not produced by the kernels before
+  float w[2 * E];
   if (kind < 2 && a.has_norm) {
     const uint8_t* nwb = reinterpret_cast<const uint8_t*>(kind == 0 ? a.q_norm_w : a.k_norm_w);
 #pragma unroll
     for (int e = 0; e < E; e++) w[e] = aux_load(nwb, a.norm_w_type, i0 + e), w[E + e] = aux_load(nwb, a.norm_w_type, HALF + i0 + e);
   }
-  pdl_wait();
-  const int64_t pos = a.row_pos ? a.row_pos[r] : a.base_pos + r;
-  const int64_t seq = a.row_seq ? a.row_seq[r] : 0;
   struct __align__(4 * E) Vec { float v[E]; };
   float x[2 * E];  // values i0 .. then HALF + i0 ..
   float* qv = a.q + r * (a.ldq ? a.ldq : a.nh * D) + head * D;
@@ -633,7 +645,7 @@ __global__ void __launch_bounds__(256) qkv_prepare_warp_kernel(const QkvPrepArgs
     for (int e = 0; e < E; e++) olo.v[e] = KvT<KV>::enc(x[e]), ohi.v[e] = KvT<KV>::enc(x[E + e]);
     *reinterpret_cast<Out*>(dst + i0) = olo;
     *reinterpret_cast<Out*>(dst + HALF + i0) = ohi;
-    return;
+    continue;
   }
   if (a.has_norm) {
     // the order of the block form's sum (thread i held elements i and i + D/2 of its head): same bits
@@ -656,9 +668,9 @@ __global__ void __launch_bounds__(256) qkv_prepare_warp_kernel(const QkvPrepArgs
   if (a.has_rope) {
 #pragma unroll
     for (int e = 0; e < E; e++) {
-      float lo, hi;
-      rope_pair(x[e], x[E + e], (float)pos, ft.f[i0 + e], &lo, &hi);
-      x[e] = lo, x[E + e] = hi;
+      const float lo = __fsub_rn(__fmul_rn(x[e], cs[e]), __fmul_rn(x[E + e], sn[e]));
+      x[E + e] = __fadd_rn(__fmul_rn(x[e], sn[e]), __fmul_rn(x[E + e], cs[e]));
+      x[e] = lo;
     }
   }
   if (kind == 0) {
@@ -674,6 +686,7 @@ __global__ void __launch_bounds__(256) qkv_prepare_warp_kernel(const QkvPrepArgs
     *reinterpret_cast<Out*>(dst + i0) = olo;
     *reinterpret_cast<Out*>(dst + HALF + i0) = ohi;
   }
+  }
 }
 
 template <int KV>
@@ -684,7 +697,8 @@ static int run_qkv_prepare(const QkvPrepArgs& a, const FreqTable& ft, cudaStream
                      !((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v) |
                         reinterpret_cast<uintptr_t>(a.dq.partial) | reinterpret_cast<uintptr_t>(a.dk.partial) |
                         reinterpret_cast<uintptr_t>(a.dv.partial)) & 7);
-  const dim3 warps((unsigned)a.rows, (heads + 7) / 8);
+  // many rows: two blocks per row, a warp taking several heads
+  const dim3 warps((unsigned)a.rows, a.rows >= 128 ? std::min(2u, (heads + 7) / 8) : (heads + 7) / 8);
   if (a.d == 128 && pairs)
     DYN_CUDA(launch_pdl(qkv_prepare_warp_kernel<KV, 128>, warps, dim3(256), 0, s, a, ft));
   else if (a.d == 64)

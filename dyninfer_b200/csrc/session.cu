@@ -74,6 +74,7 @@ struct dyninfer_cuda_session_t {
   uint8_t* kcache = nullptr;  // [layer][seq][nkv][cap][d]
   uint8_t* vcache = nullptr;
   size_t kv_bytes_each = 0;
+  int64_t kv_high = 0;      // rows [0, kv_high) of a plane may have been written since the last reset
   void* pair_ws = nullptr;  // f32 cache: one sequence's keys and values as f16 pairs (prefill attention)
   size_t pair_ws_bytes = 0;
   // scratch
@@ -1567,10 +1568,15 @@ int dyninfer_cuda_session_reset_paged_kv(dyninfer_cuda_session_t* s) {
   DYN_CHECK(s->kv_configured, "paged KV is not configured");
   if (!s->pages) return 0;
   DYN_CUDA(cudaSetDevice(s->device));
-  // zero-fill in place, the pool is kept (wrapper.c:1273-1303)
-  DYN_CUDA(cudaMemsetAsync(s->kcache, 0, s->kv_bytes_each, s->stream));
-  DYN_CUDA(cudaMemsetAsync(s->vcache, 0, s->kv_bytes_each, s->stream));
-  DYN_CUDA(cudaStreamSynchronize(s->stream));
+  // zero-fill in place, the pool is kept (wrapper.c:1273-1303). The rows that were written, not the whole pool (a short
+  // prompt cleared 2 x 235 MB of a 0.6B session's f32 pool, 85 us), and ordered on the stream instead of waited for.
+  if (!s->kv_high) return 0;
+  const ModelCfg& c = s->cfg;
+  const size_t planes = (size_t)c.layers * c.batch * c.kv_heads, row = (size_t)c.head_dim * s->kv_elem;
+  const size_t pitch = s->pages * s->page_size * row;
+  DYN_CUDA(cudaMemset2DAsync(s->kcache, pitch, 0, (size_t)s->kv_high * row, planes, s->stream));
+  DYN_CUDA(cudaMemset2DAsync(s->vcache, pitch, 0, (size_t)s->kv_high * row, planes, s->stream));
+  s->kv_high = 0;
   return 0;
 }
 
@@ -1676,6 +1682,7 @@ int dyninfer_cuda_session_invoke_paged_chunk_slot(dyninfer_cuda_session_t* s, co
               (long long)tokens[i], (long long)i, s->cfg.vocab);
   CounterScope scope(s);
   DYN_CUDA(cudaSetDevice(s->device));
+  s->kv_high = std::max(s->kv_high, start_pos + rows);
   if (rows == 1 && s->mega) {
     s->stage_host[0] = tokens[0];
     s->stage_host[1] = start_pos;
@@ -1765,6 +1772,7 @@ int dyninfer_cuda_session_decode_batch(dyninfer_cuda_session_t* s, const int64_t
   }
   int64_t* st = s->stage_host + 8;
   for (int64_t i = 0; i < rows; i++) {
+    s->kv_high = std::max(s->kv_high, positions[i] + 1);
     st[i] = tokens[i];
     st[rows + i] = positions[i];
     st[2 * rows + i] = slots[i];
@@ -1888,6 +1896,7 @@ int dyninfer_cuda_session_decode_loop(dyninfer_cuda_session_t* s, int64_t first_
   CounterScope scope(s);
   DYN_CUDA(cudaSetDevice(s->device));
   if (ensure_hist(s, steps)) return 1;
+  s->kv_high = std::max(s->kv_high, start_pos + (int64_t)steps);
   if (s->mega) {
     s->stage_host[0] = first_token;
     s->stage_host[1] = start_pos;
