@@ -291,7 +291,7 @@ struct ProfT {
 // ---- staging the activation vector of a phase ---------------------------------------------------
 // Item i = (block kb = i / 4, lane quarter t = i % 4) holds 8 elements of the vector: A = 4
 // elements at baseA, B = 4 elements at baseB (the items partition the vector). An item's elements
-// come from polled pairs, from the split-KV partials, or from xs (the embedding row).
+// come from polled pairs or from xs (the embedding row).
 //
 // Two ways of staging:
 //   * per warp (stage_local): a warp stages exactly the 32-blocks its own K-slice of the phase's
@@ -303,13 +303,12 @@ struct ProfT {
 //     finished sums; each warp leaves its sum of squares in `red` for the finishing threads.
 //   * whole block (stage_phase): one scale for the vector, RMSNorm applied here; for encodings whose
 //     units share 32-blocks between warps (Q6_K quarters) and for phases of mixed encodings.
-enum { SRC_XS = 0, SRC_LL = 1, SRC_PARTIALS = 2 };
+enum { SRC_XS = 0, SRC_LL = 1 };
 
 struct StageSrc {
   int kind;
-  const float* ll;  // SRC_LL: the pair buffer; SRC_PARTIALS: a.ll_part
+  const float* ll;  // SRC_LL: the pair buffer
   unsigned ep;
-  int nsplit, max_split, d;  // SRC_PARTIALS
 };
 
 __device__ __forceinline__ void item_bases(int layout, int kb, int t, int* baseA, int* baseB) {
@@ -322,27 +321,6 @@ __device__ __forceinline__ void item_fetch(const StageSrc& src, int baseA, int b
   if (src.kind == SRC_LL) {
     const int64_t idx[4] = {baseA, baseA + 2, baseB, baseB + 2};
     ll_poll<4>(src.ll, idx, src.ep, v, sm.abort);
-  } else if (src.kind == SRC_PARTIALS) {
-    // merge the split-KV partial outputs of this item's head in split order (online softmax merge)
-    const int head = baseA / src.d, ia = baseA - head * src.d, ib = baseB - head * src.d;
-    float M = -3.40282347e38f, Lsum = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; j++) v[j] = 0.f;
-    for (int s = 0; s < src.nsplit; s++) {
-      const int64_t pb = ((int64_t)head * src.max_split + s) * (src.d + 4);
-      const int64_t idx[5] = {pb + ia, pb + ia + 2, pb + ib, pb + ib + 2, pb + src.d};
-      float p[10];
-      ll_poll<5>(src.ll, idx, src.ep, p, sm.abort);
-      const float ms = p[8], ls = p[9];
-      const float mn = fmaxf(M, ms);
-      const float f = expf(M - mn), wgt = expf(ms - mn);
-#pragma unroll
-      for (int j = 0; j < 8; j++) v[j] = v[j] * f + p[j] * wgt;
-      Lsum = Lsum * f + ls * wgt;
-      M = mn;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j++) v[j] = v[j] / Lsum;
   } else {
     const float4 a4 = *reinterpret_cast<const float4*>(sm.xs + baseA);
     const float4 b4 = *reinterpret_cast<const float4*>(sm.xs + baseB);
@@ -692,6 +670,48 @@ __device__ __forceinline__ void stage_kv(const MegaArgs& a, const AttGeo& g, int
   cp_async_commit();
 }
 
+// The slices of a head meet in the head's own CTAs, each of which finishes every nsplit-th run of the head's dims and
+// hands it on as part of one context vector. One hop more than letting every reader of the vector merge for itself, but
+// that read nsplit times the vector in every CTA, one round trip after the other: with five slices 3.8 us per layer, with
+// nine 8 us. A run is whole 32-byte sectors (four pairs). Four lanes share a pair of dims and take the slices in turn.
+__device__ __forceinline__ void merge_splits(const MegaArgs& a, const AttGeo& G, int nsplit, int64_t pbase, unsigned ep,
+                                             const Smem& sm, int tid) {
+  const int nu = a.d >> 2, upc = (nu + nsplit - 1) / nsplit;
+  const int x = tid ^ (MK_CT - 32);  // the last warps first: the first ones are storing the partial output
+  const int line = x >> 2, q = x & 3;
+  if (((x & ~31) >> 2) >= 2 * upc) return;  // whole warps
+  const int dim = 4 * upc * G.sp + 2 * line;
+  const bool live = line < 2 * upc && dim < a.d;
+  const int di = live ? dim : 0;
+  int64_t idx[8];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int s = q + 4 * i < nsplit ? q + 4 * i : nsplit - 1;
+    idx[2 * i] = pbase + (int64_t)s * (a.d + 4) + di;
+    idx[2 * i + 1] = pbase + (int64_t)s * (a.d + 4) + a.d;
+  }
+  float v[16];
+  ll_poll<8>(a.ll_part, idx, ep, v, sm.abort);
+  float M = -3.40282347e38f;
+#pragma unroll
+  for (int i = 0; i < 4; i++) M = fmaxf(M, v[4 * i + 2]);
+  M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 1));
+  M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, 2));
+  float o0 = 0.f, o1 = 0.f, lsum = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float w = q + 4 * i < nsplit ? expf(v[4 * i + 2] - M) : 0.f;
+    o0 = fmaf(v[4 * i], w, o0), o1 = fmaf(v[4 * i + 1], w, o1), lsum = fmaf(v[4 * i + 3], w, lsum);
+  }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    o0 += __shfl_xor_sync(0xffffffffu, o0, o);
+    o1 += __shfl_xor_sync(0xffffffffu, o1, o);
+    lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+  }
+  if (live && q < 2) ll_store(a.ll_ctx, (int64_t)G.h * a.d + dim + q, (q ? o1 : o0) / lsum, ep);
+}
+
 // Attention of one (head, split) over the keys [k_lo, k_hi), in batches of 64 (32 for an f32 cache)
 // staged in shared memory. The code is deliberately compact (rolled loops, no per-key unrolling): it
 // runs once per layer, and instructions that are not in the instruction cache cost more than the
@@ -912,6 +932,7 @@ __device__ __forceinline__ void phase_attention_t(const MegaArgs& a, int l, cons
     ll_store(a.ll_part, pbase + d, m_run, ep);
     ll_store(a.ll_part, pbase + d + 1, l_run, ep);
   }
+  if (nsplit > 1) merge_splits(a, G, nsplit, pbase - (int64_t)sp * (d + 4), ep, sm, tid);
   prof.stamp(4);
   prof.toc(15, tp);
   // the next layer's first batch: every warp is past its reads of the staging buffers (barrier above)
@@ -1215,7 +1236,6 @@ __device__ __forceinline__ void decode_mega_body(const MegaArgs& a) {
   prof.mark(0);
 
   StageSrc src;
-  src.nsplit = nsplit, src.max_split = a.max_split, src.d = a.d;
   // One loop over the 4 * layers + 1 products (q/k/v, o, gate/up, down per layer, then the head) so
   // that the product code exists once in the kernel: the five products of a layer run the same
   // instructions, which then stay in the instruction cache from layer to layer.
@@ -1251,7 +1271,7 @@ __device__ __forceinline__ void decode_mega_body(const MegaArgs& a) {
     } else if (k == 1) {
       phase_attention(a, l, L, AG, pos, nsplit, ep, sm, tid, lane, warp, prof);
       prof.mark(2);
-      src.kind = nsplit > 1 ? SRC_PARTIALS : SRC_LL, src.ll = nsplit > 1 ? a.ll_part : a.ll_ctx, src.ep = ep;
+      src.kind = SRC_LL, src.ll = a.ll_ctx, src.ep = ep;
       n_in = (int)qd, lenc = L->enc_o;
     } else if (k == 2) {
       src.kind = SRC_LL, src.ll = a.ll_hidden[0], src.ep = ep;

@@ -104,7 +104,7 @@ struct MegaArgs {
   // polls the pairs themselves until they carry the epoch it expects.
   float* ll_hidden[2];  // [H]: after o_proj + residual / after down + residual
   float* ll_qkv;        // [nh*d + 2*nkv*d]
-  float* ll_ctx;        // [nh*d]: attention output when one CTA holds all keys of a head
+  float* ll_ctx;        // [nh*d]: attention output
   float* ll_part;       // [nh][max_split][d + 4]: split-KV partial outputs, then (max, sum), two unused
   float* ll_act;        // [I]
   float* ll_amax;       // [grid][4]: (value, row) of each CTA's best logit, two unused (one sector per CTA)

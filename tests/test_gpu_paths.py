@@ -3,6 +3,8 @@ import numpy as np
 import pytest
 
 import helpers
+from dyninfer_b200 import synth
+from dyninfer_b200.runtime import ModelLoader, SessionConfig
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -77,3 +79,19 @@ def test_linear_exact_rows(native_lib, oracle, enc, m, n, k):
         want = oracle.linear(ow, t.float().numpy(), fast=True)
         for r in range(m):
             assert helpers.rel_err(got[r], want[r]) < 2e-5 if r != 1 else not got[r].any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("keys", [63, 64, 128, 129, 575, 1030])
+def test_persistent_attention_slices(native_lib, tmp_path, keys):
+    """One, two, three and the most slices of a head's keys, merged by the head's own blocks, against the operator path."""
+    path = synth.write_qwen3_gguf(str(tmp_path / "q.gguf"), synth.SMALL_D128, seed=5)
+    prompt = np.random.default_rng(keys).integers(0, 512, size=keys).tolist()
+    got = []
+    for kernel in ("persistent", "graph"):
+        model = ModelLoader().load(path, max_kv=1152, kv_dtype="bf16", chunk_size=128, decode_kernel=kernel)
+        with model.create_session(SessionConfig(max_sequence_length=1152)) as s:
+            assert s.uses_persistent_kernel() == (kernel == "persistent")
+            s.prefill(prompt)
+            got.append(np.stack([s.decode(t).values.copy() for t in (7, 11)]))
+    assert np.abs(got[0] - got[1]).max() <= 1e-3
