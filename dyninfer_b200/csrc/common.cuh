@@ -297,7 +297,23 @@ struct TgIo {
   float* partial = nullptr;
   size_t partial_bytes = 0;
   int splits = 0;  // out: > 1 when the sums were left in `partial` (y untouched)
+  // for products that finish their own sums (gemm_stream.cu): scratch, and one counter per SM, zero
+  float* work = nullptr;
+  size_t work_bytes = 0;
+  unsigned* counts = nullptr;
+  bool grouped = false;  // add up K in the groups of gemm_tcgen05.cu's split, whatever the tiling: the same bits on either kernel
 };
+// Dequant GEMM over boxes of raw weights (gemm_stream.cu): its tiling of a product.
+struct GsPlan {
+  int mtiles, bn, nunits, grid, gran;
+  int64_t total;
+  size_t part_bytes;
+};
+bool gemm_stream_takes(const WRef& w);
+GsPlan gemm_stream_plan(const WRef& w, int64_t M, bool whole_tiles = false);
+size_t gemm_stream_scratch_bytes(const WRef& w, int64_t M);
+int launch_gemm_stream(const WRef& w, const GsPlan& p, const __half* xh, const float* inv_s, int64_t M, float* y, const float* residual,
+                       float* part, unsigned* count, cudaStream_t s);
 int launch_dqgemm_tc(const WRef& w, const void* x, int x_type, int64_t M, float* y, const float* residual,
                      cudaStream_t s, bool* handled, TgIo* io = nullptr);
 // Whether launch_dqgemm_tc takes the product, and the activation rows its tiling pads M to.

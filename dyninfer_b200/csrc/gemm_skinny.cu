@@ -893,9 +893,10 @@ int sk_run_enc(const SkArgs& a, const SkPlan& p, const CUtensorMap& wm, const CU
 // kernels (they carry 22 bits of an activation); K a multiple of 256 (of 512 for MLX-U4 and Q6_K).
 bool gemm_skinny_takes(const WRef& w, int64_t M) {
   if (M < 1 || M > 64 || w.rows < 1 || w.rows > (1LL << 30)) return false;
-  // more than 32 rows of a large matrix are bound by the mma.sync rate and by the activations every CTA reads:
-  // the tcgen05 GEMM is ahead (24576 x 4096 Q4_0: 61 us on both at 32 rows, 63 against 150 at 64)
-  if (M > 32 && w.rows * w.cols > (16LL << 20)) return false;
+  // more rows of a large matrix are bound by the mma.sync rate and by the activations every CTA reads: the tcgen05 GEMMs
+  // are ahead, from 17 rows where raw weights arrive in boxes (a step of 24 sequences through eight layers of the 8B
+  // shape 1.99 against 1.51 ms), from 33 with the others (24576 x 4096 Q6_K)
+  if (M > (gemm_stream_takes(w) ? 16 : 32) && w.rows * w.cols > (16LL << 20)) return false;
   {  // the activations of an eighth of K have to fit beside one warp's ring
     const int ku = sk_ku(w.enc), nt = M <= 8 ? 1 : M <= 16 ? 2 : M <= 32 ? 4 : 8;
     const int64_t stages = (w.cols + ku * SK_UNIT - 1) / (ku * SK_UNIT);

@@ -26,16 +26,17 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <cstring>
 
 #include "codec.cuh"
 #include "ring.cuh"
+#include "tensor_map.cuh"
+#include "umma.cuh"
 
 namespace dyn {
 
 namespace {
 
-constexpr int TG_BM = 128;          // weight rows per CTA (MMA M)
-constexpr int TG_BK = 64;           // K elements per stage: 128 bytes of f16 per row
 constexpr int TG_GROUPS = 4;         // producer groups; group g fills stage g with chunks g, g + 4, ...
 constexpr int TG_GWARPS = 4;         // warps per group
 constexpr int TG_A_WARPS = TG_GROUPS * TG_GWARPS, TG_B_WARPS = 1;
@@ -56,48 +57,9 @@ __host__ __device__ constexpr bool tg_a_in_tmem(int enc) {
          enc == E_IQ4_XS;
 }
 __host__ __device__ constexpr bool tg_kquant(int enc) { return enc == E_Q4_K || enc == E_Q5_K || enc == E_IQ4_XS; }
-constexpr int TG_TMEM_A_COL = 256;        // first column of the A ring (32 columns per slot) behind the accumulator
 constexpr int TG_RAW_WORDS = 32 * 21;     // per-warp staging of raw row words (Q5_K: 20 words per row and chunk, odd stride)
 constexpr int TG_MAX_SLOTS = 2 * TG_GROUPS;  // a group owns one pipeline slot, or two when they fit
 constexpr int TG_A_BYTES = TG_BM * 128;
-constexpr long long TG_SPINS = 1LL << 24;
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// K-major, 128-byte swizzle: start >> 4, LBO = 1 (unused for swizzled K-major), SBO = 1024 bytes
-// between 8-row groups, descriptor version 1, layout type 2 (SWIZZLE_128B).
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
-  return (uint64_t)((smem_addr >> 4) & 0x3fff) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-         (2ull << 61);
-}
-// kind::f16: D = f32, A = B = f16, both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
-__device__ __forceinline__ uint32_t umma_idesc(int n) {
-  return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TG_BM >> 4) << 24);
-}
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same with the A operand in tensor memory: lane = row, a 32-bit column holds two consecutive K elements.
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -108,24 +70,66 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 // ---- activations -> f16 [Mpad, K] (rows >= M are zero) ------------------------------------------
 // Every row is scaled by a power of two that puts its largest magnitude in [2^12, 2^13), so the
 // conversion can neither overflow nor push ordinary entries into the f16 subnormals; inv_s[m]
-// undoes the scale in the epilogue (exact). One block per row.
+// undoes the scale in the epilogue (exact). One block per row, runs of eight elements per thread, rows of up to 8192
+// elements read once (element by element and twice 6 us of a 12288 x 4096 x 512 product). count: words to clear for
+// the product behind.
+template <bool WIDE>  // rows on 16-byte boundaries
 __global__ void __launch_bounds__(256)
-tg_prepare_x_kernel(const void* __restrict__ x, int x_bf16, int64_t M, int64_t K, __half* xh, float* inv_s) {
+tg_prepare_x_kernel(const void* __restrict__ x, int x_bf16, int64_t M, int64_t K, __half* xh, float* inv_s, unsigned* count, int ncount) {
   __shared__ float red[8];
   const int64_t m = blockIdx.x;
   const int tid = threadIdx.x;
   __half* dst = xh + m * K;
+  pdl_trigger();
+  pdl_wait();
+  if (m == 0)
+    for (int i = tid; i < ncount; i += 256) count[i] = 0;
   if (m >= M) {
     for (int64_t i = tid * 8; i < K; i += 256 * 8) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
     if (tid == 0) inv_s[m] = 0.f;
     return;
   }
-  auto ld = [&](int64_t i) -> float {
-    return x_bf16 ? bf16_bits_to_f32(reinterpret_cast<const uint16_t*>(x)[m * K + i])
-                  : reinterpret_cast<const float*>(x)[m * K + i];
+  constexpr int R = 4;
+  float v[R][8];
+  const int runs = (int)((K / 8 + 255) / 256);
+  auto load = [&](int i0) {
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+      const int64_t k = ((int64_t)tid + (i0 + i) * 256) * 8;
+      if (k >= K) {
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[i][e] = 0.f;
+      } else if (x_bf16) {
+        const uint16_t* p = reinterpret_cast<const uint16_t*>(x) + m * K + k;
+        if constexpr (WIDE) {
+          const uint4 q = *reinterpret_cast<const uint4*>(p);
+          const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+          for (int e = 0; e < 4; e++) v[i][2 * e] = __uint_as_float(w[e] << 16), v[i][2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; e++) v[i][e] = bf16_bits_to_f32(p[e]);
+        }
+      } else {
+        const float* p = reinterpret_cast<const float*>(x) + m * K + k;
+        if constexpr (WIDE) {
+          const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+          v[i][0] = a.x, v[i][1] = a.y, v[i][2] = a.z, v[i][3] = a.w, v[i][4] = b.x, v[i][5] = b.y, v[i][6] = b.z, v[i][7] = b.w;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; e++) v[i][e] = p[e];
+        }
+      }
+    }
   };
   float mx = 0.f;
-  for (int64_t i = tid; i < K; i += 256) mx = fmaxf(mx, fabsf(ld(i)));
+  for (int i0 = 0; i0 < runs; i0 += R) {
+    load(i0);
+#pragma unroll
+    for (int i = 0; i < R; i++)
+#pragma unroll
+      for (int e = 0; e < 8; e++) mx = fmaxf(mx, fabsf(v[i][e]));
+  }
   mx = warp_max(mx);
   if ((tid & 31) == 0) red[tid >> 5] = mx;
   __syncthreads();
@@ -136,10 +140,27 @@ tg_prepare_x_kernel(const void* __restrict__ x, int x_bf16, int64_t M, int64_t K
   if (mx > 0.f && mx < 3.0e38f) frexpf(mx, &e);
   const float sc = ldexpf(1.0f, 13 - e);
   if (tid == 0) inv_s[m] = ldexpf(1.0f, e - 13);
-  for (int64_t i = tid * 2; i < K; i += 512) {
-    const __half2 h = __floats2half2_rn(ld(i) * sc, ld(i + 1) * sc);
-    *reinterpret_cast<__half2*>(dst + i) = h;
+  for (int i0 = 0; i0 < runs; i0 += R) {
+    if (runs > R) load(i0);
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+      const int64_t k = ((int64_t)tid + (i0 + i) * 256) * 8;
+      if (k >= K) continue;
+      uint4 o;
+      __half2 h[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) h[q] = __floats2half2_rn(v[i][2 * q] * sc, v[i][2 * q + 1] * sc);
+      memcpy(&o, h, 16);
+      *reinterpret_cast<uint4*>(dst + k) = o;
+    }
   }
+}
+
+int tg_prepare(const void* x, int x_type, int64_t M, int64_t Mpad, int64_t K, __half* xh, float* inv_s, unsigned* count, int ncount, cudaStream_t s) {
+  auto kernel = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? tg_prepare_x_kernel<true> : tg_prepare_x_kernel<false>;
+  DYN_CUDA(launch_pdl(kernel, dim3((unsigned)Mpad), dim3(256), 0, s, x, x_type == E_BF16 ? 1 : 0, M, K, xh, inv_s, count, ncount));
+  count_launch();
+  return 0;
 }
 
 struct TgArgs {
@@ -354,11 +375,7 @@ dqgemm_tc_kernel(const TgArgs a, const __grid_constant__ CUtensorMap xmap) {
               out[2 * wq] = h2u(__floats2half2_rn(f[0], f[1])), out[2 * wq + 1] = h2u(__floats2half2_rn(f[2], f[3]));
             }
           }
-          asm volatile(
-              "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-              ::"r"(taddr + 16u * h), "r"(out[0]), "r"(out[1]), "r"(out[2]), "r"(out[3]), "r"(out[4]), "r"(out[5]), "r"(out[6]),
-                "r"(out[7]), "r"(out[8]), "r"(out[9]), "r"(out[10]), "r"(out[11]), "r"(out[12]), "r"(out[13]), "r"(out[14]), "r"(out[15])
-              : "memory");
+          tmem_st16(taddr + 16u * h, out);
         }
         __syncwarp();  // the scratch is read; the next chunk may overwrite it
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -487,11 +504,7 @@ dqgemm_tc_kernel(const TgArgs a, const __grid_constant__ CUtensorMap xmap) {
               }
             }
           }
-          asm volatile(
-              "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-              ::"r"(taddr + 16u * b), "r"(out[0]), "r"(out[1]), "r"(out[2]), "r"(out[3]), "r"(out[4]), "r"(out[5]), "r"(out[6]),
-                "r"(out[7]), "r"(out[8]), "r"(out[9]), "r"(out[10]), "r"(out[11]), "r"(out[12]), "r"(out[13]), "r"(out[14]), "r"(out[15])
-              : "memory");
+          tmem_st16(taddr + 16u * b, out);
         }
         __syncwarp();  // the scratch is read; the next chunk may overwrite it
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -676,11 +689,7 @@ dqgemm_tc_kernel(const TgArgs a, const __grid_constant__ CUtensorMap xmap) {
       const int quarter_warps = (TG_WARPS - quarter + 3) / 4;
       for (int j0 = (warp >> 2) * 16; j0 < mleft; j0 += quarter_warps * 16) {
         uint32_t v[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(tbase + (uint32_t)j0));
+        tmem_ld16(tbase + (uint32_t)j0, v);
         float r[16];
         if (res && n < N) {
           const float* rp = res + (int64_t)j0 * N;
@@ -843,7 +852,50 @@ TgPlan tg_plan(const WRef& w, int64_t M) {
 }  // namespace
 
 bool dqgemm_tc_takes(const WRef& w, int64_t M) { return tg_shape_ok(w, M); }
-int64_t dqgemm_tc_padded_rows(const WRef& w, int64_t M) { return tg_shape_ok(w, M) ? tg_plan(w, M).Mpad : 0; }
+int64_t dqgemm_tc_padded_rows(const WRef& w, int64_t M) {
+  if (!tg_shape_ok(w, M)) return 0;
+  int64_t rows = tg_plan(w, M).Mpad;
+  if (gemm_stream_takes(w))
+    for (const bool whole : {false, true}) {
+      const GsPlan p = gemm_stream_plan(w, M, whole);
+      rows = std::max<int64_t>(rows, (int64_t)p.mtiles * p.bn);
+    }
+  return rows;
+}
+
+// Scratch of run_gemm_stream for plain rows.
+size_t gemm_stream_scratch_bytes(const WRef& w, int64_t M) {
+  if (!gemm_stream_takes(w)) return 0;
+  const GsPlan p = gemm_stream_plan(w, M);
+  const size_t rows = (size_t)p.mtiles * p.bn;
+  return rows * w.cols * 2 + rows * 4 + p.part_bytes + (size_t)p.grid * 4 + 1024;
+}
+
+// The product through gemm_stream.cu: activation pass unless the caller has done it, one launch.
+static int run_gemm_stream(const WRef& w, const void* x, int x_type, int64_t M, float* y, const float* residual, cudaStream_t s, TgIo* io) {
+  const GsPlan p = gemm_stream_plan(w, M, io && io->grouped);
+  const int64_t K = w.cols, Mpad = (int64_t)p.mtiles * p.bn;
+  const bool prepared = io && io->xh;
+  DYN_CHECK(!prepared || Mpad <= io->rows_alloc, "dequant GEMM: %lld prepared rows, %lld needed", (long long)(io ? io->rows_alloc : 0),
+            (long long)Mpad);
+  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+  const size_t xh_bytes = prepared ? 0 : up((size_t)Mpad * K * 2), inv_bytes = prepared ? 0 : up((size_t)Mpad * 4);
+  const bool own_part = !(io && io->work && io->work_bytes >= p.part_bytes), own_count = !(io && io->counts);
+  const size_t part_bytes = own_part ? p.part_bytes : 0, count_bytes = own_count ? up((size_t)p.grid * 4) : 0;
+  TgScratch ws(s);
+  if (xh_bytes + inv_bytes + part_bytes + count_bytes && ws.take(xh_bytes + inv_bytes + part_bytes + count_bytes)) return 1;
+  const __half* xh = prepared ? io->xh : reinterpret_cast<__half*>(ws.ptr);
+  const float* inv_s = prepared ? io->inv_s : reinterpret_cast<float*>(ws.ptr + xh_bytes);
+  float* part = own_part ? reinterpret_cast<float*>(ws.ptr + xh_bytes + inv_bytes) : io->work;
+  unsigned* count = own_count ? reinterpret_cast<unsigned*>(ws.ptr + xh_bytes + inv_bytes + part_bytes) : io->counts;
+  if (!prepared) {
+    if (tg_prepare(x, x_type, M, Mpad, K, const_cast<__half*>(xh), const_cast<float*>(inv_s), own_count ? count : nullptr, own_count ? p.grid : 0, s))
+      return 1;
+  } else if (own_count) {
+    DYN_CUDA(cudaMemsetAsync(count, 0, count_bytes, s));
+  }
+  return launch_gemm_stream(w, p, xh, inv_s, M, y, residual, part, count, s);
+}
 
 // Tensor-core dequant GEMM. *handled = false when the encoding or shape does not qualify.
 int launch_dqgemm_tc(const WRef& w, const void* x, int x_type, int64_t M, float* y, const float* residual,
@@ -851,6 +903,15 @@ int launch_dqgemm_tc(const WRef& w, const void* x, int x_type, int64_t M, float*
   *handled = false;
   if (io) io->splits = 0;
   if (!tg_shape_ok(w, M)) return 0;
+  // A prompt's chunks keep the grouping of their sums: few tiles go on through the K split below (whose sums the next
+  // kernel adds up: 1024 x 2048, 512 rows 10 against 17 us), all others in whole tiles. So do very few tiles of a long K
+  // (1024 x 12288, 512 rows: 37 against 40 us), where the last arriver would add up eight wide parts.
+  const int old_splits = gemm_stream_takes(w) ? tg_plan(w, M).splits : 0;
+  const bool few_tiles = old_splits == 8 && M > 256 && w.cols >= 8192;
+  if (gemm_stream_takes(w) && !few_tiles && !(io && io->grouped && old_splits > 1)) {
+    *handled = true;
+    return run_gemm_stream(w, x, x_type, M, y, residual, s, io);
+  }
   const int64_t K = w.cols;
   const TgPlan pl = tg_plan(w, M);
   const int64_t mtiles = pl.mtiles, Mpad = pl.Mpad;
@@ -871,9 +932,8 @@ int launch_dqgemm_tc(const WRef& w, const void* x, int x_type, int64_t M, float*
   float* partial = part_out ? io->partial : (splits > 1 ? reinterpret_cast<float*>(ws.ptr + xh_bytes + inv_bytes) : nullptr);
   int* err = device_error_word();
   if (!err) return 1;
-  if (!prepared)
-    tg_prepare_x_kernel<<<(unsigned)Mpad, 256, 0, s>>>(x, x_type == E_BF16 ? 1 : 0, M, K, reinterpret_cast<__half*>(ws.ptr),
-                                                       reinterpret_cast<float*>(ws.ptr + xh_bytes));
+  if (!prepared && tg_prepare(x, x_type, M, Mpad, K, reinterpret_cast<__half*>(ws.ptr), reinterpret_cast<float*>(ws.ptr + xh_bytes), nullptr, 0, s))
+    return 1;
   TgArgs a;
   a.w = w, a.xh = xh, a.inv_s = inv_s, a.M = M, a.bn = bn, a.tmem_cols = cols, a.y = y, a.residual = residual, a.error = err;
   CUtensorMap xmap;
@@ -903,7 +963,7 @@ int launch_dqgemm_tc(const WRef& w, const void* x, int x_type, int64_t M, float*
     default: break;
   }
   if (rc) return rc;
-  count_launch(prepared ? 1 : 2);
+  count_launch();
   if (part_out) {
     io->splits = splits;
   } else if (splits > 1) {

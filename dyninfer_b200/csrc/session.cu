@@ -87,6 +87,7 @@ struct dyninfer_cuda_session_t {
   float *xinv = nullptr, *gpart = nullptr;
   int64_t xh_rows = 0, xh_cols = 0;
   size_t gpart_bytes = 0;
+  unsigned* tile_counts = nullptr;  // one per SM, zero between products
   __half* sk_x = nullptr;   // few-row steps: one product's activations in fragment order, and their inverse scales
   float* sk_inv = nullptr;
   float *qkv1 = nullptr, *gu1 = nullptr;  // rows of [q | k | v] and of [gate | up] for the fused products
@@ -399,9 +400,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   // sums of o / down are added inside the following residual + RMSNorm kernel, those of a single [q; k; v]
   // product inside QKV prepare -- 10 instead of 16 launches
   // per layer and five passes over the activations fewer, with the same bits as the separate kernels.
-  // (one block per row: with few rows -- batched decode steps -- the separate multi-block kernels are faster:
-  // 32 rows of the 32B shape 13.5 against 14.4 ms per step)
-  bool fuse_n = !skinny && rows >= 64 && !tp && s->xh && H <= 8192 && silu_prepare_takes(c.inter);
+  bool fuse_n = !skinny && rows > 16 && !tp && s->xh && H <= 8192 && silu_prepare_takes(c.inter);
   for (int l = 0; l < c.layers && fuse_n; l++) {
     const LayerW& L = s->layers[l];
     const WRef* ws[8] = {L.qkv_parts >= 2 ? &L.qkv : &L.q, L.qkv_parts >= 2 ? nullptr : &L.k, L.qkv_parts == 3 ? nullptr : &L.v,
@@ -431,6 +430,8 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
     TgIo local;
     if (!io) io = &local;
     if (prepared) io->xh = s->xh, io->inv_s = s->xinv, io->rows_alloc = s->xh_rows;
+    io->grouped = chunk_start >= 0;
+    io->work = s->gpart, io->work_bytes = s->gpart_bytes, io->counts = s->tile_counts;
     bool handled = false;
     if (launch_dqgemm_tc(w, x, E_F32, rows, y, residual, st, &handled, io)) return 1;
     DYN_CHECK(handled, "dequant GEMM refused a product it had accepted");
@@ -1301,6 +1302,7 @@ int dyninfer_cuda_session_create_with_file_params(
     size_t need = 0;
     auto grow = [&](const WRef& w) {
       for (int m = 1; m <= 8; m++) need = std::max(need, gemv_mma_workspace_bytes(w, E_F32, m));
+      if (cfg.batch > 16) need = std::max(need, (gemm_stream_scratch_bytes(w, cfg.batch) + 2) / 3);
     };
     grow(s->lm_head);
     for (const LayerW& L : s->layers) {
@@ -1392,7 +1394,7 @@ void dyninfer_cuda_session_destroy(dyninfer_cuda_session_t* s) {
                  s->logits, s->tokens_dev, s->out_token_dev,
                  s->hist_dev, s->hist_count_dev, s->argmax_scratch, s->mega_layers, s->io_dev,
                  s->prof_dev, s->trace_dev, s->prog_dev, s->ll_dev, s->batch_logits, s->batch_tokens_dev, s->tp_part, s->tp_logits,
-                 s->tp_gather, s->scratch, s->pair_ws, s->sk_x, s->sk_inv, s->qkv1, s->gu1, s->xh, s->xinv, s->gpart};
+                 s->tp_gather, s->scratch, s->pair_ws, s->sk_x, s->sk_inv, s->qkv1, s->gu1, s->xh, s->xinv, s->gpart, s->tile_counts};
   for (void* p : dev)
     if (p) cudaFree(p);
   if (s->logits_host) cudaFreeHost(s->logits_host);
@@ -1441,6 +1443,9 @@ int dyninfer_cuda_session_configure_paged_kv(dyninfer_cuda_session_t* s, size_t 
   const int64_t rows = std::max<int64_t>((int64_t)chunk_size, c.batch);
   const int64_t qd = (int64_t)c.heads * c.head_dim, kvd = (int64_t)c.kv_heads * c.head_dim;
   if (!s->kv_configured) {
+    // sums of K-split products: eight slices of a chunk's rows, or two tiles of up to 256 rows per SM
+    const size_t gpart_bytes = std::max<size_t>((size_t)8 * rows * std::max<int64_t>(c.hidden, qd + 2 * kvd) * 4,
+                                                (size_t)2 * sm_count() * std::min<int64_t>(256, rows + 16) * 128 * 4);
     if (dev_alloc(s, (void**)&s->hidden, (size_t)rows * c.hidden * 4) ||
         dev_alloc(s, (void**)&s->xn, (size_t)rows * c.hidden * 4) ||
         dev_alloc(s, (void**)&s->ctx, (size_t)rows * qd * 4) ||
@@ -1448,7 +1453,7 @@ int dyninfer_cuda_session_configure_paged_kv(dyninfer_cuda_session_t* s, size_t 
         (c.tp_world == 1 && rows >= 64 &&
          (dev_alloc(s, (void**)&s->xh, (size_t)(rows + rows / 2 + 64) * std::max(c.hidden, c.inter) * 2) ||
           dev_alloc(s, (void**)&s->xinv, (size_t)(rows + rows / 2 + 64) * 4) ||
-          dev_alloc(s, (void**)&s->gpart, (size_t)8 * rows * std::max<int64_t>(c.hidden, qd + 2 * kvd) * 4))) ||
+          dev_alloc(s, (void**)&s->gpart, gpart_bytes) || dev_alloc(s, (void**)&s->tile_counts, (size_t)sm_count() * 4))) ||
         (c.tp_world == 1 && (dev_alloc(s, (void**)&s->sk_x, (size_t)64 * std::max({(int64_t)c.hidden, (int64_t)c.inter, qd}) * 2) ||
                              dev_alloc(s, (void**)&s->sk_inv, 64 * 4))) ||
         dev_alloc(s, (void**)&s->qkv1, (size_t)rows * (qd + 2 * kvd) * 4) ||
@@ -1457,7 +1462,8 @@ int dyninfer_cuda_session_configure_paged_kv(dyninfer_cuda_session_t* s, size_t 
         dev_alloc(s, (void**)&s->tokens_dev, (size_t)3 * rows * 8) ||
         host_alloc(s, (void**)&s->stage_host, (size_t)(8 + 3 * rows) * 8))
       return 1;
-    if (s->xh) s->xh_rows = rows + rows / 2 + 64, s->xh_cols = std::max(c.hidden, c.inter), s->gpart_bytes = (size_t)8 * rows * std::max<int64_t>(c.hidden, qd + 2 * kvd) * 4;
+    if (s->xh) s->xh_rows = rows + rows / 2 + 64, s->xh_cols = std::max(c.hidden, c.inter), s->gpart_bytes = gpart_bytes;
+    if (s->tile_counts) DYN_CUDA(cudaMemset(s->tile_counts, 0, (size_t)sm_count() * 4));
     // the separate-product path writes dense q, k, v and `up` into the same buffers
     s->q = s->qkv1, s->k = s->q + rows * qd, s->v = s->k + rows * kvd;
     s->up = s->gu1;

@@ -95,3 +95,27 @@ def test_persistent_attention_slices(native_lib, tmp_path, keys):
             s.prefill(prompt)
             got.append(np.stack([s.decode(t).values.copy() for t in (7, 11)]))
     assert np.abs(got[0] - got[1]).max() <= 1e-3
+
+
+@pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q4_1", "gguf.q8_0", "gguf.q4_k", "gguf.q5_k", "mlx.affine.u4"])
+@pytest.mark.parametrize("m,n,k", [(65, 40, 256), (70, 129, 5120), (100, 19000, 512), (129, 640, 4096), (257, 257, 1024),
+                                   (600, 4096, 768)])
+def test_linear_many_rows(native_lib, oracle, enc, m, n, k):
+    """Ragged rows and tiles, one and several tiles of activation rows, tiles finished by one block and by several, more
+    tiles than blocks; rows of zeros and one far outside the f16 range; the same bits from call to call."""
+    from dyninfer_b200 import ops
+    from test_gpu_ops import make_pair
+    dw, ow = make_pair(oracle, enc, n, k, seed=n + m)
+    x = np.random.default_rng(m).normal(size=(m, k)).astype(np.float32)
+    x[1] = 0.0
+    x[2] *= 1e7
+    rows = [0, 2, 3, 63, 64, m // 2, m - 2, m - 1]
+    for t in (torch.from_numpy(x), torch.from_numpy(x).to(torch.bfloat16)):
+        dev = t.cuda()
+        first = ops.linear(dw, dev)
+        got = first.cpu().numpy()
+        want = oracle.linear(ow, t.float().numpy()[rows], fast=True)
+        assert np.isfinite(got).all() and not got[1].any()
+        for i, r in enumerate(rows):
+            assert helpers.rel_err(got[r], want[i]) < 1e-3
+        assert torch.equal(first, ops.linear(dw, dev))
