@@ -473,8 +473,15 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       void* part = thread_scratch(attention_split_scratch_bytes(rows, c.heads, c.head_dim, attention_decode_splits(aa)));
       // (the rows of a chunk see one another's keys: their preparation is a launch of its own)
       const bool decode = chunk_start < 0;
-      if (!(decode && attention_decode_takes(aa) && part) && launch_qkv_prepare(pa, s->freq, st)) return 1;
-      if (attention_decode_takes(aa) && part && (decode || rows < 32)) {
+      if (!(decode && attention_decode_takes(aa) && (part || rows * c.kv_heads <= sm_count())) && launch_qkv_prepare(pa, s->freq, st)) return 1;
+      if (decode && attention_decode_takes(aa) && rows * c.kv_heads <= sm_count()) {
+        // up to a CTA per SM and (row, kv head): slices merged over a cluster, then the activation pass (eight sequences
+        // of the 0.6B shape at 512: 9 us less per layer than slices through memory and their merge; with more CTAs than SMs
+        // the smaller ones of that form are ahead)
+        if (launch_attention_decode(aa, &pa, &s->freq, nullptr, nullptr, nullptr, 0, st) ||
+            launch_skinny_prepare(L.o, s->ctx, E_F32, rows, s->sk_x, s->sk_inv, st))
+          return 1;
+      } else if (attention_decode_takes(aa) && part && (decode || rows < 32)) {
         if (launch_attention_decode(aa, decode ? &pa : nullptr, &s->freq, reinterpret_cast<float*>(part), s->sk_x, s->sk_inv, L.o.enc, st))
           return 1;
       } else if (launch_attention(aa, st) || launch_skinny_prepare(L.o, s->ctx, E_F32, rows, s->sk_x, s->sk_inv, st)) {

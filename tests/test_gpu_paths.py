@@ -119,3 +119,25 @@ def test_linear_many_rows(native_lib, oracle, enc, m, n, k):
         for i, r in enumerate(rows):
             assert helpers.rel_err(got[r], want[i]) < 1e-3
         assert torch.equal(first, ops.linear(dw, dev))
+
+
+@pytest.mark.parametrize("slots", [5, 33, 64])
+def test_batched_attention_few_and_many_rows(native_lib, tmp_path, slots):
+    """Slices merged over a cluster (up to a block per SM) and through memory (more), against one sequence at a time."""
+    cfg = dict(synth.SMALL_D128, heads=8, kv_heads=4)
+    path = synth.write_qwen3_gguf(str(tmp_path / "q.gguf"), cfg, seed=9)
+    model = ModelLoader().load(path, max_kv=640, kv_dtype="bf16", chunk_size=64, decode_kernel="graph")
+    rng = np.random.default_rng(slots)
+    prompts = [rng.integers(0, 512, size=int(n)).tolist() for n in rng.integers(1, 600, size=slots)]
+    with model.create_batched_session(SessionConfig(max_sequence_length=640, batch_size=slots)) as s:
+        for b, p in enumerate(prompts):
+            s.prefill_slot(b, p, want_logits=True)
+        s.step({b: 7 for b in range(slots)})
+        _, logits = s.step({b: 11 for b in range(slots)}, want_logits=True)
+        logits = np.array([logits[b] for b in (0, 1, slots - 1)])
+    for i, b in enumerate((0, 1, slots - 1)):
+        with model.create_session(SessionConfig(max_sequence_length=640)) as s:
+            s.prefill(prompts[b])
+            s.decode(7)
+            want = s.decode(11).values
+        assert np.abs(logits[i] - want).max() <= 1e-2 and helpers.cosine(logits[i], want) >= 0.9999
