@@ -93,6 +93,13 @@ __device__ __forceinline__ void fa_pow2_scale(float mx, float* sc, float* inv) {
   *inv = ldexpf(1.0f, e - 13);
 }
 
+__device__ __forceinline__ void fa_ldsm4(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d, uint32_t at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at));
+}
+__device__ __forceinline__ void fa_ldsm4t(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d, uint32_t at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at));
+}
+
 // f32 cache -> f16 pairs: out[plane][kv head][key][hi 128 | lo 128], inv[plane][kv head][tile]; plane 0 = keys,
 // 1 = values. One block per (tile of 64 keys, kv head, plane); 64 bytes in flight per thread and load step.
 __global__ void __launch_bounds__(256)
@@ -254,34 +261,48 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
       vf = fminf(vunit / vi, 0x1p100f);  // powers of two: exact (the bound keeps 0 * inf out)
       vunit = vi;
     }
-    // ---- S = Q K^T for 16 rows x the keys of the step
+    // ---- S = Q K^T for 16 rows x the keys of the step. All key groups of a k-step in turn, so that consecutive MMAs do not
+    // wait for one another; one ldmatrix brings the fragments of two groups
     float s[NT][4];
 #pragma unroll
-    for (int nt = 0; nt < NT; nt++) {
-      s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
-      const T* krow = &ks[nt * 8 + g][0];
+    for (int nt = 0; nt < NT; nt++) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+    {
+      const uint32_t ka = (uint32_t)__cvta_generic_to_shared(&ks[(lane & 7) + 8 * (lane >> 4)][8 * ((lane >> 3) & 1)]);
+      constexpr int GR = NT < 4 ? NT : 4;  // groups at a time
 #pragma unroll
-      for (int kk = 0; kk < 8; kk++) {
-        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(krow + 16 * kk + 2 * t);
-        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(krow + 16 * kk + 8 + 2 * t);
-        M::mma(s[nt], qh[kk], b0, b1);
-        M::mma(s[nt], ql[kk], b0, b1);
-        if constexpr (SPLIT) {
-          const uint32_t c0 = *reinterpret_cast<const uint32_t*>(krow + LO + 16 * kk + 2 * t);
-          const uint32_t c1 = *reinterpret_cast<const uint32_t*>(krow + LO + 16 * kk + 8 + 2 * t);
-          M::mma(s[nt], qh[kk], c0, c1);
+      for (int n0 = 0; n0 < NT; n0 += GR)
+#pragma unroll
+        for (int kk = 0; kk < 8; kk++) {
+          uint32_t b[GR][2], c[GR][2];
+#pragma unroll
+          for (int n = 0; n < GR; n += 2) {
+            const uint32_t at = ka + (uint32_t)(((n0 + n) * 8 * FA_PITCH + 16 * kk) * 2);
+            fa_ldsm4(b[n][0], b[n][1], b[n + 1][0], b[n + 1][1], at);
+            if constexpr (SPLIT) fa_ldsm4(c[n][0], c[n][1], c[n + 1][0], c[n + 1][1], at + LO * 2);
+          }
+#pragma unroll
+          for (int n = 0; n < GR; n++) M::mma(s[n0 + n], qh[kk], b[n][0], b[n][1]);
+#pragma unroll
+          for (int n = 0; n < GR; n++) M::mma(s[n0 + n], ql[kk], b[n][0], b[n][1]);
+          if constexpr (SPLIT) {
+#pragma unroll
+            for (int n = 0; n < GR; n++) M::mma(s[n0 + n], qh[kk], c[n][0], c[n][1]);
+          }
         }
-      }
     }
-    // ---- scale, causal mask, running maximum
+    // ---- scale, causal mask (blocks that reach past the warp's first row), running maximum
     float bm0 = -3.40282347e38f, bm1 = -3.40282347e38f;
+    const bool masked = kb * FA_BC + FA_BC - 1 > a.base_pos + row_lo;
+    const int lim0 = (int)(pos0 - kb * FA_BC) - 2 * t, lim1 = (int)(pos1 - kb * FA_BC) - 2 * t;
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) {
 #pragma unroll
       for (int e = 0; e < 2; e++) {
-        const int64_t key = kb * FA_BC + nt * 8 + 2 * t + e;
-        s[nt][e] = key <= pos0 ? s[nt][e] * ks0 : -3.40282347e38f;
-        s[nt][2 + e] = key <= pos1 ? s[nt][2 + e] * ks1 : -3.40282347e38f;
+        s[nt][e] = __fmul_rn(s[nt][e], ks0), s[nt][2 + e] = __fmul_rn(s[nt][2 + e], ks1);  // rounded on its own, not inside the difference below
+        if (masked) {
+          if (nt * 8 + e > lim0) s[nt][e] = -3.40282347e38f;
+          if (nt * 8 + e > lim1) s[nt][2 + e] = -3.40282347e38f;
+        }
         bm0 = fmaxf(bm0, s[nt][e]);
         bm1 = fmaxf(bm1, s[nt][2 + e]);
       }
@@ -295,10 +316,12 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
     m0 = mn0, m1 = mn1;
     l0 *= f0, l1 *= f1;
     const float of0 = f0 * vf, of1 = f1 * vf;
+    if (__any_sync(0xffffffffu, of0 != 1.0f || of1 != 1.0f)) {
 #pragma unroll
-    for (int dt = 0; dt < 16; dt++) {
-      o[dt][0] *= of0, o[dt][1] *= of0;
-      o[dt][2] *= of1, o[dt][3] *= of1;
+      for (int dt = 0; dt < 16; dt++) {
+        o[dt][0] *= of0, o[dt][1] *= of0;
+        o[dt][2] *= of1, o[dt][3] *= of1;
+      }
     }
     // ---- P = exp(S - m) (masked keys give exactly 0 once a real key has been seen), hi/lo fragments
     uint32_t ph[NT / 2][4], pl[NT / 2][4];
@@ -307,9 +330,12 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
       float p[4];
 #pragma unroll
       for (int e = 0; e < 2; e++) {
-        const int64_t key = kb * FA_BC + nt * 8 + 2 * t + e;
-        p[e] = key <= pos0 ? expf(s[nt][e] - m0) : 0.f;
-        p[2 + e] = key <= pos1 ? expf(s[nt][2 + e] - m1) : 0.f;
+        p[e] = expf(s[nt][e] - m0);
+        p[2 + e] = expf(s[nt][2 + e] - m1);
+        if (masked) {
+          if (nt * 8 + e > lim0) p[e] = 0.f;
+          if (nt * 8 + e > lim1) p[2 + e] = 0.f;
+        }
       }
       l0 += p[0] + p[1];
       l1 += p[2] + p[3];
@@ -318,23 +344,26 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
       M::split2(p[0], p[1], &ph[j][2 * half], &pl[j][2 * half]);          // row g
       M::split2(p[2], p[3], &ph[j][2 * half + 1], &pl[j][2 * half + 1]);  // row g + 8
     }
-    // ---- O += P V: B fragments come transposed out of the [key][dim] tile
+    // ---- O += P V: B fragments come transposed out of the [key][dim] tile, four groups of eight dims at a time
+    const uint32_t va = (uint32_t)__cvta_generic_to_shared(&vs[lane & 15][8 * (lane >> 4)]);
 #pragma unroll
-    for (int dt = 0; dt < 16; dt++) {
+    for (int d0 = 0; d0 < 16; d0 += 4) {
 #pragma unroll
       for (int j = 0; j < NT / 2; j++) {
-        uint32_t b0, b1;
-        const T* vrow = &vs[16 * j + (lane & 15)][dt * 8];  // lanes 0..7: keys 16j.., 8..15: keys 16j+8..
-        asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
-                     : "=r"(b0), "=r"(b1)
-                     : "r"((uint32_t)__cvta_generic_to_shared(vrow)));
-        M::mma(o[dt], ph[j], b0, b1);
-        M::mma(o[dt], pl[j], b0, b1);
+        uint32_t b[4][2], c[4][2];
+#pragma unroll
+        for (int i = 0; i < 4; i += 2) {
+          const uint32_t at = va + (uint32_t)((16 * j * FA_PITCH + (d0 + i) * 8) * 2);
+          fa_ldsm4t(b[i][0], b[i][1], b[i + 1][0], b[i + 1][1], at);
+          if constexpr (SPLIT) fa_ldsm4t(c[i][0], c[i][1], c[i + 1][0], c[i + 1][1], at + LO * 2);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) M::mma(o[d0 + i], ph[j], b[i][0], b[i][1]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) M::mma(o[d0 + i], pl[j], b[i][0], b[i][1]);
         if constexpr (SPLIT) {
-          asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
-                       : "=r"(b0), "=r"(b1)
-                       : "r"((uint32_t)__cvta_generic_to_shared(vrow + LO)));
-          M::mma(o[dt], ph[j], b0, b1);
+#pragma unroll
+          for (int i = 0; i < 4; i++) M::mma(o[d0 + i], ph[j], c[i][0], c[i][1]);
         }
       }
     }
