@@ -1073,6 +1073,7 @@ __device__ __forceinline__ void run_phase_t(const MegaArgs& a, const Smem& sm, W
           const float hnew = res[orow - hid_lo] + s0;
           res[orow - hid_lo] = hnew;
           ll_store(a.ll_hidden[T.ep == MEGA_EP_RESID_O ? 0 : 1], orow, hnew, ep);
+          if (a.hidden_out) a.hidden_out[orow] = hnew;  // the last layer's stays
         } else if (T.ep == MEGA_EP_SWIGLU) {
           const float* p2 = pb + (int)T.acc2 * MK_CW * 16 + row;
           float s1 = 0.f;
@@ -1184,7 +1185,7 @@ __device__ __forceinline__ void decode_mega_body(const MegaArgs& a) {
   sm.nchunks = hdr->nchunks;
   if (warp == MK_CW) {
     // ------------------------------ producer: stream this CTA's weight tiles --------------
-    const int total = *sm.abort ? 0 : (int)hdr->nchunks;
+    const int total = *sm.abort ? 0 : (int)(a.hidden_out ? hdr->layer_chunks : hdr->nchunks);
     int slot = 0;
     uint32_t lap = 0;
     for (int step = 0; step < a.steps; step++)  // the same program for every token of the launch
@@ -1242,7 +1243,8 @@ __device__ __forceinline__ void decode_mega_body(const MegaArgs& a) {
   const int nprod = 4 * a.layers;
   const MegaLayerHot* L = sm.hot;
   unsigned ep = epoch_base;
-  for (int ph = 0; ph <= nprod; ph++) {
+  const int nrun = a.hidden_out ? nprod : nprod + 1;
+  for (int ph = 0; ph < nrun; ph++) {
     const int l = ph >> 2, k = ph & 3;
     const bool head = ph == nprod;
     const void* nw = nullptr;
@@ -1283,6 +1285,7 @@ __device__ __forceinline__ void decode_mega_body(const MegaArgs& a) {
     run_phase(a, sm, wk, ph, ep, src, nw, nw_type, n_in, lenc, res, hid_lo, tid, lane, warp, prof);
     prof.mark(head ? 6 : (k == 0 ? 1 : 2 + k));
   }
+  if (a.hidden_out) break;  // one token per launch
   const unsigned ep_last = epoch_base + (unsigned)a.layers;
   {
     // the (at most 128) finishing threads hold this CTA's candidates
@@ -1487,6 +1490,7 @@ void add_tile_chunks(const WRef& w, int64_t r, int n, int acc, std::vector<MegaC
 
 struct CtaProgram {
   std::vector<MegaChunk> chunks;
+  size_t layer_chunks = 0;  // those before the head
   std::vector<MegaTile> tiles;
   std::vector<MegaRound> rounds;
   std::vector<uint16_t> phase_rounds;
@@ -1591,6 +1595,7 @@ int mega_build_program(const MegaBuildLayer* layers, const MegaLayer* full, int 
       pc.begin_phase();
       pc.add_rows(L.down, nullptr, h0, h1, 0, MEGA_EP_RESID_DOWN);
     }
+    pc.layer_chunks = pc.chunks.size();
     pc.begin_phase();
     pc.add_rows(lm_head, nullptr, (int64_t)V * cta / grid, (int64_t)V * (cta + 1) / grid, 0, MEGA_EP_LOGITS);
   }
@@ -1641,7 +1646,7 @@ int mega_build_program(const MegaBuildLayer* layers, const MegaLayer* full, int 
   for (int cta = 0; cta < grid; cta++) {
     const CtaProgram& pc = per[cta];
     uint8_t* b = blob->data() + (size_t)cta * lay->bytes;
-    MegaProgHeader h{(uint32_t)pc.chunks.size(), (uint32_t)split4(H, cta + 1, grid), (uint32_t)pc.rounds.size(),
+    MegaProgHeader h{(uint32_t)pc.chunks.size(), (uint32_t)split4(H, cta + 1, grid), (uint32_t)pc.layer_chunks,
                      (uint32_t)split4(H, cta, grid)};
     memcpy(b, &h, sizeof h);
     if (!pc.chunks.empty()) memcpy(b + sizeof h, pc.chunks.data(), pc.chunks.size() * sizeof(MegaChunk));

@@ -70,7 +70,7 @@ struct MegaRound {
 //   MegaProgHeader | chunks[max_chunks] | tiles[max_tiles] | rounds[max_rounds] | phase_rounds[nph] |
 //   MegaLayerHot[layers]
 struct MegaProgHeader {
-  uint32_t nchunks, hid_hi, nrounds, hid_lo;  // [hid_lo, hid_hi): the hidden rows this CTA owns
+  uint32_t nchunks, hid_hi, layer_chunks, hid_lo;  // layer_chunks: those before the head; [hid_lo, hid_hi): the hidden rows this CTA owns
 };
 // What the kernel needs of a layer besides its weights, kept in shared memory (part of the blob)
 // so that no layer begins with a fetch of its descriptor.
@@ -100,6 +100,7 @@ struct MegaArgs {
   const void* out_norm;
   int out_norm_type;
   float* logits;  // f32 [V], plain
+  float* hidden_out;  // nullable [H]: the launch ends with the last layer's output here; norm and head are launches of their own
   // Hand-off vectors between the CTAs: arrays of (value, epoch) pairs, 8 bytes each; a reader
   // polls the pairs themselves until they carry the epoch it expects.
   float* ll_hidden[2];  // [H]: after o_proj + residual / after down + residual

@@ -874,6 +874,7 @@ void fill_mega_args(Session* s, MegaArgs* a, int advance, int steps = 1) {
   a->layer_stride = (uint64_t)c.batch * c.kv_heads * (uint64_t)a->cap * c.head_dim * s->kv_elem;
   a->kv_type = s->kv_type;
   a->io = s->io_dev;
+  a->hidden_out = nullptr;
   a->inline_io = 0, a->in_token = a->in_pos = a->in_seq = 0, a->out_host = nullptr;
   a->hist = s->hist_dev, a->hist_count = s->hist_count_dev, a->hist_cap = (int64_t)s->hist_cap;
   a->advance = advance;
@@ -1707,7 +1708,15 @@ int dyninfer_cuda_session_invoke_paged_chunk_slot(dyninfer_cuda_session_t* s, co
     ma.inline_io = 1, ma.in_token = tokens[0], ma.in_pos = start_pos, ma.in_seq = slot;
     DYN_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&ma.out_host), s->stage_host + 3, 0));
     s->stage_host[4] = 0;
-    if (launch_decode_mega(ma, s->mega_grid, s->mega_smem, s->stream)) return 1;
+    // The head is a launch of its own: its streaming kernels keep all of an SM's warps on the weights, where the eight
+    // consumer warps of the persistent kernel are bound by their arithmetic (Q6_K, 151936 x 1024: 68 against 34 us; bf16
+    // 124 against 60), which outweighs three launches. Loops of several tokens per launch keep it inside.
+    ma.hidden_out = s->hidden;
+    if (launch_decode_mega(ma, s->mega_grid, s->mega_smem, s->stream) ||
+        launch_rms_norm(s->hidden, s->out_norm.ptr, s->out_norm.type, 1, s->cfg.hidden, s->cfg.eps, s->xn, s->stream) ||
+        launch_linear(s->lm_head, s->xn, E_F32, 1, s->logits, nullptr, s->stream) ||
+        launch_argmax_rows(s->logits, 1, s->cfg.vocab, ma.out_host, s->stream))
+      return 1;
   } else if (rows == 1) {
     if (!s->decode_graph && capture(s, false, &s->decode_graph, &s->graph_nodes)) return 1;
     s->stage_host[0] = tokens[0];
