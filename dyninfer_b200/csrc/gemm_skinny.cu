@@ -817,28 +817,12 @@ bool sk_make_plan(const WRef& w, int64_t M, bool swiglu, SkPlan* best) {
       }
     }
   if (best_cost > 1e29) return false;
-#ifdef SK_TUNE
-  if (const char* e = getenv("SK_PLAN")) {
-    SkPlan q = *best;
-    if (sscanf(e, "%d,%d,%d,%d,%d", &q.RT, &q.RW, &q.KW, &q.CK, &q.nst) == 5) {
-      q.cstages = (q.kstages + q.CK - 1) / q.CK;
-      q.smem = sk_smem(w, q, (int)M);
-      q.groups = (N + (swiglu ? 8 : 16) * q.RT * q.RW - 1) / ((swiglu ? 8 : 16) * q.RT * q.RW);
-      if (q.smem > (size_t)SK_MAX_SMEM || q.cstages * (q.CK - 1) >= q.kstages || q.KW > q.cstages || (swiglu && q.RW < 2)) return false;
-      *best = q;
-    }
-  }
-  if (getenv("SK_PRINT")) fprintf(stderr, "plan M %d N %d K %d: NT %d RT %d RW %d KW %d CK %d nst %d groups %d smem %d cost %.2f\n", (int)M, (int)N, (int)w.cols, best->NT, best->RT, best->RW, best->KW, best->CK, best->nst, (int)best->groups, (int)best->smem, best_cost);
-#endif
   return true;
 }
 
 // Plans are looked up, not searched, after the first product of a shape (a search costs the host several
 // microseconds). Per thread; dropped when a program with very many shapes fills it.
 bool sk_plan(const WRef& w, int64_t M, bool swiglu, SkPlan* p) {
-#ifdef SK_TUNE
-  return sk_make_plan(w, M, swiglu, p);
-#endif
   typedef std::array<int64_t, 4> Key;
   static thread_local std::map<Key, std::pair<bool, SkPlan>> plans;
   const Key key = {w.rows, w.cols, M, (int64_t)w.enc * 4 + (w.group == 32 ? 2 : 0) + (swiglu ? 1 : 0)};

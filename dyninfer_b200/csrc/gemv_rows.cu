@@ -694,28 +694,12 @@ bool gr_make_plan(const WRef& w, int64_t M, bool swiglu, GrPlan* best) {
   const int rows = (swiglu ? 8 : 16) * best->RW;
   best->groups = (N + rows - 1) / rows;
   if (best->groups * best->CK > 0x7fffffff) return false;
-#ifdef SK_TUNE
-  if (const char* e = getenv("GR_PLAN")) {
-    GrPlan q = *best;
-    if (sscanf(e, "%d,%d,%d,%d", &q.RW, &q.KW, &q.CK, &q.nst) == 4) {
-      q.cstages = (q.kstages + q.CK - 1) / q.CK;
-      q.smem = gr_smem(w, q);
-      q.groups = (N + (swiglu ? 8 : 16) * q.RW - 1) / ((swiglu ? 8 : 16) * q.RW);
-      if (q.smem > (size_t)GR_MAX_SMEM || q.cstages * (q.CK - 1) >= q.kstages || q.KW > q.cstages || (swiglu && q.RW < 2)) return false;
-      *best = q;
-    }
-  }
-  if (getenv("SK_PRINT")) fprintf(stderr, "plan M %d N %d K %d: NM %d RW %d KW %d CK %d nst %d groups %d smem %d\n", (int)M, (int)N, (int)w.cols, best->NM, best->RW, best->KW, best->CK, best->nst, (int)best->groups, (int)best->smem);
-#endif
   return true;
 }
 
 // Plans are looked up, not searched, after the first product of a shape. Per thread; dropped when a program with
 // very many shapes fills it.
 bool gr_plan(const WRef& w, int64_t M, bool swiglu, GrPlan* p) {
-#ifdef SK_TUNE
-  return gr_make_plan(w, M, swiglu, p);
-#endif
   typedef std::array<int64_t, 4> Key;
   static thread_local std::map<Key, std::pair<bool, GrPlan>> plans;
   const Key key = {w.rows, w.cols, M, (int64_t)w.enc * 4 + (w.group == 32 ? 2 : 0) + (swiglu ? 1 : 0)};
