@@ -264,10 +264,11 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 // Power of two that puts a row's largest magnitude into [2^12, 2^13) -- no f16 overflow, ordinary entries stay out
-// of the subnormals -- and its inverse.
+// of the subnormals -- and its inverse. Rows below 2^-101 share a scale: 2^(13 - e) of a smaller one is infinite.
 __device__ __forceinline__ void f16_scale_for(float mx, float* s, float* inv_s) {
   int e = 0;
-  if (mx > 0.f && mx < 3.0e38f) frexpf(mx, &e);
+  if (mx > 0.f && mx <= 3.40282347e38f) frexpf(mx, &e);
+  e = max(e, -100);
   *s = ldexpf(1.0f, 13 - e);
   *inv_s = ldexpf(1.0f, e - 13);
 }

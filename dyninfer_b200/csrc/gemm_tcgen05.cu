@@ -136,10 +136,9 @@ tg_prepare_x_kernel(const void* __restrict__ x, int x_bf16, int64_t M, int64_t K
   mx = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; i++) mx = fmaxf(mx, red[i]);
-  int e = 0;
-  if (mx > 0.f && mx < 3.0e38f) frexpf(mx, &e);
-  const float sc = ldexpf(1.0f, 13 - e);
-  if (tid == 0) inv_s[m] = ldexpf(1.0f, e - 13);
+  float sc, inv;
+  f16_scale_for(mx, &sc, &inv);
+  if (tid == 0) inv_s[m] = inv;
   for (int i0 = 0; i0 < runs; i0 += R) {
     if (runs > R) load(i0);
 #pragma unroll

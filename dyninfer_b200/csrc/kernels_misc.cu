@@ -135,10 +135,7 @@ __device__ __forceinline__ void f16_row_scale(float mx, float* red, float* sc, f
   __syncthreads();
   mx = 0.f;
   for (int i = 0; i < nw; i++) mx = fmaxf(mx, red[i]);
-  int e = 0;
-  if (mx > 0.f && mx < 3.0e38f) frexpf(mx, &e);
-  *sc = ldexpf(1.0f, 13 - e);
-  *inv = ldexpf(1.0f, e - 13);
+  f16_scale_for(mx, sc, inv);
 }
 
 // FULL: the row is exactly PER x 256 elements, so that every access is a constant offset from a thread's own pointers

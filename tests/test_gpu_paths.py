@@ -141,3 +141,25 @@ def test_batched_attention_few_and_many_rows(native_lib, tmp_path, slots):
             s.decode(7)
             want = s.decode(11).values
         assert np.abs(logits[i] - want).max() <= 1e-2 and helpers.cosine(logits[i], want) >= 0.9999
+
+
+@pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q8_0", "gguf.q6_k", "mlx.affine.u4", "plain.bf16", "plain.f16"])
+@pytest.mark.parametrize("m", [1, 4, 5, 16, 40, 100])
+def test_linear_rows_at_the_ends_of_the_range(native_lib, oracle, enc, m):
+    """Rows are scaled into the f16 range by a power of two: it stays finite for rows of 1e-36 and, where more than four
+    rows are scaled by it alone, for a row that holds the largest f32."""
+    from dyninfer_b200 import ops
+    from test_gpu_ops import make_pair
+    n, k = 96, 512
+    dw, ow = make_pair(oracle, enc, n, k, seed=m)
+    x = np.random.default_rng(m).normal(size=(m, k)).astype(np.float32)
+    x[0] *= 1e-36
+    if m > 4:
+        x[1] = 0.0
+        x[1, 77] = 3.4e38
+    got = ops.linear(dw, torch.from_numpy(x).cuda()).cpu().numpy()
+    want = oracle.linear(ow, x, fast=True).astype(np.float64)
+    assert np.isfinite(got).all()
+    for r in range(min(m, 3)):
+        f = 1e30 if r == 0 else 1.0
+        assert helpers.rel_err(got[r] * f, want[r] * f) < 1e-3
