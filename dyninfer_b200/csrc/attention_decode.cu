@@ -6,15 +6,23 @@
 // ONE head), so instruction issue and not the cache's bytes set the pace (8 rows of 32 heads at context 2048:
 // 113 us for 67 MB). Here a CTA takes (row, kv head, slice of the keys); its warps walk 16 keys at a time:
 //   S = Q K^T  A operand: the G <= 8 query heads as rows, row g = leading term of head g, row g + 8 = the second
-//              term (Q enters as two or three terms of the cache's type, so an f32 query keeps its bits);
+//              term (Q enters as three terms of bf16, or as two of f16 after a power of two that keeps the second
+//              term out of the subnormals, so an f32 query keeps its bits at any magnitude);
 //              B operand: K rows as they lie in memory, 16 bytes per lane -- the order of the head
 //              dimensions inside the product is free, so a lane's eight consecutive dimensions serve two steps.
 //   O += P V   the accumulator layout of S is the A layout of P (terms again in rows g and g + 8);
 //              V comes through shared memory (cp.async, a ring per warp) and ldmatrix.trans.
-// Scores, maxima, sums and the output stay f32; each slice leaves (unnormalised output, max, sum) and the
-// slices are combined in a fixed order: by the CTAs of a cluster through shared memory, or (many rows) by a merge
-// kernel straight into the f16 operand of the following product. Per-head RMSNorm, rotation and the write of the new
-// cache row happen here too: the preparation kernel they used to be cost a launch (3.4 us) per layer.
+// Scores, maxima, sums and the output stay f32. An mma truncates where it adds to its accumulator (about 1.5e-8 of the
+// sum each time, always toward zero), so a step's P V starts from zero, smallest terms first, and joins the running
+// output by a rounded fma: as exact as the per-row kernel in f32, at the time per call it had (one row of 32 heads at
+// 8191: f16 14.4, bf16 15.7 us). On f16 caches the weights, their sum included, enter times 2^14: what lies below 2^-14
+// of the largest weight would lose its bits to the subnormals. Error against 64 bits with the mma adding up the output
+// and nothing scaled / now / per-row kernel, f16, 256 rows at 7936: one-sided values 5.5e-6 / 1.0e-7 / 4.7e-7, a long
+// tail 1.9e-5 / 8.1e-7 / 2.4e-6; one row at 300, small queries 1.7e-5 / 2.5e-7 / 1.6e-7.
+// Each slice leaves (unnormalised output, max, sum) and the slices are combined in a fixed order: by the CTAs of a
+// cluster through shared memory, or (many rows) by a merge kernel straight into the f16 operand of the following product.
+// Per-head RMSNorm, rotation and the write of the new cache row happen here too: the preparation kernel they used to be
+// cost a launch (3.4 us) per layer.
 #include <algorithm>
 
 #include "common.cuh"
@@ -31,6 +39,8 @@ struct AdT;
 template <>
 struct AdT<E_BF16> {
   static constexpr int TERMS = 3;  // 8 bits each
+  static constexpr bool SCALED = false;  // f32's range
+  static constexpr float PMUL = 1.0f;
   __device__ static __forceinline__ uint16_t bits(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
   __device__ static __forceinline__ uint32_t pack(float& x, float& y) {  // leading terms; x and y keep what is left
     const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
@@ -46,6 +56,8 @@ struct AdT<E_BF16> {
 template <>
 struct AdT<E_F16> {
   static constexpr int TERMS = 2;  // 11 bits each
+  static constexpr bool SCALED = true;
+  static constexpr float PMUL = 16384.0f;
   __device__ static __forceinline__ uint16_t bits(float x) { return __half_as_ushort(__float2half_rn(x)); }
   __device__ static __forceinline__ uint32_t pack(float& x, float& y) {
     const __half2 h = __floats2half2_rn(x, y);
@@ -209,11 +221,29 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
   __syncthreads();
   // Q: chunk j of lane t = dims 32 j + 8 t ..; products 2j and 2j + 1 take its first and last four
   uint32_t q[TERMS][CH][4];
+  float scale = 1.0f / sqrtf((float)D);
   {
     const float* qv = s_q[g < G ? g : 0] + 8 * t;
+    float qs = 1.0f;
+    if constexpr (T::SCALED) {
+      float mx = 0.f;
+#pragma unroll
+      for (int j = 0; j < CH; j++)
+#pragma unroll
+        for (int e = 0; e < 8; e++) mx = fmaxf(mx, fabsf(qv[32 * j + e]));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      float inv;
+      f16_scale_for(mx, &qs, &inv);
+      scale *= inv;
+    }
 #pragma unroll
     for (int j = 0; j < CH; j++) {
       float4 x = *reinterpret_cast<const float4*>(qv + 32 * j), y = *reinterpret_cast<const float4*>(qv + 32 * j + 4);
+      if constexpr (T::SCALED) {
+        x.x *= qs, x.y *= qs, x.z *= qs, x.w *= qs;
+        y.x *= qs, y.y *= qs, y.z *= qs, y.w *= qs;
+      }
 #pragma unroll
       for (int k = 0; k < TERMS; k++) {
         q[k][j][0] = T::pack(x.x, x.y), q[k][j][1] = T::pack(x.z, x.w);
@@ -221,10 +251,9 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
       }
     }
   }
-  const float scale = 1.0f / sqrtf((float)D);
-  float o[NT][4];
+  float o[NT][2];  // head g, dims 8 i + 2 t, + 1
 #pragma unroll
-  for (int i = 0; i < NT; i++) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  for (int i = 0; i < NT; i++) o[i][0] = o[i][1] = 0.f;
   float m = -3.40282347e38f, l = 0.f;  // head g's running maximum, this lane's share of the sum
 
   // 16 keys key0 .. (those below k_end count): K in kr, V in stage st
@@ -234,16 +263,21 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
     for (int h = 0; h < 2; h++)
 #pragma unroll
       for (int e = 0; e < 2; e++) c[h][e][0] = c[h][e][1] = c[h][e][2] = c[h][e][3] = 0.f;
+    if constexpr (TERMS > 2) {
+#pragma unroll
+      for (int j = 0; j < CH; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          T::mma(c[h][0], q[2][j][0], 0u, q[2][j][1], 0u, kr[h][j].x, kr[h][j].y);
+          T::mma(c[h][1], q[2][j][2], 0u, q[2][j][3], 0u, kr[h][j].z, kr[h][j].w);
+        }
+    }
 #pragma unroll
     for (int j = 0; j < CH; j++)
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         T::mma(c[h][0], q[0][j][0], q[1][j][0], q[0][j][1], q[1][j][1], kr[h][j].x, kr[h][j].y);
         T::mma(c[h][1], q[0][j][2], q[1][j][2], q[0][j][3], q[1][j][3], kr[h][j].z, kr[h][j].w);
-        if constexpr (TERMS > 2) {
-          T::mma(c[h][0], q[2][j][0], 0u, q[2][j][1], 0u, kr[h][j].x, kr[h][j].y);
-          T::mma(c[h][1], q[2][j][2], 0u, q[2][j][3], 0u, kr[h][j].z, kr[h][j].w);
-        }
       }
     after_scores();
     // head g's scores of keys 8 h + 2 t, + 1
@@ -254,25 +288,20 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const int key = key0 + 8 * h + 2 * t + e;
-        const float v = (c[h][0][e] + c[h][1][e]) + (c[h][0][2 + e] + c[h][1][2 + e]);
+        const float v = (c[h][0][e] + c[h][0][2 + e]) + (c[h][1][e] + c[h][1][2 + e]);
         pr[h][e] = key < k_end ? v * scale : -3.40282347e38f;
         bm = fmaxf(bm, pr[h][e]);
       }
     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
     const float mn = fmaxf(m, bm), f = expf(m - mn);
-    const bool rescale = __any_sync(0xffffffffu, f != 1.0f);
     m = mn, l *= f;
-    if (rescale) {
-#pragma unroll
-      for (int i = 0; i < NT; i++) o[i][0] *= f, o[i][1] *= f, o[i][2] *= f, o[i][3] *= f;
-    }
 #pragma unroll
     for (int h = 0; h < 2; h++)
 #pragma unroll
       for (int e = 0; e < 2; e++) {
         const int key = key0 + 8 * h + 2 * t + e;
-        pr[h][e] = key < k_end ? expf(pr[h][e] - m) : 0.f;
+        pr[h][e] = key < k_end ? expf(pr[h][e] - m) * T::PMUL : 0.f;
         l += pr[h][e];
       }
     uint32_t pa[TERMS][2];
@@ -287,11 +316,17 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
       asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                    : "=r"(b0), "=r"(b1), "=r"(b2), "=r"(b3)
                    : "r"(vrow + i * 16));
-      T::mma(o[i], pa[0][0], pa[1][0], pa[0][1], pa[1][1], b0, b1);
-      T::mma(o[i + 1], pa[0][0], pa[1][0], pa[0][1], pa[1][1], b2, b3);
+      float u[4] = {0.f, 0.f, 0.f, 0.f}, v[4] = {0.f, 0.f, 0.f, 0.f};
       if constexpr (TERMS > 2) {
-        T::mma(o[i], pa[2][0], 0u, pa[2][1], 0u, b0, b1);
-        T::mma(o[i + 1], pa[2][0], 0u, pa[2][1], 0u, b2, b3);
+        T::mma(u, pa[2][0], 0u, pa[2][1], 0u, b0, b1);
+        T::mma(v, pa[2][0], 0u, pa[2][1], 0u, b2, b3);
+      }
+      T::mma(u, pa[0][0], pa[1][0], pa[0][1], pa[1][1], b0, b1);
+      T::mma(v, pa[0][0], pa[1][0], pa[0][1], pa[1][1], b2, b3);
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        o[i][e] = fmaf(o[i][e], f, u[e] + u[2 + e]);
+        o[i + 1][e] = fmaf(o[i + 1][e], f, v[e] + v[2 + e]);
       }
     }
     __syncwarp();  // the stage is read; the next round may overwrite it
@@ -334,7 +369,7 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
 #pragma unroll
   for (int i = 0; i < NT; i++)
     *reinterpret_cast<float2*>(so + (warp * 8 + g) * D + i * 8 + 2 * t) =
-        make_float2((o[i][0] + o[i][2]) * wgt, (o[i][1] + o[i][3]) * wgt);
+        make_float2(o[i][0] * wgt, o[i][1] * wgt);
   __syncthreads();
   for (int i = threadIdx.x; i < G * D; i += W * 32) {
     const int h = i / D, d = i % D;

@@ -163,3 +163,49 @@ def test_linear_rows_at_the_ends_of_the_range(native_lib, oracle, enc, m):
     for r in range(min(m, 3)):
         f = 1e30 if r == 0 else 1.0
         assert helpers.rel_err(got[r] * f, want[r] * f) < 1e-3
+
+
+def attention_64(q, kc, vc, start):
+    """Causal attention of rows at start .. in 64 bits, and the caches as the kernel reads them: q [s, heads, d]."""
+    s, nh, _ = q.shape
+    n, rep = start + s, nh // kc.shape[0]
+    k, v = (t[:, :n].double().numpy().repeat(rep, 0) for t in (kc, vc))
+    sc = np.einsum("shd,hkd->hsk", q.astype(np.float64), k) / np.sqrt(q.shape[2])
+    sc[:, np.arange(n)[None] > start + np.arange(s)[:, None]] = -np.inf
+    p = np.exp(sc - sc.max(-1, keepdims=True))
+    return np.einsum("hsk,hkd->shd", p / p.sum(-1, keepdims=True), v).reshape(s, -1)
+
+
+def attention_inputs(kind, s, nh, nkv, d, n):
+    rng = np.random.default_rng(s + n)
+    q, k, v = (rng.normal(size=shape).astype(np.float32) for shape in ((s, nh, d), (nkv, n, d), (nkv, n, d)))
+    if kind == "small queries":      # products of ordinary size out of queries that are small in their own type
+        q, k = q * 1e-3, k * 1e3
+    elif kind == "one-sided values":  # sums that only grow: roundings toward zero add up
+        v += 2
+    elif kind == "long tail":        # one key far ahead of many whose weights are 1e-6 of its own
+        q[:], k, v = 1.0, k * 0.01, v * 0.01 + 1
+        k[:, 0] += 14.0 / np.sqrt(d)
+        v[:, 0] = -1
+    elif kind == "large queries":    # beyond the range of f16
+        q, k = q * 1e6, k * 1e-6
+    return q, k, v
+
+
+def rel_64(got, want):
+    return np.linalg.norm(got - want) / np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("kind", ["normal", "small queries", "large queries", "one-sided values", "long tail"])
+@pytest.mark.parametrize("s,start,d", [(1, 4095, 128), (1, 300, 64), (3, 4000, 64), (20, 1000, 128)])
+def test_attention_decode_keeps_f32_accuracy(native_lib, dtype, kind, s, start, d):
+    """Few rows on 2-byte caches (queries and weights as sums of two or three terms of the cache's type) against 64 bits:
+    the terms hold 2^-24 of a query or weight, a step of 16 keys adds at most a handful of truncations of 2^-25, and the
+    steps are added up with roundings of 2^-25 either way, which for one-sided sums of 300 steps stays under 2^-20."""
+    from dyninfer_b200 import ops
+    q, k, v = attention_inputs(kind, s, 8, 2, d, start + s)
+    tt = {"bf16": torch.bfloat16, "f16": torch.float16}[dtype]
+    kt, vt = torch.from_numpy(k).to(tt), torch.from_numpy(v).to(tt)
+    got = ops.attention(torch.from_numpy(q).cuda(), kt.cuda(), vt.cuda(), start).cpu().numpy()
+    assert rel_64(got, attention_64(q, kt, vt, start)) < 2.0 ** -20
