@@ -17,11 +17,17 @@
 //
 // f32 caches: a first pass turns the sequence's keys and values into (hi, lo) pairs of f16, every 64-key
 // tile of a head scaled by a power of two of its own (no overflow, nothing lost to subnormals), so a pair
-// holds the entry to 2^-23 of its magnitude; the query rows are scaled and split the same way. The
-// products take three mma per tile (hi hi, lo hi, hi lo; what is dropped is 2^-22 of a term). The tile
-// scales are exact: the keys' multiply the scores, the values' enter with the running rescaling of the
-// output. Tiles are twice as wide, so a step takes 32 keys. One-row-per-block evaluation of the same chunk
-// (what f32 caches used before) read every key once per query row: 0.6B, 2048-token prompt 102 -> 25 ms.
+// holds the entry to 2^-24 of its magnitude; the query rows are scaled and split the same way. The
+// products take three mma per tile (hi hi, lo hi, hi lo; what is dropped is 2^-24 of a term). The tile
+// scales are exact: the keys' multiply the scores, the values' a step's share of the output. Tiles are
+// twice as wide, so a step takes 32 keys. One-row-per-block evaluation of the same chunk (what f32 caches
+// used before) read every key once per query row: 0.6B, 2048-token prompt 102 -> 25 ms.
+// An mma truncates where it adds to its accumulator (about 1.5e-8 of the sum each time, always toward
+// zero). With f16 pairs the scores are therefore added up in chains of four, the products with a lo term
+// apart, and the P V of a step starts from zero and joins the running output by a rounded fma. Error against
+// 64 bits, 256 rows at 7936, mma adding up everything / now / per-row kernel in f32: normal values 1.5e-5 /
+// 3.9e-7 / 8.9e-7, values of one sign 3.2e-5 / 2.0e-7 / 4.7e-7. Cost: 512 rows of 16 heads at 1536
+// 125.5 -> 129.8 us.
 #include <algorithm>
 
 #include "common.cuh"
@@ -87,7 +93,7 @@ struct Mma<E_F32> : Mma<E_F16> {};  // operands are f16 pairs
 // Power of two that puts `mx` into [2^12, 2^13), and its inverse; magnitudes below 2^-41 share one scale.
 __device__ __forceinline__ void fa_pow2_scale(float mx, float* sc, float* inv) {
   int e = 0;
-  if (mx > 0.f && mx < 3.0e38f) frexpf(mx, &e);
+  if (mx > 0.f && mx <= 3.40282347e38f) frexpf(mx, &e);
   e = max(e, -40);
   *sc = ldexpf(1.0f, 13 - e);
   *inv = ldexpf(1.0f, e - 13);
@@ -100,12 +106,24 @@ __device__ __forceinline__ void fa_ldsm4t(uint32_t& a, uint32_t& b, uint32_t& c,
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at));
 }
 
+// (a, b) = (a, b) * f + (x, y) * s, two values per instruction; s is a power of two.
+__device__ __forceinline__ void fa_fold2(float& a, float& b, float f, float x, float y, float s) {
+  asm("{\n\t.reg .b64 o, g, u, t;\n\t"
+      "mov.b64 o, {%0, %1};\n\tmov.b64 g, {%2, %2};\n\tmov.b64 u, {%3, %4};\n\tmov.b64 t, {%5, %5};\n\t"
+      "mul.rn.f32x2 u, u, t;\n\tfma.rn.f32x2 o, o, g, u;\n\tmov.b64 {%0, %1}, o;\n\t}"
+      : "+f"(a), "+f"(b)
+      : "f"(f), "f"(x), "f"(y), "f"(s));
+}
+
 // f32 cache -> f16 pairs: out[plane][kv head][key][hi 128 | lo 128], inv[plane][kv head][tile]; plane 0 = keys,
 // 1 = values. One block per (tile of 64 keys, kv head, plane); 64 bytes in flight per thread and load step.
+// Entries that are not finite have no part in the scale. Among the values they become zeros and the key is marked in
+// `lost`: weight 0 times such an entry would reach the rows that do not see the key. (A key's own reach its scores only.)
 __global__ void __launch_bounds__(256)
 fa_split_kernel(const float* __restrict__ kc, const float* __restrict__ vc, int64_t nkv, int64_t cap, int64_t seq,
-                int64_t nkeys, __half* __restrict__ out, float* __restrict__ inv) {
+                int64_t nkeys, __half* __restrict__ out, float* __restrict__ inv, unsigned* __restrict__ lost) {
   __shared__ float red[8];
+  __shared__ unsigned s_lost[2];
   const int64_t tile = blockIdx.x, kvh = blockIdx.y, plane = blockIdx.z;
   const float* src = (plane ? vc : kc) + ((seq * nkv + kvh) * cap + tile * FA_SPLIT_TILE) * FA_D;
   const int left = (int)min((int64_t)FA_SPLIT_TILE, nkeys - tile * FA_SPLIT_TILE) * (FA_D / 4);  // float4s
@@ -116,9 +134,25 @@ fa_split_kernel(const float* __restrict__ kc, const float* __restrict__ vc, int6
     const int i = threadIdx.x + 256 * k;
     v[k] = i < left ? reinterpret_cast<const float4*>(src)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
+  if (threadIdx.x < 2) s_lost[threadIdx.x] = 0;
+  __syncthreads();
 #pragma unroll
-  for (int k = 0; k < 8; k++)
-    mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v[k].x), fabsf(v[k].y)), fmaxf(fabsf(v[k].z), fabsf(v[k].w))));
+  for (int k = 0; k < 8; k++) {
+    float m = fmaxf(fmaxf(fabsf(v[k].x), fabsf(v[k].y)), fmaxf(fabsf(v[k].z), fabsf(v[k].w)));
+    const float sum = fabsf(v[k].x * 0.f + v[k].y * 0.f) + fabsf(v[k].z * 0.f + v[k].w * 0.f);  // 0 unless one is not finite
+    if (sum != 0.f) {
+      float* e = reinterpret_cast<float*>(&v[k]);
+      m = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (fabsf(e[i]) <= 3.40282347e38f) m = fmaxf(m, fabsf(e[i]));
+        else if (plane) e[i] = 0.f;
+      }
+      const int key = (threadIdx.x + 256 * k) / (FA_D / 4);
+      atomicOr(&s_lost[key >> 5], 1u << (key & 31));
+    }
+    mx = fmaxf(mx, m);
+  }
   mx = warp_max(mx);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
   __syncthreads();
@@ -128,6 +162,7 @@ fa_split_kernel(const float* __restrict__ kc, const float* __restrict__ vc, int6
   float sc, is;
   fa_pow2_scale(mx, &sc, &is);
   if (threadIdx.x == 0) inv[(plane * nkv + kvh) * (cap / FA_SPLIT_TILE) + tile] = is;
+  if (plane && threadIdx.x < 2) lost[kvh * (cap / 32) + 2 * tile + threadIdx.x] = s_lost[threadIdx.x];
   __half* dst = out + ((plane * nkv + kvh) * cap + tile * FA_SPLIT_TILE) * (2 * FA_D);
 #pragma unroll
   for (int k = 0; k < 8; k++) {
@@ -148,6 +183,7 @@ struct FaArgs {
   const void* vcache;
   const float* kinv;  // f32 caches: inverse tile scales [kv head][cap / 64]
   const float* vinv;
+  const unsigned* vlost;  // f32 caches: a bit per key whose values are not all finite [kv head][cap / 32]
   float* ctx;         // [rows, nh * d]
   int64_t rows, nh, nkv, cap, base_pos, seq;
   int64_t ldq;        // floats between consecutive rows of q
@@ -157,6 +193,8 @@ template <int KV, int HALVES>
 __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(const FaArgs a) {
   constexpr int FA_THREADS = fa_threads(HALVES);
   constexpr bool SPLIT = KV == E_F32;
+  constexpr bool SCALED = KV != E_BF16;                // f16 terms: the query rows and the weights need scales
+  constexpr float PMUL = SCALED ? 16384.0f : 1.0f;     // the weights' (the sum carries it too)
   constexpr int FA_BC = fa_keys(KV), FA_TILE = fa_tile(KV), NP = fa_planes(KV), NT = FA_BC / 8;
   constexpr int LO = FA_BC * FA_PITCH;  // the lo half of a tile
   using M = Mma<KV>;
@@ -173,6 +211,7 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
   const T* vplane = reinterpret_cast<const T*>(a.vcache) + plane;
   const float* kinv = SPLIT ? a.kinv + kvh * (a.cap / FA_SPLIT_TILE) : nullptr;
   const float* vinv = SPLIT ? a.vinv + kvh * (a.cap / FA_SPLIT_TILE) : nullptr;
+  const unsigned* vlost = SPLIT ? a.vlost + kvh * (a.cap / 32) : nullptr;
   const int64_t row_lo = rb * FA_BR + warp * 16;   // this warp's first query row
   const int64_t r0 = row_lo + g, r1 = r0 + 8;      // the lane's two rows
   const int64_t r0c = r0 < a.rows ? r0 : a.rows - 1, r1c = r1 < a.rows ? r1 : a.rows - 1;
@@ -182,12 +221,11 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
   // Q fragments (hi, lo) for the 8 k-steps over the head dim
   uint32_t qh[8][4], ql[8][4];
   float scale0 = scale, scale1 = scale;  // per query row: 1 / sqrt(d), with f16 pairs times the row's inverse scale
-  float vunit = 1.0f;                    // f16 pairs: the accumulated output counts in units of the last tile's inverse scale
   {
     const float* q0 = a.q + r0c * a.ldq + h * FA_D;
     const float* q1 = a.q + r1c * a.ldq + h * FA_D;
     float s0 = 1.f, s1 = 1.f;
-    if constexpr (SPLIT) {
+    if constexpr (SCALED) {
       float x0 = 0.f, x1 = 0.f;
 #pragma unroll
       for (int kk = 0; kk < 16; kk++) {
@@ -253,41 +291,63 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
     const T(*ks)[FA_PITCH] = reinterpret_cast<const T(*)[FA_PITCH]>(tiles + ((pr & 1) * 2 * HALVES + half * 2) * FA_TILE);
     const T(*vs)[FA_PITCH] = reinterpret_cast<const T(*)[FA_PITCH]>(tiles + ((pr & 1) * 2 * HALVES + half * 2 + 1) * FA_TILE);
     if (kb * FA_BC > warp_last) continue;  // every key of the block lies after this warp's rows
-    float ks0 = scale0, ks1 = scale1, vf = 1.0f;
+    float ks0 = scale0, ks1 = scale1, vi = 1.0f;
+    unsigned lost = 0;  // keys of the step whose values are not finite
     if constexpr (SPLIT) {
       const int64_t tile = kb * FA_BC / FA_SPLIT_TILE;
-      const float ki = __ldg(kinv + tile), vi = __ldg(vinv + tile);
+      const float ki = __ldg(kinv + tile);
+      vi = __ldg(vinv + tile) * (1.0f / PMUL);
+      lost = __ldg(vlost + 2 * tile + (kb & 1));
       ks0 *= ki, ks1 *= ki;
-      vf = fminf(vunit / vi, 0x1p100f);  // powers of two: exact (the bound keeps 0 * inf out)
-      vunit = vi;
     }
     // ---- S = Q K^T for 16 rows x the keys of the step. All key groups of a k-step in turn, so that consecutive MMAs do not
     // wait for one another; one ldmatrix brings the fragments of two groups
     float s[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; nt++) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
-    {
-      const uint32_t ka = (uint32_t)__cvta_generic_to_shared(&ks[(lane & 7) + 8 * (lane >> 4)][8 * ((lane >> 3) & 1)]);
+    const uint32_t ka = (uint32_t)__cvta_generic_to_shared(&ks[(lane & 7) + 8 * (lane >> 4)][8 * ((lane >> 3) & 1)]);
+    if constexpr (SPLIT) {
+#pragma unroll
+      for (int n0 = 0; n0 < NT; n0 += 2) {
+        float x[2][2][4], lo[2][2][4];  // group, chain
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) x[n][h][e] = lo[n][h][e] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < 8; kk++) {
+          uint32_t b[2][2], c[2][2];
+          const uint32_t at = ka + (uint32_t)((n0 * 8 * FA_PITCH + 16 * kk) * 2);
+          fa_ldsm4(b[0][0], b[0][1], b[1][0], b[1][1], at);
+          fa_ldsm4(c[0][0], c[0][1], c[1][0], c[1][1], at + LO * 2);
+#pragma unroll
+          for (int n = 0; n < 2; n++) M::mma(x[n][kk & 1], qh[kk], b[n][0], b[n][1]);
+#pragma unroll
+          for (int n = 0; n < 2; n++) M::mma(lo[n][0], ql[kk], b[n][0], b[n][1]);
+#pragma unroll
+          for (int n = 0; n < 2; n++) M::mma(lo[n][1], qh[kk], c[n][0], c[n][1]);
+        }
+#pragma unroll
+        for (int n = 0; n < 2; n++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) s[n0 + n][e] = (x[n][0][e] + x[n][1][e]) + (lo[n][0][e] + lo[n][1][e]);
+      }
+    } else {
       constexpr int GR = NT < 4 ? NT : 4;  // groups at a time
 #pragma unroll
       for (int n0 = 0; n0 < NT; n0 += GR)
 #pragma unroll
         for (int kk = 0; kk < 8; kk++) {
-          uint32_t b[GR][2], c[GR][2];
+          uint32_t b[GR][2];
 #pragma unroll
-          for (int n = 0; n < GR; n += 2) {
-            const uint32_t at = ka + (uint32_t)(((n0 + n) * 8 * FA_PITCH + 16 * kk) * 2);
-            fa_ldsm4(b[n][0], b[n][1], b[n + 1][0], b[n + 1][1], at);
-            if constexpr (SPLIT) fa_ldsm4(c[n][0], c[n][1], c[n + 1][0], c[n + 1][1], at + LO * 2);
-          }
+          for (int n = 0; n < GR; n += 2)
+            fa_ldsm4(b[n][0], b[n][1], b[n + 1][0], b[n + 1][1], ka + (uint32_t)(((n0 + n) * 8 * FA_PITCH + 16 * kk) * 2));
 #pragma unroll
           for (int n = 0; n < GR; n++) M::mma(s[n0 + n], qh[kk], b[n][0], b[n][1]);
 #pragma unroll
           for (int n = 0; n < GR; n++) M::mma(s[n0 + n], ql[kk], b[n][0], b[n][1]);
-          if constexpr (SPLIT) {
-#pragma unroll
-            for (int n = 0; n < GR; n++) M::mma(s[n0 + n], qh[kk], c[n][0], c[n][1]);
-          }
         }
     }
     // ---- scale, causal mask (blocks that reach past the warp's first row), running maximum
@@ -315,12 +375,11 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
     const float f0 = expf(m0 - mn0), f1 = expf(m1 - mn1);
     m0 = mn0, m1 = mn1;
     l0 *= f0, l1 *= f1;
-    const float of0 = f0 * vf, of1 = f1 * vf;
-    if (__any_sync(0xffffffffu, of0 != 1.0f || of1 != 1.0f)) {
+    if (!SPLIT && __any_sync(0xffffffffu, f0 != 1.0f || f1 != 1.0f)) {
 #pragma unroll
       for (int dt = 0; dt < 16; dt++) {
-        o[dt][0] *= of0, o[dt][1] *= of0;
-        o[dt][2] *= of1, o[dt][3] *= of1;
+        o[dt][0] *= f0, o[dt][1] *= f0;
+        o[dt][2] *= f1, o[dt][3] *= f1;
       }
     }
     // ---- P = exp(S - m) (masked keys give exactly 0 once a real key has been seen), hi/lo fragments
@@ -330,8 +389,8 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
       float p[4];
 #pragma unroll
       for (int e = 0; e < 2; e++) {
-        p[e] = expf(s[nt][e] - m0);
-        p[2 + e] = expf(s[nt][2 + e] - m1);
+        p[e] = expf(s[nt][e] - m0) * PMUL;
+        p[2 + e] = expf(s[nt][2 + e] - m1) * PMUL;
         if (masked) {
           if (nt * 8 + e > lim0) p[e] = 0.f;
           if (nt * 8 + e > lim1) p[2 + e] = 0.f;
@@ -348,6 +407,7 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
     const uint32_t va = (uint32_t)__cvta_generic_to_shared(&vs[lane & 15][8 * (lane >> 4)]);
 #pragma unroll
     for (int d0 = 0; d0 < 16; d0 += 4) {
+      float u[4][4];
 #pragma unroll
       for (int j = 0; j < NT / 2; j++) {
         uint32_t b[4][2], c[4][2];
@@ -357,20 +417,40 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
           fa_ldsm4t(b[i][0], b[i][1], b[i + 1][0], b[i + 1][1], at);
           if constexpr (SPLIT) fa_ldsm4t(c[i][0], c[i][1], c[i + 1][0], c[i + 1][1], at + LO * 2);
         }
-#pragma unroll
-        for (int i = 0; i < 4; i++) M::mma(o[d0 + i], ph[j], b[i][0], b[i][1]);
-#pragma unroll
-        for (int i = 0; i < 4; i++) M::mma(o[d0 + i], pl[j], b[i][0], b[i][1]);
         if constexpr (SPLIT) {
+          if (j == 0) {
 #pragma unroll
-          for (int i = 0; i < 4; i++) M::mma(o[d0 + i], ph[j], c[i][0], c[i][1]);
+            for (int i = 0; i < 4; i++) u[i][0] = u[i][1] = u[i][2] = u[i][3] = 0.f;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; i++) M::mma(u[i], ph[j], c[i][0], c[i][1]);
+#pragma unroll
+          for (int i = 0; i < 4; i++) M::mma(u[i], pl[j], b[i][0], b[i][1]);
+#pragma unroll
+          for (int i = 0; i < 4; i++) M::mma(u[i], ph[j], b[i][0], b[i][1]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; i++) M::mma(o[d0 + i], ph[j], b[i][0], b[i][1]);
+#pragma unroll
+          for (int i = 0; i < 4; i++) M::mma(o[d0 + i], pl[j], b[i][0], b[i][1]);
+        }
+      }
+      if constexpr (SPLIT) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          fa_fold2(o[d0 + i][0], o[d0 + i][1], f0, u[i][0], u[i][1], vi);
+          fa_fold2(o[d0 + i][2], o[d0 + i][3], f1, u[i][2], u[i][3], vi);
         }
       }
     }
-  }
-  if constexpr (SPLIT) {
+    if (SPLIT && lost) {  // their pairs are zeros: rows that see one of them get no number, earlier rows are not touched
+      const int64_t key = kb * FA_BC + __ffs(lost) - 1;
 #pragma unroll
-    for (int dt = 0; dt < 16; dt++) o[dt][0] *= vunit, o[dt][1] *= vunit, o[dt][2] *= vunit, o[dt][3] *= vunit;
+      for (int dt = 0; dt < 16; dt++) {
+        if (key <= pos0) o[dt][0] = o[dt][1] = __int_as_float(0x7fffffff);
+        if (key <= pos1) o[dt][2] = o[dt][3] = __int_as_float(0x7fffffff);
+      }
+    }
   }
   // ---- merge the two halves' running states (thread for thread: both cover the same rows and columns)
   if constexpr (HALVES == 2) {
@@ -403,7 +483,7 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
   l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-  const float i0 = 1.0f / l0, i1 = 1.0f / l1;
+  const float i0 = (SPLIT ? PMUL : 1.0f) / l0, i1 = (SPLIT ? PMUL : 1.0f) / l1;  // pairs: o left the weights' scale with each step
 #pragma unroll
   for (int dt = 0; dt < 16; dt++) {
     if (r0 < a.rows)
@@ -417,10 +497,10 @@ __global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(c
 
 }  // namespace
 
-// Scratch of the f16 pairs of an f32 cache: the pairs, then the inverse tile scales.
+// Scratch of the f16 pairs of an f32 cache: the pairs, the inverse tile scales, a bit per key.
 size_t attention_prefill_scratch_bytes(const AttnArgs& a) {
   if (a.kv_type != E_F32) return 0;
-  return (size_t)(2 * a.nkv * a.cap) * (2 * FA_D) * 2 + (size_t)(2 * a.nkv * (a.cap / FA_SPLIT_TILE)) * 4;
+  return (size_t)(2 * a.nkv * a.cap) * (2 * FA_D) * 2 + (size_t)(2 * a.nkv * (a.cap / FA_SPLIT_TILE)) * 4 + (size_t)(a.nkv * (a.cap / 32)) * 4;
 }
 
 // Tensor-core attention for `a.rows` query rows of sequence `seq` at positions base_pos + row.
@@ -433,7 +513,7 @@ int launch_attention_prefill(const AttnArgs& a, int64_t base_pos, int64_t seq, c
   f.q = a.q, f.kcache = a.kcache, f.vcache = a.vcache, f.ctx = a.ctx;
   f.rows = a.rows, f.nh = a.nh, f.nkv = a.nkv, f.cap = a.cap, f.base_pos = base_pos, f.seq = seq;
   f.ldq = a.ldq ? a.ldq : a.nh * FA_D;
-  f.kinv = f.vinv = nullptr;
+  f.kinv = f.vinv = nullptr, f.vlost = nullptr;
   const dim3 grid((unsigned)a.nh, (unsigned)((a.rows + FA_BR - 1) / FA_BR));
   // a grid that fits the GPU in one round: eight warps and pairs of key blocks; larger: four warps, two CTAs per
   // SM (2-byte caches; the f16 pairs of an f32 cache fill an SM's shared memory either way)
@@ -450,12 +530,13 @@ int launch_attention_prefill(const AttnArgs& a, int64_t base_pos, int64_t seq, c
     __half* const out = reinterpret_cast<__half*>(ws);
     const size_t plane = (size_t)a.nkv * a.cap * 2 * FA_D;
     float* const inv = reinterpret_cast<float*>(out + 2 * plane);
+    unsigned* const lost = reinterpret_cast<unsigned*>(inv + 2 * a.nkv * (a.cap / FA_SPLIT_TILE));
     const int64_t nkeys = base_pos + a.rows;
     fa_split_kernel<<<dim3((unsigned)((nkeys + FA_SPLIT_TILE - 1) / FA_SPLIT_TILE), (unsigned)a.nkv, 2), 256, 0, s>>>(
-        reinterpret_cast<const float*>(a.kcache), reinterpret_cast<const float*>(a.vcache), a.nkv, a.cap, seq, nkeys, out, inv);
+        reinterpret_cast<const float*>(a.kcache), reinterpret_cast<const float*>(a.vcache), a.nkv, a.cap, seq, nkeys, out, inv, lost);
     count_launch();
     f.kcache = out, f.vcache = out + plane;
-    f.kinv = inv, f.vinv = inv + a.nkv * (a.cap / FA_SPLIT_TILE);
+    f.kinv = inv, f.vinv = inv + a.nkv * (a.cap / FA_SPLIT_TILE), f.vlost = lost;
   }
   auto run = [&](auto kernel, int halves) -> int {
     const int bytes = fa_smem_bytes(a.kv_type, halves);

@@ -209,3 +209,36 @@ def test_attention_decode_keeps_f32_accuracy(native_lib, dtype, kind, s, start, 
     kt, vt = torch.from_numpy(k).to(tt), torch.from_numpy(v).to(tt)
     got = ops.attention(torch.from_numpy(q).cuda(), kt.cuda(), vt.cuda(), start).cpu().numpy()
     assert rel_64(got, attention_64(q, kt, vt, start)) < 2.0 ** -20
+
+
+@pytest.mark.parametrize("kind", ["normal", "small queries", "large queries", "one-sided values", "long tail"])
+@pytest.mark.parametrize("s,start,nh,nkv", [(64, 0, 8, 2), (45, 4000, 4, 1), (200, 500, 8, 4)])
+def test_attention_prefill_f32_cache_keeps_f32_accuracy(native_lib, kind, s, start, nh, nkv):
+    """f16 pairs against 64 bits: a pair holds 2^-24 of a value, scores take chains of four mma, the steps of 32 keys are
+    added up with roundings; the bound is the decode kernel's. Equal small addends on a large sum round the same way each
+    time: a long tail adds 2^-24 for each of a half's (start + s) / 64 steps, in the sum and in the output."""
+    from dyninfer_b200 import ops
+    q, k, v = attention_inputs(kind, s, nh, nkv, 128, (start + s + 63) // 64 * 64)
+    kt, vt = torch.from_numpy(k), torch.from_numpy(v)
+    got = ops.attention(torch.from_numpy(q).cuda(), kt.cuda(), vt.cuda(), start).cpu().numpy()
+    bound = 2.0 ** -20 + ((start + s) / 64 * 2.0 ** -23 if kind == "long tail" else 0)
+    assert rel_64(got, attention_64(q, kt, vt, start)) < bound
+
+
+@pytest.mark.parametrize("plane", ["keys", "values"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_attention_prefill_f32_cache_entries_that_are_not_finite(native_lib, plane, bad):
+    """A key or value that is not finite reaches the rows that see it and no earlier one, also of the same tile; values far
+    beyond f16 beside it keep their accuracy."""
+    from dyninfer_b200 import ops
+    s, start, at = 100, 20, 70              # row 50 of the chunk writes key 70, in the middle of the second tile
+    q, k, v = attention_inputs("normal", s, 4, 2, 128, 128)
+    k[:, 64:128] *= 1e3
+    v[:, 64:128] *= 1e6
+    want = attention_64(q, torch.from_numpy(k), torch.from_numpy(v), start)
+    (k if plane == "keys" else v)[1, at, 5] = bad
+    got = ops.attention(*(torch.from_numpy(t).cuda() for t in (q, k, v)), start).cpu().numpy().reshape(s, 4, 128)
+    want = want.reshape(s, 4, 128)
+    assert rel_64(got[:, :2], want[:, :2]) < 2.0 ** -20          # the other kv head
+    assert rel_64(got[:at - start], want[:at - start]) < 2.0 ** -20
+    assert not np.isfinite(got[at - start:, 2:, 5]).any()
