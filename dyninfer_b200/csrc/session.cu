@@ -376,6 +376,11 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
     if (d->S) thread_scratch_hold(d->ws_bytes);
     return 0;
   };
+  // the matrices a layer multiplies with: those that lie back to back as one
+  auto products = [](const LayerW& L) {
+    return std::array<const WRef*, 7>{L.qkv_parts >= 2 ? &L.qkv : &L.q, L.qkv_parts >= 2 ? nullptr : &L.k, L.qkv_parts == 3 ? nullptr : &L.v,
+                                      &L.o, L.gate_up.data ? &L.gate_up : &L.gate, L.gate_up.data ? nullptr : &L.up, &L.down};
+  };
   // 5 to 64 rows on one GPU (batched decode steps, short prompts): the skinny GEMM, its operands written by the
   // kernels in front of it (norm, attention merge), the residuals and the SwiGLU applied behind it: ten launches
   // per layer, each a programmatic dependent of the one before, so that weights stream while it drains. (0.6B
@@ -385,8 +390,8 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   bool skinny = rows > 4 && rows <= 64 && !tp && s->sk_x && H % 256 == 0 && H <= 8192 && c.inter % 32 == 0;
   for (int l = 0; l < c.layers && skinny; l++) {
     const LayerW& L = s->layers[l];
-    for (const WRef* w : {&L.q, &L.k, &L.v, &L.o, &L.gate, &L.up, &L.down})
-      skinny = skinny && gemm_skinny_takes(*w, rows) && gemm_skinny_terms(*w, rows) == 1;
+    for (const WRef* w : products(L))
+      if (w) skinny = skinny && gemm_skinny_takes(*w, rows) && gemm_skinny_terms(*w, rows) == 1;
     skinny = skinny && frag_class(L.q.enc) == frag_class(L.k.enc) && frag_class(L.q.enc) == frag_class(L.v.enc) && L.gate_up.data;
   }
   auto few = [&](const WRef& w, float* y, const float* residual, bool swiglu) -> int {
@@ -403,9 +408,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   bool fuse_n = !skinny && rows > 16 && !tp && s->xh && H <= 8192 && silu_prepare_takes(c.inter);
   for (int l = 0; l < c.layers && fuse_n; l++) {
     const LayerW& L = s->layers[l];
-    const WRef* ws[8] = {L.qkv_parts >= 2 ? &L.qkv : &L.q, L.qkv_parts >= 2 ? nullptr : &L.k, L.qkv_parts == 3 ? nullptr : &L.v,
-                         &L.o, L.gate_up.data ? &L.gate_up : &L.gate, L.gate_up.data ? nullptr : &L.up, &L.down, nullptr};
-    for (const WRef* w : ws)
+    for (const WRef* w : products(L))
       if (w && !(dqgemm_tc_takes(*w, rows) && dqgemm_tc_padded_rows(*w, rows) <= s->xh_rows)) fuse_n = false;
     if (H > s->xh_cols || c.inter > s->xh_cols) fuse_n = false;
   }

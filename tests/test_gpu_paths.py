@@ -242,3 +242,25 @@ def test_attention_prefill_f32_cache_entries_that_are_not_finite(native_lib, pla
     assert rel_64(got[:, :2], want[:, :2]) < 2.0 ** -20          # the other kv head
     assert rel_64(got[:at - start], want[:at - start]) < 2.0 ** -20
     assert not np.isfinite(got[at - start:, 2:, 5]).any()
+
+
+@pytest.mark.parametrize("hidden,inter", [(2048, 4608), (1024, 4608)])
+def test_few_row_steps_where_only_the_fused_matrix_is_large(native_lib, oracle, tmp_path, hidden, inter):
+    """gate and up pass for the few-row GEMM one by one, [gate; up] as one matrix does not: prompts and batched steps of 17
+    and more rows take another path, as steps of a larger model do."""
+    from dyninfer_b200 import checkpoint as ck
+    from test_gpu_model import oracle_run
+    cfg = dict(synth.SMALL_D128, layers=1, hidden=hidden, intermediate=inter, vocab=512)
+    path = synth.write_qwen3_gguf(str(tmp_path / "q.gguf"), cfg, seed=11)
+    cat = ck.open_catalog(path)
+    prompt = np.random.default_rng(1).integers(0, 512, size=40).tolist()
+    want, toks, _ = oracle_run(oracle, cat, prompt, 1, kv_round=2, kv_cap=64)
+    model = ModelLoader().load(path, max_kv=64, kv_dtype="bf16", chunk_size=64)
+    slots = 18
+    with model.create_batched_session(SessionConfig(max_sequence_length=64, batch_size=slots)) as s:
+        for b in range(slots):
+            lg, _ = s.prefill_slot(b, prompt, want_logits=True)
+            assert np.abs(lg - want[0]).max() <= 1e-2
+        _, logits = s.step({b: toks[0] for b in range(slots)}, want_logits=True)
+        for b in range(slots):
+            assert np.abs(logits[b] - want[1]).max() <= 1e-2 and helpers.cosine(logits[b], want[1]) >= 0.9999
