@@ -324,6 +324,7 @@ int64_t dqgemm_tc_padded_rows(const WRef& w, int64_t M);
 // Activations: f16 rows in the fragment order of the weight's encoding (sk_frag_off), gemm_skinny_terms planes of
 // [M, K], scaled by a power of two per row, with the inverse scales beside them.
 bool gemm_skinny_takes(const WRef& w, int64_t M);
+bool gemm_skinny_prefers(const WRef& w, int64_t M, bool chain);  // chain: inside a layer's chain of fused products
 int gemm_skinny_terms(const WRef& w, int64_t M);
 int launch_gemm_skinny(const WRef& w, const __half* x, const float* x_inv, int64_t M, float* y, const float* residual,
                        bool swiglu, cudaStream_t s, bool* handled);

@@ -877,10 +877,6 @@ int sk_run_enc(const SkArgs& a, const SkPlan& p, const CUtensorMap& wm, const CU
 // kernels (they carry 22 bits of an activation); K a multiple of 256 (of 512 for MLX-U4 and Q6_K).
 bool gemm_skinny_takes(const WRef& w, int64_t M) {
   if (M < 1 || M > 64 || w.rows < 1 || w.rows > (1LL << 30)) return false;
-  // more rows of a large matrix are bound by the mma.sync rate and by the activations every CTA reads: the tcgen05 GEMMs
-  // are ahead, from 17 rows where raw weights arrive in boxes (a step of 24 sequences through eight layers of the 8B
-  // shape 1.99 against 1.51 ms), from 33 with the others (24576 x 4096 Q6_K)
-  if (M > (gemm_stream_takes(w) ? 16 : 32) && w.rows * w.cols > (16LL << 20)) return false;
   {  // the activations of an eighth of K have to fit beside one warp's ring
     const int ku = sk_ku(w.enc), nt = M <= 8 ? 1 : M <= 16 ? 2 : M <= 32 ? 4 : 8;
     const int64_t stages = (w.cols + ku * SK_UNIT - 1) / (ku * SK_UNIT);
@@ -901,6 +897,21 @@ bool gemm_skinny_takes(const WRef& w, int64_t M) {
              ((reinterpret_cast<uintptr_t>(w.scales) | reinterpret_cast<uintptr_t>(w.biases)) & 15) == 0;
     default: return false;
   }
+}
+
+// Where the kernel is ahead of the tcgen05 GEMMs. More rows of a large matrix are bound by the mma.sync rate and by the
+// activations every CTA reads, from 17 rows where raw weights arrive in boxes, from 33 with the others.
+// A product by itself: over 100 shapes of 512 x 512 to 57344 x 8192 at 17 to 64 rows a line at 8 M weights costs 4.0 %
+// against the faster kernel of each shape, at 4 M 3.9, at 12 M 5.0, at 16 M 6.8 %; Q6_K at 33 to 64 rows 2.6, 2.7, 2.7 and
+// 4.7 % (4096 x 4096, 48 rows, here / there: Q4_0 19 / 14 us, Q6_K 46 / 26 us). Plain weights keep more of an f32 row here
+// than the GEMM's one f16 term, so they stay as long as they can.
+// In a chain of layers, where norm, residual and SwiGLU ride on the products, the line is higher: eight layers of
+// 2048 x 3072 ([gate; up] 12 M) take 0.50 against 0.65 ms at 24 rows, Q6_K 0.80 against 0.86 at 40 (Q4_0 0.78 against 0.72
+// there); eight layers of the 8B shape (100 M) 1.99 against 1.51 ms.
+bool gemm_skinny_prefers(const WRef& w, int64_t M, bool chain) {
+  if (!gemm_skinny_takes(w, M)) return false;
+  const int64_t line = (chain || sk_plain(w.enc) ? 16LL : 8LL) << 20;
+  return M <= (gemm_stream_takes(w) ? 16 : 32) || w.rows * w.cols <= line;
 }
 
 // y[M, N] = x w^T + residual, or with `swiglu` (the matrix is [gate; up], N = rows / 2) silu(x gate^T) * (x up^T).
@@ -984,7 +995,6 @@ int launch_skinny_prepare(const WRef& w, const void* x, int x_type, int64_t M, _
 int launch_linear_skinny(const WRef& w, const void* x, int x_type, int64_t M, float* y, const float* residual, cudaStream_t s,
                          bool* handled) {
   *handled = false;
-  if (!gemm_skinny_takes(w, M)) return 0;
   const size_t xb = ((size_t)gemm_skinny_terms(w, M) * M * w.cols * 2 + 255) / 256 * 256, bytes = xb + (size_t)M * 4;
   uint8_t* ws = reinterpret_cast<uint8_t*>(thread_scratch(bytes));
   const bool pooled = ws == nullptr;

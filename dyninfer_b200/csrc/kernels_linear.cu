@@ -123,24 +123,21 @@ int launch_linear(const WRef& w, const void* x, int x_type, int64_t m, float* y,
   DYN_CHECK(x_type == E_F32 || x_type == E_BF16, "linear: x_type must be f32 or bf16, got %d",
             x_type);
   DYN_CHECK(m >= 1, "linear: m must be >= 1");
-  // more rows than one pass of the tensor-core GEMV takes (4 with f32 activations, 8 with bf16):
-  // dequant-in-shared-memory tensor-core GEMM, one pass over the weights for all rows
-  // (below 17 rows only for the encodings with a word-fetching GEMM producer, which beats repeated GEMV
-  // passes: the GEMM's dequantisation cost does not shrink with the row count)
   // few rows, exact weights and 22-bit activations: f32 rows up to 4, bf16 rows up to 8
   if (m <= (x_type == E_BF16 ? 8 : 4) && gemv_rows_prefers(w, m)) {
     bool handled = false;
     if (launch_gemv_rows(w, x, x_type, m, nullptr, 0, 0.f, y, residual, false, s, &handled)) return 1;
     if (handled) return 0;
   }
-  // up to 64 rows beyond what the exact few-row kernels take: one launch, weights streamed once. From 17 rows of a large
-  // matrix the tensor-memory GEMM is ahead (4096 x 4096 Q4_0, 24 rows: 12 against 19 us; 40000 x 2560: 35 against 45 us).
-  const bool stream = m > 16 && w.rows * w.cols > (8LL << 20) && gemm_stream_takes(w);
-  if (!stream && m <= 64 && m > (x_type == E_BF16 ? 8 : 4)) {
+  // up to 64 rows beyond what the exact few-row kernels take: one activation pass, weights streamed once
+  if (m > (x_type == E_BF16 ? 8 : 4) && gemm_skinny_prefers(w, m, false)) {
     bool handled = false;
     if (launch_linear_skinny(w, x, x_type, m, y, residual, s, &handled)) return 1;
     if (handled) return 0;
   }
+  // what is left of more rows than one pass of the tensor-core GEMV takes (4 with f32 activations, 8 with bf16): dequant
+  // GEMM, one pass over the weights for all rows (below 17 rows only for the encodings with a word-fetching producer, which
+  // beats repeated GEMV passes: the GEMM's dequantisation cost does not shrink with the row count)
   const bool cheap_producer = w.enc == E_Q4_0 || w.enc == E_Q4_1 || w.enc == E_Q8_0 || w.enc == E_Q6_K ||
                               w.enc == E_Q4_K || w.enc == E_Q5_K || w.enc == E_IQ4_XS || w.enc == E_MLX_U4;
   if (m > 16 || (cheap_producer && m > (x_type == E_BF16 ? 8 : 4))) {

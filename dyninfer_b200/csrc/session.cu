@@ -391,7 +391,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   for (int l = 0; l < c.layers && skinny; l++) {
     const LayerW& L = s->layers[l];
     for (const WRef* w : products(L))
-      if (w) skinny = skinny && gemm_skinny_takes(*w, rows) && gemm_skinny_terms(*w, rows) == 1;
+      if (w) skinny = skinny && gemm_skinny_prefers(*w, rows, true) && gemm_skinny_terms(*w, rows) == 1;
     skinny = skinny && frag_class(L.q.enc) == frag_class(L.k.enc) && frag_class(L.q.enc) == frag_class(L.v.enc) && L.gate_up.data;
   }
   auto few = [&](const WRef& w, float* y, const float* residual, bool swiglu) -> int {
@@ -717,7 +717,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   }
   if (all_rows) {
     // batched decode: every row is the last token of its own sequence
-    if (rows > 4 && rows <= 64 && !tp && s->sk_x && H % 256 == 0 && H <= 8192 && gemm_skinny_takes(s->lm_head, rows) &&
+    if (rows > 4 && rows <= 64 && !tp && s->sk_x && H % 256 == 0 && H <= 8192 && gemm_skinny_prefers(s->lm_head, rows, true) &&
         gemm_skinny_terms(s->lm_head, rows) == 1) {
       if (launch_norm_frag(s->hidden, s->out_norm.ptr, s->out_norm.type, rows, H, c.eps, s->lm_head.enc, s->sk_x, s->sk_inv, st) ||
           few(s->lm_head, s->batch_logits, nullptr, false))
