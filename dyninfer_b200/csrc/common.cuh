@@ -333,7 +333,7 @@ int launch_linear_skinny(const WRef& w, const void* x, int x_type, int64_t M, fl
                          bool* handled);
 // The exact few-row product (gemv_rows.cu): 1 to 8 rows, optionally RMSNorm in front, residual or SwiGLU behind.
 bool gemv_rows_takes(const WRef& w, int64_t M);
-bool gemv_rows_prefers(const WRef& w, int64_t M);
+bool gemv_rows_prefers(const WRef& w, int64_t M, bool fused);  // fused: with the norm in front
 int launch_gemv_rows(const WRef& w, const void* x, int x_type, int64_t M, const void* norm_w, int norm_type, float eps, float* y,
                      const float* residual, bool swiglu, cudaStream_t s, bool* handled);
 bool gemv_cs_q8_0_shape_ok(const WRef& w, int M);

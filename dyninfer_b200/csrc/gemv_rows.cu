@@ -21,6 +21,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
 #include <array>
 #include <map>
 
@@ -635,6 +636,7 @@ struct GrPlan {
   int NM, RW, KW, CK, nst, kstages, cstages;
   int64_t groups;
   size_t smem;
+  int per_sm;  // CTAs that share an SM
 };
 
 int gr_ku(int enc) { return enc == E_MLX_U4 || enc == E_Q6_K ? 2 : 1; }
@@ -656,6 +658,26 @@ size_t gr_smem(const WRef& w, const GrPlan& p) {
   const size_t x = (size_t)p.NM * 2 * (units * 512 + 64) + (size_t)gr_ku(w.enc) * 512 + (size_t)p.NM * units * 4 * gr_ng(w.enc) * 4;
   const size_t red = ((size_t)p.KW + 1) * p.NM * rows * 4;
   return 1024 + std::max(ring + x, red);
+}
+
+template <int ENC>
+const void* gr_kernel_of(int nm) {
+  switch (nm) {
+    case 1: return reinterpret_cast<const void*>(gemv_rows_kernel<ENC, 1>);
+    case 2: return reinterpret_cast<const void*>(gemv_rows_kernel<ENC, 2>);
+    case 4: return reinterpret_cast<const void*>(gemv_rows_kernel<ENC, 4>);
+    default: return reinterpret_cast<const void*>(gemv_rows_kernel<ENC, 8>);
+  }
+}
+const void* gr_kernel(int enc, int nm) {
+  switch (enc) {
+    case E_Q4_1: return gr_kernel_of<E_Q4_1>(nm);
+    case E_Q8_0: return gr_kernel_of<E_Q8_0>(nm);
+    case E_Q6_K: return gr_kernel_of<E_Q6_K>(nm);
+    case E_Q4_K: return gr_kernel_of<E_Q4_K>(nm);
+    case E_MLX_U4: return gr_kernel_of<E_MLX_U4>(nm);
+    default: return gr_kernel_of<E_Q4_0>(nm);
+  }
 }
 
 // The split of the work, from sweeps of all plans over eleven shapes at 1 to 4 rows: eight warps per CTA (four where
@@ -691,6 +713,10 @@ bool gr_make_plan(const WRef& w, int64_t M, bool swiglu, GrPlan* best) {
     if (found) break;
   }
   if (!found) return false;
+  const void* kernel = gr_kernel(w.enc, best->NM);
+  if (ensure_dynamic_smem(kernel, GR_MAX_SMEM) ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&best->per_sm, kernel, best->RW * best->KW * 32, best->smem) != cudaSuccess || best->per_sm < 1)
+    best->per_sm = 1;
   const int rows = (swiglu ? 8 : 16) * best->RW;
   best->groups = (N + rows - 1) / rows;
   if (best->groups * best->CK > 0x7fffffff) return false;
@@ -771,18 +797,56 @@ bool gemv_rows_takes(const WRef& w, int64_t M) {
   }
 }
 
-// Where this kernel is ahead of the ones that split K over CTAs and add the sums in a second launch (they keep one
-// CTA per SM alive over all its tiles): one row, all but the vocabulary-sized matrices, whose tiles are done before
-// a CTA's prologue has paid off (151936 x 1024 Q4_0 28 against 24 us, Q6_K 39 against 36), and the widest rows
-// (5120 x 25600: 40 against 29); three and four rows, all but large 4-bit matrices (24576 x 4096: 43 against 39); five to eight bf16 rows, which the
-// other kernel multiplies as one term, small matrices only (3072 x 1024: 14 against 19, 4096 x 4096: 39 against 24).
-bool gemv_rows_prefers(const WRef& w, int64_t M) {
-  if (!gemv_rows_takes(w, M) || w.cols >= 16384) return false;
+// Where this kernel is ahead of those that split K over CTAs and add the sums in a second launch (they keep one CTA per SM
+// alive over all its tiles). Both sides measured on 100 shapes of 512 x 512 to 57344 x 8192 per encoding, us here / there.
+// What decides is the plan, not the size: CTAs that do not fit the SMs at once leave a second round, and one that is
+// nearly empty costs as much as a full one. 5120 x 13824 Q4_0 has 320 CTAs for 296 places: 26 / 17 (4096 x 14336, 256
+// CTAs: 14.5 / 14.7); with eight tiles per CTA there are so many that it does not show (40745 x 1536: 14 / 15).
+//   One row: vocabulary-sized matrices are done before a prologue has paid off (151936 x 1024 Q4_0 27 / 23, Q6_K 40 / 35;
+//     between 65536 and 128256 rows the two are within 10 % either way); with rows of 16384 and more the others have to fall
+//     back for Q8_0 and Q6_K (8192 x 28672 52 / 117 and 70 / 174; Q4_0 5120 x 25600 39 / 25); wide rows need more than a
+//     CTA per SM (1288 x 12800 Q4_0 13 / 10). Q6_K, four warps per CTA, needs the SMs filled by one round from 4096 wide on
+//     (4096 x 14336 21 / 23, 12288 x 4096 21 / 17, 2560 x 9728 17 / 15). MLX-U4 has the slower kernel on the other side.
+//   Two rows: nearly always (12288 x 4096 Q4_0 15 / 38).
+//   Three and four: the others are bound by arithmetic, so all but large matrices (24576 x 4096 Q4_0 43 / 39); Q8_0 also
+//     those, unless clusters of four are left with short shares (27648 x 5120 80 / 69, 10240 x 5120 39 / 53); Q4_K, whose
+//     other side is the row kernel, the large ones (24576 x 4096 45 / 87, 1024 x 1024 9 / 7, 5120 x 5120 with its second
+//     round 42 / 29).
+//   Five to eight bf16 rows, which the other kernel multiplies as one term: small matrices only (3072 x 1024 Q4_0 14 / 25,
+//     4096 x 4096 40 / 38), Q4_K none (1024 x 1024 14 / 9).
+//   Q6_K rows that are not multiples of 8 bytes (K an odd multiple of 512) come in a copy per row here; the row kernel on
+//     the other side is ahead on few rows (2560 x 2560, four rows 20 / 12, eight bf16 rows 48 / 18).
+// `fused`: the norm in front rides on this kernel, which saves a launch (3 us): below 32 MB of weights that is worth more
+// than the differences above (a step of four 14B-sized layers 374 -> 338 us with this rule, of Q6_K 606 -> 507).
+bool gemv_rows_prefers(const WRef& w, int64_t M, bool fused) {
+  GrPlan p;
+  if (!gemv_rows_takes(w, M) || !gr_plan(w, M, false, &p)) return false;
+  const bool six = w.enc == E_Q6_K, odd = six && w.row_bytes() % 8, wide = w.cols >= 16384;
   const int64_t units = ((w.rows + 15) / 16) * (w.cols / GR_UNIT);
-  if (M == 1) return w.rows < 100000;
-  if (M == 2) return true;
-  if (M <= 4) return w.enc == E_Q6_K || w.enc == E_Q8_0 || units < 16384;
-  return w.enc == E_Q6_K ? units < 8192 : units < 1024;  // bf16 rows, whose second term is zero
+  const double places = (double)p.per_sm * std::max(1, sm_count()), rounds = p.groups * p.CK / places;
+  const bool tail = rounds > 1 && rounds < 0.7 * std::ceil(rounds) && p.RW < (six ? 4 : 8);
+  const bool chain = fused && !wide && w.total_bytes() < ((int64_t)32 << 20);
+  if (M == 1) {
+    if (w.rows >= 100000) return false;
+    if (chain) return true;
+    if (wide) return six || (w.enc == E_Q8_0 && !tail);
+    if (six && w.cols >= 4096) return rounds >= 0.55 && rounds <= 1;
+    if (tail && !(w.enc == E_MLX_U4 && w.cols <= 6144)) return false;
+    return w.cols <= 12288 || p.groups * p.CK > sm_count();
+  }
+  if (wide) return false;
+  if (M == 2) return chain || !odd || w.rows > 5200;
+  if (M <= 4) {
+    if (chain && (six || w.enc == E_Q8_0)) return true;
+    if (odd) return w.cols < 2048 && w.rows >= 18000;
+    if (six) return units < 65536;
+    if (w.enc == E_Q8_0) return units < 32768 || p.CK < 4 || p.cstages > 5;
+    if (w.enc == E_Q4_K) return chain || ((w.rows >= 8000 || w.cols >= 2048) && !(tail && units < 8192));
+    return units < 16384 && !(p.per_sm == 1 && rounds > 1);
+  }
+  if (w.enc == E_Q4_K) return false;
+  if (odd) return w.cols < 2048 && w.rows >= 18000 && M < 8;
+  return units < (six ? 8192 : 1024);
 }
 
 // y[M, N] = x w^T + residual, or with `swiglu` (the matrix is [gate; up], N = rows / 2) silu(x gate^T) * (x up^T);

@@ -124,7 +124,7 @@ int launch_linear(const WRef& w, const void* x, int x_type, int64_t m, float* y,
             x_type);
   DYN_CHECK(m >= 1, "linear: m must be >= 1");
   // few rows, exact weights and 22-bit activations: f32 rows up to 4, bf16 rows up to 8
-  if (m <= (x_type == E_BF16 ? 8 : 4) && gemv_rows_prefers(w, m)) {
+  if (m <= (x_type == E_BF16 ? 8 : 4) && gemv_rows_prefers(w, m, false)) {
     bool handled = false;
     if (launch_gemv_rows(w, x, x_type, m, nullptr, 0, 0.f, y, residual, false, s, &handled)) return 1;
     if (handled) return 0;

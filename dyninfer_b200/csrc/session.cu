@@ -419,7 +419,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   const NormW* normed_by = nullptr;  // which norm of `hidden` xn holds
   auto norm_product = [&](const WRef& w, const NormW& nw, float* y, bool swiglu) -> int {
     bool handled = false;
-    if (gemv_rows_prefers(w, rows) &&
+    if (gemv_rows_prefers(w, rows, true) &&
         launch_gemv_rows(w, s->hidden, E_F32, rows, nw.ptr, nw.type, c.eps, y, nullptr, swiglu, st, &handled))
       return 1;
     if (handled) return 0;

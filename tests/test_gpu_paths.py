@@ -264,3 +264,17 @@ def test_few_row_steps_where_only_the_fused_matrix_is_large(native_lib, oracle, 
         _, logits = s.step({b: toks[0] for b in range(slots)}, want_logits=True)
         for b in range(slots):
             assert np.abs(logits[b] - want[1]).max() <= 1e-2 and helpers.cosine(logits[b], want[1]) >= 0.9999
+
+
+@pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q8_0", "gguf.q6_k", "gguf.q4_k", "mlx.affine.u4"])
+@pytest.mark.parametrize("m,n,k", [(1, 5120, 13824), (1, 4096, 4608), (1, 640, 16384), (1, 1288, 12800), (3, 2560, 2560),
+                                   (4, 5120, 5120), (2, 700, 1536)])
+def test_linear_few_rows_on_both_sides_of_the_plan_rule(native_lib, oracle, enc, m, n, k):
+    """Products whose plan leaves a nearly empty round, too few blocks, or copies per row, and their neighbours: whichever
+    kernel takes them, f32 rows keep f32 accuracy."""
+    from dyninfer_b200 import ops
+    from test_gpu_ops import make_pair
+    dw, ow = make_pair(oracle, enc, n, k, seed=n + m)
+    x = np.random.default_rng(m).normal(size=(m, k)).astype(np.float32)
+    got = ops.linear(dw, torch.from_numpy(x).cuda()).cpu().numpy()
+    assert helpers.rel_err(got, oracle.linear(ow, x, fast=True)) < 2e-5
