@@ -138,9 +138,9 @@ __device__ __forceinline__ void f16_row_scale(float mx, float* red, float* sc, f
   f16_scale_for(mx, sc, inv);
 }
 
-// FULL: the row is exactly PER x 256 elements, so that every access is a constant offset from a thread's own pointers
-// (with bounds and 64-bit indices per element the kernel took 130 registers and one block per SM: 512 rows x 4096
-// with two slices 36 us).
+// FULL: the row is a multiple of 256 elements, at most PER of them per thread, so that every access is a constant offset
+// from a thread's own pointers under a condition that the whole block shares (with bounds and 64-bit indices per element
+// the kernel took 130 registers and one block per SM: 512 rows x 4096 with two slices 36 us).
 template <int PER, bool FULL>
 __global__ void __launch_bounds__(256, PER <= 8 ? 6 : PER <= 16 ? 4 : 2)
 norm_prepare_kernel(const float* __restrict__ x, const float* __restrict__ partial, int S, int64_t rows,
@@ -149,7 +149,8 @@ norm_prepare_kernel(const float* __restrict__ x, const float* __restrict__ parti
   __shared__ float red[32];
   const int T = FULL ? 256 : (int)blockDim.x, tid = threadIdx.x;
   const int64_t at = (int64_t)blockIdx.x * width + tid;
-  auto in = [&](int k) { return FULL || tid + k * T < width; };
+  const int runs = width >> 8;
+  auto in = [&](int k) { return FULL ? k < runs : tid + k * T < width; };
   pdl_trigger();
   float v[PER];
   pdl_wait();
@@ -220,13 +221,24 @@ int launch_norm_prepare(const float* x, const float* partial, int splits, const 
                       eps, xh, inv_s);
   };
   cudaError_t e;
-  if (width == 1024) e = run(norm_prepare_kernel<4, true>);
-  else if (width == 2048) e = run(norm_prepare_kernel<8, true>);
-  else if (width == 4096) e = run(norm_prepare_kernel<16, true>);
-  else if (width == 5120) e = run(norm_prepare_kernel<20, true>);
-  else if (width <= 8 * threads) e = run(norm_prepare_kernel<8, false>);
-  else if (width <= 16 * threads) e = run(norm_prepare_kernel<16, false>);
-  else e = run(norm_prepare_kernel<32, false>);
+  if (width >= 1024 && width % 256 == 0) {  // elements per thread, rounded up to a multiple of four
+    switch ((width + 1023) / 1024) {
+      case 1: e = run(norm_prepare_kernel<4, true>); break;
+      case 2: e = run(norm_prepare_kernel<8, true>); break;
+      case 3: e = run(norm_prepare_kernel<12, true>); break;
+      case 4: e = run(norm_prepare_kernel<16, true>); break;
+      case 5: e = run(norm_prepare_kernel<20, true>); break;
+      case 6: e = run(norm_prepare_kernel<24, true>); break;
+      case 7: e = run(norm_prepare_kernel<28, true>); break;
+      default: e = run(norm_prepare_kernel<32, true>);
+    }
+  } else if (width <= 8 * threads) {
+    e = run(norm_prepare_kernel<8, false>);
+  } else if (width <= 16 * threads) {
+    e = run(norm_prepare_kernel<16, false>);
+  } else {
+    e = run(norm_prepare_kernel<32, false>);
+  }
   DYN_CUDA(e);
   count_launch();
   DYN_CUDA(cudaGetLastError());
