@@ -903,11 +903,22 @@ int launch_dqgemm_tc(const WRef& w, const void* x, int x_type, int64_t M, float*
   if (io) io->splits = 0;
   if (!tg_shape_ok(w, M)) return 0;
   // A prompt's chunks keep the grouping of their sums: few tiles go on through the K split below (whose sums the next
-  // kernel adds up: 1024 x 2048, 512 rows 10 against 17 us), all others in whole tiles. So do very few tiles of a long K
-  // (1024 x 12288, 512 rows: 37 against 40 us), where the last arriver would add up eight wide parts.
-  const int old_splits = gemm_stream_takes(w) ? tg_plan(w, M).splits : 0;
-  const bool few_tiles = old_splits == 8 && M > 256 && w.cols >= 8192;
-  if (gemm_stream_takes(w) && !few_tiles && !(io && io->grouped && old_splits > 1)) {
+  // kernel adds up: 1024 x 2048, 512 rows 10 against 17 us), all others in whole tiles. Other products stay below where the
+  // split of a long K gives most SMs one wide tile: in gemm_stream the last arriver of a shared tile would add up as many
+  // wide parts. Over 360 shapes of 640 x 6144 to 4096 x 20480 at 96 to 2048 rows per encoding this rule costs 1.6 % against
+  // the faster kernel of each, gemm_stream always 2.8. us, below / gemm_stream: Q4_0 1024 x 12288, 512 rows 31 / 34,
+  // 2048 x 12288, 512 rows 41 / 51, 4096 x 12288, 256 rows 41 / 50; where the split leaves a third of the SMs idle
+  // 512 x 12288, 300 rows 28 / 26; Q4_K and Q5_K convert faster in gemm_stream (2048 x 20480, 300 rows 72 / 55, 108 / 60).
+  int old_splits = 0;
+  bool split_fills = false;
+  if (gemm_stream_takes(w)) {
+    const TgPlan old = tg_plan(w, M);
+    const int64_t ctas = (w.rows + TG_BM - 1) / TG_BM * old.mtiles * old.splits, sms = std::max(1, sm_count());
+    old_splits = old.splits;
+    split_fills = old.splits >= 4 && ctas <= sms && 10 * ctas >= 7 * sms && old.bn >= 160 && w.cols >= 8192 &&
+                  w.enc != E_Q4_K && w.enc != E_Q5_K;
+  }
+  if (gemm_stream_takes(w) && !(io && io->grouped ? old_splits > 1 : split_fills)) {
     *handled = true;
     return run_gemm_stream(w, x, x_type, M, y, residual, s, io);
   }

@@ -297,3 +297,17 @@ def test_many_row_norm_widths(native_lib, oracle, tmp_path, hidden):
     with model.create_session(SessionConfig(max_sequence_length=128)) as s:
         got = s.prefill(prompt).values
     assert np.abs(got - want[0]).max() <= 1e-2 and helpers.cosine(got, want[0]) >= 0.9999
+
+
+@pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q8_0", "gguf.q4_k", "mlx.affine.u4"])
+@pytest.mark.parametrize("m,n,k", [(256, 4096, 8192), (300, 1024, 8192), (300, 640, 8192), (160, 3500, 8192)])
+def test_linear_many_rows_where_a_k_split_fills_the_gpu(native_lib, oracle, enc, m, n, k):
+    """A long K split over about as many blocks as there are SMs, and its neighbours that are cut into equal shares."""
+    from dyninfer_b200 import ops
+    from test_gpu_ops import make_pair
+    dw, ow = make_pair(oracle, enc, n, k, seed=n + m)
+    x = np.random.default_rng(m).normal(size=(m, k)).astype(np.float32)
+    rows = [0, 63, 127, 128, m - 1]
+    got = ops.linear(dw, torch.from_numpy(x).cuda()).cpu().numpy()
+    want = oracle.linear(ow, x[rows], fast=True)
+    assert helpers.rel_err(got[rows], want) < 1e-3
