@@ -397,6 +397,21 @@ gemm_skinny_kernel(const SkArgs a, const __grid_constant__ CUtensorMap wmap, con
         for (int h = 0; h + 1 < CH; h++) accx[h][rt][nt][e] = 0.f;
       }
     }
+  // Plain weights: an mma truncates where it adds to its accumulator (about 1.5e-8 of the sum each time, always toward
+  // zero), so the sums start from zero with every unit and are added up with rounded adds, up to 16 rows with the lower
+  // terms in accumulators of their own. Error against 64 bits of a 4096 x 4096 bf16 matrix, 16 f32 rows: 1.7e-6 with one
+  // chain, now 1.4e-7 (row kernel in f32: 2.1e-7); 151936 x 1024, 16 rows 135 -> 145 us, 8 rows 82 as before. Quantised weights
+  // are rounded to 2^-12, which hides this.
+  constexpr bool APART = PLAIN && NT <= 2;
+  float tot[PLAIN ? NT : 1][4], low[APART ? 2 : 1][APART ? NT : 1][4];
+#pragma unroll
+  for (int nt = 0; nt < (PLAIN ? NT : 1); nt++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) tot[nt][e] = 0.f;
+#pragma unroll
+  for (int nt = 0; nt < (APART ? NT : 1); nt++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) low[0][nt][e] = low[APART ? 1 : 0][nt][e] = 0.f;
   auto give_up = [&]() {
     if (!s_abort) {
       s_abort = 1;
@@ -497,8 +512,9 @@ gemm_skinny_kernel(const SkArgs a, const __grid_constant__ CUtensorMap wmap, con
             for (int rt = 0; rt < RT; rt++) {
               constexpr bool BF = ENC == E_BF16;
               const int h0 = CH == 4 ? 2 * (c & 1) : 0, h1 = CH == 4 ? h0 + 1 : CH == 2 ? 1 : 0;
-              float(&c0)[4] = h0 == 0 ? acc[rt][nt] : accx[h0 > 0 ? h0 - 1 : 0][rt][nt];
-              float(&c1)[4] = h1 == 0 ? acc[rt][nt] : accx[h1 > 0 ? h1 - 1 : 0][rt][nt];
+              const bool second = APART && k > 0;
+              float(&c0)[4] = second ? low[0][APART ? nt : 0] : h0 == 0 ? acc[rt][nt] : accx[h0 > 0 ? h0 - 1 : 0][rt][nt];
+              float(&c1)[4] = second ? low[APART ? 1 : 0][APART ? nt : 0] : h1 == 0 ? acc[rt][nt] : accx[h1 > 0 ? h1 - 1 : 0][rt][nt];
               const uint32_t(&q0)[4] = p0[pc][rt], (&q1)[4] = p1[pc][rt];
               if constexpr (BF) {
                 mma_bf16_16816(c0, q0[0], q1[0], q0[1], q1[1], b.x, b.y);
@@ -514,13 +530,27 @@ gemm_skinny_kernel(const SkArgs a, const __grid_constant__ CUtensorMap wmap, con
       if constexpr (PLAIN) {
         __syncwarp();
         issue();
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            float v = acc[0][nt][e];
+#pragma unroll
+            for (int h = 0; h + 1 < CH; h++) v += accx[h][0][nt][e], accx[h][0][nt][e] = 0.f;
+            tot[nt][e] += v, acc[0][nt][e] = 0.f;
+          }
       }
     }
     if (!ok) break;
     xu += a.KW * KU * 512;
     if (++slot == nst) slot = 0, parity ^= 1u;
   }
-  if constexpr (CH > 1) {
+  if constexpr (PLAIN) {
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) acc[0][nt][e] = APART ? tot[nt][e] + (low[0][APART ? nt : 0][e] + low[APART ? 1 : 0][APART ? nt : 0][e]) : tot[nt][e];
+  } else if constexpr (CH > 1) {
 #pragma unroll
     for (int h = 0; h + 1 < CH; h++)
 #pragma unroll

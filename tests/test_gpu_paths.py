@@ -311,3 +311,15 @@ def test_linear_many_rows_where_a_k_split_fills_the_gpu(native_lib, oracle, enc,
     got = ops.linear(dw, torch.from_numpy(x).cuda()).cpu().numpy()
     want = oracle.linear(ow, x[rows], fast=True)
     assert helpers.rel_err(got[rows], want) < 1e-3
+
+
+@pytest.mark.parametrize("enc", ["plain.bf16", "plain.f16"])
+@pytest.mark.parametrize("m,n,k", [(5, 4096, 4096), (8, 3072, 1024), (9, 520, 2560), (16, 4096, 4096)])
+def test_linear_few_rows_of_plain_weights_keep_f32_accuracy(native_lib, enc, m, n, k):
+    """5 to 16 f32 rows against 64 bits: the terms hold 2^-24 of a value, a unit of K adds chains of up to eight mma at 2^-26
+    of the sum each, the units are added with roundings of 2^-25."""
+    from dyninfer_b200 import ops
+    w = ops.DeviceWeight(enc, n, k, synth.random_weight(enc, n, k, seed=m)["data"])
+    x = torch.randn(m, k, generator=torch.Generator("cuda").manual_seed(m), device="cuda")
+    want = (x.double() @ ops.dequant(w).double().T).cpu().numpy()
+    assert rel_64(ops.linear(w, x).double().cpu().numpy(), want) < 2.0 ** -21
