@@ -46,7 +46,6 @@ class DeviceWeight:
         self.data = buf
         self.scales = _dev(np.ascontiguousarray(scales).view(np.uint8).reshape(-1), device) if scales is not None else None
         self.biases = _dev(np.ascontiguousarray(biases).view(np.uint8).reshape(-1), device) if biases is not None else None
-        self._ref = None
         self.nbytes = raw.size + (self.scales.numel() if self.scales is not None else 0) + \
             (self.biases.numel() if self.biases is not None else 0)
 
@@ -54,11 +53,16 @@ class DeviceWeight:
         return _lib.Weight(ENC[self.encoding], ENC.get(self.aux, 2), self.group, 0, self.rows,
                            self.cols, _p(self.data), _p(self.scales), _p(self.biases))
 
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        object.__setattr__(self, "_ref", None)     # whatever was described may have changed
+
     def ref(self):
-        """The descriptor by reference, built once: a small product's time is mostly the host's."""
-        key = (self.data.data_ptr(), self.scales.data_ptr() if self.scales is not None else 0)
+        """The descriptor by reference, built once for what it describes: a small product's time is mostly the host's."""
+        key = (self.data.data_ptr(), None if self.scales is None else self.scales.data_ptr(),
+               None if self.biases is None else self.biases.data_ptr())
         if self._ref is None or self._ref[0] != key:
-            self._ref = (key, C.byref(self.c()))
+            object.__setattr__(self, "_ref", (key, C.byref(self.c())))
         return self._ref[1]
 
 
