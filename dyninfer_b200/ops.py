@@ -15,8 +15,15 @@ from . import _lib
 from ._lib import ENC, check, lib
 
 
+# torch's current stream as an integer: 0.2 us through its raw getters (3.2 us through a Stream object), which are not
+# part of its public interface, so a torch without them takes the public way
+_raw_stream, _raw_device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream():
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    if _raw_stream is None or _raw_device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_raw_device())
 
 
 def _p(t):

@@ -36,3 +36,12 @@ def test_changed_fields_are_described_anew(weight, field, value, name):
     weight.ref()
     setattr(weight, field, value)
     assert getattr(described(weight), name) == (_lib.ENC[value] if isinstance(value, str) else value)
+
+
+@pytest.mark.parametrize("missing", ["_raw_stream", "_raw_device"])
+def test_the_stream_comes_the_public_way_from_a_torch_without_raw_getters(monkeypatch, missing):
+    class Stream:
+        cuda_stream = 1234
+    monkeypatch.setattr(ops, missing, None)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: Stream)
+    assert ops._stream() == 1234
