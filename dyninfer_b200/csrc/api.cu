@@ -5,7 +5,6 @@
 #include <stdarg.h>
 #include <stdio.h>
 
-#include <atomic>
 #include <map>
 #include <mutex>
 #include <string>
@@ -194,8 +193,6 @@ int wref_from_api(const dyninfer_cuda_weight_t* w, WRef* out) {
 }
 
 static int require_device() {
-  static std::atomic<bool> usable{false};  // asked once: a process does not lose its devices
-  if (usable.load(std::memory_order_relaxed)) return 0;
   int n = 0;
   cudaError_t e = cudaGetDeviceCount(&n);
   if (e != cudaSuccess || n <= 0) {
