@@ -363,12 +363,11 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   const size_t layer_stride = (size_t)c.batch * c.kv_heads * cap * c.head_dim * s->kv_elem;
   if (launch_gather(s->embed, s->tokens_dev, rows, s->hidden, st)) return 1;
   bool normed = false;  // xn already holds this layer's attn_norm rows (fused into the last exchange)
-  // One row: the q / k / v and [gate; up] products (local also under tensor parallelism), when their K is
-  // split over CTAs, leave the
-  // addition of the K-slice sums to the kernel that consumes the result (QKV prepare, SwiGLU): three
-  // launches fewer per layer (8B mixed: 3.24 -> 2.90 ms per step). The sums wait in the session's scratch,
-  // held until that kernel is enqueued. The same for o / down with residual + RMSNorm in one single-block
-  // kernel was slower (3.39 ms): their reductions stay separate, multi-block launches.
+  // One row on a tensor-parallel rank (one GPU takes the chain of exact products below): a q / k / v or [gate; up] product
+  // whose K is split over CTAs, which is where the one-launch kernel hands over to the column-split ones, leaves the addition
+  // of its K-slice sums to the kernel that consumes the result (QKV prepare, SwiGLU). The sums wait in the session's scratch,
+  // held until that kernel is enqueued. The same for o / down with residual + RMSNorm in one single-block kernel was slower
+  // (8B mixed: 3.39 against 3.24 ms per step): their reductions stay separate, multi-block launches.
   const bool fuse1 = rows == 1;
   auto linear_deferred = [&](const WRef& w, const float* x, float* y, Deferred* d) -> int {
     DeferScope scope(d);
@@ -428,6 +427,32 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
     if (!swiglu) return launch_linear(w, s->xn, E_F32, rows, y, nullptr, st);
     return launch_linear(w, s->xn, E_F32, rows, s->gu1, nullptr, st) || launch_silu_mul_rows(s->gu1, rows, c.inter, y, st);
   };
+  // a layer's q, k, v rows (row strides 0: dense) with its norms and its planes of the cache, and the attention over them
+  auto qkv_args = [&](int l, float* q, float* k, float* v, int64_t ldq, int64_t ldk, int64_t ldv) {
+    const LayerW& L = s->layers[l];
+    QkvPrepArgs pa{};
+    pa.q = q, pa.k = k, pa.v = v;
+    pa.kcache = s->kcache + (size_t)l * layer_stride, pa.vcache = s->vcache + (size_t)l * layer_stride;
+    pa.q_norm_w = L.q_norm.ptr, pa.k_norm_w = L.k_norm.ptr, pa.norm_w_type = L.q_norm.type;
+    pa.row_pos = s->row_pos_dev, pa.row_seq = s->row_seq_dev, pa.base_pos = 0;
+    pa.rows = rows, pa.nh = c.heads, pa.nkv = c.kv_heads, pa.d = c.head_dim, pa.cap = cap;
+    pa.kv_type = s->kv_type, pa.has_norm = c.qk_norm ? 1 : 0, pa.has_rope = c.rope ? 1 : 0;
+    pa.eps = c.eps;
+    pa.ldq = ldq, pa.ldk = ldk, pa.ldv = ldv;
+    return pa;
+  };
+  auto attn_args = [&](const QkvPrepArgs& pa) {
+    AttnArgs aa{};
+    aa.q = pa.q, aa.kcache = pa.kcache, aa.vcache = pa.vcache;
+    aa.row_pos = pa.row_pos, aa.row_seq = pa.row_seq, aa.base_pos = 0;
+    aa.ctx = s->ctx;
+    aa.rows = rows, aa.nh = pa.nh, aa.nkv = pa.nkv, aa.d = pa.d, aa.cap = cap;
+    aa.kv_type = pa.kv_type;
+    aa.ldq = pa.ldq;
+    aa.pair_ws = s->pair_ws, aa.pair_ws_bytes = s->pair_ws_bytes;
+    aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;  // a prefill chunk: consecutive positions
+    return aa;
+  };
   bool xh_ready = false;  // xh already holds this layer's normalised rows (written by the layer before)
   auto gemm = [&](const WRef& w, const float* x, bool prepared, float* y, const float* residual, TgIo* io) -> int {
     TgIo local;
@@ -455,24 +480,8 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       } else if (few(L.q, qp, nullptr, false) || few(L.k, kp, nullptr, false) || few(L.v, vp, nullptr, false)) {
         return 1;
       }
-      QkvPrepArgs pa{};
-      pa.q = qp, pa.k = kp, pa.v = vp;
-      pa.kcache = s->kcache + (size_t)l * layer_stride, pa.vcache = s->vcache + (size_t)l * layer_stride;
-      pa.q_norm_w = L.q_norm.ptr, pa.k_norm_w = L.k_norm.ptr, pa.norm_w_type = L.q_norm.type;
-      pa.row_pos = s->row_pos_dev, pa.row_seq = s->row_seq_dev, pa.base_pos = 0;
-      pa.rows = rows, pa.nh = c.heads, pa.nkv = c.kv_heads, pa.d = c.head_dim, pa.cap = cap;
-      pa.kv_type = s->kv_type, pa.has_norm = c.qk_norm ? 1 : 0, pa.has_rope = c.rope ? 1 : 0;
-      pa.eps = c.eps;
-      pa.ldq = ldq, pa.ldk = ldk, pa.ldv = ldv;
-      AttnArgs aa{};
-      aa.q = qp, aa.kcache = pa.kcache, aa.vcache = pa.vcache;
-      aa.row_pos = s->row_pos_dev, aa.row_seq = s->row_seq_dev, aa.base_pos = 0;
-      aa.ctx = s->ctx;
-      aa.rows = rows, aa.nh = c.heads, aa.nkv = c.kv_heads, aa.d = c.head_dim, aa.cap = cap;
-      aa.kv_type = s->kv_type;
-      aa.ldq = ldq;
-      aa.pair_ws = s->pair_ws, aa.pair_ws_bytes = s->pair_ws_bytes;
-      aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;
+      QkvPrepArgs pa = qkv_args(l, qp, kp, vp, ldq, ldk, ldv);
+      const AttnArgs aa = attn_args(pa);
       void* part = thread_scratch(attention_split_scratch_bytes(rows, c.heads, c.head_dim, attention_decode_splits(aa)));
       // (the rows of a chunk see one another's keys: their preparation is a launch of its own)
       const bool decode = chunk_start < 0;
@@ -516,16 +525,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
                  gemm(L.v, nullptr, true, vp, nullptr, nullptr)) {
         return 1;
       }
-      QkvPrepArgs pa{};
-      pa.q = qp, pa.k = kp, pa.v = vp;
-      pa.kcache = s->kcache + (size_t)l * layer_stride;
-      pa.vcache = s->vcache + (size_t)l * layer_stride;
-      pa.q_norm_w = L.q_norm.ptr, pa.k_norm_w = L.k_norm.ptr, pa.norm_w_type = L.q_norm.type;
-      pa.row_pos = s->row_pos_dev, pa.row_seq = s->row_seq_dev, pa.base_pos = 0;
-      pa.rows = rows, pa.nh = c.heads, pa.nkv = c.kv_heads, pa.d = c.head_dim, pa.cap = cap;
-      pa.kv_type = s->kv_type, pa.has_norm = c.qk_norm ? 1 : 0, pa.has_rope = c.rope ? 1 : 0;
-      pa.eps = c.eps;
-      pa.ldq = ldq, pa.ldk = ldk, pa.ldv = ldv;
+      QkvPrepArgs pa = qkv_args(l, qp, kp, vp, ldq, ldk, ldv);
       if (io_q.splits > 1) {
         DeferredCols dc;
         dc.partial = s->gpart, dc.S = io_q.splits, dc.N = qd + 2 * kvd, dc.rows = rows;
@@ -533,15 +533,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
         pa.dk.col = qd, pa.dv.col = qd + kvd;
       }
       if (launch_qkv_prepare(pa, s->freq, st)) return 1;
-      AttnArgs aa{};
-      aa.q = qp, aa.kcache = pa.kcache, aa.vcache = pa.vcache;
-      aa.row_pos = s->row_pos_dev, aa.row_seq = s->row_seq_dev, aa.base_pos = 0;
-      aa.ctx = s->ctx;
-      aa.rows = rows, aa.nh = c.heads, aa.nkv = c.kv_heads, aa.d = c.head_dim, aa.cap = cap;
-      aa.kv_type = s->kv_type;
-      aa.ldq = ldq;
-      aa.pair_ws = s->pair_ws, aa.pair_ws_bytes = s->pair_ws_bytes;
-      aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;
+      const AttnArgs aa = attn_args(pa);
       if (launch_attention(aa, st)) return 1;
       // o: hidden += W ctx, then the FFN norm straight into the GEMM's operand
       TgIo io_o;
@@ -589,23 +581,8 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
                  norm_product(L.v, L.attn_norm, vp, false)) {
         return 1;
       }
-      QkvPrepArgs pa{};
-      pa.q = qp, pa.k = kp, pa.v = vp;
-      pa.kcache = s->kcache + (size_t)l * layer_stride, pa.vcache = s->vcache + (size_t)l * layer_stride;
-      pa.q_norm_w = L.q_norm.ptr, pa.k_norm_w = L.k_norm.ptr, pa.norm_w_type = L.q_norm.type;
-      pa.row_pos = s->row_pos_dev, pa.row_seq = s->row_seq_dev, pa.base_pos = 0;
-      pa.rows = rows, pa.nh = c.heads, pa.nkv = c.kv_heads, pa.d = c.head_dim, pa.cap = cap;
-      pa.kv_type = s->kv_type, pa.has_norm = c.qk_norm ? 1 : 0, pa.has_rope = c.rope ? 1 : 0;
-      pa.eps = c.eps;
-      pa.ldq = ldq, pa.ldk = ldk, pa.ldv = ldv;
-      AttnArgs aa{};
-      aa.q = qp, aa.kcache = pa.kcache, aa.vcache = pa.vcache;
-      aa.row_pos = s->row_pos_dev, aa.row_seq = s->row_seq_dev, aa.base_pos = 0;
-      aa.ctx = s->ctx;
-      aa.rows = rows, aa.nh = c.heads, aa.nkv = c.kv_heads, aa.d = c.head_dim, aa.cap = cap;
-      aa.kv_type = s->kv_type;
-      aa.ldq = ldq;
-      aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;
+      QkvPrepArgs pa = qkv_args(l, qp, kp, vp, ldq, ldk, ldv);
+      const AttnArgs aa = attn_args(pa);
       if (attention_decode_takes(aa) && (rows == 1 || chunk_start < 0)) {
         if (launch_attention_decode(aa, &pa, &s->freq, nullptr, nullptr, nullptr, 0, st)) return 1;
       } else if (launch_qkv_prepare(pa, s->freq, st) || launch_attention(aa, st)) {
@@ -656,28 +633,11 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       if (launch_linear(L.k, s->xn, E_F32, rows, kp, nullptr, st)) return 1;
       if (launch_linear(L.v, s->xn, E_F32, rows, vp, nullptr, st)) return 1;
     }
-    QkvPrepArgs pa{};
-    pa.q = qp, pa.k = kp, pa.v = vp;
-    pa.kcache = s->kcache + (size_t)l * layer_stride;
-    pa.vcache = s->vcache + (size_t)l * layer_stride;
-    pa.q_norm_w = L.q_norm.ptr, pa.k_norm_w = L.k_norm.ptr, pa.norm_w_type = L.q_norm.type;
-    pa.row_pos = s->row_pos_dev, pa.row_seq = s->row_seq_dev, pa.base_pos = 0;
-    pa.rows = rows, pa.nh = c.heads, pa.nkv = c.kv_heads, pa.d = c.head_dim, pa.cap = cap;
-    pa.kv_type = s->kv_type, pa.has_norm = c.qk_norm ? 1 : 0, pa.has_rope = c.rope ? 1 : 0;
-    pa.eps = c.eps;
-    pa.ldq = ldq, pa.ldk = ldk, pa.ldv = ldv;
+    QkvPrepArgs pa = qkv_args(l, qp, kp, vp, ldq, ldk, ldv);
     pa.dq = deferred_cols(dq, 0), pa.dk = deferred_cols(dk, colk), pa.dv = deferred_cols(dv, colv);
     if (launch_qkv_prepare(pa, s->freq, st)) return 1;
     thread_scratch_release_all();
-    AttnArgs aa{};
-    aa.q = qp, aa.kcache = pa.kcache, aa.vcache = pa.vcache;
-    aa.row_pos = s->row_pos_dev, aa.row_seq = s->row_seq_dev, aa.base_pos = 0;
-    aa.ctx = s->ctx;
-    aa.rows = rows, aa.nh = c.heads, aa.nkv = c.kv_heads, aa.d = c.head_dim, aa.cap = cap;
-    aa.kv_type = s->kv_type;
-    aa.ldq = ldq;
-    aa.pair_ws = s->pair_ws, aa.pair_ws_bytes = s->pair_ws_bytes;
-    aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;  // a prefill chunk: consecutive positions
+    const AttnArgs aa = attn_args(pa);
     if (launch_attention(aa, st)) return 1;
     bool ffn_normed = false;
     if (tp ? tp_row_parallel(s, L.o, s->ctx, rows, 0, &L.ffn_norm, &ffn_normed, st)
