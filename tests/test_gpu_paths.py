@@ -323,3 +323,84 @@ def test_linear_few_rows_of_plain_weights_keep_f32_accuracy(native_lib, enc, m, 
     x = torch.randn(m, k, generator=torch.Generator("cuda").manual_seed(m), device="cuda")
     want = (x.double() @ ops.dequant(w).double().T).cpu().numpy()
     assert rel_64(ops.linear(w, x).double().cpu().numpy(), want) < 2.0 ** -21
+
+
+EDGES = [0, 1, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 299]
+
+
+def one_by_one(oracle, path, tokens, at, kv):
+    """The oracle's logits after each of the positions in `at`, the cache rounded to its type."""
+    from dyninfer_b200 import checkpoint as ck
+    cat = ck.open_catalog(path)
+    m = oracle.Model(cat.config, helpers.catalog_weights(oracle, cat), kv_cap=len(tokens), kv_round={"f16": 1, "bf16": 2, "f32": 0}[kv], fast=True)
+    out = {}
+    for i, t in enumerate(tokens):
+        lg, _ = m.forward([t])
+        if i in at:
+            out[i] = lg
+    return out
+
+
+@pytest.mark.parametrize("kv", ["bf16", "f16"])
+@pytest.mark.parametrize("d,slots", [(128, 1), (64, 1), (128, 3)])
+def test_decode_attention_prepares_its_own_rows(native_lib, oracle, tmp_path, kv, d, slots):
+    """Decode attention with the QKV preparation inside (norm, rotation, cache write, the slice that owns the new key) at
+    every position around the ends of its slices, token by token against the oracle. The products in front keep 22 bits of
+    their rows and the attention 24, so what is left are roundings of single cache entries that fall the other way:
+    2^-9 (bf16) or 2^-12 of an entry."""
+    cfg = dict(synth.TINY, layers=1, heads=8, kv_heads=2, head_dim=d, hidden=512)
+    path = synth.write_qwen3_gguf(str(tmp_path / "q.gguf"), cfg, seed=17)
+    rng = np.random.default_rng(d + slots)
+    tokens = [rng.integers(0, cfg["vocab"], size=max(EDGES) + 1).tolist() for _ in range(slots)]
+    want = [one_by_one(oracle, path, t, EDGES, kv) for t in tokens]
+    model = ModelLoader().load(path, max_kv=512, kv_dtype=kv, chunk_size=1, decode_kernel="graph")
+    if slots == 1:
+        with model.create_session(SessionConfig(max_sequence_length=512)) as s:
+            for i, t in enumerate(tokens[0]):
+                lg = (s.prefill([t]) if i == 0 else s.decode(t)).values
+                if i in want[0]:
+                    assert np.abs(lg - want[0][i]).max() <= 1e-3, i
+        return
+    with model.create_batched_session(SessionConfig(max_sequence_length=512, batch_size=slots)) as s:
+        for b in range(slots):
+            s.prefill_slot(b, tokens[b][:1])
+        for i in range(1, len(tokens[0])):
+            _, logits = s.step({b: tokens[b][i] for b in range(slots)}, want_logits=True)
+            if i in want[0]:
+                for b in range(slots):
+                    assert np.abs(logits[b] - want[b][i]).max() <= 1e-3, (i, b)
+
+
+@pytest.mark.parametrize("kv", ["bf16", "f16"])
+@pytest.mark.parametrize("slots", [8, 40])
+def test_batched_decode_attention_at_the_ends_of_slices(native_lib, oracle, tmp_path, kv, slots):
+    """Steps of many sequences (slices that meet in a cluster, and more blocks than SMs: slices through memory) whose
+    contexts end around the ends of the slices, against the oracle; f16 operands of the products in front: 1e-2."""
+    cfg = dict(synth.SMALL_D128, layers=1, heads=8, kv_heads=4, vocab=512)
+    path = synth.write_qwen3_gguf(str(tmp_path / "q.gguf"), cfg, seed=19)
+    rng = np.random.default_rng(slots)
+    lengths = [EDGES[1:][(5 * b) % (len(EDGES) - 1)] for b in range(slots)]
+    tokens = [rng.integers(0, 512, size=n + 1).tolist() for n in lengths]
+    model = ModelLoader().load(path, max_kv=320, kv_dtype=kv, chunk_size=64, decode_kernel="graph")
+    with model.create_batched_session(SessionConfig(max_sequence_length=320, batch_size=slots)) as s:
+        for b in range(slots):
+            s.prefill_slot(b, tokens[b][:-1])
+        _, logits = s.step({b: tokens[b][-1] for b in range(slots)}, want_logits=True)
+    for b in range(slots):
+        want = one_by_one(oracle, path, tokens[b], [lengths[b]], kv)[lengths[b]]
+        assert np.abs(logits[b] - want).max() <= 1e-2 and helpers.cosine(logits[b], want) >= 0.9999, (b, lengths[b])
+
+
+def test_persistent_attention_slices_against_the_oracle(native_lib, oracle, tmp_path):
+    """One slice of a head's keys up to the most there are (nine, then several batches per slice), token by token."""
+    path = synth.write_qwen3_gguf(str(tmp_path / "q.gguf"), dict(synth.SMALL_D128, vocab=512), seed=5)
+    at = [0, 62, 63, 64, 127, 128, 191, 192, 511, 512, 575, 576, 577, 1030]
+    tokens = np.random.default_rng(3).integers(0, 512, size=max(at) + 1).tolist()
+    want = one_by_one(oracle, path, tokens, at, "bf16")
+    model = ModelLoader().load(path, max_kv=1152, kv_dtype="bf16", chunk_size=128, decode_kernel="persistent")
+    with model.create_session(SessionConfig(max_sequence_length=1152)) as s:
+        assert s.uses_persistent_kernel()
+        for i, t in enumerate(tokens):
+            lg = (s.prefill([t]) if i == 0 else s.decode(t)).values
+            if i in want:
+                assert np.abs(lg - want[i]).max() <= 1e-2 and helpers.cosine(lg, want[i]) >= 0.9999, i
