@@ -114,7 +114,6 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
   const int g = lane >> 2, t = lane & 3, G = p.G, nsplit = p.nsplit;
   const int64_t kvh = blockIdx.x, r = blockIdx.y;
   const int sp = blockIdx.z;
-  pdl_trigger();
   const int64_t pos = a.row_pos ? a.row_pos[r] : a.base_pos + r;
   const int64_t seq = a.row_seq ? a.row_seq[r] : 0;
   const int n = (int)pos + (p.prep ? 0 : 1);  // keys that lie in the cache
@@ -148,7 +147,7 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
       for (int j = 0; j < CH; j++) kr[h][j] = *reinterpret_cast<const uint4*>(kb + (int64_t)key * (D * 2) + 64 * j + 16 * t);
     }
   };
-  if (!p.prep) pdl_wait();  // the kernel in front may have written cache rows
+  if (!p.prep) pdl_wait_then_trigger();  // the kernel in front may have written cache rows
   if (warp < steps) load_k(warp);
   load_v(warp, 0);
 
@@ -171,7 +170,7 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
 #pragma unroll
         for (int e = 0; e < E; e++) w[e] = aux_load(nw, p.norm_type, i0 + e), w[E + e] = aux_load(nw, p.norm_type, D / 2 + i0 + e);
       }
-      if (!waited) pdl_wait();
+      if (!waited) pdl_wait_then_trigger();
       waited = true;
       const float* src = query ? a.q + r * (a.ldq ? a.ldq : a.nh * D) + (kvh * G + job) * D
                                : key ? p.k + r * p.ldk + kvh * D : p.v + r * p.ldv + kvh * D;
@@ -216,7 +215,7 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
         }
       }
     }
-    if (!waited) pdl_wait();  // the results may still be read by the kernels in front
+    if (!waited) pdl_wait_then_trigger();  // the results may still be read by the kernels in front
   }
   __syncthreads();
   // Q: chunk j of lane t = dims 32 j + 8 t ..; products 2j and 2j + 1 take its first and last four
@@ -428,16 +427,14 @@ attention_decode_kernel(const AdArgs p, const __grid_constant__ FreqTable ft) {
 // Slices -> the f16 operand of the following product (fragment order of `enc`, power-of-two scale, inverse in
 // inv_s). One block per row, because the scale is the row's; a thread takes eight consecutive dims of a head.
 __global__ void __launch_bounds__(1024)
-attention_merge_frag_kernel(const float* __restrict__ part, int nsplit, int nh, int d, __half* __restrict__ frag,
-                            float* __restrict__ inv_s, int enc) {
+attention_merge_frag_kernel(const float* part, int nsplit, int nh, int d, __half* frag, float* inv_s, int enc) {
   __shared__ float red[32];
-  pdl_trigger();
   const int64_t r = blockIdx.x;
   const int k = threadIdx.x * 8, h = k / d, d0 = k - h * d;
   float o[8];
 #pragma unroll
   for (int e = 0; e < 8; e++) o[e] = 0.f;
-  pdl_wait();
+  pdl_wait_then_trigger();
   if (k < nh * d) {
     const float* p0 = part + (r * nh + h) * nsplit * (d + 2);
     float gm = -3.40282347e38f, gl = 0.f;

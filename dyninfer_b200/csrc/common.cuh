@@ -74,10 +74,22 @@ inline DeferredCols deferred_cols(const Deferred& d, int64_t col) {
 
 // Programmatic dependent launch (sm_90+). A kernel launched with launch_pdl may start while the
 // kernel before it in the stream is still running; it must not touch anything that kernel (or an
-// earlier one) produces, nor write global memory, before pdl_wait(). pdl_trigger() lets the next
-// kernel of the stream start early; kernels that never call it release it when they exit.
+// earlier one) produces, nor write global memory, before pdl_wait(). The next kernel of the stream
+// starts early once every block has triggered or exited. Kernels that wait trigger behind the wait
+// (pdl_wait_then_trigger), so that at most two kernels of a stream are on the GPU and the third finds
+// all that lies two kernels back complete. With the trigger at a kernel's top a chain of small kernels
+// started a whole layer ahead: steps of 17 to 31 rows of a Q4_0 model gave NaN now and then, and no
+// longer did when any one kernel of the layer was launched plainly. pdl_trigger() alone is for kernels
+// launched plainly, which start behind everything.
+// What another kernel of the chain produces is read through ordinary pointers or __ldcg: a const
+// __restrict__ pointer or __ldg promises data that does not change while the kernel runs, which is not
+// so for a kernel that starts before its inputs are written.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait_then_trigger() {
+  pdl_wait();
+  pdl_trigger();
+}
 bool pdl_enabled();  // DYNINFER_CUDA_PDL=0 turns the attribute off (plain launches)
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,

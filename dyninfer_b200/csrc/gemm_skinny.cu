@@ -298,7 +298,6 @@ gemm_skinny_kernel(const SkArgs a, const __grid_constant__ CUtensorMap wmap, con
   uint8_t* after = smem + nwarps * nst * RT * (S::STAGE + aux_stage);
   uint64_t* bars = reinterpret_cast<uint64_t*>(after) + warp * nst;
   uint8_t* xs = after + (nwarps * nst * 8 + 127) / 128 * 128;
-  pdl_trigger();
   if (tid == 0) {
     s_abort = 0;
     mbar_init(&xbar, 1);
@@ -371,7 +370,7 @@ gemm_skinny_kernel(const SkArgs a, const __grid_constant__ CUtensorMap wmap, con
   if (warp == nwarps) {
     // this CTA's K share of the activations, one bulk copy per row and term (columns n >= M of the products are
     // never stored, so those rows stay unwritten)
-    pdl_wait();
+    pdl_wait_then_trigger();
     const int units = (st_hi - st_lo) * KU;
     if (lane == 0) mbar_expect_tx(&xbar, (unsigned)(TERMS * a.M * units * 512));
     __syncwarp();
@@ -695,15 +694,13 @@ gemm_skinny_kernel(const SkArgs a, const __grid_constant__ CUtensorMap wmap, con
 // ---- activation pass for many rows: rows -> f16 fragment order + inverse scales ------------------------
 // One block per row; a thread takes runs of eight elements.
 __global__ void __launch_bounds__(256)
-sk_prepare_kernel(const void* __restrict__ x, int x_bf16, int K, int enc, int terms, int64_t plane, __half* __restrict__ out,
-                  float* __restrict__ inv_s) {
+sk_prepare_kernel(const void* x, int x_bf16, int K, int enc, int terms, int64_t plane, __half* out, float* inv_s) {
   __shared__ float red[8];
-  pdl_trigger();
   const int64_t m = blockIdx.x;
   const int tid = threadIdx.x;
   constexpr int R = 4;  // runs in registers at a time: rows of up to 8192 elements are loaded once
   float v[R][8];
-  pdl_wait();
+  pdl_wait_then_trigger();
   auto load = [&](int i0) {
 #pragma unroll
     for (int i = 0; i < R; i++) {

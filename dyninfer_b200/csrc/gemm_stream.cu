@@ -235,7 +235,6 @@ gemm_stream_kernel(const GsArgs a, const __grid_constant__ CUtensorMap wmap, con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
-  pdl_trigger();  // not before this CTA has its tensor memory: a CTA of the next kernel must not get ahead of it
 
   if (warp < GS_CONV) {
     const int quarter = warp & 3, g = warp >> 2;
@@ -299,7 +298,7 @@ gemm_stream_kernel(const GsArgs a, const __grid_constant__ CUtensorMap wmap, con
       if (!waited) pdl_wait();
       waited = true;
       auto sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(GS_CONV * 32) : "memory"); };
-      if (tid < bn) s_inv[tid] = m0 + tid < a.M ? __ldg(a.inv_s + m0 + tid) : 0.f;
+      if (tid < bn) s_inv[tid] = m0 + tid < a.M ? __ldcg(a.inv_s + m0 + tid) : 0.f;
       const bool whole = sg.k1 - sg.k0 == nunits;
       int first = 0, last = 0;
       if (!whole) {
@@ -409,7 +408,7 @@ gemm_stream_kernel(const GsArgs a, const __grid_constant__ CUtensorMap wmap, con
   } else if (warp == GS_X_WARP) {
     // ---------------- activations -------------------------------------------------------------------------------------
     if (lane == 0) {
-      pdl_wait();
+      pdl_wait_then_trigger();
       int xs = 0;
       unsigned phase = 1, i = 0;
       bool ok = true;

@@ -75,13 +75,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 // the product behind.
 template <bool WIDE>  // rows on 16-byte boundaries
 __global__ void __launch_bounds__(256)
-tg_prepare_x_kernel(const void* __restrict__ x, int x_bf16, int64_t M, int64_t K, __half* xh, float* inv_s, unsigned* count, int ncount) {
+tg_prepare_x_kernel(const void* x, int x_bf16, int64_t M, int64_t K, __half* xh, float* inv_s, unsigned* count, int ncount) {
   __shared__ float red[8];
   const int64_t m = blockIdx.x;
   const int tid = threadIdx.x;
   __half* dst = xh + m * K;
-  pdl_trigger();
-  pdl_wait();
+  pdl_wait_then_trigger();
   if (m == 0)
     for (int i = tid; i < ncount; i += 256) count[i] = 0;
   if (m >= M) {

@@ -82,13 +82,13 @@ constexpr int CS_MAX_SMEM = 226 * 1024;  // dynamic shared memory the kernel may
 // order 2 (Q4_K): a 32-element sub-block is one nibble plane of 32 bytes; step s = 2i+o takes the plane's
 //   elements of word s: b0 = (x[4s], x[4s+2]), b1 = (x[4s+1], x[4s+3]), all of them / 16 for the odd
 //   sub-blocks (the high-nibble plane).
-__device__ __forceinline__ float cs_stage_x(const void* __restrict__ x, int x_bf16, int K, int k0, int kspan, uint2* xq,
+__device__ __forceinline__ float cs_stage_x(const void* x, int x_bf16, int K, int k0, int kspan, uint2* xq,
                                             float* sx8, float* red, float sum_factor, int order = 0) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   auto ld = [&](int i) -> float {
     if (i >= K) return 0.f;
-    return x_bf16 ? bf16_bits_to_f32(__ldg(reinterpret_cast<const uint16_t*>(x) + i))
-                  : __ldg(reinterpret_cast<const float*>(x) + i);
+    return x_bf16 ? bf16_bits_to_f32(__ldcg(reinterpret_cast<const uint16_t*>(x) + i))
+                  : __ldcg(reinterpret_cast<const float*>(x) + i);
   };
   float mx = 0.f;
   for (int i = tid; i < K; i += CS_WARPS * 32) mx = fmaxf(mx, fabsf(ld(i)));
@@ -161,7 +161,6 @@ gemv_cs_q4_kernel(const CsArgs a, const __grid_constant__ CUtensorMap wmap) {
   uint4* xq = reinterpret_cast<uint4*>(cs_smem + G::RING_BYTES);
   float* sx8 = reinterpret_cast<float*>(xq + (size_t)a.span_units * 64);
   float* red = sx8 + a.span_units * 8;
-  pdl_trigger();  // the next kernel of the stream may start its own weight fetch
   if (threadIdx.x == 0) s_abort = 0;
   if (lane == 0) {
     for (int i = 0; i < CS_NST; i++) mbar_init(bars + i, 1);
@@ -209,7 +208,7 @@ gemv_cs_q4_kernel(const CsArgs a, const __grid_constant__ CUtensorMap wmap) {
 
   // The weights do not depend on the kernels before this one: the first stages are already in
   // flight. Everything else (the activation row, the scratch words) does.
-  pdl_wait();
+  pdl_wait_then_trigger();
   // while the first stages are in flight: arrange the activation row in shared memory
   const float out_scale = cs_stage_x(a.x, a.x_bf16, a.K, U_base * 256, (sl_last - sl_first + 1) * nst * 512,
                                      reinterpret_cast<uint2*>(xq), sx8, red, ENC == E_Q4_0 ? 8.0f : 1.0f);
@@ -354,7 +353,6 @@ gemv_cs_mlx_kernel(const CsArgs a, const __grid_constant__ CUtensorMap wmap, con
   uint4* xq = reinterpret_cast<uint4*>(smem + (size_t)CS_WARPS * CS_NST * (CM_WSTAGE + aux_stage + 8));
   float* sx8 = reinterpret_cast<float*>(xq + (size_t)a.span_units * 64);
   float* red = sx8 + a.span_units * 8;
-  pdl_trigger();  // the next kernel of the stream may start its own weight fetch
   if (threadIdx.x == 0) s_abort = 0;
   if (lane == 0) {
     for (int i = 0; i < CS_NST; i++) mbar_init(bars + i, 1);
@@ -397,7 +395,7 @@ gemv_cs_mlx_kernel(const CsArgs a, const __grid_constant__ CUtensorMap wmap, con
 #pragma unroll
   for (int q = 0; q < CS_NST; q++) issue();
 
-  pdl_wait();
+  pdl_wait_then_trigger();
   const float out_scale = cs_stage_x(a.x, a.x_bf16, a.K, U_base * 256, (sl_last - sl_first + 1) * nst * 512,
                                      reinterpret_cast<uint2*>(xq), sx8, red, 1.0f, 1);
   if (blockIdx.x == 0 && threadIdx.x == 0) a.misc[0] = out_scale;
@@ -519,7 +517,6 @@ gemv_cs_q4k_kernel(const CsArgs a, const __grid_constant__ CUtensorMap wmap) {
   uint4* xq = reinterpret_cast<uint4*>(cs_smem_q4k + G::RING_BYTES);
   float* sx8 = reinterpret_cast<float*>(xq + (size_t)a.span_units * 64);
   float* red = sx8 + a.span_units * 8;
-  pdl_trigger();  // the next kernel of the stream may start its own weight fetch
   if (threadIdx.x == 0) s_abort = 0;
   if (lane == 0) {
     for (int i = 0; i < CS_NST; i++) mbar_init(bars + i, 1);
@@ -559,7 +556,7 @@ gemv_cs_q4k_kernel(const CsArgs a, const __grid_constant__ CUtensorMap wmap) {
 #pragma unroll
   for (int q = 0; q < CS_NST; q++) issue();
 
-  pdl_wait();
+  pdl_wait_then_trigger();
   const float out_scale = cs_stage_x(a.x, a.x_bf16, a.K, U_base * 256, (sl_last - sl_first + 1) * nst * 512,
                                      reinterpret_cast<uint2*>(xq), sx8, red, 1.0f, 2);
   if (blockIdx.x == 0 && threadIdx.x == 0) a.misc[0] = out_scale;
@@ -663,10 +660,9 @@ gemv_cs_q4k_kernel(const CsArgs a, const __grid_constant__ CUtensorMap wmap) {
 
 // partial sums over the K-slices, fixed order
 __global__ void __launch_bounds__(256)
-cs_reduce_kernel(const float* __restrict__ partial, int S, int64_t N, const float* __restrict__ misc,
+cs_reduce_kernel(const float* partial, int S, int64_t N, const float* misc,
                  float* y, const float* residual) {
-  pdl_trigger();
-  pdl_wait();  // the partial sums come from the kernel before this one
+  pdl_wait_then_trigger();  // the partial sums come from the kernel before this one
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= N) return;
   float v = 0.f;

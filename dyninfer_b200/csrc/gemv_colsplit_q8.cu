@@ -47,12 +47,12 @@ struct Q8Args {
 // Activation row -> shared memory: xhi[K], 16 bytes of padding, xlo[K] (f16, natural order, scaled
 // so the largest magnitude sits in [2^12, 2^13)); sx[K/32] = 128 * 2^-24 * sum of each block.
 // Returns 2^24 / scale.
-__device__ __forceinline__ float q8_stage_x(const void* __restrict__ x, int x_bf16, int K, __half* xhi,
+__device__ __forceinline__ float q8_stage_x(const void* x, int x_bf16, int K, __half* xhi,
                                             __half* xlo, float* sx, float* red) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   auto ld = [&](int i) -> float {
-    return x_bf16 ? bf16_bits_to_f32(__ldg(reinterpret_cast<const uint16_t*>(x) + i))
-                  : __ldg(reinterpret_cast<const float*>(x) + i);
+    return x_bf16 ? bf16_bits_to_f32(__ldcg(reinterpret_cast<const uint16_t*>(x) + i))
+                  : __ldcg(reinterpret_cast<const float*>(x) + i);
   };
   float mx = 0.f;
   for (int i = tid; i < K; i += Q8_WARPS * 32) mx = fmaxf(mx, fabsf(ld(i)));
@@ -96,7 +96,6 @@ gemv_cs_q8_0_kernel(const Q8Args a, const __grid_constant__ CUtensorMap wmap) {
   __half* xlo = xhi + a.K + 8;  // 16 bytes off a multiple of 128: hi and lo lanes hit different banks
   float* sx = reinterpret_cast<float*>(xlo + a.K + 8);
   float* red = sx + (a.K >> 5);
-  pdl_trigger();  // the next kernel of the stream may start its own weight fetch
   if (threadIdx.x == 0) s_abort = 0;
   if (lane == 0) {
     for (int i = 0; i < Q8_NST; i++) mbar_init(bars + i, 1);
@@ -132,7 +131,7 @@ gemv_cs_q8_0_kernel(const Q8Args a, const __grid_constant__ CUtensorMap wmap) {
 
   // the weights do not depend on the kernels before this one (their first stages are in flight);
   // the activation row and the scratch words do
-  pdl_wait();
+  pdl_wait_then_trigger();
   const float out_scale = q8_stage_x(a.x, a.x_bf16, a.K, xhi, xlo, sx, red);
   if (blockIdx.x == 0 && threadIdx.x == 0) a.misc[0] = out_scale;
   __syncthreads();
@@ -230,10 +229,9 @@ gemv_cs_q8_0_kernel(const Q8Args a, const __grid_constant__ CUtensorMap wmap) {
 }
 
 __global__ void __launch_bounds__(256)
-q8_reduce_kernel(const float* __restrict__ partial, int S, int64_t N, const float* __restrict__ misc, float* y,
+q8_reduce_kernel(const float* partial, int S, int64_t N, const float* misc, float* y,
                  const float* residual) {
-  pdl_trigger();
-  pdl_wait();  // the partial sums come from the kernel before this one
+  pdl_wait_then_trigger();  // the partial sums come from the kernel before this one
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= N) return;
   float v = 0.f;

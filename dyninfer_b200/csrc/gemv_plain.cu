@@ -38,14 +38,13 @@ __device__ __forceinline__ void widen8(const uint4& w, float (&f)[8]) {
 // y[m][n] = sum_k x[m][k] * w[n][k] (+ residual). K % 256 == 0, M <= 4.
 template <bool BF16, int M>
 __global__ void __launch_bounds__(GP_WARPS * 32) gemv_plain_kernel(const uint8_t* __restrict__ w, int64_t N, int K,
-                                                                   const void* __restrict__ x, int x_bf16,
-                                                                   float* __restrict__ y,
-                                                                   const float* __restrict__ residual) {
+                                                                   const void* x, int x_bf16,
+                                                                   float* y,
+                                                                   const float* residual) {
   extern __shared__ __align__(16) float gp_xs[];  // [M][K]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  pdl_trigger();
   // the weights do not depend on earlier kernels of the stream; the activations do
-  pdl_wait();
+  pdl_wait_then_trigger();
   for (int i = tid; i < M * K; i += GP_WARPS * 32)
     gp_xs[i] = x_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[i])
                       : reinterpret_cast<const float*>(x)[i];

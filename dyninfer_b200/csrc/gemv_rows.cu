@@ -262,7 +262,6 @@ gemv_rows_kernel(const GrArgs a, const __grid_constant__ CUtensorMap wmap, const
   uint8_t* after = smem + nwarps * nst * (S::STAGE + aux_stage);
   uint64_t* bars = reinterpret_cast<uint64_t*>(after) + warp * nst;
   uint8_t* xs = after + (nwarps * nst * 8 + 127) / 128 * 128;
-  pdl_trigger();
   if (tid == 0) s_abort = 0;
   if (lane == 0) {
     for (int i = 0; i < nst; i++) mbar_init(bars + i, 1);
@@ -317,7 +316,7 @@ gemv_rows_kernel(const GrArgs a, const __grid_constant__ CUtensorMap wmap, const
   for (int q = 0; q < nst; q++) issue();
 
   // the weights do not depend on the kernels before this one; everything else does
-  pdl_wait();
+  pdl_wait_then_trigger();
 
   // ---- activations: largest magnitude (and sum of squares) of every row, then hi / lo fragments of the K share ----
   const int units = (st_hi - st_lo) * KU, u_lo = st_lo * KU, all_units = a.K / GR_UNIT;

@@ -104,7 +104,7 @@ int launch_rms_norm(const float* x, const void* w, int w_type, int64_t rows, int
 // reduction kernels), four slices' loads in flight at a time for all NE elements: a plain loop would wait
 // for one L2 round trip per slice and element.
 template <int NE>
-__device__ __forceinline__ void deferred_sums(const float* __restrict__ partial, int S, int64_t N,  // N: floats between slices
+__device__ __forceinline__ void deferred_sums(const float* partial, int S, int64_t N,  // N: floats between slices
                                               const int64_t (&idx)[NE], const bool (&live)[NE], float (&out)[NE]) {
 #pragma unroll
   for (int e = 0; e < NE; e++) out[e] = 0.f;
@@ -143,17 +143,16 @@ __device__ __forceinline__ void f16_row_scale(float mx, float* red, float* sc, f
 // the kernel took 130 registers and one block per SM: 512 rows x 4096 with two slices 36 us).
 template <int PER, bool FULL>
 __global__ void __launch_bounds__(256, PER <= 8 ? 6 : PER <= 16 ? 4 : 2)
-norm_prepare_kernel(const float* __restrict__ x, const float* __restrict__ partial, int S, int64_t rows,
+norm_prepare_kernel(const float* x, const float* partial, int S, int64_t rows,
                     const float* residual, float* hidden, const void* __restrict__ w, int w_type, int width,
-                    float eps, __half* __restrict__ xh, float* __restrict__ inv_s) {
+                    float eps, __half* xh, float* inv_s) {
   __shared__ float red[32];
   const int T = FULL ? 256 : (int)blockDim.x, tid = threadIdx.x;
   const int64_t at = (int64_t)blockIdx.x * width + tid;
   const int runs = width >> 8;
   auto in = [&](int k) { return FULL ? k < runs : tid + k * T < width; };
-  pdl_trigger();
   float v[PER];
-  pdl_wait();
+  pdl_wait_then_trigger();
   // the slices outermost: all of a slice's loads are in flight together
   if (S) {
     const float* p = partial + at;
@@ -249,10 +248,9 @@ int launch_norm_prepare(const float* x, const float* partial, int splits, const 
 // per row, a thread takes R runs of eight elements and keeps them in registers.
 template <int R>
 __global__ void __launch_bounds__(256)
-norm_frag_kernel(const float* __restrict__ x, const void* __restrict__ w, int w_type, int width, float eps, int enc,
-                 __half* __restrict__ xh, float* __restrict__ inv_s) {
+norm_frag_kernel(const float* x, const void* __restrict__ w, int w_type, int width, float eps, int enc,
+                 __half* xh, float* inv_s) {
   __shared__ float red[32];
-  pdl_trigger();
   const int64_t row = blockIdx.x;
   float v[R][8], wv[R][8];
 #pragma unroll
@@ -261,7 +259,7 @@ norm_frag_kernel(const float* __restrict__ x, const void* __restrict__ w, int w_
 #pragma unroll
     for (int e = 0; e < 8; e++) wv[i][e] = k < width ? aux_load(reinterpret_cast<const uint8_t*>(w), w_type, k + e) : 0.f;
   }
-  pdl_wait();
+  pdl_wait_then_trigger();
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < R; i++) {
@@ -316,9 +314,8 @@ int launch_norm_frag(const float* x, const void* w, int w_type, int64_t rows, in
 // over the row, each waiting for its loads, took 50 us on 512 x 12288; now 13).
 template <int PER4>
 __global__ void __launch_bounds__(1024)
-silu_prepare_kernel(const float* __restrict__ gu, int64_t I, __half* __restrict__ xh, float* __restrict__ inv_s) {
+silu_prepare_kernel(const float* gu, int64_t I, __half* xh, float* inv_s) {
   __shared__ float red[32];
-  pdl_trigger();
   const int64_t row = blockIdx.x;
   const float4* g = reinterpret_cast<const float4*>(gu + row * 2 * I);
   const float4* u = reinterpret_cast<const float4*>(gu + row * 2 * I + I);
@@ -326,7 +323,7 @@ silu_prepare_kernel(const float* __restrict__ gu, int64_t I, __half* __restrict_
   auto val = [](float gv, float uv) { return (gv / (1.0f + expf(-gv))) * uv; };
   float4 v[PER4];
   float mx = 0.f;
-  pdl_wait();
+  pdl_wait_then_trigger();
 #pragma unroll
   for (int k0 = 0; k0 < PER4; k0 += 4) {  // at most four pairs in flight: 1024 threads leave 64 registers each
     float4 w[4];
@@ -592,8 +589,7 @@ __global__ void __launch_bounds__(256, 4) qkv_prepare_warp_kernel(const QkvPrepA
   const int lane = threadIdx.x & 31;
   const int64_t r = blockIdx.x;
   const int i0 = E * lane;
-  pdl_trigger();
-  pdl_wait();
+  pdl_wait_then_trigger();
   const int64_t pos = a.row_pos ? a.row_pos[r] : a.base_pos + r;
   const int64_t seq = a.row_seq ? a.row_seq[r] : 0;
   // the rotation is the row's: a warp that takes several heads evaluates it once
@@ -1069,15 +1065,14 @@ argmax_final_kernel(const ArgPair* part, int count, int64_t* out) {
 // block per row left most SMs idle: 8 rows of 151936 logits 30 us, now 6); candidates meet in rank 0's shared memory.
 constexpr int AR_CL = 8, AR_T = 512;
 __global__ void __cluster_dims__(AR_CL, 1, 1) __launch_bounds__(AR_T)
-argmax_rows_kernel(const float* __restrict__ v, int64_t n, int shards, int64_t* out) {
+argmax_rows_kernel(const float* v, int64_t n, int shards, int64_t* out) {
   __shared__ float sv[AR_T / 32], cv[AR_CL];
   __shared__ long long si[AR_T / 32], ci[AR_CL];
   const int rank = blockIdx.x % AR_CL;
   const int64_t r = blockIdx.x / AR_CL, rows = gridDim.x / AR_CL;
   float bv = -INFINITY;
   long long bi = 0x7fffffffffffffffLL;
-  pdl_trigger();
-  pdl_wait();
+  pdl_wait_then_trigger();
   // slice w of this row sits at [w][row][n]; its elements are indices w * n + j
   for (int w = 0; w < shards; w++) {
     const float* row = v + ((int64_t)w * rows + r) * n;

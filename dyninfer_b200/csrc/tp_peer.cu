@@ -50,10 +50,9 @@ __global__ void __launch_bounds__(TP_THREADS, 1) tp_exchange_kernel(const PeerAr
   __shared__ float red[32];
   __shared__ float s_inv;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  pdl_trigger();  // a product launched next may begin fetching its weights
   // launched as a programmatic dependent: everything above and the launch itself overlap the tail
   // of the product before; its partial rows (and this kernel's own epoch word) are there after the wait
-  pdl_wait();
+  pdl_wait_then_trigger();
   const unsigned e = a.epochs[blockIdx.x] + 1;
   // arrival: this rank's partial rows were written by the kernel before this one
   if (tid < a.world) {

@@ -404,3 +404,34 @@ def test_persistent_attention_slices_against_the_oracle(native_lib, oracle, tmp_
             lg = (s.prefill([t]) if i == 0 else s.decode(t)).values
             if i in want:
                 assert np.abs(lg - want[i]).max() <= 1e-2 and helpers.cosine(lg, want[i]) >= 0.9999, i
+
+
+@pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q8_0"])
+@pytest.mark.parametrize("kv", ["bf16", "f16", "f32"])
+def test_few_row_chains_give_the_same_bits_every_time(native_lib, tmp_path, enc, kv):
+    """Many small layers as one chain of dependent launches: prompts and batched steps of every kind of row count, repeated
+    on a session whose buffers hold other values from prompt to prompt, are finite and do not change by a bit."""
+    cfg = dict(synth.SMALL_D128, layers=16, heads=8, kv_heads=4, intermediate=3072, vocab=512)
+    path = synth.write_qwen3_gguf(str(tmp_path / "q.gguf"), cfg, seed=23, encodings=dict.fromkeys(synth.linear_shapes(cfg), enc),
+                                  repeat_layers=True)
+    rng = np.random.default_rng(7)
+    model = ModelLoader().load(path, max_kv=256, kv_dtype=kv, chunk_size=64)
+    prompts = {n: rng.integers(0, 512, size=n).tolist() for n in (2, 4, 5, 9, 16, 17, 20, 24, 28, 31, 32, 48, 64, 92)}
+    first = {}
+    with model.create_session(SessionConfig(max_sequence_length=256)) as s:
+        for _ in range(6):
+            for n, p in prompts.items():
+                got = s.prefill(p).values
+                assert np.isfinite(got).all(), n
+                assert np.array_equal(got, first.setdefault(n, got)), n
+    for slots in (3, 8, 24, 40):
+        with model.create_batched_session(SessionConfig(max_sequence_length=256, batch_size=slots)) as s:
+            seen = None
+            for _ in range(4):
+                for b in range(slots):
+                    s.prefill_slot(b, prompts[28])
+                _, logits = s.step({b: 5 + b for b in range(slots)}, want_logits=True)
+                logits = np.array([logits[b] for b in range(slots)])
+                assert np.isfinite(logits).all()
+                seen = logits if seen is None else seen
+                assert np.array_equal(logits, seen), slots
