@@ -902,20 +902,25 @@ int launch_dqgemm_tc(const WRef& w, const void* x, int x_type, int64_t M, float*
   if (io) io->splits = 0;
   if (!tg_shape_ok(w, M)) return 0;
   // A prompt's chunks keep the grouping of their sums: few tiles go on through the K split below (whose sums the next
-  // kernel adds up: 1024 x 2048, 512 rows 10 against 17 us), all others in whole tiles. Other products stay below where the
-  // split of a long K gives most SMs one wide tile: in gemm_stream the last arriver of a shared tile would add up as many
-  // wide parts. Over 360 shapes of 640 x 6144 to 4096 x 20480 at 96 to 2048 rows per encoding this rule costs 1.6 % against
-  // the faster kernel of each, gemm_stream always 2.8. us, below / gemm_stream: Q4_0 1024 x 12288, 512 rows 31 / 34,
-  // 2048 x 12288, 512 rows 41 / 51, 4096 x 12288, 256 rows 41 / 50; where the split leaves a third of the SMs idle
-  // 512 x 12288, 300 rows 28 / 26; Q4_K and Q5_K convert faster in gemm_stream (2048 x 20480, 300 rows 72 / 55, 108 / 60).
+  // kernel adds up: 1024 x 2048, 512 rows 10 against 17 us), all others in whole tiles. Other products of a long K stay below
+  // where its blocks, one wide tile or a part of its K each, fill the SMs: gemm_stream works at an activation tile for longer
+  // than this kernel, and where it cuts tiles the last arriver adds up as many wide parts. us, below / gemm_stream, Q4_0:
+  //   K split four ways and more, one round of blocks: 1024 x 12288, 512 rows 31 / 34, 2048 x 12288, 512 rows 41 / 51,
+  //     4096 x 12288, 256 rows 41 / 50; with a third of the SMs idle 512 x 12288, 300 rows 28 / 26. 360 shapes per encoding of
+  //     640 x 6144 to 4096 x 20480 at 96 to 2048 rows: 1.6 % off the faster kernel of each (gemm_stream always 2.8).
+  //   A thousand rows and more, Q4_0 and Q4_1 (the others convert faster there): 4096 x 12288, 2048 rows 188 / 220 (rounds
+  //     filled to 86 %), 8192 x 8192 244 / 281, 2048 x 20480 166 / 222; 5120 x 13824, 1024 rows 198 / 141 (54 %).
+  //   Q4_K and Q5_K always convert faster in gemm_stream (2048 x 20480, 300 rows 72 / 55, 108 / 60).
   int old_splits = 0;
   bool split_fills = false;
   if (gemm_stream_takes(w)) {
     const TgPlan old = tg_plan(w, M);
     const int64_t ctas = (w.rows + TG_BM - 1) / TG_BM * old.mtiles * old.splits, sms = std::max(1, sm_count());
+    const int64_t places = (ctas + sms - 1) / sms * sms;
     old_splits = old.splits;
-    split_fills = old.splits >= 4 && ctas <= sms && 10 * ctas >= 7 * sms && old.bn >= 160 && w.cols >= 8192 &&
-                  w.enc != E_Q4_K && w.enc != E_Q5_K;
+    split_fills = old.bn >= 160 && w.cols >= 8192 && w.enc != E_Q4_K && w.enc != E_Q5_K &&
+                  ((old.splits >= 4 && ctas <= sms && 10 * ctas >= 7 * places) ||
+                   (M >= 1000 && (w.enc == E_Q4_0 || w.enc == E_Q4_1) && 10 * ctas >= 8 * places));
   }
   if (gemm_stream_takes(w) && !(io && io->grouped ? old_splits > 1 : split_fills)) {
     *handled = true;
