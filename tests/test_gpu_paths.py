@@ -301,7 +301,7 @@ def test_many_row_norm_widths(native_lib, oracle, tmp_path, hidden):
 
 @pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q8_0", "gguf.q4_k", "mlx.affine.u4"])
 @pytest.mark.parametrize("m,n,k", [(256, 4096, 8192), (300, 1024, 8192), (300, 640, 8192), (160, 3500, 8192),
-                                   (1100, 3500, 8192)])
+                                   (1100, 3500, 8192), (1100, 3500, 12288), (2048, 2300, 12288)])
 def test_linear_many_rows_where_a_k_split_fills_the_gpu(native_lib, oracle, enc, m, n, k):
     """A long K split over about as many blocks as there are SMs, and its neighbours that are cut into equal shares."""
     from dyninfer_b200 import ops
