@@ -908,12 +908,12 @@ int launch_dqgemm_tc(const WRef& w, const void* x, int x_type, int64_t M, float*
   //   K split four ways and more, one round of blocks: 1024 x 12288, 512 rows 31 / 34, 2048 x 12288, 512 rows 41 / 51,
   //     4096 x 12288, 256 rows 41 / 50; with a third of the SMs idle 512 x 12288, 300 rows 28 / 26. 360 shapes per encoding of
   //     640 x 6144 to 4096 x 20480 at 96 to 2048 rows: 1.6 % off the faster kernel of each (gemm_stream always 2.8).
-  //   A thousand rows and more where the work fills 78 % of the rounds (a short last activation tile counts by its rows), over
-  //     54 products of 1024 to 4096 rows per encoding: Q4_0 and Q4_1 from 12 M activations on, 0.87 and 0.89 of gemm_stream's
-  //     time (4096 x 12288, 2048 rows 189 / 218, 4096 rows 402 / 478, 2048 x 20480, 2048 rows 168 / 227; below the line 4096 x
-  //     8192, 1024 rows 86 / 79; 4096 x 8192, 1800 rows fill 76 % 159 / 137); Q8_0, which converts faster there, from 2048 rows
-  //     of K = 12288 on, 0.94 (2048 x 20480 189 / 249, 4096 x 12288 223 / 239; 8192 x 8192 300 / 293). MLX-U4 is even (1.00)
-  //     with losses of up to a quarter (5120 x 25600, 2304 rows 862 / 730) and stays with gemm_stream.
+  //   A thousand rows and more where the work fills 78 % of the rounds (a short last activation tile counts by its rows). Of 54
+  //     products of 1024 to 4096 rows per encoding those that this moves take, in gemm_stream's time: Q4_0 and Q4_1 from 12 M
+  //     activations on 0.86 and 0.88 (4096 x 12288, 2048 rows 189 / 218, 4096 rows 402 / 478, 2048 x 20480, 2048 rows 168 /
+  //     227; below the line 4096 x 8192, 1024 rows 86 / 79; 4096 x 8192, 1800 rows fill 76 % 159 / 137); Q8_0, which converts
+  //     faster there, from 2048 rows of K = 12288 on 0.94 (2048 x 20480 189 / 249, 4096 x 12288 223 / 239; 8192 x 8192 300 /
+  //     293). MLX-U4 would be even (1.00) with losses of up to a quarter (5120 x 25600, 2304 rows 862 / 730) and stays there.
   //   Q4_K and Q5_K always convert faster in gemm_stream (2048 x 20480, 300 rows 72 / 55, 108 / 60).
   int old_splits = 0;
   bool split_fills = false;
