@@ -228,13 +228,16 @@ __device__ __forceinline__ int sk_frag_off(int enc, int k) {
   }
   return unit + (c * 4 + t) * 8 + b * 4;
 }
+constexpr int SK_NATURAL = -1;  // as `enc`: rows in natural order (gemm_cluster.cu)
 // Eight elements k .. k + 7 (k a multiple of 8) times `sc` into a row in fragment order.
 __device__ __forceinline__ void sk_store_frag8(__half* row, int enc, int k, const float (&v)[8], float sc) {
   auto pk = [&](int i, int j) {
     const __half2 h = __floats2half2_rn(v[i] * sc, v[j] * sc);
     return *reinterpret_cast<const uint32_t*>(&h);
   };
-  if (enc == E_MLX_U4) {
+  if (enc == SK_NATURAL) {
+    *reinterpret_cast<uint4*>(row + k) = make_uint4(pk(0, 1), pk(2, 3), pk(4, 5), pk(6, 7));
+  } else if (enc == E_MLX_U4) {
     *reinterpret_cast<uint4*>(row + sk_frag_off(enc, k)) = make_uint4(pk(0, 4), pk(1, 5), pk(2, 6), pk(3, 7));
   } else if (enc == E_Q4_0 || enc == E_Q4_1 || enc == E_Q4_K) {
     *reinterpret_cast<uint2*>(row + sk_frag_off(enc, k)) = make_uint2(pk(0, 2), pk(1, 3));
@@ -338,9 +341,15 @@ int64_t dqgemm_tc_padded_rows(const WRef& w, int64_t M);
 bool gemm_skinny_takes(const WRef& w, int64_t M);
 bool gemm_skinny_prefers(const WRef& w, int64_t M, bool chain);  // chain: inside a layer's chain of fused products
 int gemm_skinny_terms(const WRef& w, int64_t M);
+// The dequant GEMM of 33..64 activation rows with K split over a cluster (gemm_cluster.cu). Activations: f16 rows in natural
+// order, gemm_cluster_rows(M) of them allocated, scaled by a power of two per row, with the inverse scales beside them.
+bool gemm_cluster_prefers(const WRef& w, int64_t M, bool swiglu);
+int64_t gemm_cluster_rows(int64_t M);
+int launch_gemm_cluster(const WRef& w, const __half* x, const float* x_inv, int64_t M, float* y, const float* residual, bool swiglu,
+                        cudaStream_t s);
 int launch_gemm_skinny(const WRef& w, const __half* x, const float* x_inv, int64_t M, float* y, const float* residual,
                        bool swiglu, cudaStream_t s, bool* handled);
-int launch_skinny_prepare(const WRef& w, const void* x, int x_type, int64_t M, __half* out, float* inv_s, cudaStream_t s);
+int launch_skinny_prepare(const WRef& w, const void* x, int x_type, int64_t M, __half* out, float* inv_s, cudaStream_t s, bool natural = false);
 int launch_linear_skinny(const WRef& w, const void* x, int x_type, int64_t M, float* y, const float* residual, cudaStream_t s,
                          bool* handled);
 // The exact few-row product (gemv_rows.cu): 1 to 8 rows, optionally RMSNorm in front, residual or SwiGLU behind.

@@ -1011,9 +1011,9 @@ int launch_gemm_skinny(const WRef& w, const __half* x, const float* x_inv, int64
 
 int gemm_skinny_terms(const WRef& w, int64_t M) { return sk_terms(w.enc, M <= 8 ? 1 : M <= 16 ? 2 : M <= 32 ? 4 : 8); }
 
-int launch_skinny_prepare(const WRef& w, const void* x, int x_type, int64_t M, __half* out, float* inv_s, cudaStream_t s) {
-  DYN_CUDA(launch_pdl(sk_prepare_kernel, dim3((unsigned)M), dim3(256), 0, s, x, x_type == E_BF16 ? 1 : 0, (int)w.cols, w.enc,
-                      gemm_skinny_terms(w, M), M * w.cols, out, inv_s));
+int launch_skinny_prepare(const WRef& w, const void* x, int x_type, int64_t M, __half* out, float* inv_s, cudaStream_t s, bool natural) {
+  DYN_CUDA(launch_pdl(sk_prepare_kernel, dim3((unsigned)M), dim3(256), 0, s, x, x_type == E_BF16 ? 1 : 0, (int)w.cols,
+                      natural ? SK_NATURAL : w.enc, natural ? 1 : gemm_skinny_terms(w, M), M * w.cols, out, inv_s));
   count_launch();
   return 0;
 }
@@ -1022,7 +1022,9 @@ int launch_skinny_prepare(const WRef& w, const void* x, int x_type, int64_t M, _
 int launch_linear_skinny(const WRef& w, const void* x, int x_type, int64_t M, float* y, const float* residual, cudaStream_t s,
                          bool* handled) {
   *handled = false;
-  const size_t xb = ((size_t)gemm_skinny_terms(w, M) * M * w.cols * 2 + 255) / 256 * 256, bytes = xb + (size_t)M * 4;
+  const bool cluster = gemm_cluster_prefers(w, M, false);
+  const size_t x_rows = cluster ? (size_t)gemm_cluster_rows(M) : (size_t)gemm_skinny_terms(w, M) * M;
+  const size_t xb = (x_rows * w.cols * 2 + 255) / 256 * 256, bytes = xb + (size_t)M * 4;
   uint8_t* ws = reinterpret_cast<uint8_t*>(thread_scratch(bytes));
   const bool pooled = ws == nullptr;
   if (pooled) {
@@ -1030,8 +1032,11 @@ int launch_linear_skinny(const WRef& w, const void* x, int x_type, int64_t M, fl
     DYN_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&ws), bytes, s));
   }
   float* inv = reinterpret_cast<float*>(ws + xb);
-  int rc = launch_skinny_prepare(w, x, x_type, M, reinterpret_cast<__half*>(ws), inv, s);
-  if (!rc) rc = launch_gemm_skinny(w, reinterpret_cast<const __half*>(ws), inv, M, y, residual, false, s, handled);
+  int rc = launch_skinny_prepare(w, x, x_type, M, reinterpret_cast<__half*>(ws), inv, s, cluster);
+  if (!rc && cluster) {
+    rc = launch_gemm_cluster(w, reinterpret_cast<const __half*>(ws), inv, M, y, residual, false, s);
+    *handled = true;
+  } else if (!rc) rc = launch_gemm_skinny(w, reinterpret_cast<const __half*>(ws), inv, M, y, residual, false, s, handled);
   const cudaError_t fe = pooled ? cudaFreeAsync(ws, s) : cudaSuccess;
   if (rc) return 1;
   if (fe != cudaSuccess) return cuda_fail(fe, "cudaFreeAsync", __FILE__, __LINE__);

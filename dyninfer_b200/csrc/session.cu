@@ -393,7 +393,8 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       if (w) skinny = skinny && gemm_skinny_prefers(*w, rows, true) && gemm_skinny_terms(*w, rows) == 1;
     skinny = skinny && frag_class(L.q.enc) == frag_class(L.k.enc) && frag_class(L.q.enc) == frag_class(L.v.enc) && L.gate_up.data;
   }
-  auto few = [&](const WRef& w, float* y, const float* residual, bool swiglu) -> int {
+  auto few = [&](const WRef& w, float* y, const float* residual, bool swiglu, bool cluster = false) -> int {
+    if (cluster) return launch_gemm_cluster(w, s->sk_x, s->sk_inv, rows, y, residual, swiglu, st);
     bool handled = false;
     if (launch_gemm_skinny(w, s->sk_x, s->sk_inv, rows, y, residual, swiglu, st, &handled)) return 1;
     DYN_CHECK(handled, "skinny GEMM refused a product it had accepted");
@@ -468,16 +469,22 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   for (int l = 0; l < c.layers; l++) {
     const LayerW& L = s->layers[l];
     if (skinny) {
-      if (launch_norm_frag(s->hidden, L.attn_norm.ptr, L.attn_norm.type, rows, H, c.eps, L.q.enc, s->sk_x, s->sk_inv, st)) return 1;
+      // products of one operand read it in one order: natural where the cluster GEMM takes them all
+      const auto ws = products(L);
+      bool cq = true;
+      for (int i = 0; i < 3; i++) cq = cq && (!ws[i] || gemm_cluster_prefers(*ws[i], rows, false));
+      const bool co = gemm_cluster_prefers(L.o, rows, false), cg = gemm_cluster_prefers(L.gate_up, rows, true),
+                 cd = gemm_cluster_prefers(L.down, rows, false);
+      if (launch_norm_frag(s->hidden, L.attn_norm.ptr, L.attn_norm.type, rows, H, c.eps, cq ? SK_NATURAL : L.q.enc, s->sk_x, s->sk_inv, st)) return 1;
       float *qp = s->q, *kp = s->k, *vp = s->v;
       int64_t ldq = 0, ldk = 0, ldv = 0;
       if (L.qkv_parts >= 2) {
         qp = s->qkv1, kp = qp + qd;
         ldq = ldk = L.qkv_parts == 3 ? qd + 2 * kvd : qd + kvd;
-        if (few(L.qkv, qp, nullptr, false)) return 1;
+        if (few(L.qkv, qp, nullptr, false, cq)) return 1;
         if (L.qkv_parts == 3) vp = kp + kvd, ldv = ldq;
-        else if (few(L.v, vp, nullptr, false)) return 1;
-      } else if (few(L.q, qp, nullptr, false) || few(L.k, kp, nullptr, false) || few(L.v, vp, nullptr, false)) {
+        else if (few(L.v, vp, nullptr, false, cq)) return 1;
+      } else if (few(L.q, qp, nullptr, false, cq) || few(L.k, kp, nullptr, false, cq) || few(L.v, vp, nullptr, false, cq)) {
         return 1;
       }
       QkvPrepArgs pa = qkv_args(l, qp, kp, vp, ldq, ldk, ldv);
@@ -491,18 +498,18 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
         // of the 0.6B shape at 512: 9 us less per layer than slices through memory and their merge; with more CTAs than SMs
         // the smaller ones of that form are ahead)
         if (launch_attention_decode(aa, &pa, &s->freq, nullptr, nullptr, nullptr, 0, st) ||
-            launch_skinny_prepare(L.o, s->ctx, E_F32, rows, s->sk_x, s->sk_inv, st))
+            launch_skinny_prepare(L.o, s->ctx, E_F32, rows, s->sk_x, s->sk_inv, st, co))
           return 1;
       } else if (attention_decode_takes(aa) && part && (decode || rows < 32)) {
-        if (launch_attention_decode(aa, decode ? &pa : nullptr, &s->freq, reinterpret_cast<float*>(part), s->sk_x, s->sk_inv, L.o.enc, st))
+        if (launch_attention_decode(aa, decode ? &pa : nullptr, &s->freq, reinterpret_cast<float*>(part), s->sk_x, s->sk_inv, co ? SK_NATURAL : L.o.enc, st))
           return 1;
-      } else if (launch_attention(aa, st) || launch_skinny_prepare(L.o, s->ctx, E_F32, rows, s->sk_x, s->sk_inv, st)) {
+      } else if (launch_attention(aa, st) || launch_skinny_prepare(L.o, s->ctx, E_F32, rows, s->sk_x, s->sk_inv, st, co)) {
         return 1;
       }
-      if (few(L.o, s->hidden, s->hidden, false) ||
-          launch_norm_frag(s->hidden, L.ffn_norm.ptr, L.ffn_norm.type, rows, H, c.eps, L.gate.enc, s->sk_x, s->sk_inv, st) ||
-          few(L.gate_up, s->act, nullptr, true) || launch_skinny_prepare(L.down, s->act, E_F32, rows, s->sk_x, s->sk_inv, st) ||
-          few(L.down, s->hidden, s->hidden, false))
+      if (few(L.o, s->hidden, s->hidden, false, co) ||
+          launch_norm_frag(s->hidden, L.ffn_norm.ptr, L.ffn_norm.type, rows, H, c.eps, cg ? SK_NATURAL : L.gate.enc, s->sk_x, s->sk_inv, st) ||
+          few(L.gate_up, s->act, nullptr, true, cg) || launch_skinny_prepare(L.down, s->act, E_F32, rows, s->sk_x, s->sk_inv, st, cd) ||
+          few(L.down, s->hidden, s->hidden, false, cd))
         return 1;
       continue;
     }

@@ -280,6 +280,24 @@ def test_linear_few_rows_on_both_sides_of_the_plan_rule(native_lib, oracle, enc,
     assert helpers.rel_err(got, oracle.linear(ow, x, fast=True)) < 2e-5
 
 
+@pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q4_1", "gguf.q8_0", "gguf.q4_k", "mlx.affine.u4"])
+@pytest.mark.parametrize("m,n,k", [(33, 130, 256), (48, 127, 768), (49, 1000, 2560), (64, 257, 3072), (47, 2049, 1792),
+                                   (64, 6000, 1024), (40, 128, 6144), (64, 129, 6400)])
+def test_linear_rows_over_a_cluster(native_lib, oracle, enc, m, n, k):
+    """33 to 64 rows, K over clusters of two to eight blocks with one to three units each (and sizes beyond): ragged
+    tiles and row groups, a last block with fewer units, odd row counts per finishing block. Both operands are rounded to
+    2^-12 of a value; over k products the error of a sum, relative to its size, is about 2^-12 * sqrt(2 / 3) = 2.0e-4 (rounding
+    errors are uniform), so 4e-4 over all outputs holds with room."""
+    from dyninfer_b200 import ops
+    from test_gpu_ops import make_pair
+    if enc == "mlx.affine.u4" and k % 512:
+        pytest.skip("the few-row kernels take MLX rows of whole 512s")
+    dw, ow = make_pair(oracle, enc, n, k, seed=n + m)
+    x = np.random.default_rng(m).normal(size=(m, k)).astype(np.float32)
+    got = ops.linear(dw, torch.from_numpy(x).cuda()).cpu().numpy()
+    assert helpers.rel_err(got, oracle.linear(ow, x, fast=True)) < 4e-4
+
+
 @pytest.mark.parametrize("hidden", [1280, 1536, 2816, 3584, 7168, 1344])
 def test_many_row_norm_widths(native_lib, oracle, tmp_path, hidden):
     """Rows that are multiples of 256 but not of 1024 elements (the last runs of a thread stay empty), and one that is
