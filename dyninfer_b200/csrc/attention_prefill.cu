@@ -1,94 +1,65 @@
 // Causal GQA attention for prefill chunks: many query rows of ONE sequence at consecutive
-// positions against an f32, bf16 or f16 KV cache, on the tensor cores.
+// positions against an f32, bf16 or f16 KV cache, on the 5th-generation tensor cores.
 //
 // Same mathematics as the per-row kernel (kernels.rs:310-458: s = (q.k) * 1/sqrt(d), keys beyond the
 // row's position masked, online max / sum merge, out / sum at the end), restructured the usual
-// flash-attention way: one CTA = one query head x 64 consecutive rows. The 64-key blocks stream through
-// shared memory with cp.async, the next group of blocks in flight while the current one is used.
-// Two shapes of CTA: when the grid is no larger than the GPU (a 512-row chunk of a 16-head model: 128
-// CTAs), eight warps -- warp w takes the 16 rows of group w mod 4 and, of every PAIR of blocks, block
-// w / 4, so two blocks are worked on at once and the two halves' running (max, sum, out) are merged at
-// the end (four K + V tiles resident, one CTA per SM); for larger grids four warps and one block at a
-// time (two tiles resident, two CTAs per SM). S = Q K^T and O += P V run on mma.sync.m16n8k16 with f32
-// accumulators. The cache entries are used
-// in their stored type (exact); the f32 operands Q and P enter as hi + lo pairs of that type
-// (two mma per tile), so the products carry ~16 significant bits of Q / P and the result stays
-// within ~1e-4 of the f32 evaluation.
+// flash-attention way. One CTA = 128 consecutive rows of one query head = the 128 lanes of tensor memory, a thread = a row:
+//   * Q lies in tensor memory as (hi, lo) pairs (128 columns). 64-key tiles of K and V arrive as tensor copies.
+//   * Two streams of four warps take the tiles in turn, each with its own running (max, sum, out), so that one's softmax runs
+//     under the other's MMAs. A fifth warp per stream asks for its tiles and issues its MMAs. Per tile: S (64 columns) = Qhi Khi, a second
+//     accumulator for the terms with a lo part; the thread reads its row twice (maximum, then weights), leaves P as (hi, lo)
+//     pairs in place of S; U (128 columns) = P V, with V's tile as an operand that is contiguous along N; the thread folds U into its 128
+//     f32 sums. The second score accumulator uses U's columns, so a stream needs 192, and 512 hold everything.
+//   * Keys are also dealt over the CTAs of a cluster where there are few (head, row block) pairs (16 heads x 512 rows: 64); all streams'
+//     states meet through shared memory at the end and are merged in a fixed order.
+// On mma.sync (16 rows per warp, 64 per CTA) the MMAs alone kept an SM busy four times as long: 512 rows of 16 heads at 1536, f32
+// cache, 92 us.
 //
+// The cache entries are used in their stored type (exact); the f32 operands Q and P enter as hi + lo pairs of that type. f16
+// operands: query rows are scaled by a power of two, weights by 2^14.
 // f32 caches: a first pass turns the sequence's keys and values into (hi, lo) pairs of f16, every 64-key
 // tile of a head scaled by a power of two of its own (no overflow, nothing lost to subnormals), so a pair
-// holds the entry to 2^-24 of its magnitude; the query rows are scaled and split the same way. The
-// products take three mma per tile (hi hi, lo hi, hi lo; what is dropped is 2^-24 of a term). The tile
-// scales are exact: the keys' multiply the scores, the values' a step's share of the output. Tiles are
-// twice as wide, so a step takes 32 keys. One-row-per-block evaluation of the same chunk (what f32 caches
-// used before) read every key once per query row: 0.6B, 2048-token prompt 102 -> 25 ms.
-// An mma truncates where it adds to its accumulator (about 1.5e-8 of the sum each time, always toward
-// zero). With f16 pairs the scores are therefore added up in chains of four, the products with a lo term
-// apart, and the P V of a step starts from zero and joins the running output by a rounded fma. Error against
-// 64 bits, 256 rows at 7936, mma adding up everything / now / per-row kernel in f32: normal values 1.5e-5 /
-// 3.9e-7 / 8.9e-7, values of one sign 3.2e-5 / 2.0e-7 / 4.7e-7. Cost: 512 rows of 16 heads at 1536
-// 125.5 -> 129.8 us.
+// holds the entry to 2^-24 of its magnitude. The products take three MMAs (hi hi, lo hi, hi lo; what is dropped is 2^-24 of a
+// term). The tile scales are exact: the keys' multiply the scores, the values' a tile's share of the output.
+// Every tile's products start from zero and join the running output by a rounded fma, because a tensor-core accumulation
+// truncates.
 #include <algorithm>
 
 #include "common.cuh"
+#include "tensor_map.cuh"
+#include "umma.cuh"
 
 namespace dyn {
 
 namespace {
 
-constexpr int FA_D = 128;      // head dim handled by this kernel
-constexpr int FA_BR = 64;      // query rows per CTA
-constexpr int FA_PITCH = FA_D + 8;  // elements per shared-memory row (272 bytes: conflict-free fragment loads)
-constexpr int FA_SPLIT_TILE = 64;   // keys per scale of the (hi, lo) form
-constexpr int fa_keys(int kv) { return kv == E_F32 ? 32 : 64; }       // keys per step
-constexpr int fa_planes(int kv) { return kv == E_F32 ? 2 : 1; }       // (hi, lo) or the entries themselves
-constexpr int fa_tile(int kv) { return fa_keys(kv) * FA_PITCH * fa_planes(kv); }  // elements of one K (or V) tile
-constexpr int fa_threads(int halves) { return 128 * halves; }
-constexpr int fa_smem_bytes(int kv, int halves) { return 2 * halves * 2 * fa_tile(kv) * 2; }  // buffers x blocks of a group x (K, V) x 2 bytes
+constexpr int FA_D = 128;           // head dim handled by this kernel
+constexpr int FA_BR = 128;          // query rows per CTA
+constexpr int FA_SPLIT_TILE = 64;   // keys per tile = per scale of the (hi, lo) form
+constexpr int FA_BOX = 64 * 128;    // bytes of a tensor copy: 64 keys x 64 two-byte elements
+constexpr int FA_WORKERS = 576;     // two streams of eight softmax warps, one issuing warp each
+constexpr int FA_THREADS = 640;     // whole warpgroups: registers are dealt out per group
+// 640 threads start with 96 registers each = 61440; 512 x 112 + 128 x 32 = 61440
+constexpr int FA_SOFTMAX_REGS = 112, FA_ISSUE_REGS = 32;
+static_assert(512 * FA_SOFTMAX_REGS + 128 * FA_ISSUE_REGS <= FA_THREADS * 96, "the groups' shares come out of the launch's registers");
+constexpr int fa_items(int kv) { return kv == E_F32 ? 3 : 6; }             // K or V tiles a stream keeps in shared memory
+constexpr int fa_item_bytes(int kv) { return (kv == E_F32 ? 4 : 2) * FA_BOX; }
+constexpr int FA_Q_BYTES = 32768;   // half of the query rows' dims in f32, in the last places of a stream's tiles
+constexpr int FA_PITCH = FA_D + 4;  // floats per row of a stream's final state
+constexpr int FA_SMEM = 2 * 3 * 4 * FA_BOX + 1024;
+static_assert(2 * FA_BR * FA_PITCH * 4 <= FA_SMEM - 1024, "the streams' final states reuse the tiles' memory");
 
-__device__ __forceinline__ void fa_cp16(void* dst, const void* src, bool live) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const int n = live ? 16 : 0;  // 0 source bytes: the 16 destination bytes are zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+// (hi, lo) packed pairs of two f32 values. The packing conversions matter: scalar ones share the unit of the exponentials.
+template <bool BF>
+__device__ __forceinline__ void fa_split2(float x, float y, uint32_t* hi, uint32_t* lo) {
+  if constexpr (BF) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y), l = __floats2bfloat162_rn(x - __low2float(h), y - __high2float(h));
+    *hi = *reinterpret_cast<const uint32_t*>(&h), *lo = *reinterpret_cast<const uint32_t*>(&l);
+  } else {
+    const __half2 h = __floats2half2_rn(x, y), l = __floats2half2_rn(x - __low2float(h), y - __high2float(h));
+    *hi = *reinterpret_cast<const uint32_t*>(&h), *lo = *reinterpret_cast<const uint32_t*>(&l);
+  }
 }
-
-template <int KV>
-struct Mma;
-template <>
-struct Mma<E_BF16> {
-  using T = __nv_bfloat16;
-  __device__ static __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-  }
-  // (hi, lo) packed pairs of two f32 values
-  __device__ static __forceinline__ void split2(float x, float y, uint32_t* hi, uint32_t* lo) {
-    const __nv_bfloat16 hx = __float2bfloat16_rn(x), hy = __float2bfloat16_rn(y);
-    const __nv_bfloat16 lx = __float2bfloat16_rn(x - __bfloat162float(hx));
-    const __nv_bfloat16 ly = __float2bfloat16_rn(y - __bfloat162float(hy));
-    *hi = (uint32_t)__bfloat16_as_ushort(hx) | ((uint32_t)__bfloat16_as_ushort(hy) << 16);
-    *lo = (uint32_t)__bfloat16_as_ushort(lx) | ((uint32_t)__bfloat16_as_ushort(ly) << 16);
-  }
-};
-template <>
-struct Mma<E_F16> {
-  using T = __half;
-  __device__ static __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-  }
-  __device__ static __forceinline__ void split2(float x, float y, uint32_t* hi, uint32_t* lo) {
-    const __half hx = __float2half_rn(x), hy = __float2half_rn(y);
-    const __half lx = __float2half_rn(x - __half2float(hx)), ly = __float2half_rn(y - __half2float(hy));
-    *hi = (uint32_t)__half_as_ushort(hx) | ((uint32_t)__half_as_ushort(hy) << 16);
-    *lo = (uint32_t)__half_as_ushort(lx) | ((uint32_t)__half_as_ushort(ly) << 16);
-  }
-};
-
-template <>
-struct Mma<E_F32> : Mma<E_F16> {};  // operands are f16 pairs
 
 // Power of two that puts `mx` into [2^12, 2^13), and its inverse; magnitudes below 2^-41 share one scale.
 __device__ __forceinline__ void fa_pow2_scale(float mx, float* sc, float* inv) {
@@ -97,13 +68,6 @@ __device__ __forceinline__ void fa_pow2_scale(float mx, float* sc, float* inv) {
   e = max(e, -40);
   *sc = ldexpf(1.0f, 13 - e);
   *inv = ldexpf(1.0f, e - 13);
-}
-
-__device__ __forceinline__ void fa_ldsm4(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d, uint32_t at) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at));
-}
-__device__ __forceinline__ void fa_ldsm4t(uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d, uint32_t at) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at));
 }
 
 // (a, b) = (a, b) * f + (x, y) * s, two values per instruction; s is a power of two.
@@ -120,8 +84,8 @@ __device__ __forceinline__ void fa_fold2(float& a, float& b, float f, float x, f
 // Entries that are not finite have no part in the scale. Among the values they become zeros and the key is marked in
 // `lost`: weight 0 times such an entry would reach the rows that do not see the key. (A key's own reach its scores only.)
 __global__ void __launch_bounds__(256)
-fa_split_kernel(const float* __restrict__ kc, const float* __restrict__ vc, int64_t nkv, int64_t cap, int64_t seq,
-                int64_t nkeys, __half* __restrict__ out, float* __restrict__ inv, unsigned* __restrict__ lost) {
+fa_split_kernel(const float* kc, const float* vc, int64_t nkv, int64_t cap, int64_t seq,
+                int64_t nkeys, __half* out, float* inv, unsigned* lost) {
   __shared__ float red[8];
   __shared__ unsigned s_lost[2];
   const int64_t tile = blockIdx.x, kvh = blockIdx.y, plane = blockIdx.z;
@@ -129,10 +93,11 @@ fa_split_kernel(const float* __restrict__ kc, const float* __restrict__ vc, int6
   const int left = (int)min((int64_t)FA_SPLIT_TILE, nkeys - tile * FA_SPLIT_TILE) * (FA_D / 4);  // float4s
   float4 v[8];
   float mx = 0.f;
+  pdl_wait_then_trigger();
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     const int i = threadIdx.x + 256 * k;
-    v[k] = i < left ? reinterpret_cast<const float4*>(src)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[k] = i < left ? __ldcg(reinterpret_cast<const float4*>(src) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (threadIdx.x < 2) s_lost[threadIdx.x] = 0;
   __syncthreads();
@@ -169,8 +134,8 @@ fa_split_kernel(const float* __restrict__ kc, const float* __restrict__ vc, int6
     const int i = threadIdx.x + 256 * k;
     if (i >= left) continue;
     uint2 hi, lo;
-    Mma<E_F16>::split2(v[k].x * sc, v[k].y * sc, &hi.x, &lo.x);
-    Mma<E_F16>::split2(v[k].z * sc, v[k].w * sc, &hi.y, &lo.y);
+    fa_split2<false>(v[k].x * sc, v[k].y * sc, &hi.x, &lo.x);
+    fa_split2<false>(v[k].z * sc, v[k].w * sc, &hi.y, &lo.y);
     __half* row = dst + (i / (FA_D / 4)) * (2 * FA_D) + (i % (FA_D / 4)) * 4;
     *reinterpret_cast<uint2*>(row) = hi;
     *reinterpret_cast<uint2*>(row + FA_D) = lo;
@@ -179,320 +144,443 @@ fa_split_kernel(const float* __restrict__ kc, const float* __restrict__ vc, int6
 
 struct FaArgs {
   const float* q;     // [rows, nh, d]
-  const void* kcache; // plane of (seq, kv head): [cap, d]; f32 caches: the f16 pairs, [kv head][cap][hi d | lo d]
-  const void* vcache;
+  int64_t krow, vrow; // row of the tensor maps at which the sequence's keys (values) of kv head 0 start
   const float* kinv;  // f32 caches: inverse tile scales [kv head][cap / 64]
   const float* vinv;
   const unsigned* vlost;  // f32 caches: a bit per key whose values are not all finite [kv head][cap / 32]
   float* ctx;         // [rows, nh * d]
-  int64_t rows, nh, nkv, cap, base_pos, seq;
+  int* error;
+  int64_t rows, nh, nkv, cap, base_pos;
   int64_t ldq;        // floats between consecutive rows of q
+  int splits;         // CTAs of a cluster that share the keys
 };
 
-template <int KV, int HALVES>
-__global__ void __launch_bounds__(fa_threads(HALVES)) attention_prefill_kernel(const FaArgs a) {
-  constexpr int FA_THREADS = fa_threads(HALVES);
-  constexpr bool SPLIT = KV == E_F32;
-  constexpr bool SCALED = KV != E_BF16;                // f16 terms: the query rows and the weights need scales
-  constexpr float PMUL = SCALED ? 16384.0f : 1.0f;     // the weights' (the sum carries it too)
-  constexpr int FA_BC = fa_keys(KV), FA_TILE = fa_tile(KV), NP = fa_planes(KV), NT = FA_BC / 8;
-  constexpr int LO = FA_BC * FA_PITCH;  // the lo half of a tile
-  using M = Mma<KV>;
-  using T = typename M::T;
-  extern __shared__ __align__(16) uint8_t fa_smem[];
-  T* const tiles = reinterpret_cast<T*>(fa_smem);  // [buffer][block of the pair][K, V][hi, lo][FA_BC][FA_PITCH]
-  const int tid = threadIdx.x, lane = tid & 31, warp8 = tid >> 5;
-  const int warp = warp8 & 3, half = warp8 >> 2;   // row group; which block of a group
-  const int g = lane >> 2, t = lane & 3;
-  const int64_t h = blockIdx.x, rb = gridDim.y - 1 - blockIdx.y;  // the longest row blocks start first
+// kind::f16 descriptor: M = 128, N = n, f32 accumulation; BF: bf16 operands; mn: B contiguous along N.
+__device__ __forceinline__ uint32_t fa_idesc(int n, bool bf, bool mn) {
+  return umma_idesc(n) | (bf ? (1u << 7) | (1u << 10) : 0u) | (mn ? 1u << 16 : 0u);
+}
+// B operand contiguous along N, 128-byte swizzle: 64 elements of N per 128-byte row, a row per K element; LBO = the next 64 of N (the
+// next box), SBO = the next eight of K.
+__device__ __forceinline__ uint64_t fa_desc_mn(uint32_t smem_addr) {
+  return (uint64_t)((smem_addr >> 4) & 0x3fff) | ((uint64_t)(FA_BOX >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
+template <int KV>
+__global__ void __launch_bounds__(FA_THREADS, 1)
+attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
+                         const __grid_constant__ CUtensorMap vmap) {
+  constexpr bool SPLIT = KV == E_F32, BF = KV == E_BF16;
+  constexpr bool SCALED = !BF;                      // f16 terms: the query rows and the weights need scales
+  constexpr float PMUL = SCALED ? 16384.0f : 1.0f;  // the weights' (the sum carries it too)
+  constexpr int R = fa_items(KV), ITEM = fa_item_bytes(KV);
+  // parts of a tile's keys that are folded into the output one by one: with f32 caches the tensor cores' truncation is the largest
+  // error (4 large terms in a chain: 1.7 times that of 2 for values of one sign)
+  constexpr int FOLDS = SPLIT ? 2 : 1;
+  constexpr uint32_t Q_COL = 384;                   // hi in 64 columns, lo in 64; stream i: S at 192 i, U at 192 i + 64
+  constexpr float LOWEST = -3.40282347e38f;
+  extern __shared__ __align__(1024) uint8_t fa_smem[];
+  __shared__ uint64_t item_full[2][6], q_full[2], s_full[2], p_full[2], u_full[2], u_free[2];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int s_abort;
+  __shared__ float s_x[4][FA_BR];         // largest magnitude of a quarter of the dims
+  __shared__ float s_mx[2][2][2][FA_BR];  // [tile parity][stream][half of the keys]: a row's maximum
+  __shared__ float s_m[2][FA_BR], s_l[2][2][FA_BR];
+  uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fa_smem) + 1023) & ~uintptr_t(1023));
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int ns = a.splits, rank = (int)(blockIdx.x % (unsigned)ns);
+  const int64_t h = blockIdx.x / (unsigned)ns, rb = gridDim.y - 1 - blockIdx.y;  // the longest row blocks start first
   const int64_t kvh = h / (a.nh / a.nkv);
-  const int64_t plane = (SPLIT ? kvh : a.seq * a.nkv + kvh) * a.cap * (FA_D * NP);
-  const T* kplane = reinterpret_cast<const T*>(a.kcache) + plane;
-  const T* vplane = reinterpret_cast<const T*>(a.vcache) + plane;
-  const float* kinv = SPLIT ? a.kinv + kvh * (a.cap / FA_SPLIT_TILE) : nullptr;
-  const float* vinv = SPLIT ? a.vinv + kvh * (a.cap / FA_SPLIT_TILE) : nullptr;
-  const unsigned* vlost = SPLIT ? a.vlost + kvh * (a.cap / 32) : nullptr;
-  const int64_t row_lo = rb * FA_BR + warp * 16;   // this warp's first query row
-  const int64_t r0 = row_lo + g, r1 = r0 + 8;      // the lane's two rows
-  const int64_t r0c = r0 < a.rows ? r0 : a.rows - 1, r1c = r1 < a.rows ? r1 : a.rows - 1;
-  const int64_t pos0 = a.base_pos + r0, pos1 = a.base_pos + r1;
-  const float scale = 1.0f / sqrtf((float)FA_D);
+  // keys 0 .. last position of the CTA's rows, in tiles of 64; tile i belongs to stream i & 1 of CTA (i >> 1) mod splits
+  const int64_t row_lo = rb * FA_BR, row_hi = min(row_lo + FA_BR, a.rows) - 1;
+  const int last = (int)(a.base_pos + row_hi), ntiles = last / FA_SPLIT_TILE + 1;
+  const int stream = warp < 16 ? warp >> 3 : warp & 1;
+  const int first = 2 * rank + stream, step = 2 * ns, mine = first < ntiles ? (ntiles - first + step - 1) / step : 0;
 
-  // Q fragments (hi, lo) for the 8 k-steps over the head dim
-  uint32_t qh[8][4], ql[8][4];
-  float scale0 = scale, scale1 = scale;  // per query row: 1 / sqrt(d), with f16 pairs times the row's inverse scale
-  {
-    const float* q0 = a.q + r0c * a.ldq + h * FA_D;
-    const float* q1 = a.q + r1c * a.ldq + h * FA_D;
-    float s0 = 1.f, s1 = 1.f;
-    if constexpr (SCALED) {
-      float x0 = 0.f, x1 = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < 16; kk++) {
-        const float2 a0 = *reinterpret_cast<const float2*>(q0 + 8 * kk + 2 * t);
-        const float2 a1 = *reinterpret_cast<const float2*>(q1 + 8 * kk + 2 * t);
-        x0 = fmaxf(x0, fmaxf(fabsf(a0.x), fabsf(a0.y)));
-        x1 = fmaxf(x1, fmaxf(fabsf(a1.x), fabsf(a1.y)));
-      }
-      x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, 1));
-      x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, 2));
-      x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, 1));
-      x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, 2));
-      float i0, i1;
-      fa_pow2_scale(x0, &s0, &i0);
-      fa_pow2_scale(x1, &s1, &i1);
-      scale0 *= i0, scale1 *= i1;
+  if (tid == 0) {
+    s_abort = 0;
+    for (int i = 0; i < 2; i++) {
+      for (int j = 0; j < 6; j++) mbar_init(&item_full[i][j], 1);
+      mbar_init(q_full + i, 1), mbar_init(s_full + i, 1), mbar_init(p_full + i, 8), mbar_init(u_full + i, 1), mbar_init(u_free + i, 8);
     }
-#pragma unroll
-    for (int kk = 0; kk < 8; kk++) {
-      const float2 a0 = *reinterpret_cast<const float2*>(q0 + 16 * kk + 2 * t);
-      const float2 a1 = *reinterpret_cast<const float2*>(q1 + 16 * kk + 2 * t);
-      const float2 a2 = *reinterpret_cast<const float2*>(q0 + 16 * kk + 8 + 2 * t);
-      const float2 a3 = *reinterpret_cast<const float2*>(q1 + 16 * kk + 8 + 2 * t);
-      M::split2(a0.x * s0, a0.y * s0, &qh[kk][0], &ql[kk][0]);
-      M::split2(a1.x * s1, a1.y * s1, &qh[kk][1], &ql[kk][1]);
-      M::split2(a2.x * s0, a2.y * s0, &qh[kk][2], &ql[kk][2]);
-      M::split2(a3.x * s1, a3.y * s1, &qh[kk][3], &ql[kk][3]);
-    }
+    mbar_fence_init();
   }
-  float o[16][4];
-#pragma unroll
-  for (int dt = 0; dt < 16; dt++) o[dt][0] = o[dt][1] = o[dt][2] = o[dt][3] = 0.f;
-  float m0 = -3.40282347e38f, m1 = -3.40282347e38f, l0 = 0.f, l1 = 0.f;
+  // Tensor memory is taken before this block lets the next kernel start, so that kernel cannot take it first and then wait for this one.
+  if (warp == 16) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base_s, s_col = tmem + 192u * stream, u_col = s_col + 64u;
+  pdl_wait();
+  if (tid == 0) pdl_trigger();
 
-  // keys 0 .. last position of the CTA's rows
-  int64_t cta_last = a.base_pos + rb * FA_BR + FA_BR - 1;
-  if (cta_last > a.base_pos + a.rows - 1) cta_last = a.base_pos + a.rows - 1;
-  const int64_t warp_last = a.base_pos + (row_lo + 15 < a.rows ? row_lo + 15 : a.rows - 1);
-  const int64_t nkb = cta_last / FA_BC + 1, npairs = (nkb + HALVES - 1) / HALVES;
-  // HALVES blocks x (K, V) x keys of a step x 16 (pairs: 32) pieces of 16 bytes per group, coalesced; rows past the last written
-  // position may hold anything: they are masked, but 0 * NaN must not happen, so they arrive as zeros
-  auto load_pair = [&](int64_t pr) {
-    T* dst = tiles + (pr & 1) * 2 * HALVES * FA_TILE;
-    constexpr int PC = NP * FA_D / 8;  // pieces per key
-    for (int i = tid; i < HALVES * FA_BC * PC; i += FA_THREADS) {
-      const int blk = i / (FA_BC * PC), key = (i / PC) % FA_BC, c = i % PC;
-      const int64_t gk = (HALVES * pr + blk) * FA_BC + key;  // < cap for every written key
-      const bool written = gk <= cta_last;
-      const int64_t src = (written ? gk : 0) * (FA_D * NP) + c * 8;
-      const int at = (c / (FA_D / 8)) * LO + key * FA_PITCH + (c % (FA_D / 8)) * 8;
-      fa_cp16(dst + (blk * 2) * FA_TILE + at, kplane + src, written);
-      fa_cp16(dst + (blk * 2 + 1) * FA_TILE + at, vplane + src, written);
+  uint8_t* const items = smem + stream * (R * ITEM);
+  float o[FA_D / 2];  // the running output of this thread's row and half of the dims
+  float m_run = LOWEST, l_run = 0.f;
+
+  // every thread's part of the ends of the loops: copies and products in flight land before shared memory is used again
+  auto drained = [&] {
+    if (s_abort) {
+      const long long t0 = clock64();
+      while (clock64() - t0 < (1LL << 22)) {
+      }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    __syncwarp();
+    __syncthreads();  // nobody reads the tiles any more
   };
-  load_pair(0);
-  for (int64_t pr = 0; pr < npairs; pr++) {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();  // pair pr has arrived for everyone, and nobody still reads the buffer the next pair goes to
-    if (pr + 1 < npairs) load_pair(pr + 1);
-    const int64_t kb = HALVES * pr + half;
-    if (kb >= nkb) continue;
-    const T(*ks)[FA_PITCH] = reinterpret_cast<const T(*)[FA_PITCH]>(tiles + ((pr & 1) * 2 * HALVES + half * 2) * FA_TILE);
-    const T(*vs)[FA_PITCH] = reinterpret_cast<const T(*)[FA_PITCH]>(tiles + ((pr & 1) * 2 * HALVES + half * 2 + 1) * FA_TILE);
-    if (kb * FA_BC > warp_last) continue;  // every key of the block lies after this warp's rows
-    float ks0 = scale0, ks1 = scale1, vi = 1.0f;
-    unsigned lost = 0;  // keys of the step whose values are not finite
-    if constexpr (SPLIT) {
-      const int64_t tile = kb * FA_BC / FA_SPLIT_TILE;
-      const float ki = __ldg(kinv + tile);
-      vi = __ldg(vinv + tile) * (1.0f / PMUL);
-      lost = __ldg(vlost + 2 * tile + (kb & 1));
-      ks0 *= ki, ks1 *= ki;
-    }
-    // ---- S = Q K^T for 16 rows x the keys of the step. All key groups of a k-step in turn, so that consecutive MMAs do not
-    // wait for one another; one ldmatrix brings the fragments of two groups
-    float s[NT][4];
+  auto cluster_sync = [] { asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory"); };
+  // row of this thread, and its half of a tile's keys and of the output's dims
+  const int row = (warp & 3) * 32 + lane, part = (warp >> 2) & 1;
+
+  if (warp < 16) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FA_SOFTMAX_REGS));
+    const uint32_t tlane = (uint32_t)((warp & 3) * 32) << 16;
+    const int pos = (int)(a.base_pos + min(row_lo + row, a.rows - 1));
+    // ---- Q: four threads share a row, 32 dims each
+    float scale = 1.0f / sqrtf((float)FA_D);
+    {
+      if (!mbar_wait_bounded(q_full + stream, 0, TG_SPINS, &s_abort) && !s_abort) s_abort = 5;
+      const uint8_t* q = items + R * ITEM - FA_Q_BYTES + part * (FA_Q_BYTES / 2) + row * 128;
+      float4 x[8];
 #pragma unroll
-    for (int nt = 0; nt < NT; nt++) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
-    const uint32_t ka = (uint32_t)__cvta_generic_to_shared(&ks[(lane & 7) + 8 * (lane >> 4)][8 * ((lane >> 3) & 1)]);
-    if constexpr (SPLIT) {
+      for (int i = 0; i < 8; i++) x[i] = *reinterpret_cast<const float4*>(q + ((i ^ (row & 7)) << 4));
+      float sc = 1.0f;
+      if constexpr (SCALED) {
+        float mx = 0.f;
 #pragma unroll
-      for (int n0 = 0; n0 < NT; n0 += 2) {
-        float x[2][2][4], lo[2][2][4];  // group, chain
-#pragma unroll
-        for (int n = 0; n < 2; n++)
-#pragma unroll
-          for (int h = 0; h < 2; h++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) x[n][h][e] = lo[n][h][e] = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < 8; kk++) {
-          uint32_t b[2][2], c[2][2];
-          const uint32_t at = ka + (uint32_t)((n0 * 8 * FA_PITCH + 16 * kk) * 2);
-          fa_ldsm4(b[0][0], b[0][1], b[1][0], b[1][1], at);
-          fa_ldsm4(c[0][0], c[0][1], c[1][0], c[1][1], at + LO * 2);
-#pragma unroll
-          for (int n = 0; n < 2; n++) M::mma(x[n][kk & 1], qh[kk], b[n][0], b[n][1]);
-#pragma unroll
-          for (int n = 0; n < 2; n++) M::mma(lo[n][0], ql[kk], b[n][0], b[n][1]);
-#pragma unroll
-          for (int n = 0; n < 2; n++) M::mma(lo[n][1], qh[kk], c[n][0], c[n][1]);
-        }
-#pragma unroll
-        for (int n = 0; n < 2; n++)
-#pragma unroll
-          for (int e = 0; e < 4; e++) s[n0 + n][e] = (x[n][0][e] + x[n][1][e]) + (lo[n][0][e] + lo[n][1][e]);
+        for (int i = 0; i < 8; i++) mx = fmaxf(mx, fmaxf(fmaxf(fabsf(x[i].x), fabsf(x[i].y)), fmaxf(fabsf(x[i].z), fabsf(x[i].w))));
+        s_x[2 * stream + part][row] = mx;
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+        mx = fmaxf(fmaxf(s_x[0][row], s_x[1][row]), fmaxf(s_x[2][row], s_x[3][row]));
+        float inv;
+        fa_pow2_scale(mx, &sc, &inv);
+        scale *= inv;
       }
-    } else {
-      constexpr int GR = NT < 4 ? NT : 4;  // groups at a time
 #pragma unroll
-      for (int n0 = 0; n0 < NT; n0 += GR)
+      for (int i = 0; i < 8; i += 4) {
+        uint32_t hi[8], lo[8];
 #pragma unroll
-        for (int kk = 0; kk < 8; kk++) {
-          uint32_t b[GR][2];
-#pragma unroll
-          for (int n = 0; n < GR; n += 2)
-            fa_ldsm4(b[n][0], b[n][1], b[n + 1][0], b[n + 1][1], ka + (uint32_t)(((n0 + n) * 8 * FA_PITCH + 16 * kk) * 2));
-#pragma unroll
-          for (int n = 0; n < GR; n++) M::mma(s[n0 + n], qh[kk], b[n][0], b[n][1]);
-#pragma unroll
-          for (int n = 0; n < GR; n++) M::mma(s[n0 + n], ql[kk], b[n][0], b[n][1]);
+        for (int j = 0; j < 4; j++) {
+          fa_split2<BF>(x[i + j].x * sc, x[i + j].y * sc, &hi[2 * j], &lo[2 * j]);
+          fa_split2<BF>(x[i + j].z * sc, x[i + j].w * sc, &hi[2 * j + 1], &lo[2 * j + 1]);
         }
+        const uint32_t at = tmem + tlane + Q_COL + 32u * stream + 16u * part + 2u * i;
+        tmem_st8(at, hi);
+        tmem_st8(at + 64u, lo);
+      }
     }
-    // ---- scale, causal mask (blocks that reach past the warp's first row), running maximum
-    float bm0 = -3.40282347e38f, bm1 = -3.40282347e38f;
-    const bool masked = kb * FA_BC + FA_BC - 1 > a.base_pos + row_lo;
-    const int lim0 = (int)(pos0 - kb * FA_BC) - 2 * t, lim1 = (int)(pos1 - kb * FA_BC) - 2 * t;
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    tc_fence_before();
+    asm volatile("bar.sync 2, %0;" ::"n"(FA_WORKERS) : "memory");  // Q is complete, and its place in shared memory free
 #pragma unroll
-    for (int nt = 0; nt < NT; nt++) {
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        s[nt][e] = __fmul_rn(s[nt][e], ks0), s[nt][2 + e] = __fmul_rn(s[nt][2 + e], ks1);  // rounded on its own, not inside the difference below
+    for (int d = 0; d < FA_D / 2; d++) o[d] = 0.f;
+    float nki = 1.f, nvi = 1.f;
+    unsigned nl0 = 0, nl1 = 0;
+    auto tile_info = [&](int i) {  // of the stream's tile i, a tile ahead
+      if constexpr (SPLIT) {
+        const int t = first + i * step;
+        nki = __ldcg(a.kinv + kvh * (a.cap / FA_SPLIT_TILE) + t), nvi = __ldcg(a.vinv + kvh * (a.cap / FA_SPLIT_TILE) + t);
+        nl0 = __ldcg(a.vlost + kvh * (a.cap / 32) + 2 * t), nl1 = __ldcg(a.vlost + kvh * (a.cap / 32) + 2 * t + 1);
+      }
+    };
+    if (mine) tile_info(0);
+    int item = 1;  // of the tile's values
+    unsigned iphase = 0;
+#pragma unroll 1
+    for (int i = 0; i < mine; i++) {
+      const int key0 = (first + i * step) * FA_SPLIT_TILE;
+      const float ks = scale * nki, vi = SPLIT ? nvi * (1.0f / PMUL) : 1.0f;
+      const unsigned lost0 = nl0, lost1 = nl1;
+      if (i + 1 < mine) tile_info(i + 1);
+      const int lim = pos - key0;  // keys 0 .. lim of the tile are seen
+      const bool masked = key0 + FA_SPLIT_TILE - 1 > a.base_pos + row_lo + (warp & 3) * 32;
+      // a failed wait is not left with a break: every warp keeps the same sequence of barriers (and the next waits return at
+      // once, because they look at s_abort)
+      if (!mbar_wait_bounded(s_full + stream, i & 1, TG_SPINS, &s_abort) && !s_abort) s_abort = 1;
+      tc_fence_after();
+      float mx = LOWEST;
+#pragma unroll 1
+      for (int c = 2 * part; c < 2 * part + 2; c++) {
+        uint32_t x[16], y[16];
+        tmem_ld16(s_col + tlane + 16u * c, x);
+        tmem_ld16(u_col + tlane + 16u * c, y);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (masked) {
-          if (nt * 8 + e > lim0) s[nt][e] = -3.40282347e38f;
-          if (nt * 8 + e > lim1) s[nt][2 + e] = -3.40282347e38f;
-        }
-        bm0 = fmaxf(bm0, s[nt][e]);
-        bm1 = fmaxf(bm1, s[nt][2 + e]);
-      }
-    }
-    bm0 = fmaxf(bm0, __shfl_xor_sync(0xffffffffu, bm0, 1));
-    bm0 = fmaxf(bm0, __shfl_xor_sync(0xffffffffu, bm0, 2));
-    bm1 = fmaxf(bm1, __shfl_xor_sync(0xffffffffu, bm1, 1));
-    bm1 = fmaxf(bm1, __shfl_xor_sync(0xffffffffu, bm1, 2));
-    const float mn0 = fmaxf(m0, bm0), mn1 = fmaxf(m1, bm1);
-    const float f0 = expf(m0 - mn0), f1 = expf(m1 - mn1);
-    m0 = mn0, m1 = mn1;
-    l0 *= f0, l1 *= f1;
-    if (!SPLIT && __any_sync(0xffffffffu, f0 != 1.0f || f1 != 1.0f)) {
 #pragma unroll
-      for (int dt = 0; dt < 16; dt++) {
-        o[dt][0] *= f0, o[dt][1] *= f0;
-        o[dt][2] *= f1, o[dt][3] *= f1;
-      }
-    }
-    // ---- P = exp(S - m) (masked keys give exactly 0 once a real key has been seen), hi/lo fragments
-    uint32_t ph[NT / 2][4], pl[NT / 2][4];
+          for (int e = 0; e < 16; e++)
+            if (16 * c + e <= lim) mx = fmaxf(mx, __fmul_rn(__uint_as_float(x[e]) + __uint_as_float(y[e]), ks));
+        } else {
+          float m1 = LOWEST;
 #pragma unroll
-    for (int nt = 0; nt < NT; nt++) {
-      float p[4];
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        p[e] = expf(s[nt][e] - m0) * PMUL;
-        p[2 + e] = expf(s[nt][2 + e] - m1) * PMUL;
-        if (masked) {
-          if (nt * 8 + e > lim0) p[e] = 0.f;
-          if (nt * 8 + e > lim1) p[2 + e] = 0.f;
+          for (int e = 0; e < 16; e += 2) {
+            mx = fmaxf(mx, __fmul_rn(__uint_as_float(x[e]) + __uint_as_float(y[e]), ks));
+            m1 = fmaxf(m1, __fmul_rn(__uint_as_float(x[e + 1]) + __uint_as_float(y[e + 1]), ks));
+          }
+          mx = fmaxf(mx, m1);
         }
       }
-      l0 += p[0] + p[1];
-      l1 += p[2] + p[3];
-      // accumulator tiles 2j, 2j+1 are the A fragment of k-step j of P V
-      const int j = nt >> 1, half = nt & 1;
-      M::split2(p[0], p[1], &ph[j][2 * half], &pl[j][2 * half]);          // row g
-      M::split2(p[2], p[3], &ph[j][2 * half + 1], &pl[j][2 * half + 1]);  // row g + 8
-    }
-    // ---- O += P V: B fragments come transposed out of the [key][dim] tile, four groups of eight dims at a time
-    const uint32_t va = (uint32_t)__cvta_generic_to_shared(&vs[lane & 15][8 * (lane >> 4)]);
+      s_mx[i & 1][stream][part][row] = mx;
+      asm volatile("bar.sync %0, 256;" ::"r"(3 + stream) : "memory");
+      mx = fmaxf(mx, s_mx[i & 1][stream][part ^ 1][row]);
+      const float mn = fmaxf(m_run, mx), f = expf(m_run - mn);
+      m_run = mn, l_run *= f;
+#pragma unroll 1
+      for (int c = 2 * part; c < 2 * part + 2; c++) {
+        uint32_t x[16], y[16];
+        tmem_ld16(s_col + tlane + 16u * c, x);
+        tmem_ld16(u_col + tlane + 16u * c, y);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        uint32_t hi[8], lo[8];
+        float sum = 0.f;
 #pragma unroll
-    for (int d0 = 0; d0 < 16; d0 += 4) {
-      float u[4][4];
+        for (int e = 0; e < 16; e++) x[e] = __float_as_uint(expf(__fmul_rn(__uint_as_float(x[e]) + __uint_as_float(y[e]), ks) - m_run) * PMUL);
+        if (masked) {  // exactly 0
 #pragma unroll
-      for (int j = 0; j < NT / 2; j++) {
-        uint32_t b[4][2], c[4][2];
-#pragma unroll
-        for (int i = 0; i < 4; i += 2) {
-          const uint32_t at = va + (uint32_t)((16 * j * FA_PITCH + (d0 + i) * 8) * 2);
-          fa_ldsm4t(b[i][0], b[i][1], b[i + 1][0], b[i + 1][1], at);
-          if constexpr (SPLIT) fa_ldsm4t(c[i][0], c[i][1], c[i + 1][0], c[i + 1][1], at + LO * 2);
+          for (int e = 0; e < 16; e++)
+            if (16 * c + e > lim) x[e] = 0;
         }
-        if constexpr (SPLIT) {
-          if (j == 0) {
 #pragma unroll
-            for (int i = 0; i < 4; i++) u[i][0] = u[i][1] = u[i][2] = u[i][3] = 0.f;
+        for (int e = 0; e < 8; e++) {
+          const float p0 = __uint_as_float(x[2 * e]), p1 = __uint_as_float(x[2 * e + 1]);
+          sum += p0 + p1;
+          fa_split2<BF>(p0, p1, &hi[e], &lo[e]);
+        }
+        l_run += sum;
+        tmem_st8(s_col + tlane + 16u * c, hi);
+        tmem_st8(s_col + tlane + 16u * c + 8u, lo);
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      if (key0 + FA_SPLIT_TILE - 1 > last) {
+        // values past the last row may hold anything, and their weight 0 must stay 0: zeros
+        if (!mbar_wait_bounded(&item_full[stream][item], iphase, TG_SPINS, &s_abort) && !s_abort) s_abort = 2;
+        const int dead = last + 1 - key0;
+        for (int e = tid & 255; e < (FA_SPLIT_TILE - dead) * 8 * (ITEM / FA_BOX); e += 256)
+          *reinterpret_cast<uint4*>(items + item * ITEM + (e / ((FA_SPLIT_TILE - dead) * 8)) * FA_BOX + dead * 128 + e % ((FA_SPLIT_TILE - dead) * 8) * 16) = make_uint4(0, 0, 0, 0);
+        fence_async_smem();
+      }
+      item += 2;
+      if (item >= R) item -= R, iphase ^= 1u;
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full + stream);
+#pragma unroll 1
+      for (int q = 0; q < FOLDS; q++) {
+        if (!mbar_wait_bounded(u_full + stream, (FOLDS * i + q) & 1, TG_SPINS, &s_abort) && !s_abort) s_abort = 3;
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < 4; c += 2) {
+          uint32_t u[2][16];
+          tmem_ld16(u_col + tlane + 64u * part + 16u * c, u[0]);
+          tmem_ld16(u_col + tlane + 64u * part + 16u * c + 16u, u[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int e = 0; e < 32; e += 2)
+            fa_fold2(o[16 * c + e], o[16 * c + e + 1], q ? 1.0f : f, __uint_as_float(u[e >> 4][e & 15]), __uint_as_float(u[e >> 4][(e & 15) + 1]), vi);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(u_free + stream);
+      }
+      if (SPLIT && (lost0 | lost1)) {  // their pairs are zeros: rows that see one of them get no number, earlier rows are not touched
+        const int key = lost0 ? __ffs(lost0) - 1 : 31 + __ffs(lost1);
+        if (key <= lim) {
+#pragma unroll
+          for (int d = 0; d < FA_D / 2; d++) o[d] = __int_as_float(0x7fffffff);
+        }
+      }
+    }
+    drained();
+    // ---- the streams' states: [stream][row][pitch]
+    float* const state = reinterpret_cast<float*>(smem);
+    {
+      float* const p = state + (stream * FA_BR + row) * FA_PITCH + part * (FA_D / 2);
+#pragma unroll
+      for (int d = 0; d < FA_D / 2; d += 4) *reinterpret_cast<float4*>(p + d) = make_float4(o[d], o[d + 1], o[d + 2], o[d + 3]);
+      s_m[stream][row] = m_run, s_l[stream][part][row] = l_run;
+    }
+    __syncwarp();
+    cluster_sync();
+    {
+      uint32_t base[4];  // of the CTAs' shared memory; what is read there lies at the same offsets as here
+#pragma unroll
+      for (int c = 0; c < 4; c++) asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[c]) : "r"(smem_u32(smem)), "r"(c < ns ? c : 0));
+      const uint32_t at_m = smem_u32(&s_m[0][0]) - smem_u32(smem), at_l = smem_u32(&s_l[0][0][0]) - smem_u32(smem);
+      // a warp's rows, two at a time; lane = four dims
+#pragma unroll 1
+      for (int r0 = rank * 16 + warp; r0 < FA_BR && row_lo + r0 < a.rows; r0 += 32 * ns) {
+        float4 acc[2];
+        float l[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          const int r = min(r0 + 16 * ns * q, FA_BR - 1);
+          float mv[8], l0[8], l1[8], M = LOWEST;
+          float4 v[8];
+#pragma unroll
+          for (int p = 0; p < 8; p++) {  // part p: stream p & 1 of CTA p >> 1
+            if (p >= 2 * ns) break;
+            const uint32_t b = base[p >> 1], sr = (uint32_t)((p & 1) * FA_BR + r);
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(mv[p]) : "r"(b + at_m + 4u * sr) : "memory");
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l0[p]) : "r"(b + at_l + 4u * (2u * FA_BR * (p & 1) + r)) : "memory");
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l1[p]) : "r"(b + at_l + 4u * (2u * FA_BR * (p & 1) + FA_BR + r)) : "memory");
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[p].x), "=f"(v[p].y), "=f"(v[p].z), "=f"(v[p].w)
+                         : "r"(b + 4u * (sr * FA_PITCH + 4 * lane))
+                         : "memory");
           }
 #pragma unroll
-          for (int i = 0; i < 4; i++) M::mma(u[i], ph[j], c[i][0], c[i][1]);
+          for (int p = 0; p < 8; p++)
+            if (p < 2 * ns) M = fmaxf(M, mv[p]);
+          acc[q] = make_float4(0.f, 0.f, 0.f, 0.f), l[q] = 0.f;
 #pragma unroll
-          for (int i = 0; i < 4; i++) M::mma(u[i], pl[j], b[i][0], b[i][1]);
+          for (int p = 0; p < 8; p++) {
+            if (p >= 2 * ns) break;
+            const float w = expf(mv[p] - M);  // a stream without tiles has sum 0 and contributes nothing
+            acc[q].x = fmaf(v[p].x, w, acc[q].x), acc[q].y = fmaf(v[p].y, w, acc[q].y);
+            acc[q].z = fmaf(v[p].z, w, acc[q].z), acc[q].w = fmaf(v[p].w, w, acc[q].w);
+            l[q] = fmaf(l0[p] + l1[p], w, l[q]);
+          }
+        }
 #pragma unroll
-          for (int i = 0; i < 4; i++) M::mma(u[i], ph[j], b[i][0], b[i][1]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; i++) M::mma(o[d0 + i], ph[j], b[i][0], b[i][1]);
-#pragma unroll
-          for (int i = 0; i < 4; i++) M::mma(o[d0 + i], pl[j], b[i][0], b[i][1]);
+        for (int q = 0; q < 2; q++) {
+          const int r = r0 + 16 * ns * q;
+          if (r >= FA_BR || row_lo + r >= a.rows) break;
+          const float i0 = (SPLIT ? PMUL : 1.0f) / l[q];  // pairs: o left the weights' scale with each tile
+          *reinterpret_cast<float4*>(a.ctx + (row_lo + r) * a.nh * FA_D + h * FA_D + 4 * lane) =
+              make_float4(acc[q].x * i0, acc[q].y * i0, acc[q].z * i0, acc[q].w * i0);
         }
       }
-      if constexpr (SPLIT) {
+    }
+    __syncwarp();
+    // nobody leaves while its state may still be read
+    cluster_sync();
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FA_ISSUE_REGS));
+    if (warp < 18) {
+    // ---- the stream's tiles and MMAs. The items K0 V0 K1 V1 .. go round R places; a place is free when the MMAs that read it are
+    // done, which the softmax warps' arrivals imply: P(i) written = S(i) done, U(i) read = P V of i done. The warp walks along
+    // together, so that addresses stay in uniform registers; one lane asks and issues.
+    int put = 0, put_at = 0, get_at = 0;
+    unsigned gphase = 0;
+    auto ask = [&]() {  // the next item
+      if (put < 2 * mine && elect_one()) {
+        const bool values = put & 1;
+        const int key0 = (first + (put >> 1) * step) * FA_SPLIT_TILE;
+        const int y = (int)((values ? a.vrow : a.krow) + kvh * a.cap + key0);
+        uint64_t* bar = &item_full[stream][put_at];
+        uint8_t* dst = items + put_at * ITEM;
+        mbar_expect_tx(bar, ITEM);
+        for (int b = 0; b < ITEM / FA_BOX; b++) tma_box_g2s(dst + b * FA_BOX, values ? &vmap : &kmap, 32 * b, y, bar);
+      }
+      __syncwarp();
+      put++;
+      if (++put_at == R) put_at = 0;
+    };
+    if (elect_one()) {
+      mbar_expect_tx(q_full + stream, FA_Q_BYTES);
+      for (int b = 0; b < 2; b++)
+        tma_box_g2s(items + R * ITEM - FA_Q_BYTES + b * (FA_Q_BYTES / 2), &qmap, (int)(h * FA_D) + stream * 64 + 32 * b, (int)row_lo, q_full + stream);
+    }
+    __syncwarp();
+    for (int i = 0; i < R - FA_Q_BYTES / ITEM; i++) ask();
+    asm volatile("bar.sync 2, %0;" ::"n"(FA_WORKERS) : "memory");
+    for (int i = 0; i < FA_Q_BYTES / ITEM; i++) ask();
+    tc_fence_after();
+    const uint32_t q_hi = tmem + Q_COL, q_lo = q_hi + 64u;
+    const uint32_t id_s = fa_idesc(FA_SPLIT_TILE, BF, false), id_u = fa_idesc(FA_D, BF, true);
+    const uint64_t k_desc0 = umma_desc(smem_u32(items)), v_desc0 = fa_desc_mn(smem_u32(items));
+    // the second stream starts half a tile later, so that the one's MMAs run under the other's softmax (in step, they would
+    // wait for the same units)
+    bool ok = !(stream && mine > 2) || mbar_wait_bounded(s_full, 0, TG_SPINS, &s_abort);
+#pragma unroll 1
+    for (int i = 0; i < mine && ok; i++) {
+      ok = mbar_wait_bounded(&item_full[stream][get_at], gphase, TG_SPINS, &s_abort) &&
+           (i == 0 || mbar_wait_bounded(u_free + stream, (FOLDS * i - 1) & 1, TG_SPINS, &s_abort));
+      if (!ok) break;
+      tc_fence_after();
+      const uint64_t k_hi = k_desc0 + (uint64_t)(get_at * (ITEM >> 4)), k_lo = k_hi + (2 * FA_BOX >> 4);
+      if (elect_one()) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          fa_fold2(o[d0 + i][0], o[d0 + i][1], f0, u[i][0], u[i][1], vi);
-          fa_fold2(o[d0 + i][2], o[d0 + i][3], f1, u[i][2], u[i][3], vi);
+        for (int k = 0; k < 8; k++) {  // sixteen dims at a time: boxes of 64 dims, 32 bytes in a row
+          const uint64_t at = (uint64_t)((k >> 2) * (FA_BOX >> 4) + 2 * (k & 3));
+          umma_f16_ts(u_col, q_lo + 8u * k, k_hi + at, id_s, k ? 1u : 0u);
+          if constexpr (SPLIT) umma_f16_ts(u_col, q_hi + 8u * k, k_lo + at, id_s, 1u);
         }
+        // the large terms in two chains of four, one of them on top of the small ones
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          umma_f16_ts(k < 4 ? s_col : u_col, q_hi + 8u * k, k_hi + (uint64_t)((k >> 2) * (FA_BOX >> 4) + 2 * (k & 3)), id_s, k ? 1u : 0u);
+        umma_commit(s_full + stream);
       }
-    }
-    if (SPLIT && lost) {  // their pairs are zeros: rows that see one of them get no number, earlier rows are not touched
-      const int64_t key = kb * FA_BC + __ffs(lost) - 1;
+      __syncwarp();
+      if (i) ask();  // in place of the values of tile i - 1
+      if (++get_at == R) get_at = 0, gphase ^= 1u;
+      ok = mbar_wait_bounded(&item_full[stream][get_at], gphase, TG_SPINS, &s_abort) &&
+           mbar_wait_bounded(p_full + stream, i & 1, TG_SPINS, &s_abort);
+      if (!ok) break;
+      tc_fence_after();
+      const uint64_t v_hi = v_desc0 + (uint64_t)(get_at * (ITEM >> 4)), v_lo = v_hi + (2 * FA_BOX >> 4);
 #pragma unroll
-      for (int dt = 0; dt < 16; dt++) {
-        if (key <= pos0) o[dt][0] = o[dt][1] = __int_as_float(0x7fffffff);
-        if (key <= pos1) o[dt][2] = o[dt][3] = __int_as_float(0x7fffffff);
+      for (int q = 0; q < FOLDS; q++) {
+        if (q && ok) ok = mbar_wait_bounded(u_free + stream, (FOLDS * i + q - 1) & 1, TG_SPINS, &s_abort);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          constexpr int KS = 4 / FOLDS;  // sixteen keys at a time; the small terms first
+#pragma unroll
+          for (int k = q * KS; k < (q + 1) * KS; k++) {
+            const uint32_t p_hi = s_col + 16u * k, p_lo = p_hi + 8u;
+            const uint64_t at = (uint64_t)(k * (2048 >> 4));
+            umma_f16_ts(u_col, p_lo, v_hi + at, id_u, k > q * KS ? 1u : 0u);
+            if constexpr (SPLIT) umma_f16_ts(u_col, p_hi, v_lo + at, id_u, 1u);
+          }
+#pragma unroll
+          for (int k = q * KS; k < (q + 1) * KS; k++) umma_f16_ts(u_col, s_col + 16u * k, v_hi + (uint64_t)(k * (2048 >> 4)), id_u, 1u);
+          umma_commit(u_full + stream);
+        }
+        __syncwarp();
       }
+      ask();  // in place of the keys
+      if (++get_at == R) get_at = 0, gphase ^= 1u;
     }
-  }
-  // ---- merge the two halves' running states (thread for thread: both cover the same rows and columns)
-  if constexpr (HALVES == 2) {
-  __syncthreads();  // the tiles are no longer read
-  float* const mg = reinterpret_cast<float*>(fa_smem) + (size_t)(warp * 32 + lane) * 68;
-  if (half == 1) {
-    mg[0] = m0, mg[1] = m1, mg[2] = l0, mg[3] = l1;
-#pragma unroll
-    for (int dt = 0; dt < 16; dt++)
-      *reinterpret_cast<float4*>(mg + 4 + 4 * dt) = make_float4(o[dt][0], o[dt][1], o[dt][2], o[dt][3]);
-  }
-  __syncthreads();
-  if (half == 1) return;
-  {
-    const float mb0 = mg[0], mb1 = mg[1];
-    const float mn0 = fmaxf(m0, mb0), mn1 = fmaxf(m1, mb1);
-    const float fa0 = expf(m0 - mn0), fb0 = expf(mb0 - mn0), fa1 = expf(m1 - mn1), fb1 = expf(mb1 - mn1);
-    l0 = l0 * fa0 + mg[2] * fb0;
-    l1 = l1 * fa1 + mg[3] * fb1;
-#pragma unroll
-    for (int dt = 0; dt < 16; dt++) {
-      const float4 ob = *reinterpret_cast<const float4*>(mg + 4 + 4 * dt);
-      o[dt][0] = o[dt][0] * fa0 + ob.x * fb0, o[dt][1] = o[dt][1] * fa0 + ob.y * fb0;
-      o[dt][2] = o[dt][2] * fa1 + ob.z * fb1, o[dt][3] = o[dt][3] * fa1 + ob.w * fb1;
+    if (!ok && !s_abort) s_abort = 4;
+    __syncwarp();
     }
+    // (the softmax warps' ends are theirs alone: these warps have given their registers away)
+    drained();
+    cluster_sync();
+    cluster_sync();
   }
+  tc_fence_after();
+  if (warp == 16) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  if (tid == 0 && s_abort) report_wait_expired(a.error, DEV_ERR_GEMM_PIPE);
+}
+
+template <int KV>
+int fa_launch(const FaArgs& f, const CUtensorMap& qmap, const CUtensorMap& kmap, const CUtensorMap& vmap, cudaStream_t s) {
+  auto kernel = attention_prefill_kernel<KV>;
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), FA_SMEM)) return 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(f.nh * f.splits), (unsigned)((f.rows + FA_BR - 1) / FA_BR)), cfg.blockDim = dim3(FA_THREADS);
+  cfg.dynamicSmemBytes = FA_SMEM, cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
   }
-  // ---- out / sum
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-  const float i0 = (SPLIT ? PMUL : 1.0f) / l0, i1 = (SPLIT ? PMUL : 1.0f) / l1;  // pairs: o left the weights' scale with each step
-#pragma unroll
-  for (int dt = 0; dt < 16; dt++) {
-    if (r0 < a.rows)
-      *reinterpret_cast<float2*>(a.ctx + r0 * a.nh * FA_D + h * FA_D + dt * 8 + 2 * t) =
-          make_float2(o[dt][0] * i0, o[dt][1] * i0);
-    if (r1 < a.rows)
-      *reinterpret_cast<float2*>(a.ctx + r1 * a.nh * FA_D + h * FA_D + dt * 8 + 2 * t) =
-          make_float2(o[dt][2] * i1, o[dt][3] * i1);
-  }
+  attr[n].id = cudaLaunchAttributeClusterDimension;
+  attr[n].val.clusterDim.x = (unsigned)f.splits, attr[n].val.clusterDim.y = 1, attr[n].val.clusterDim.z = 1;
+  n++;
+  cfg.attrs = attr, cfg.numAttrs = n;
+  DYN_CUDA(cudaLaunchKernelEx(&cfg, kernel, f, qmap, kmap, vmap));
+  return 0;
 }
 
 }  // namespace
@@ -509,16 +597,21 @@ int launch_attention_prefill(const AttnArgs& a, int64_t base_pos, int64_t seq, c
   *handled = false;
   if (a.d != FA_D || a.rows < 32 || (a.kv_type != E_BF16 && a.kv_type != E_F16 && a.kv_type != E_F32)) return 0;
   if (a.nkv <= 0 || a.nh % a.nkv || a.cap % FA_SPLIT_TILE) return 0;
-  FaArgs f;
-  f.q = a.q, f.kcache = a.kcache, f.vcache = a.vcache, f.ctx = a.ctx;
-  f.rows = a.rows, f.nh = a.nh, f.nkv = a.nkv, f.cap = a.cap, f.base_pos = base_pos, f.seq = seq;
+  if (((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.ctx) | reinterpret_cast<uintptr_t>(a.kcache) |
+        reinterpret_cast<uintptr_t>(a.vcache)) & 15) || a.ldq % 4 || 2 * a.nkv * a.cap > 0x7fffffff)
+    return 0;
+  FaArgs f{};
+  f.q = a.q, f.ctx = a.ctx, f.error = device_error_word();
+  if (!f.error) return 1;
+  f.rows = a.rows, f.nh = a.nh, f.nkv = a.nkv, f.cap = a.cap, f.base_pos = base_pos;
   f.ldq = a.ldq ? a.ldq : a.nh * FA_D;
-  f.kinv = f.vinv = nullptr, f.vlost = nullptr;
-  const dim3 grid((unsigned)a.nh, (unsigned)((a.rows + FA_BR - 1) / FA_BR));
-  // a grid that fits the GPU in one round: eight warps and pairs of key blocks; larger: four warps, two CTAs per
-  // SM (2-byte caches; the f16 pairs of an f32 cache fill an SM's shared memory either way)
-  const bool pairs = a.kv_type == E_F32 || (int64_t)grid.x * grid.y <= std::max(1, sm_count());
+  // The keys go to as many CTAs as the SMs hold besides one another, while each has a tile for both of its streams
+  const int64_t pairs = a.nh * ((a.rows + FA_BR - 1) / FA_BR), tiles = (base_pos + a.rows + FA_SPLIT_TILE - 1) / FA_SPLIT_TILE;
+  f.splits = 1;
+  while (f.splits < 4 && 2 * f.splits * pairs <= sm_count() && 4 * f.splits <= tiles) f.splits *= 2;
   void* pooled = nullptr;
+  CUtensorMap qmap, kmap, vmap;
+  if (make_row_box_map(reinterpret_cast<const uint8_t*>(a.q), (size_t)f.ldq * 4, a.rows, 32, FA_BR, &qmap, true)) return 1;
   if (a.kv_type == E_F32) {
     const size_t bytes = attention_prefill_scratch_bytes(a);
     void* ws = a.pair_ws && a.pair_ws_bytes >= bytes ? a.pair_ws : nullptr;
@@ -532,25 +625,22 @@ int launch_attention_prefill(const AttnArgs& a, int64_t base_pos, int64_t seq, c
     float* const inv = reinterpret_cast<float*>(out + 2 * plane);
     unsigned* const lost = reinterpret_cast<unsigned*>(inv + 2 * a.nkv * (a.cap / FA_SPLIT_TILE));
     const int64_t nkeys = base_pos + a.rows;
-    fa_split_kernel<<<dim3((unsigned)((nkeys + FA_SPLIT_TILE - 1) / FA_SPLIT_TILE), (unsigned)a.nkv, 2), 256, 0, s>>>(
-        reinterpret_cast<const float*>(a.kcache), reinterpret_cast<const float*>(a.vcache), a.nkv, a.cap, seq, nkeys, out, inv, lost);
+    DYN_CUDA(launch_pdl(fa_split_kernel, dim3((unsigned)((nkeys + FA_SPLIT_TILE - 1) / FA_SPLIT_TILE), (unsigned)a.nkv, 2), dim3(256), 0, s,
+                        reinterpret_cast<const float*>(a.kcache), reinterpret_cast<const float*>(a.vcache), a.nkv, a.cap, seq, nkeys, out, inv,
+                        lost));
     count_launch();
-    f.kcache = out, f.vcache = out + plane;
     f.kinv = inv, f.vinv = inv + a.nkv * (a.cap / FA_SPLIT_TILE), f.vlost = lost;
+    if (make_row_box_map(reinterpret_cast<const uint8_t*>(out), 4 * FA_D, 2 * a.nkv * a.cap, 32, FA_SPLIT_TILE, &kmap, true)) return 1;
+    vmap = kmap;
+    f.krow = 0, f.vrow = a.nkv * a.cap;
+  } else {
+    const int64_t at = seq * a.nkv * a.cap;  // row of the sequence's first plane
+    if (make_row_box_map(reinterpret_cast<const uint8_t*>(a.kcache) + at * (2 * FA_D), 2 * FA_D, a.nkv * a.cap, 32, FA_SPLIT_TILE, &kmap, true) ||
+        make_row_box_map(reinterpret_cast<const uint8_t*>(a.vcache) + at * (2 * FA_D), 2 * FA_D, a.nkv * a.cap, 32, FA_SPLIT_TILE, &vmap, true))
+      return 1;
   }
-  auto run = [&](auto kernel, int halves) -> int {
-    const int bytes = fa_smem_bytes(a.kv_type, halves);
-    if (ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), bytes)) return 1;
-    kernel<<<grid, fa_threads(halves), bytes, s>>>(f);
-    return 0;
-  };
-  int rc;
-  if (a.kv_type == E_F32)
-    rc = run(attention_prefill_kernel<E_F32, 2>, 2);
-  else if (a.kv_type == E_BF16)
-    rc = pairs ? run(attention_prefill_kernel<E_BF16, 2>, 2) : run(attention_prefill_kernel<E_BF16, 1>, 1);
-  else
-    rc = pairs ? run(attention_prefill_kernel<E_F16, 2>, 2) : run(attention_prefill_kernel<E_F16, 1>, 1);
+  const int rc = a.kv_type == E_F32 ? fa_launch<E_F32>(f, qmap, kmap, vmap, s) : a.kv_type == E_BF16 ? fa_launch<E_BF16>(f, qmap, kmap, vmap, s)
+                                                                                              : fa_launch<E_F16>(f, qmap, kmap, vmap, s);
   const cudaError_t fe = pooled ? cudaFreeAsync(pooled, s) : cudaSuccess;
   if (rc) return 1;
   if (fe != cudaSuccess) return cuda_fail(fe, "cudaFreeAsync", __FILE__, __LINE__);

@@ -280,6 +280,29 @@ def test_linear_few_rows_on_both_sides_of_the_plan_rule(native_lib, oracle, enc,
     assert helpers.rel_err(got, oracle.linear(ow, x, fast=True)) < 2e-5
 
 
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("s,start,nh,nkv", [(32, 0, 4, 2), (127, 0, 2, 1), (128, 64, 2, 2), (129, 127, 4, 1), (40, 200, 8, 2),
+                                            (257, 383, 3, 3), (64, 1087, 2, 1), (300, 20, 80, 8)])
+def test_attention_prefill_at_the_edges_of_blocks(native_lib, dtype, s, start, nh, nkv):
+    """128-row blocks and 64-key tiles that end on, before and behind a boundary; one to four blocks share the keys, some of
+    their streams without a tile; more blocks than SMs. Operands are pairs: 22 bits with f16 terms, 16 with bf16 ones, so that
+    an output, a mean of values of size one, is off by a few 2^-22 (2^-16) of their largest."""
+    from dyninfer_b200 import ops
+    d, cap = 128, 1408
+    g = torch.Generator("cuda").manual_seed(s + start)
+    q, k, v = (torch.randn(*shape, generator=g, device="cuda") for shape in ((s, nh, d), (nkv, cap, d), (nkv, cap, d)))
+    tt = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dtype]
+    k, v = k.to(tt), v.to(tt)
+    k[:, start + s:] = float("nan")                  # never-written rows must not leak into the result
+    v[:, start + s:] = float("inf")
+    got = ops.attention(q, k, v, start).reshape(s, nh, d).double()
+    hidden = torch.arange(start + s, device="cuda")[None, :] > torch.arange(s, device="cuda")[:, None] + start
+    for h in range(nh):
+        kh, vh = (c[h // (nh // nkv), :start + s].double() for c in (k, v))
+        want = (q[:, h].double() @ kh.T / d ** 0.5).masked_fill(hidden, float("-inf")).softmax(-1) @ vh
+        assert float((got[:, h] - want).abs().max()) < (1e-4 if dtype == "bf16" else 4e-6) * float(vh.abs().max())
+
+
 @pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q4_1", "gguf.q8_0", "gguf.q4_k", "mlx.affine.u4"])
 @pytest.mark.parametrize("m,n,k", [(33, 130, 256), (48, 127, 768), (49, 1000, 2560), (64, 257, 3072), (47, 2049, 1792),
                                    (64, 6000, 1024), (40, 128, 6144), (64, 129, 6400)])
