@@ -713,11 +713,27 @@ bool gr_make_plan(const WRef& w, int64_t M, bool swiglu, GrPlan* best) {
   }
   if (!found) return false;
   const void* kernel = gr_kernel(w.enc, best->NM);
-  if (ensure_dynamic_smem(kernel, GR_MAX_SMEM) ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&best->per_sm, kernel, best->RW * best->KW * 32, best->smem) != cudaSuccess || best->per_sm < 1)
-    best->per_sm = 1;
-  const int rows = (swiglu ? 8 : 16) * best->RW;
-  best->groups = (N + rows - 1) / rows;
+  if (ensure_dynamic_smem(kernel, GR_MAX_SMEM)) return false;
+  // Blocks of more rows and fewer K warps where the blocks do not fit the SMs well: eight warps on one SM get through a tile's K
+  // faster alone than beside a second block, and a second round of a few blocks costs as much as a full one. us before / with twice
+  // the rows: Q4_0, one row, 5120 x 4096 (320 blocks for 296 places) 10.1 / 6.9, 4096 x 4096 (256) 6.0 / 5.4, 3072 x 2048 (192)
+  // 4.3 / 3.9; four rows 4096 x 4096 15.5 / 14.5, 10240 x 5120 38 / 32. Beyond eight stages per warp the second block's loads count for
+  // more (4096 x 14336 14.1 / 17.4), with that second round beyond twelve (5120 x 13824 Q8_0, four rows 56 / 60).
+  const int tile_rows = swiglu ? 8 : 16;
+  for (int i = 0;; i++) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&best->per_sm, kernel, best->RW * best->KW * 32, best->smem) != cudaSuccess || best->per_sm < 1)
+      best->per_sm = 1;
+    best->groups = (N + tile_rows * best->RW - 1) / (tile_rows * best->RW);
+    const int64_t ctas = best->groups * best->CK, places = (int64_t)best->per_sm * std::max(1, sm_count());
+    const bool halves = best->KW >= 4 && ctas > sm_count() && 2 * best->cstages <= 8 * best->KW, spills = best->KW >= 2 && ctas > places && 10 * ctas <= 13 * places && 2 * best->cstages <= 12 * best->KW;
+    if (best->RW * best->KW != 8 || !(i == 0 ? halves || spills : spills)) break;
+    GrPlan q = *best;
+    q.RW *= 2, q.KW /= 2;
+    q.nst = std::min((q.cstages + q.KW - 1) / q.KW, 2);
+    q.smem = gr_smem(w, q);
+    if (q.smem > (size_t)GR_MAX_SMEM || (q.smem > (size_t)110 * 1024 && best->smem <= (size_t)110 * 1024)) break;
+    *best = q;
+  }
   if (best->groups * best->CK > 0x7fffffff) return false;
   return true;
 }
