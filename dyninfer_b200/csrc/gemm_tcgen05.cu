@@ -610,6 +610,7 @@ dqgemm_tc_kernel(const TgArgs a, const __grid_constant__ CUtensorMap xmap) {
   } else if (warp == TG_B_WARP) {
     // ---------------- B producer: one TMA tile (bn rows x 64 k, swizzled by the hardware) per stage -----
     if (lane == 0) {
+      pdl_wait_then_trigger();  // (tensor memory is taken: the next kernel cannot take it first and then wait for this one)
       int slot = 0;
       unsigned phase = 1;  // parity of the drain that frees a slot for its next chunk; the first round waits for none
       uint8_t* dst = smem + A_BYTES;
@@ -671,7 +672,8 @@ dqgemm_tc_kernel(const TgArgs a, const __grid_constant__ CUtensorMap xmap) {
   // before its first store (y may be the residual's own buffer).
   {
     __syncwarp();  // the issuing lanes of the MMA and copy warps rejoin here
-    for (int j = tid; j < bn; j += TG_THREADS) s_inv[j] = m0 + j < a.M ? __ldg(a.inv_s + m0 + j) : 0.f;
+    pdl_wait();    // inverse scales, residual; the output may still be read by the kernels before
+    for (int j = tid; j < bn; j += TG_THREADS) s_inv[j] = m0 + j < a.M ? __ldcg(a.inv_s + m0 + j) : 0.f;
     __syncthreads();
     const bool ok = mbar_wait_bounded(&accum_bar, 0, TG_SPINS, &s_abort);
     if (!ok && !s_abort) s_abort = 3;
@@ -773,8 +775,9 @@ int tg_make_xmap(__half* xh, int64_t rows, int64_t K, int bn, CUtensorMap* map) 
 
 // y = sum over the K splits (fixed order) + residual
 __global__ void __launch_bounds__(256)
-tg_split_reduce_kernel(const float* __restrict__ partial, int splits, int64_t count, float* y, const float* residual) {
+tg_split_reduce_kernel(const float* partial, int splits, int64_t count, float* y, const float* residual) {
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  pdl_wait_then_trigger();
   if (i >= count) return;
   float v = 0.f;
   for (int z = 0; z < splits; z++) v += partial[(int64_t)z * count + i];
@@ -785,7 +788,8 @@ tg_split_reduce_kernel(const float* __restrict__ partial, int splits, int64_t co
 template <int ENC>
 int tg_launch(const TgArgs& a, const CUtensorMap& xmap, dim3 grid, size_t smem, cudaStream_t s) {
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(dqgemm_tc_kernel<ENC>), 200 * 1024)) return 1;
-  dqgemm_tc_kernel<ENC><<<grid, TG_THREADS, smem, s>>>(a, xmap);
+  // weights are fetched and converted while the kernel in front still runs
+  DYN_CUDA(launch_pdl(dqgemm_tc_kernel<ENC>, grid, dim3(TG_THREADS), smem, s, a, xmap));
   return 0;
 }
 
@@ -989,7 +993,8 @@ int launch_dqgemm_tc(const WRef& w, const void* x, int x_type, int64_t M, float*
     io->splits = splits;
   } else if (splits > 1) {
     const int64_t count = M * w.rows;
-    tg_split_reduce_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(partial, splits, count, y, residual);
+    DYN_CUDA(launch_pdl(tg_split_reduce_kernel, dim3((unsigned)((count + 255) / 256)), dim3(256), 0, s, (const float*)partial, splits, count, y,
+                        residual));
     count_launch();
   }
   DYN_CUDA(cudaGetLastError());
