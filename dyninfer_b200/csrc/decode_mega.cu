@@ -348,23 +348,23 @@ __device__ __forceinline__ void item_store(const float (&sv)[8], int layout, int
     for (int j = 0; j < 8; j++) f[j] = sv[j];
     *run0 = sa, *run1 = sb;
   }
-  __half hi[8], lo[8];  // 16-bit storage: f16, or bf16 bit patterns for the plain-bf16 layout
+  // f16, or bf16 bit patterns for the plain-bf16 layout; packing conversions (scalar ones run at an eighth of their rate)
+  uint32_t hi[4], lo[4];
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
+  for (int j = 0; j < 4; j++) {
     if (layout == XL_BF16N) {
-      const __nv_bfloat16 h = __float2bfloat16_rn(f[j]);
-      const __nv_bfloat16 l = __float2bfloat16_rn(f[j] - __bfloat162float(h));
-      hi[j] = __ushort_as_half(__bfloat16_as_ushort(h));
-      lo[j] = __ushort_as_half(__bfloat16_as_ushort(l));
+      const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
+      const __nv_bfloat162 l = __floats2bfloat162_rn(f[2 * j] - __low2float(h), f[2 * j + 1] - __high2float(h));
+      hi[j] = *reinterpret_cast<const uint32_t*>(&h), lo[j] = *reinterpret_cast<const uint32_t*>(&l);
     } else {
-      const __half h = __float2half_rn(f[j]);
-      hi[j] = h;
-      lo[j] = __float2half_rn(f[j] - __half2float(h));
+      const __half2 h = __floats2half2_rn(f[2 * j], f[2 * j + 1]);
+      const __half2 l = __floats2half2_rn(f[2 * j] - __low2float(h), f[2 * j + 1] - __high2float(h));
+      hi[j] = *reinterpret_cast<const uint32_t*>(&h), lo[j] = *reinterpret_cast<const uint32_t*>(&l);
     }
   }
   uint4* dst = reinterpret_cast<uint4*>(sm.xf + ((size_t)(kb * 2) * 4 + t) * 8);
-  dst[0] = *reinterpret_cast<uint4*>(hi);
-  dst[4] = *reinterpret_cast<uint4*>(lo);
+  dst[0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+  dst[4] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
 }
 
 // Per-warp staging. ukb: 32-blocks per unit of the phase's encoding; the warp owns the units
