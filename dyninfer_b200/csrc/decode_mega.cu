@@ -151,6 +151,7 @@ struct Smem {
   const MegaRound* rounds;
   const uint16_t* phase_rounds;
   const MegaLayerHot* hot;
+  const uint4* zeros;  // 64 bytes
   volatile int* abort;
   uint32_t nchunks;  // chunks of one token's program
   int nslot;
@@ -220,8 +221,10 @@ __device__ __forceinline__ void produce_chunk(const MegaChunk* c, const Smem& sm
     const uint32_t off = ((uint32_t)c->aal + (uint32_t)i * c->aal_step) & 15u;
     const uint32_t nb = (off + c->aseg + 15u) & ~15u;
     uint8_t* d = base + 16 * c->pitch + i * c->apitch;
-    bulk_g2s(d, c->sc + (size_t)i * c->arb - off, nb, sm.full + slot);
-    bulk_g2s(d + 16 * c->apitch, c->bi + (size_t)i * c->arb - off, nb, sm.full + slot);
+    // rows 8..15 of an interleaved tile: as many rows further on as those of the words (a group has 16 << group_shift bytes of words)
+    const int64_t at = (int64_t)i * c->arb + (i >= 8 ? ((int64_t)c->jump16 * (c->aux == E_F32 ? 4 : 2)) >> c->group_shift : 0);
+    bulk_g2s(d, c->sc + at - off, nb, sm.full + slot);
+    bulk_g2s(d + 16 * c->apitch, c->bi + at - off, nb, sm.full + slot);
   }
 }
 
@@ -329,6 +332,27 @@ __device__ __forceinline__ void item_fetch(const StageSrc& src, int baseA, int b
   }
 }
 
+// The norm weights of an item: four at baseA, four at baseB (both multiples of four; 1 without a norm).
+__device__ __forceinline__ void item_norm(const void* nw, int type, int baseA, int baseB, float (&w)[8]) {
+  if (!nw) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) w[q] = 1.0f;
+  } else if (type == E_F32) {
+    const float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(nw) + baseA);
+    const float4 b = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(nw) + baseB);
+    w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
+  } else {
+    const uint2 a = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(nw) + baseA);
+    const uint2 b = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(nw) + baseB);
+    const uint32_t u[4] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      w[2 * q] = type == E_F16 ? f16_bits_to_f32(u[q] & 0xffffu) : __uint_as_float(u[q] << 16);
+      w[2 * q + 1] = type == E_F16 ? f16_bits_to_f32(u[q] >> 16) : __uint_as_float(u[q] & 0xffff0000u);
+    }
+  }
+}
+
 // Writes one item's hi/lo f16 fragments from its 8 scaled values sv and returns its share of the
 // block's two 16-element runs.
 __device__ __forceinline__ void item_store(const float (&sv)[8], int layout, int kb, int t, const Smem& sm, float* run0,
@@ -388,9 +412,7 @@ __device__ __forceinline__ void stage_local(const StageSrc& src, const void* nw,
     if (live) {
       // norm weights first: their loads are in flight while the pairs are polled
       float w[8];
-#pragma unroll
-      for (int q = 0; q < 8; q++)
-        w[q] = nw ? aux_load(reinterpret_cast<const uint8_t*>(nw), nw_type, (q < 4 ? baseA : baseB - 4) + q) : 1.0f;
+      item_norm(nw, nw_type, baseA, baseB, w);
       item_fetch(src, baseA, baseB, sm, v);
 #pragma unroll
       for (int q = 0; q < 8; q++) {
@@ -439,9 +461,7 @@ __device__ __forceinline__ void stage_phase(const StageSrc& src, const void* nw,
     int baseA, baseB;
     item_bases(layout, kb, t, &baseA, &baseB);
     float w[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-      w[j] = nw ? aux_load(reinterpret_cast<const uint8_t*>(nw), nw_type, (j < 4 ? baseA : baseB - 4) + j) : 1.0f;
+    item_norm(nw, nw_type, baseA, baseB, w);
     float v[8];
     item_fetch(src, baseA, baseB, sm, v);
     if (src.kind != SRC_XS) {
@@ -482,12 +502,10 @@ __device__ __forceinline__ void stage_phase(const StageSrc& src, const void* nw,
       const float4 a4 = *reinterpret_cast<const float4*>(sm.xs + baseA);  // written by this thread
       const float4 b4 = *reinterpret_cast<const float4*>(sm.xs + baseB);
       const float v[8] = {a4.x, a4.y, a4.z, a4.w, b4.x, b4.y, b4.z, b4.w};
-      float sv[8];
+      float sv[8], w[8];
+      item_norm(nw, nw_type, baseA, baseB, w);
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const float wj = nw ? aux_load(reinterpret_cast<const uint8_t*>(nw), nw_type, (j < 4 ? baseA : baseB - 4) + j) : 1.0f;
-        sv[j] = (nw ? __fmul_rn(__fmul_rn(v[j], inv), wj) : v[j]) * s;
-      }
+      for (int j = 0; j < 8; j++) sv[j] = (nw ? __fmul_rn(__fmul_rn(v[j], inv), w[j]) : v[j]) * s;
       item_store(sv, layout, kb, t, sm, &run0, &run1);
     }
     run0 += __shfl_xor_sync(0xffffffffu, run0, 1);
@@ -580,6 +598,43 @@ __device__ __forceinline__ void run_unit(int enc, int aux, int group_shift, cons
     case E_F16: run_unit_t<E_F16>(aux, group_shift, p0, p1, a0, a1, apitch16, u, kb0, sm, lane, acc); break;
     default: run_unit_t<E_Q6_K>(aux, group_shift, p0, p1, a0, a1, apitch16, u, kb0, sm, lane, acc); break;
   }
+}
+
+// MLX-U4, four consecutive 32-blocks of a chunk at a time (quad P: blocks 4 P .. 4 P + 3), one per lane quarter: quarter t feeds
+// the A operand with its own block of rows g and g + 8, and the B operand holds that block's activations only in columns 2 t
+// (hi) and 2 t + 1 (lo), so a lane ends up with its own block's sums and applies one scale and bias per eight MMAs. Block by block, all
+// four quarters fetched the same scales and applied them to the same sums, about 200 instructions per 128 weights of 16 rows
+// against 70 now (tile math of a 0.6B token 177 -> 117 us). The accumulator then holds the quarter's share of a row: the
+// quarters are added up when the tile ends. Q4_0, whose scale lies beside its block, gains nothing (its blocks start in the middle
+// of a word).
+__device__ __forceinline__ void run_quad(int aux, int group_shift, const uint8_t* p0, const uint8_t* p1, const uint8_t* a0,
+                                         const uint8_t* a1, int apitch16, int P, int kb0, const Smem& sm, int lane, TileAcc<true>& acc) {
+  const int g = lane >> 2, t = lane & 3, kb = kb0 + 4 * P + t;
+  const uint4* xb = (g >> 1) == t ? reinterpret_cast<const uint4*>(sm.xf + ((size_t)(kb * 2 + (g & 1)) * 4) * 8) : sm.zeros;
+  const uint4 v0 = *reinterpret_cast<const uint4*>(p0 + P * 64 + t * 16), v1 = *reinterpret_cast<const uint4*>(p1 + P * 64 + t * 16);
+  const int gi = (4 * P + t) >> group_shift;
+  float f[4];  // scales of the two rows, biases
+  if (aux == E_F32) {
+    f[0] = reinterpret_cast<const float*>(a0)[gi], f[1] = reinterpret_cast<const float*>(a1)[gi];
+    f[2] = reinterpret_cast<const float*>(a0 + apitch16)[gi], f[3] = reinterpret_cast<const float*>(a1 + apitch16)[gi];
+  } else {
+    const uint32_t u[4] = {reinterpret_cast<const uint16_t*>(a0)[gi], reinterpret_cast<const uint16_t*>(a1)[gi],
+                           reinterpret_cast<const uint16_t*>(a0 + apitch16)[gi], reinterpret_cast<const uint16_t*>(a1 + apitch16)[gi]};
+#pragma unroll
+    for (int i = 0; i < 4; i++) f[i] = aux == E_F16 ? f16_bits_to_f32(u[i]) : __uint_as_float(u[i] << 16);
+  }
+  const uint32_t w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
+  float c[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const uint4 b = xb[i];
+    const uint32_t h0 = w0[i] >> 8, h1 = w1[i] >> 8;
+    mma_f16_16816(c, w0[i] & 0x000F000Fu, w1[i] & 0x000F000Fu, w0[i] & 0x00F000F0u, w1[i] & 0x00F000F0u, b.x, b.y);
+    mma_f16_16816(e, h0 & 0x000F000Fu, h1 & 0x000F000Fu, h0 & 0x00F000F0u, h1 & 0x00F000F0u, b.z, b.w);
+  }
+  const float bs = sm.isx[kb], sx = sm.sx32[kb] * GV_2M24;
+  acc.v[0] = fmaf(f[0] * bs, (c[0] + c[1]) + (e[0] + e[1]), fmaf(f[2] * bs, sx, acc.v[0]));
+  acc.v[1] = fmaf(f[1] * bs, (c[2] + c[3]) + (e[2] + e[3]), fmaf(f[3] * bs, sx, acc.v[1]));
 }
 
 __device__ __forceinline__ float round_kv(float v, int kv_type) {
@@ -970,7 +1025,7 @@ struct Walk {
   long long bi;
 };
 
-template <int ENC, class Prof>
+template <int ENC, bool QUADS, class Prof>
 __device__ __forceinline__ void run_phase_t(const MegaArgs& a, const Smem& sm, Walk& w, int nr, unsigned ep,
                                             const float* ssq, int n_in, float* res, int hid_lo, int tid, int lane,
                                             int warp, Prof& prof, int sid) {
@@ -984,6 +1039,13 @@ __device__ __forceinline__ void run_phase_t(const MegaArgs& a, const Smem& sm, W
     t.clear();
     int cur = -1;
     auto flush = [&]() {
+      if constexpr (QUADS) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          t.v[i] += __shfl_xor_sync(0xffffffffu, t.v[i], 1);
+          t.v[i] += __shfl_xor_sync(0xffffffffu, t.v[i], 2);
+        }
+      }
       if (cur >= 0 && (lane & 3) == 0) {
         pb[(cur * MK_CW + warp) * 16 + g] = t.v[0];
         pb[(cur * MK_CW + warp) * 16 + g + 8] = t.v[1];
@@ -1037,6 +1099,9 @@ __device__ __forceinline__ void run_phase_t(const MegaArgs& a, const Smem& sm, W
       if (ok) {
         const Geo q = geometry(hot, slot);
         int u = warp;
+        if constexpr (QUADS) {
+          for (; 2 * u < q.nu; u += MK_CW) run_quad(q.aux, q.gs, q.p0, q.p1, q.a0, q.a1, q.apitch16, u, q.kb0, sm, lane, t);
+        } else
         for (; u < q.nu; u += MK_CW)
           run_unit<ENC>(q.enc, q.aux, q.gs, q.p0, q.p1, q.a0, q.a1, q.apitch16, u, q.kb0, sm, lane, t);
       }
@@ -1107,14 +1172,15 @@ __device__ __forceinline__ void run_phase(const MegaArgs& a, const Smem& sm, Wal
                                           const StageSrc& src, const void* nw, int nw_type, int n_in, int layout_enc,
                                           float* res, int hid_lo, int tid, int lane, int warp, Prof& prof) {
   const unsigned word = sm.phase_rounds[phase_index];
-  const int nr = (int)(word & 0xffu), enc = (int)(word >> 8);
+  const bool quads = (word >> 8) != 0xffu && ((word >> 8) & MEGA_QUADS);
+  const int nr = (int)(word & 0xffu), enc = quads ? (int)(word >> 8) & ~MEGA_QUADS : (int)(word >> 8);
   if (nr == 0) return;
   const unsigned long long ts = prof.tic();
   const float* ssq = nullptr;
   if (MK_OPT_LOCAL && (enc == E_Q4_0 || enc == E_Q4_1 || enc == E_Q8_0 || enc == E_MLX_U4)) {
     float* mine = sm.misc + MK_OFF_RED + 32 + (w.nlocal & 1u) * MK_CW;  // consecutive per-warp stages alternate
     w.nlocal++;
-    stage_local(src, nw, nw_type, n_in, (enc == E_Q4_0 || enc == E_Q8_0 || enc == E_MLX_U4) ? 2 : 1, xl_for_encoding(enc), sm, mine + warp,
+    stage_local(src, nw, nw_type, n_in, quads ? 4 : (enc == E_Q4_0 || enc == E_Q8_0 || enc == E_MLX_U4) ? 2 : 1, xl_for_encoding(enc), sm, mine + warp,
                 lane, warp);
     if (nw) ssq = mine;
   } else {
@@ -1125,17 +1191,19 @@ __device__ __forceinline__ void run_phase(const MegaArgs& a, const Smem& sm, Wal
   prof.toc(9, ts);
   const int sid = (phase_index & 3) == 0 ? 0 : 2 + 3 * (phase_index & 3);  // 0, 5, 8, 11
   prof.stamp(sid);
-  if (enc == E_Q4_0)
-    run_phase_t<E_Q4_0>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
+  if (quads)
+    run_phase_t<E_MLX_U4, true>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
+  else if (enc == E_Q4_0)
+    run_phase_t<E_Q4_0, false>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
 #if !defined(MK_SIZE_PROBE) || MK_SIZE_PROBE < 2
   else if (enc == E_Q6_K)
-    run_phase_t<E_Q6_K>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
+    run_phase_t<E_Q6_K, false>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
   else if (enc == E_MLX_U4)  // MLX models: every layer product is of this kind
-    run_phase_t<E_MLX_U4>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
+    run_phase_t<E_MLX_U4, false>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
 #endif
 #ifndef MK_SIZE_PROBE
   else
-    run_phase_t<-1>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
+    run_phase_t<-1, false>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
 #endif
 }
 
@@ -1160,6 +1228,9 @@ __device__ __forceinline__ void decode_mega_body(const MegaArgs& a) {
   sm.empty = sm.full + a.nslot;
   sm.prog_bar = sm.empty + a.nslot;
   uint8_t* prog_area = reinterpret_cast<uint8_t*>(sm.prog_bar + 2);
+  __shared__ uint4 s_zeros[4];
+  if (tid < 4) s_zeros[tid] = make_uint4(0, 0, 0, 0);
+  sm.zeros = s_zeros;
   sm.abort = &s_abort;
   if (tid == 0) {
     s_abort = 0;
@@ -1556,6 +1627,12 @@ static int64_t split4(int64_t n, int cta, int grid) { return 4 * ((n / 4) * cta 
 static int64_t split8(int64_t n, int cta, int grid) { return 8 * ((n / 8) * cta / grid); }
 // gate and up can share tiles when they are the same kind of matrix and 16-byte congruent
 static bool can_interleave(const WRef& g, const WRef& u, int I) {
+  if (g.enc == E_MLX_U4) {  // one matrix [gate; up]: words, scales and biases of up lie I rows behind those of gate
+    if (u.enc != g.enc || u.cols != g.cols || u.group != g.group || u.aux != g.aux || I % 8) return false;
+    const int64_t rb = g.cols / 2, arb = g.cols / g.group * (g.aux == E_F32 ? 4 : 2);
+    return u.data == g.data + I * rb && u.scales == g.scales + I * arb && u.biases == g.biases + I * arb && (I - 8) * rb % 16 == 0 &&
+           (I - 8) * arb % 16 == 0 && (I - 8) * rb / 16 < (1LL << 31);
+  }
   return (g.enc == E_Q4_0 || g.enc == E_Q4_1 || g.enc == E_Q8_0) && u.enc == g.enc && u.cols == g.cols && I % 8 == 0 &&
          ((u.data - g.data) - 8 * (int64_t)g.row_bytes()) % 16 == 0 &&
          std::llabs(((u.data - g.data) - 8 * (int64_t)g.row_bytes()) / 16) < (1LL << 31);
@@ -1657,9 +1734,14 @@ int mega_build_program(const MegaBuildLayer* layers, const MegaLayer* full, int 
     size_t ci = 0, ri = 0;
     for (size_t ph = 0; ph < pc.phase_rounds.size(); ph++) {
       int enc = -1;
+      bool quads = true;  // the phase's chunks are whole runs of four blocks
       for (int r = 0; r < pc.phase_rounds[ph]; r++, ri++)
-        for (int k = 0; k < pc.rounds[ri].nchunks; k++, ci++)
-          enc = enc == -1 ? pc.chunks[ci].enc : (enc == pc.chunks[ci].enc ? enc : 0xff);
+        for (int k = 0; k < pc.rounds[ri].nchunks; k++, ci++) {
+          const MegaChunk& c = pc.chunks[ci];
+          enc = enc == -1 ? c.enc : (enc == c.enc ? enc : 0xff);
+          quads = quads && c.enc == E_MLX_U4 && c.al == 0 && c.al_step == 0 && c.nu % 2 == 0 && c.kb0 % (4 * MK_CW) == 0;
+        }
+      if (enc >= 0 && enc != 0xff && quads) enc |= MEGA_QUADS;
       words[ph] = (uint16_t)(pc.phase_rounds[ph] | ((enc < 0 ? 0xff : enc) << 8));
     }
     memcpy(b + lay->off_phase, words.data(), words.size() * 2);

@@ -61,6 +61,7 @@ static_assert(sizeof(MegaTile) == 8, "MegaTile must stay 8 bytes");
 // A round: chunks whose sums are held in registers (at most MEGA_TA accumulators), then ONE
 // cross-warp reduction and the epilogues of its tiles.
 constexpr int MEGA_TA = 8;
+constexpr int MEGA_QUADS = 0x40;  // in a phase word's encoding: chunks are worked on four blocks at a time
 struct MegaRound {
   uint16_t nchunks;
   uint8_t ntiles;
