@@ -341,7 +341,7 @@ int64_t dqgemm_tc_padded_rows(const WRef& w, int64_t M);
 bool gemm_skinny_takes(const WRef& w, int64_t M);
 bool gemm_skinny_prefers(const WRef& w, int64_t M, bool chain);  // chain: inside a layer's chain of fused products
 int gemm_skinny_terms(const WRef& w, int64_t M);
-// The dequant GEMM of 33..64 activation rows with K split over a cluster (gemm_cluster.cu). Activations: f16 rows in natural
+// The dequant GEMM of 33..128 activation rows with K split over a cluster (gemm_cluster.cu). Activations: f16 rows in natural
 // order, gemm_cluster_rows(M) of them allocated, scaled by a power of two per row, with the inverse scales beside them.
 bool gemm_cluster_prefers(const WRef& w, int64_t M, bool swiglu);
 int64_t gemm_cluster_rows(int64_t M);

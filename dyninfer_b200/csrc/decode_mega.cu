@@ -1191,15 +1191,13 @@ __device__ __forceinline__ void run_phase(const MegaArgs& a, const Smem& sm, Wal
   prof.toc(9, ts);
   const int sid = (phase_index & 3) == 0 ? 0 : 2 + 3 * (phase_index & 3);  // 0, 5, 8, 11
   prof.stamp(sid);
-  if (quads)
+  if (quads)  // MLX models: every layer product is of this kind
     run_phase_t<E_MLX_U4, true>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
   else if (enc == E_Q4_0)
     run_phase_t<E_Q4_0, false>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
 #if !defined(MK_SIZE_PROBE) || MK_SIZE_PROBE < 2
   else if (enc == E_Q6_K)
     run_phase_t<E_Q6_K, false>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
-  else if (enc == E_MLX_U4)  // MLX models: every layer product is of this kind
-    run_phase_t<E_MLX_U4, false>(a, sm, w, nr, ep, ssq, n_in, res, hid_lo, tid, lane, warp, prof, sid);
 #endif
 #ifndef MK_SIZE_PROBE
   else

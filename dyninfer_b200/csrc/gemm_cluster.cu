@@ -1,4 +1,4 @@
-// Dequant GEMM of 33 to 64 activation rows on the 5th-generation tensor cores, K split over a cluster:
+// Dequant GEMM of 33 to 128 activation rows on the 5th-generation tensor cores, K split over a cluster:
 // y[m, n] = sum_k x[m, k] * w[n, k], f32 accumulation, the residual or SwiGLU behind it, one launch.
 //
 // A product of a few dozen rows with a layer's matrix of a small model is over in a few microseconds; what it costs is the
@@ -13,6 +13,7 @@
 //   * SwiGLU: a tile is 64 rows of gate and the same 64 of up, so both sums of an output are in one CTA.
 // All waits are bounded; one that runs out sets the device error word.
 #include <algorithm>
+#include <atomic>
 
 #include "raw_box.cuh"
 #include "tensor_map.cuh"
@@ -25,8 +26,8 @@ constexpr int GC_CONV = 16;  // conversion warps: lane quarter = warp % 4, quart
 constexpr int GC_MMA_WARP = GC_CONV;
 constexpr int GC_THREADS = (GC_CONV + 1) * 32;
 constexpr int GC_MAX_UPC = 3;      // units of A operands in tensor memory (128 columns each) behind the accumulator
-constexpr int GC_ACC_COLS = 64;
-constexpr int GC_SMEM = 220 * 1024;
+constexpr int GC_MAX_BN = 128;
+constexpr int GC_SMEM = 222 * 1024;
 
 struct GcArgs {
   WRef w;
@@ -35,7 +36,7 @@ struct GcArgs {
   float* y;               // [M, N]
   int* error;
   int64_t N;              // columns of y (SwiGLU: rows of gate = rows of up)
-  int M, bn, nunits, upc, CK, slice, tmem_cols, swiglu;
+  int M, bn, nunits, upc, CK, slice, nx, acc_cols, tmem_cols, swiglu;
 };
 
 __device__ __forceinline__ void gc_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
@@ -62,10 +63,10 @@ __global__ void __launch_bounds__(GC_THREADS, 2)
 gemm_cluster_kernel(const GcArgs a, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap) {
   constexpr uint32_t RAW_BYTES = TG_BM * gs_words(ENC) * 4;
   extern __shared__ __align__(1024) uint8_t gc_smem[];
-  __shared__ uint64_t raw_full[GC_MAX_UPC], a_full, x_full, acc_full;
+  __shared__ uint64_t raw_full[GC_MAX_UPC], a_full, x_full[GC_MAX_UPC], x_free[GC_MAX_UPC], acc_full;
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_abort;
-  __shared__ uint32_t s_dst[64];  // where row m is finished: its first sum of this CTA's part
+  __shared__ uint32_t s_dst[GC_MAX_BN];  // where row m is finished: its first sum of this CTA's part
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int bn = a.bn, CK = a.CK, M = a.M, slice = a.slice;
   const int rank = (int)(blockIdx.x % (unsigned)CK);
@@ -74,15 +75,15 @@ gemm_cluster_kernel(const GcArgs a, const __grid_constant__ CUtensorMap wmap, co
   const int64_t n0 = tile * (a.swiglu ? 64 : TG_BM);            // first column of y
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gc_smem) + 1023) & ~uintptr_t(1023));
   const uint32_t xb = (uint32_t)bn * 128;                       // bytes of a 64-wide chunk of x
-  uint8_t* const xs = smem;                                     // operand: [unit][chunk][row][128 bytes, swizzled]
+  uint8_t* const xs = smem;                                     // operand: [stage][chunk][row][128 bytes, swizzled]
   // one region in turn: raw weights [unit]; the cluster's sums [rank][row of the slice][128]
-  uint8_t* const raw = smem + (size_t)a.upc * 4 * xb;
+  uint8_t* const raw = smem + (size_t)a.nx * 4 * xb;
   float* const red = reinterpret_cast<float*>(raw);
 
   if (tid == GC_MMA_WARP * 32) {
     s_abort = 0;
-    for (int i = 0; i < GC_MAX_UPC; i++) mbar_init(raw_full + i, 1);
-    mbar_init(&a_full, GC_CONV), mbar_init(&x_full, 1), mbar_init(&acc_full, 1);
+    for (int i = 0; i < GC_MAX_UPC; i++) mbar_init(raw_full + i, 1), mbar_init(x_full + i, 1), mbar_init(x_free + i, 1);
+    mbar_init(&a_full, GC_CONV), mbar_init(&acc_full, 1);
     mbar_fence_init();
     // weights are not produced by the kernels before: they are asked for at once
     for (int u = 0; u < nu; u++) {
@@ -135,7 +136,7 @@ gemm_cluster_kernel(const GcArgs a, const __grid_constant__ CUtensorMap wmap, co
       r.load(raw + (size_t)u * RAW_BYTES, row, g);
       r.align();
       uint32_t out[16];
-      const uint32_t taddr = tlane + GC_ACC_COLS + (uint32_t)(4 * u + g) * 32u;
+      const uint32_t taddr = tlane + (uint32_t)a.acc_cols + (uint32_t)(4 * u + g) * 32u;
       r.half(0, out);
       tmem_st16(taddr, out);
       r.half(1, out);
@@ -148,30 +149,46 @@ gemm_cluster_kernel(const GcArgs a, const __grid_constant__ CUtensorMap wmap, co
     pdl_wait();  // inverse scales, residual; y may still be read by the kernels before
   } else {
     // ---- MMA issue ----------------------------------------------------------------------------------------------------------
+    auto ask = [&](int u, int stage) {  // the activations of a unit
+      mbar_expect_tx(x_full + stage, 4 * xb);
+#pragma unroll 1
+      for (int c = 0; c < 4; c++) tma_box_g2s(xs + (size_t)(stage * 4 + c) * xb, &xmap, ((k0 + u) * 4 + c) * (TG_BK / 2), 0, x_full + stage);
+    };
     if (lane == 0) {
       pdl_wait_then_trigger();
-      mbar_expect_tx(&x_full, (unsigned)nu * 4 * xb);
-#pragma unroll 1
-      for (int c = 0; c < 4 * nu; c++) tma_box_g2s(xs + (size_t)c * xb, &xmap, (k0 * 4 + c) * (TG_BK / 2), 0, &x_full);
+      for (int u = 0; u < min(nu, a.nx); u++) ask(u, u);
     }
     __syncwarp();
     const uint32_t idesc = umma_idesc(bn);
-    const uint64_t dchunk = xb >> 4;
-    uint64_t desc = umma_desc(smem_u32(xs));
-    const bool ok = mbar_wait_bounded(&a_full, 0, TG_SPINS, &s_abort) && mbar_wait_bounded(&x_full, 0, TG_SPINS, &s_abort);
-    if (!ok && !s_abort) s_abort = 7;
-    tc_fence_after();
-    if (elect_one()) {
-      if (ok) {
-        uint32_t acol = tmem + GC_ACC_COLS;
+    const uint64_t dchunk = xb >> 4, desc0 = umma_desc(smem_u32(xs));
+    bool ok = mbar_wait_bounded(&a_full, 0, TG_SPINS, &s_abort);
+    int stage = 0;
+    unsigned phase = 0;
 #pragma unroll 1
-        for (int c = 0; c < 4 * nu; c++, acol += 32u, desc += dchunk) {
+    for (int u = 0; u < nu && ok; u++) {
+      ok = mbar_wait_bounded(x_full + stage, phase, TG_SPINS, &s_abort);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
+        uint32_t acol = tmem + (uint32_t)(a.acc_cols + 128 * u);
+        uint64_t desc = desc0 + dchunk * (4 * stage);
+#pragma unroll 1
+        for (int c = 0; c < 4; c++, acol += 32u, desc += dchunk) {
 #pragma unroll
-          for (int k4 = 0; k4 < TG_BK / 16; k4++) umma_f16_ts(tmem, acol + 8u * k4, desc + 2 * k4, idesc, (c | k4) ? 1u : 0u);
+          for (int k4 = 0; k4 < TG_BK / 16; k4++) umma_f16_ts(tmem, acol + 8u * k4, desc + 2 * k4, idesc, (u | c | k4) ? 1u : 0u);
         }
+        umma_commit(x_free + stage);
       }
-      umma_commit(&acc_full);
+      __syncwarp();
+      if (u + a.nx < nu) {  // the stage's next unit, when the MMAs have read it
+        ok = mbar_wait_bounded(x_free + stage, phase, TG_SPINS, &s_abort);
+        if (ok && elect_one()) ask(u + a.nx, stage);
+        __syncwarp();
+      }
+      if (++stage == a.nx) stage = 0, phase ^= 1u;
     }
+    if (!ok && !s_abort) s_abort = 7;
+    if (elect_one()) umma_commit(&acc_full);
     __syncwarp();
   }
   // this warp has used up its raw weights: when every warp has, the cluster's sums may take their place (awaited before the first write)
@@ -249,12 +266,38 @@ gemm_cluster_kernel(const GcArgs a, const __grid_constant__ CUtensorMap wmap, co
 }
 
 struct GcPlan {
-  int bn, CK, upc, nunits, slice;
+  int bn, CK, upc, nunits, slice, nx;
   int64_t tiles;
   size_t smem;
 };
+// CTAs in clusters of `ck` that the device holds at a time, one per SM: GPCs differ in size, and a cluster does not span two.
+int gc_places(int ck) {
+  static std::atomic<int> kept[16][9];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::atomic<int>* const slot = dev < 16 ? &kept[dev][ck] : nullptr;
+  int n = slot ? slot->load(std::memory_order_relaxed) : 0;
+  if (n) return n;
+  const void* kernel = reinterpret_cast<const void*>(gemm_cluster_kernel<E_Q4_0>);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(ck * 64)), cfg.blockDim = dim3(GC_THREADS), cfg.dynamicSmemBytes = 116 * 1024;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)ck, attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr, cfg.numAttrs = 1;
+  int clusters = 0;
+  if (ensure_dynamic_smem(kernel, GC_SMEM) || cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    clusters = sm_count() * 3 / 4 / ck;
+  }
+  n = std::max(1, clusters * ck);
+  if (slot) slot->store(n, std::memory_order_relaxed);
+  return n;
+}
 // K is split as far as one CTA per SM allows (two of a product on an SM take almost twice as long), with an eighth of the SMs left
-// over because clusters do not fill every GPC (6144 x 1280 in 144 CTAs of three: 16.2 us, 64 rows, against 12.8 on mma.sync).
+// over because clusters do not fill every GPC (6144 x 1280 in 144 CTAs of three: 16.2 us, 64 rows, against 12.8 on mma.sync). With more
+// than 64 rows, whose CTAs have an SM each, what does not fit at once costs a whole second round (2048 x 2048, 100 rows, in 16
+// clusters of eight 15.3 us).
 bool gc_plan(const WRef& w, int64_t M, bool swiglu, GcPlan* p) {
   p->bn = (int)((M + 15) / 16 * 16);
   p->nunits = (int)(w.cols / GS_UNIT);
@@ -264,16 +307,21 @@ bool gc_plan(const WRef& w, int64_t M, bool swiglu, GcPlan* p) {
   for (int ck = 1; ck <= 8; ck++) {
     const int upc = (p->nunits + ck - 1) / ck;
     if (8 * p->tiles * ck > 7 * sms || upc > GC_MAX_UPC || (ck - 1) * upc >= p->nunits) continue;
+    if (M > 64 && p->tiles * ck > gc_places(ck)) continue;
     p->CK = ck, p->upc = upc;
   }
   if (!p->CK) return false;
   p->slice = (int)((M + p->CK - 1) / p->CK);  // rows of y that a CTA finishes
-  p->smem = 1024 + (size_t)p->upc * p->bn * 512 +
-            std::max((size_t)p->upc * TG_BM * gs_words(w.enc) * 4, (size_t)p->CK * p->slice * TG_BM * 4);
+  for (p->nx = p->upc; p->nx >= 1; p->nx--) {  // units of activations at a time
+    p->smem = 1024 + (size_t)p->nx * p->bn * 512 +
+              std::max((size_t)p->upc * TG_BM * gs_words(w.enc) * 4, (size_t)p->CK * p->slice * TG_BM * 4);
+    if (p->smem <= (size_t)GC_SMEM) break;
+  }
+  if (!p->nx) return false;
   // Several units take all of an SM's tensor memory: two such CTAs of one cluster on an SM would wait for one another, so
   // their shared memory does not let them.
-  if (p->upc > 1) p->smem = std::max<size_t>(p->smem, 116 * 1024);
-  return p->smem <= (size_t)GC_SMEM;
+  if (p->upc > 1 || p->bn > 64) p->smem = std::max<size_t>(p->smem, 116 * 1024);
+  return true;
 }
 
 template <int ENC>
@@ -303,11 +351,13 @@ int gc_launch(const GcArgs& a, const CUtensorMap& wmap, const CUtensorMap& xmap,
 
 // Where the kernel is ahead of gemm_skinny.cu among the products that one takes: more rows than 32 (with up to 32 the activations that
 // every CTA of that kernel reads weigh less: 1024 x 2048 Q4_0, activation pass included, 24 rows 6.6 there and 6.9 us here, 37
-// rows 8.2 and 7.0, 64 rows 9.7 and 7.4), and a K that four CTAs share, or two with a third of the SMs to spare (6144 x 1024, 64
+// rows 8.2 and 7.0, 64 rows 9.7 and 7.4; 65 rows, against the kernels behind that one, 13.1 and 7.8, 128 rows 13.5 and 9.8; a
+// second tile of 128 rows is slower than they are), and a K that four CTAs share, or two with a third of the SMs to spare (6144 x 1024, 64
 // rows 12.4 and 8.7; 12288 x 512 in whole tiles 11.6 and 12.9, 8192 x 768 Q8_0 in 128 CTAs 11.5 and 11.8).
 bool gemm_cluster_prefers(const WRef& w, int64_t M, bool swiglu) {
   GcPlan p;
-  if (M <= 32 || M > 64 || !gemm_stream_takes(w) || w.rows > (1 << 30) || (swiglu && w.rows % 2) || !gc_plan(w, M, swiglu, &p)) return false;
+  if (M <= 32 || M > GC_MAX_BN || !gemm_stream_takes(w) || w.rows > (1 << 30) || (swiglu && w.rows % 2) || !gc_plan(w, M, swiglu, &p)) return false;
+  if (M > 64) return !swiglu && p.CK >= 2 && w.cols >= 1536 && p.tiles <= 20;
   return p.CK >= 4 || (p.CK >= 2 && p.upc <= 2 && 3 * p.tiles * p.CK <= 2 * sm_count());
 }
 
@@ -324,9 +374,10 @@ int launch_gemm_cluster(const WRef& w, const __half* x, const float* x_inv, int6
   a.w = w, a.inv_s = x_inv;
   a.residual = residual, a.y = y, a.error = device_error_word();
   if (!a.error) return 1;
-  a.N = swiglu ? w.rows / 2 : w.rows, a.M = (int)M, a.bn = p.bn, a.nunits = p.nunits, a.upc = p.upc, a.CK = p.CK, a.slice = p.slice;
+  a.N = swiglu ? w.rows / 2 : w.rows, a.M = (int)M, a.bn = p.bn, a.nunits = p.nunits, a.upc = p.upc, a.CK = p.CK, a.slice = p.slice, a.nx = p.nx;
   a.swiglu = swiglu ? 1 : 0;
-  a.tmem_cols = GC_ACC_COLS + 128 * p.upc <= 256 ? 256 : 512;
+  a.acc_cols = p.bn <= 64 ? 64 : 128;
+  a.tmem_cols = a.acc_cols + 128 * p.upc <= 256 ? 256 : 512;
   CUtensorMap wmap, xmap;
   if (make_row_box_map(w.data, w.enc == E_MLX_U4 ? (size_t)w.cols / 2 : (size_t)w.row_bytes(), w.rows, gs_words(w.enc), swiglu ? 64 : TG_BM,
                        &wmap, w.enc == E_MLX_U4) ||

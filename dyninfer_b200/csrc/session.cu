@@ -454,6 +454,7 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
     aa.uniform_base = chunk_start, aa.uniform_seq = chunk_slot;  // a prefill chunk: consecutive positions
     return aa;
   };
+  auto clustered = [&](const WRef& w) { return gemm_cluster_prefers(w, rows, false) && gemm_cluster_rows(rows) <= s->xh_rows && w.cols <= s->xh_cols; };
   bool xh_ready = false;  // xh already holds this layer's normalised rows (written by the layer before)
   auto gemm = [&](const WRef& w, const float* x, bool prepared, float* y, const float* residual, TgIo* io) -> int {
     TgIo local;
@@ -545,7 +546,13 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       // o: hidden += W ctx, then the FFN norm straight into the GEMM's operand
       TgIo io_o;
       io_o.partial = s->gpart, io_o.partial_bytes = s->gpart_bytes;
-      if (gemm(L.o, s->ctx, false, s->hidden, s->hidden, &io_o)) return 1;
+      if (clustered(L.o)) {
+        if (launch_skinny_prepare(L.o, s->ctx, E_F32, rows, s->xh, s->xinv, st, true) ||
+            launch_gemm_cluster(L.o, s->xh, s->xinv, rows, s->hidden, s->hidden, false, st))
+          return 1;
+      } else if (gemm(L.o, s->ctx, false, s->hidden, s->hidden, &io_o)) {
+        return 1;
+      }
       if (io_o.splits > 1 ? launch_norm_prepare(nullptr, s->gpart, io_o.splits, s->hidden, s->hidden, L.ffn_norm.ptr,
                                                 L.ffn_norm.type, rows, H, c.eps, s->xh, s->xinv, st)
                           : launch_norm_prepare(s->hidden, nullptr, 0, nullptr, nullptr, L.ffn_norm.ptr, L.ffn_norm.type, rows,
@@ -565,7 +572,11 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
       // down: hidden += W act; with another layer to come, its attention norm rides on the addition
       TgIo io_d;
       if (l + 1 < c.layers) io_d.partial = s->gpart, io_d.partial_bytes = s->gpart_bytes;
-      if (gemm(L.down, act_prepared ? nullptr : s->act, act_prepared, s->hidden, s->hidden, &io_d)) return 1;
+      if (act_prepared && clustered(L.down)) {
+        if (launch_gemm_cluster(L.down, s->xh, s->xinv, rows, s->hidden, s->hidden, false, st)) return 1;
+      } else if (gemm(L.down, act_prepared ? nullptr : s->act, act_prepared, s->hidden, s->hidden, &io_d)) {
+        return 1;
+      }
       if (io_d.splits > 1) {
         const NormW& nw = s->layers[l + 1].attn_norm;
         if (launch_norm_prepare(nullptr, s->gpart, io_d.splits, s->hidden, s->hidden, nw.ptr, nw.type, rows, H, c.eps, s->xh,

@@ -305,9 +305,10 @@ def test_attention_prefill_at_the_edges_of_blocks(native_lib, dtype, s, start, n
 
 @pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q4_1", "gguf.q8_0", "gguf.q4_k", "mlx.affine.u4"])
 @pytest.mark.parametrize("m,n,k", [(33, 130, 256), (48, 127, 768), (49, 1000, 2560), (64, 257, 3072), (47, 2049, 1792),
-                                   (64, 6000, 1024), (40, 128, 6144), (64, 129, 6400)])
+                                   (64, 6000, 1024), (40, 128, 6144), (64, 129, 6400), (65, 1024, 2048), (128, 257, 1536),
+                                   (100, 2048, 2048), (127, 1000, 3072)])
 def test_linear_rows_over_a_cluster(native_lib, oracle, enc, m, n, k):
-    """33 to 64 rows, K over clusters of two to eight blocks with one to three units each (and sizes beyond): ragged
+    """33 to 128 rows, K over clusters of two to eight blocks with one to three units each (and sizes beyond): ragged
     tiles and row groups, a last block with fewer units, odd row counts per finishing block. Both operands are rounded to
     2^-12 of a value; over k products the error of a sum, relative to its size, is about 2^-12 * sqrt(2 / 3) = 2.0e-4 (rounding
     errors are uniform), so 4e-4 over all outputs holds with room."""
@@ -446,6 +447,23 @@ def test_persistent_attention_slices_against_the_oracle(native_lib, oracle, tmp_
             lg = (s.prefill([t]) if i == 0 else s.decode(t)).values
             if i in want:
                 assert np.abs(lg - want[i]).max() <= 1e-2 and helpers.cosine(lg, want[i]) >= 0.9999, i
+
+
+@pytest.mark.parametrize("hidden,inter,group", [(1024, 1536, 64), (1024, 1536, 32), (1024, 1536, 128), (1536, 2304, 64),
+                                                (512, 768, 32), (512, 4096, 64), (2048, 256, 128)])
+def test_persistent_mlx_widths_and_groups(native_lib, tmp_path, hidden, inter, group):
+    """One slice of K and several, shares of two to sixteen blocks per warp, every group size, gate and up rows in one tile: the
+    persistent kernel against the operator path (both keep f32 rows to 22 bits)."""
+    cfg = dict(synth.SMALL_D64, hidden=hidden, intermediate=inter, vocab=512)
+    path = synth.write_qwen3_mlx(str(tmp_path / "mlx"), cfg, seed=9, group=group)
+    got = []
+    for kernel in ("persistent", "graph"):
+        model = ModelLoader().load(path, max_kv=64, kv_dtype="f32", chunk_size=64, decode_kernel=kernel)
+        with model.create_session(SessionConfig(max_sequence_length=64)) as s:
+            assert s.uses_persistent_kernel() == (kernel == "persistent")
+            s.prefill([3])
+            got.append(np.stack([s.decode(t).values.copy() for t in (7, 11, 400)]))
+    assert np.abs(got[0] - got[1]).max() <= 1e-4 * np.abs(got[1]).max()
 
 
 @pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q8_0"])
