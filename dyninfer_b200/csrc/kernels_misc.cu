@@ -702,8 +702,12 @@ static int run_qkv_prepare(const QkvPrepArgs& a, const FreqTable& ft, cudaStream
                      !((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v) |
                         reinterpret_cast<uintptr_t>(a.dq.partial) | reinterpret_cast<uintptr_t>(a.dk.partial) |
                         reinterpret_cast<uintptr_t>(a.dv.partial)) & 7);
-  // many rows: two blocks per row, a warp taking several heads
-  const dim3 warps((unsigned)a.rows, a.rows >= 128 ? std::min(2u, (heads + 7) / 8) : (heads + 7) / 8);
+  // Many rows: fewer blocks per row, a warp taking several heads, so that the row's rotation is evaluated by fewer
+  // warps: two blocks while they all fit the SMs at once (four of these blocks to an SM), one beyond. A 2048-token
+  // prompt in chunks of 512 rows of 32 heads: two blocks 12.41 ms, one 12.20; two heads of a warp at a time (their
+  // loads in flight together) needs more than the 64 registers of four blocks per SM and takes 12.66 and 12.33.
+  const unsigned per_row = a.rows > 2 * sm_count() ? 1 : a.rows >= 128 ? 2 : heads;
+  const dim3 warps((unsigned)a.rows, std::min(per_row, (heads + 7) / 8));
   if (a.d == 128 && pairs)
     DYN_CUDA(launch_pdl(qkv_prepare_warp_kernel<KV, 128>, warps, dim3(256), 0, s, a, ft));
   else if (a.d == 64)

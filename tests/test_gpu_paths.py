@@ -414,6 +414,21 @@ def test_decode_attention_prepares_its_own_rows(native_lib, oracle, tmp_path, kv
                     assert np.abs(logits[b] - want[b][i]).max() <= 1e-3, (i, b)
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("rows", [127, 128, 296, 297, 593])
+def test_prompt_rows_prepared_by_fewer_blocks(native_lib, oracle, tmp_path, rows, d):
+    """Prompts of one chunk whose rows are prepared for the attention by a block per eight heads, two blocks, one block, and
+    more blocks than fit at once; 20 heads, so the last warps of a block have fewer. f16 operands of the products: 1e-2."""
+    cfg = dict(synth.TINY, layers=1, heads=12, kv_heads=4, head_dim=d, hidden=512)
+    path = synth.write_qwen3_gguf(str(tmp_path / "q.gguf"), cfg, seed=23)
+    prompt = np.random.default_rng(rows).integers(0, cfg["vocab"], size=rows).tolist()
+    want = one_by_one(oracle, path, prompt, [rows - 1], "bf16")[rows - 1]
+    model = ModelLoader().load(path, max_kv=1024, kv_dtype="bf16", chunk_size=1024)
+    with model.create_session(SessionConfig(max_sequence_length=1024)) as s:
+        got = s.prefill(prompt).values
+    assert np.abs(got - want).max() <= 1e-2 and helpers.cosine(got, want) >= 0.9999
+
+
 @pytest.mark.parametrize("kv", ["bf16", "f16"])
 @pytest.mark.parametrize("slots", [8, 40])
 def test_batched_decode_attention_at_the_ends_of_slices(native_lib, oracle, tmp_path, kv, slots):
