@@ -384,7 +384,8 @@ int enqueue_forward(Session* s, int64_t rows, int64_t logits_row, bool all_rows 
   // kernels in front of it (norm, attention merge), the residuals and the SwiGLU applied behind it: ten launches
   // per layer, each a programmatic dependent of the one before, so that weights stream while it drains. (0.6B
   // MLX-U4, 8 sequences at context 512: 3.2 ms per step on the tcgen05 GEMM with its activation passes and
-  // K-split reductions.) Four rows and fewer stay on the kernels that carry 22 bits of an activation.
+  // K-split reductions.) Above 32 rows each product may go to the GEMM over a cluster instead,
+  // whose operand is the same rows in natural order. Four rows and fewer stay on the kernels that carry 22 bits of an activation.
   auto frag_class = [](int enc) { return enc == E_Q4_1 ? (int)E_Q4_0 : enc; };
   bool skinny = rows > 4 && rows <= 64 && !tp && s->sk_x && H % 256 == 0 && H <= 8192 && c.inter % 32 == 0;
   for (int l = 0; l < c.layers && skinny; l++) {
