@@ -11,10 +11,12 @@
 //   * The sums meet through distributed shared memory: every CTA writes its accumulator into the CTA of the cluster that
 //     finishes the rows; one cluster barrier; then the parts are added in the order of K, scaled back and stored.
 //   * SwiGLU: a tile is 64 rows of gate and the same 64 of up, so both sums of an output are in one CTA.
-// All waits are bounded; one that runs out sets the device error word.
+// Waits for copies and products are bounded; one that runs out sets the device error word. The allocation of tensor memory and the
+// cluster barriers have no bound: gemm_cluster_plan.h says why they end.
 #include <algorithm>
 #include <atomic>
 
+#include "gemm_cluster_plan.h"
 #include "raw_box.cuh"
 #include "tensor_map.cuh"
 
@@ -25,9 +27,7 @@ namespace {
 constexpr int GC_CONV = 16;  // conversion warps: lane quarter = warp % 4, quarter of the box = warp / 4
 constexpr int GC_MMA_WARP = GC_CONV;
 constexpr int GC_THREADS = (GC_CONV + 1) * 32;
-constexpr int GC_MAX_UPC = 3;      // units of A operands in tensor memory (128 columns each) behind the accumulator
-constexpr int GC_MAX_BN = 128;
-constexpr int GC_SMEM = 222 * 1024;
+static_assert(GC_TILE == TG_BM && GC_UNIT == GS_UNIT, "the plan's tile is the kernel's");
 
 struct GcArgs {
   WRef w;
@@ -265,11 +265,6 @@ gemm_cluster_kernel(const GcArgs a, const __grid_constant__ CUtensorMap wmap, co
   if (tid == 0 && s_abort) report_wait_expired(a.error, DEV_ERR_GEMM_PIPE);
 }
 
-struct GcPlan {
-  int bn, CK, upc, nunits, slice, nx;
-  int64_t tiles;
-  size_t smem;
-};
 // CTAs in clusters of `ck` that the device holds at a time, one per SM: GPCs differ in size, and a cluster does not span two.
 int gc_places(int ck) {
   static std::atomic<int> kept[16][9];
@@ -280,7 +275,7 @@ int gc_places(int ck) {
   if (n) return n;
   const void* kernel = reinterpret_cast<const void*>(gemm_cluster_kernel<E_Q4_0>);
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(ck * 64)), cfg.blockDim = dim3(GC_THREADS), cfg.dynamicSmemBytes = 116 * 1024;
+  cfg.gridDim = dim3((unsigned)(ck * 64)), cfg.blockDim = dim3(GC_THREADS), cfg.dynamicSmemBytes = GC_SMEM_OWN;
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = (unsigned)ck, attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
@@ -294,34 +289,8 @@ int gc_places(int ck) {
   if (slot) slot->store(n, std::memory_order_relaxed);
   return n;
 }
-// K is split as far as one CTA per SM allows (two of a product on an SM take almost twice as long), with an eighth of the SMs left
-// over because clusters do not fill every GPC (6144 x 1280 in 144 CTAs of three: 16.2 us, 64 rows, against 12.8 on mma.sync). With more
-// than 64 rows, whose CTAs have an SM each, what does not fit at once costs a whole second round (2048 x 2048, 100 rows, in 16
-// clusters of eight 15.3 us).
 bool gc_plan(const WRef& w, int64_t M, bool swiglu, GcPlan* p) {
-  p->bn = (int)((M + 15) / 16 * 16);
-  p->nunits = (int)(w.cols / GS_UNIT);
-  p->tiles = swiglu ? (w.rows / 2 + 63) / 64 : (w.rows + TG_BM - 1) / TG_BM;
-  const int64_t sms = std::max(1, sm_count());
-  p->CK = 0;
-  for (int ck = 1; ck <= 8; ck++) {
-    const int upc = (p->nunits + ck - 1) / ck;
-    if (8 * p->tiles * ck > 7 * sms || upc > GC_MAX_UPC || (ck - 1) * upc >= p->nunits) continue;
-    if (M > 64 && p->tiles * ck > gc_places(ck)) continue;
-    p->CK = ck, p->upc = upc;
-  }
-  if (!p->CK) return false;
-  p->slice = (int)((M + p->CK - 1) / p->CK);  // rows of y that a CTA finishes
-  for (p->nx = p->upc; p->nx >= 1; p->nx--) {  // units of activations at a time
-    p->smem = 1024 + (size_t)p->nx * p->bn * 512 +
-              std::max((size_t)p->upc * TG_BM * gs_words(w.enc) * 4, (size_t)p->CK * p->slice * TG_BM * 4);
-    if (p->smem <= (size_t)GC_SMEM) break;
-  }
-  if (!p->nx) return false;
-  // Several units take all of an SM's tensor memory: two such CTAs of one cluster on an SM would wait for one another, so
-  // their shared memory does not let them.
-  if (p->upc > 1 || p->bn > 64) p->smem = std::max<size_t>(p->smem, 116 * 1024);
-  return true;
+  return gc_plan(w.rows, w.cols, gs_words(w.enc), M, swiglu, std::max(1, sm_count()), gc_places, p);
 }
 
 template <int ENC>
@@ -376,8 +345,7 @@ int launch_gemm_cluster(const WRef& w, const __half* x, const float* x_inv, int6
   if (!a.error) return 1;
   a.N = swiglu ? w.rows / 2 : w.rows, a.M = (int)M, a.bn = p.bn, a.nunits = p.nunits, a.upc = p.upc, a.CK = p.CK, a.slice = p.slice, a.nx = p.nx;
   a.swiglu = swiglu ? 1 : 0;
-  a.acc_cols = p.bn <= 64 ? 64 : 128;
-  a.tmem_cols = a.acc_cols + 128 * p.upc <= 256 ? 256 : 512;
+  a.acc_cols = p.acc_cols, a.tmem_cols = p.tmem_cols;
   CUtensorMap wmap, xmap;
   if (make_row_box_map(w.data, w.enc == E_MLX_U4 ? (size_t)w.cols / 2 : (size_t)w.row_bytes(), w.rows, gs_words(w.enc), swiglu ? 64 : TG_BM,
                        &wmap, w.enc == E_MLX_U4) ||
