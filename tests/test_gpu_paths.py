@@ -244,6 +244,35 @@ def test_attention_prefill_f32_cache_entries_that_are_not_finite(native_lib, pla
     assert not np.isfinite(got[at - start:, 2:, 5]).any()
 
 
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("s,start,nkv,lost", [(100, 20, 2, [(70, 5)]), (128, 0, 2, [(0, 64), (127, 127)]), (33, 0, 1, [(32, 0), (1, 3)]),
+                                              (300, 20, 2, [(31, 5), (32, 5), (190, 77), (319, 0)]), (128, 64, 80, [(65, 1), (130, 2), (191, 126)])])
+def test_attention_prefill_2_byte_cache_values_that_are_not_finite(native_lib, dtype, bad, s, start, nkv, lost):
+    """A value that is not finite reaches its dim of the rows that see its key, and nothing else: not the earlier rows of
+    the same block or tile, not the other dims. First and last keys of tiles and blocks, several in a tile, one and more blocks
+    per head; the keys behind the last row are not finite either. Bounds as at the edges of blocks below."""
+    from dyninfer_b200 import ops
+    d, cap, nh = 128, 1408, 2 * nkv
+    g = torch.Generator("cuda").manual_seed(s + start)
+    tt = torch.bfloat16 if dtype == "bf16" else torch.float16
+    q, k, v = (torch.randn(*shape, generator=g, device="cuda") for shape in ((s, nh, d), (nkv, cap, d), (nkv, cap, d)))
+    k, v = k.to(tt), v.to(tt)
+    n = start + s
+    scores = torch.einsum("shd,hkd->hsk", q.double(), k[:, :n].double().repeat_interleave(2, 0)) / d ** 0.5
+    hidden = torch.arange(n, device="cuda")[None, :] > torch.arange(s, device="cuda")[:, None] + start
+    want = scores.masked_fill(hidden, float("-inf")).softmax(-1) @ v[:, :n].double().repeat_interleave(2, 0)     # [nh, s, d]
+    touched = torch.zeros(nh, s, d, dtype=torch.bool, device="cuda")
+    largest = float(v[:, :n].abs().max())
+    v[:, n:] = bad
+    for key, dim in lost:
+        v[0, key, dim] = bad
+        touched[:2, max(0, key - start):, dim] = True
+    got = ops.attention(q, k, v, start).reshape(s, nh, d).double().transpose(0, 1)
+    assert torch.equal(~got.isfinite(), touched)
+    assert float((got - want)[~touched].abs().max()) < (1e-4 if dtype == "bf16" else 4e-6) * largest
+
+
 @pytest.mark.parametrize("hidden,inter", [(2048, 4608), (1024, 4608)])
 def test_few_row_steps_where_only_the_fused_matrix_is_large(native_lib, oracle, tmp_path, hidden, inter):
     """gate and up pass for the few-row GEMM one by one, [gate; up] as one matrix does not: prompts and batched steps of 17
