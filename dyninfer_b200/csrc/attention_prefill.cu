@@ -214,7 +214,7 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
   constexpr uint32_t Q_COL = 384;                   // hi in 64 columns, lo in 64; stream i: S at 192 i, U at 192 i + 64
   constexpr float LOWEST = -3.40282347e38f;
   extern __shared__ __align__(1024) uint8_t fa_smem[];
-  __shared__ uint64_t item_full[2][6], q_full[2], s_full[2], p_full[2], u_full[2], u_free[2];
+  __shared__ uint64_t item_full[2][6], q_full[2], s_full[2], p_full[2], u_full[2], u_free[2], started;
   __shared__ uint32_t tmem_base_s;
   __shared__ int s_abort;
   __shared__ float s_x[4][FA_BR];         // largest magnitude of a quarter of the dims
@@ -241,6 +241,7 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
       for (int j = 0; j < 6; j++) mbar_init(&item_full[i][j], 1);
       mbar_init(q_full + i, 1), mbar_init(s_full + i, 1), mbar_init(p_full + i, SPLIT ? 8 : 9), mbar_init(u_full + i, 1), mbar_init(u_free + i, 8);
     }
+    mbar_init(&started, 1);
     mbar_fence_init();
   }
   // Tensor memory is taken before this block lets the next kernel start, so that kernel cannot take it first and then wait for this one.
@@ -547,8 +548,8 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
     const uint32_t id_s = fa_idesc(FA_SPLIT_TILE, BF, false), id_u = fa_idesc(FA_D, BF, true);
     const uint64_t k_desc0 = umma_desc(smem_u32(items)), v_desc0 = fa_desc_mn(smem_u32(items));
     // the second stream starts half a tile later, so that the one's MMAs run under the other's softmax (in step, they would
-    // wait for the same units)
-    bool ok = !(stream && mine > 2) || mbar_wait_bounded(s_full, 0, TG_SPINS, &s_abort);
+    // wait for the same units). The barrier has this one phase: a warp that comes late finds it done whatever has gone on since.
+    bool ok = !(stream && mine > 2) || mbar_wait_bounded(&started, 0, TG_SPINS, &s_abort);
 #pragma unroll 1
     for (int i = 0; i < mine && ok; i++) {
       ok = mbar_wait_bounded(&item_full[stream][get_at], gphase, TG_SPINS, &s_abort) &&
@@ -568,6 +569,7 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
         for (int k = 0; k < 8; k++)
           umma_f16_ts(k < 4 ? s_col : u_col, q_hi + 8u * k, k_hi + (uint64_t)((k >> 2) * (FA_BOX >> 4) + 2 * (k & 3)), id_s, k ? 1u : 0u);
         umma_commit(s_full + stream);
+        if (!stream && i == 0) umma_commit(&started);
       }
       __syncwarp();
       if (i) ask();  // in place of the values of tile i - 1
