@@ -700,7 +700,16 @@ int launch_attention_prefill(const AttnArgs& a, int64_t base_pos, int64_t seq, c
   const int64_t pairs = a.nh * ((a.rows + FA_BR - 1) / FA_BR), tiles = (base_pos + a.rows + FA_SPLIT_TILE - 1) / FA_SPLIT_TILE;
   f.splits = 1;
   while (f.splits < 4 && 2 * f.splits * pairs <= sm_count() && 4 * f.splits <= tiles) f.splits *= 2;
-  void* pooled = nullptr;
+  struct Pooled {  // given back however the call ends
+    void* ptr = nullptr;
+    cudaStream_t s;
+    cudaError_t give_back() {
+      void* const p = ptr;
+      ptr = nullptr;
+      return p ? cudaFreeAsync(p, s) : cudaSuccess;
+    }
+    ~Pooled() { give_back(); }
+  } pooled{nullptr, s};
   CUtensorMap qmap, kmap, vmap;
   if (make_row_box_map(reinterpret_cast<const uint8_t*>(a.q), (size_t)f.ldq * 4, a.rows, 32, FA_BR, &qmap, true)) return 1;
   if (a.kv_type == E_F32) {
@@ -708,8 +717,8 @@ int launch_attention_prefill(const AttnArgs& a, int64_t base_pos, int64_t seq, c
     void* ws = a.pair_ws && a.pair_ws_bytes >= bytes ? a.pair_ws : nullptr;
     if (!ws) {
       if (keep_scratch_pool_cached()) return 1;
-      DYN_CUDA(cudaMallocAsync(&pooled, bytes, s));
-      ws = pooled;
+      DYN_CUDA(cudaMallocAsync(&pooled.ptr, bytes, s));
+      ws = pooled.ptr;
     }
     __half* const out = reinterpret_cast<__half*>(ws);
     const size_t plane = (size_t)a.nkv * a.cap * 2 * FA_D;
@@ -733,7 +742,7 @@ int launch_attention_prefill(const AttnArgs& a, int64_t base_pos, int64_t seq, c
   }
   const int rc = a.kv_type == E_F32 ? fa_launch<E_F32>(f, qmap, kmap, vmap, s) : a.kv_type == E_BF16 ? fa_launch<E_BF16>(f, qmap, kmap, vmap, s)
                                                                                               : fa_launch<E_F16>(f, qmap, kmap, vmap, s);
-  const cudaError_t fe = pooled ? cudaFreeAsync(pooled, s) : cudaSuccess;
+  const cudaError_t fe = pooled.give_back();
   if (rc) return 1;
   if (fe != cudaSuccess) return cuda_fail(fe, "cudaFreeAsync", __FILE__, __LINE__);
   count_launch();
