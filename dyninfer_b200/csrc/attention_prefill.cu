@@ -67,11 +67,10 @@ __device__ __forceinline__ void fa_split2(float x, float y, uint32_t* hi, uint32
 
 // Power of two that puts `mx` into [2^12, 2^13), and its inverse; magnitudes below 2^-41 share one scale.
 __device__ __forceinline__ void fa_pow2_scale(float mx, float* sc, float* inv) {
-  int e = 0;
-  if (mx > 0.f && mx <= 3.40282347e38f) frexpf(mx, &e);
-  e = max(e, -40);
-  *sc = ldexpf(1.0f, 13 - e);
-  *inv = ldexpf(1.0f, e - 13);
+  int e = 0;  // mx = [0.5, 1) * 2^e
+  if (mx > 0.f && mx <= 3.40282347e38f) e = max((int)(__float_as_uint(mx) >> 23) - 126, -40);
+  *sc = __uint_as_float((uint32_t)(127 + 13 - e) << 23);
+  *inv = __uint_as_float((uint32_t)(127 - 13 + e) << 23);
 }
 
 // (a, b) = (a, b) * f + (x, y) * s, two values per instruction; s is a power of two.
@@ -157,7 +156,6 @@ struct FaArgs {
   int* error;
   int64_t rows, nh, nkv, cap, base_pos;
   int64_t ldq;        // floats between consecutive rows of q
-  int splits;         // CTAs of a cluster that share the keys
 };
 
 // kind::f16 descriptor: M = 128, N = n, f32 accumulation; BF: bf16 operands; mn: B contiguous along N.
@@ -200,7 +198,8 @@ __device__ __forceinline__ void fa_add_not_finite8(float* o, const uint4& v) {
   }
 }
 
-template <int KV>
+// NS CTAs share the keys of a row block (a template: each count's merge, and the loop in front of it, in as few registers as it needs).
+template <int KV, int NS>
 __global__ void __launch_bounds__(FA_THREADS, 1)
 attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                          const __grid_constant__ CUtensorMap vmap) {
@@ -224,14 +223,16 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
   unsigned* const s_lost = reinterpret_cast<unsigned*>(s_lost4);
   uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fa_smem) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const int ns = a.splits, rank = (int)(blockIdx.x % (unsigned)ns);
-  const int64_t h = blockIdx.x / (unsigned)ns, rb = gridDim.y - 1 - blockIdx.y;  // the longest row blocks start first
+  const int rank = (int)(blockIdx.x % (unsigned)NS);
+  const int64_t h = blockIdx.x / (unsigned)NS, rb = gridDim.y - 1 - blockIdx.y;  // the longest row blocks start first
   const int64_t kvh = h / (a.nh / a.nkv);
-  // keys 0 .. last position of the CTA's rows, in tiles of 64; tile i belongs to stream i & 1 of CTA (i >> 1) mod splits
+  // keys 0 .. last position of the CTA's rows, in tiles of 64; in turn to the first streams of the NS CTAs of a cluster,
+  // then to the second ones: with two to eight tiles, streams of one CTA get in each other's way (96 rows at 0 on an f16 cache, two tiles: 11.3 us
+  // in one CTA, 9.0 in two; 128 at 5, three: 14.6 in one, 9.9 in four)
   const int64_t row_lo = rb * FA_BR, row_hi = min(row_lo + FA_BR, a.rows) - 1;
   const int last = (int)(a.base_pos + row_hi), ntiles = last / FA_SPLIT_TILE + 1;
   const int stream = warp < 16 ? warp >> 3 : warp & 1;
-  const int first = 2 * rank + stream, step = 2 * ns, mine = first < ntiles ? (ntiles - first + step - 1) / step : 0;
+  const int first = rank + NS * stream, step = 2 * NS, mine = first < ntiles ? (ntiles - first + step - 1) / step : 0;
   const int diag0 = (int)(a.base_pos + row_lo + 1) / FA_SPLIT_TILE;  // the first of up to three tiles whose keys not all rows see
 
   if (tid == 0) {
@@ -243,6 +244,10 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
     }
     mbar_init(&started, 1);
     mbar_fence_init();
+  }
+  if (warp == 17 && lane < 3) {  // (their first use is 0.1 us shorter for it)
+    const CUtensorMap* const m = lane == 0 ? &qmap : lane == 1 ? &kmap : &vmap;
+    asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
   }
   // Tensor memory is taken before this block lets the next kernel start, so that kernel cannot take it first and then wait for this one.
   if (warp == 16) {
@@ -270,7 +275,10 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
     __syncwarp();
     __syncthreads();  // nobody reads the tiles any more
   };
-  auto cluster_sync = [] { asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory"); };
+  auto cluster_sync = [] {
+    if constexpr (NS > 1) asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    else __syncthreads();
+  };
   // row of this thread, and its half of a tile's keys and of the output's dims
   const int row = (warp & 3) * 32 + lane, part = (warp >> 2) & 1;
 
@@ -451,7 +459,7 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
     }
     // ---- the streams' states: [stream][row][pitch]
     float* const state = reinterpret_cast<float*>(smem);
-    {
+    if (mine && row_lo + (row & ~31) < a.rows) {  // (what is read below)
       float* const p = state + (stream * FA_BR + row) * FA_PITCH + part * (FA_D / 2);
 #pragma unroll
       for (int d = 0; d < FA_D / 2; d += 4) *reinterpret_cast<float4*>(p + d) = make_float4(o[d], o[d + 1], o[d + 2], o[d + 3]);
@@ -460,40 +468,47 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
     __syncwarp();
     cluster_sync();
     {
-      uint32_t base[4];  // of the CTAs' shared memory; what is read there lies at the same offsets as here
+      constexpr int NP = 2 * NS;
+      const int np = min(NP, ntiles);  // parts that had tiles
+      uint32_t base[NS];  // of the CTAs' shared memory; what is read there lies at the same offsets as here
 #pragma unroll
-      for (int c = 0; c < 4; c++) asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[c]) : "r"(smem_u32(smem)), "r"(c < ns ? c : 0));
+      for (int c = 0; NS > 1 && c < NS; c++) asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[c]) : "r"(smem_u32(smem)), "r"(c));
       const uint32_t at_m = smem_u32(&s_m[0][0]) - smem_u32(smem), at_l = smem_u32(&s_l[0][0][0]) - smem_u32(smem);
       // a warp's rows, two at a time; lane = four dims
 #pragma unroll 1
-      for (int r0 = rank * 16 + warp; r0 < FA_BR && row_lo + r0 < a.rows; r0 += 32 * ns) {
+      for (int r0 = rank * 16 + warp; r0 < FA_BR && row_lo + r0 < a.rows; r0 += 32 * NS) {
         float4 acc[2];
         float l[2];
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-          const int r = min(r0 + 16 * ns * q, FA_BR - 1);
-          float mv[8], l0[8], l1[8], M = LOWEST;
-          float4 v[8];
+          const int r = min(r0 + 16 * NS * q, FA_BR - 1);
+          float mv[NP], l0[NP], l1[NP], M = LOWEST;
+          float4 v[NP];
 #pragma unroll
-          for (int p = 0; p < 8; p++) {  // part p: stream p & 1 of CTA p >> 1
-            if (p >= 2 * ns) break;
-            const uint32_t b = base[p >> 1], sr = (uint32_t)((p & 1) * FA_BR + r);
+          for (int p = 0; p < NP; p++) {  // part p: stream p / NS of CTA p mod NS
+            if (p >= np) break;
+            if constexpr (NS == 1) {
+              mv[p] = s_m[p][r], l0[p] = s_l[p][0][r], l1[p] = s_l[p][1][r];
+              v[p] = *reinterpret_cast<const float4*>(state + (p * FA_BR + r) * FA_PITCH + 4 * lane);
+              continue;
+            }
+            const uint32_t b = base[p % NS], st = p / NS, sr = st * FA_BR + r;
             asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(mv[p]) : "r"(b + at_m + 4u * sr) : "memory");
-            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l0[p]) : "r"(b + at_l + 4u * (2u * FA_BR * (p & 1) + r)) : "memory");
-            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l1[p]) : "r"(b + at_l + 4u * (2u * FA_BR * (p & 1) + FA_BR + r)) : "memory");
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l0[p]) : "r"(b + at_l + 4u * (2u * FA_BR * st + r)) : "memory");
+            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(l1[p]) : "r"(b + at_l + 4u * (2u * FA_BR * st + FA_BR + r)) : "memory");
             asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
                          : "=f"(v[p].x), "=f"(v[p].y), "=f"(v[p].z), "=f"(v[p].w)
                          : "r"(b + 4u * (sr * FA_PITCH + 4 * lane))
                          : "memory");
           }
 #pragma unroll
-          for (int p = 0; p < 8; p++)
-            if (p < 2 * ns) M = fmaxf(M, mv[p]);
+          for (int p = 0; p < NP; p++)
+            if (p < np) M = fmaxf(M, mv[p]);
           acc[q] = make_float4(0.f, 0.f, 0.f, 0.f), l[q] = 0.f;
 #pragma unroll
-          for (int p = 0; p < 8; p++) {
-            if (p >= 2 * ns) break;
-            const float w = expf(mv[p] - M);  // a stream without tiles has sum 0 and contributes nothing
+          for (int p = 0; p < NP; p++) {
+            if (p >= np) break;
+            const float w = expf(mv[p] - M);  // a part whose keys the row does not see has sum 0 and contributes nothing
             acc[q].x = fmaf(v[p].x, w, acc[q].x), acc[q].y = fmaf(v[p].y, w, acc[q].y);
             acc[q].z = fmaf(v[p].z, w, acc[q].z), acc[q].w = fmaf(v[p].w, w, acc[q].w);
             l[q] = fmaf(l0[p] + l1[p], w, l[q]);
@@ -501,7 +516,7 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
         }
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-          const int r = r0 + 16 * ns * q;
+          const int r = r0 + 16 * NS * q;
           if (r >= FA_BR || row_lo + r >= a.rows) break;
           const float i0 = (SPLIT ? PMUL : 1.0f) / l[q];  // pairs: o left the weights' scale with each tile
           *reinterpret_cast<float4*>(a.ctx + (row_lo + r) * a.nh * FA_D + h * FA_D + 4 * lane) =
@@ -510,8 +525,7 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
       }
     }
     __syncwarp();
-    // nobody leaves while its state may still be read
-    cluster_sync();
+    if constexpr (NS > 1) cluster_sync();  // nobody leaves while its state may still be read
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FA_ISSUE_REGS));
     if (warp < 18) {
@@ -646,19 +660,19 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
     // (the softmax warps' ends are theirs alone: these warps have given their registers away)
     drained();
     cluster_sync();
-    cluster_sync();
+    if constexpr (NS > 1) cluster_sync();
   }
   tc_fence_after();
   if (warp == 16) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   if (tid == 0 && s_abort) report_wait_expired(a.error, DEV_ERR_GEMM_PIPE);
 }
 
-template <int KV>
+template <int KV, int NS>
 int fa_launch(const FaArgs& f, const CUtensorMap& qmap, const CUtensorMap& kmap, const CUtensorMap& vmap, cudaStream_t s) {
-  auto kernel = attention_prefill_kernel<KV>;
+  auto kernel = attention_prefill_kernel<KV, NS>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), FA_SMEM)) return 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(f.nh * f.splits), (unsigned)((f.rows + FA_BR - 1) / FA_BR)), cfg.blockDim = dim3(FA_THREADS);
+  cfg.gridDim = dim3((unsigned)(f.nh * NS), (unsigned)((f.rows + FA_BR - 1) / FA_BR)), cfg.blockDim = dim3(FA_THREADS);
   cfg.dynamicSmemBytes = FA_SMEM, cfg.stream = s;
   cudaLaunchAttribute attr[2];
   int n = 0;
@@ -666,9 +680,11 @@ int fa_launch(const FaArgs& f, const CUtensorMap& qmap, const CUtensorMap& kmap,
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n++].val.programmaticStreamSerializationAllowed = 1;
   }
-  attr[n].id = cudaLaunchAttributeClusterDimension;
-  attr[n].val.clusterDim.x = (unsigned)f.splits, attr[n].val.clusterDim.y = 1, attr[n].val.clusterDim.z = 1;
-  n++;
+  if (NS > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = NS, attr[n].val.clusterDim.y = 1, attr[n].val.clusterDim.z = 1;
+    n++;
+  }
   cfg.attrs = attr, cfg.numAttrs = n;
   DYN_CUDA(cudaLaunchKernelEx(&cfg, kernel, f, qmap, kmap, vmap));
   return 0;
@@ -696,10 +712,10 @@ int launch_attention_prefill(const AttnArgs& a, int64_t base_pos, int64_t seq, c
   if (!f.error) return 1;
   f.rows = a.rows, f.nh = a.nh, f.nkv = a.nkv, f.cap = a.cap, f.base_pos = base_pos;
   f.ldq = a.ldq ? a.ldq : a.nh * FA_D;
-  // The keys go to as many CTAs as the SMs hold besides one another, while each has a tile for both of its streams
+  // The keys go to as many CTAs as the SMs hold besides one another, while there is a tile for each of half of them
   const int64_t pairs = a.nh * ((a.rows + FA_BR - 1) / FA_BR), tiles = (base_pos + a.rows + FA_SPLIT_TILE - 1) / FA_SPLIT_TILE;
-  f.splits = 1;
-  while (f.splits < 4 && 2 * f.splits * pairs <= sm_count() && 4 * f.splits <= tiles) f.splits *= 2;
+  int splits = 1;
+  while (splits < 4 && 2 * splits * pairs <= sm_count() && splits < tiles) splits *= 2;
   struct Pooled {  // given back however the call ends
     void* ptr = nullptr;
     cudaStream_t s;
@@ -740,8 +756,10 @@ int launch_attention_prefill(const AttnArgs& a, int64_t base_pos, int64_t seq, c
         make_row_box_map(reinterpret_cast<const uint8_t*>(a.vcache) + at * (2 * FA_D), 2 * FA_D, a.nkv * a.cap, 32, FA_SPLIT_TILE, &vmap, true))
       return 1;
   }
-  const int rc = a.kv_type == E_F32 ? fa_launch<E_F32>(f, qmap, kmap, vmap, s) : a.kv_type == E_BF16 ? fa_launch<E_BF16>(f, qmap, kmap, vmap, s)
-                                                                                              : fa_launch<E_F16>(f, qmap, kmap, vmap, s);
+  auto launch = [&](auto n1, auto n2, auto n4) { return (splits == 1 ? n1 : splits == 2 ? n2 : n4)(f, qmap, kmap, vmap, s); };
+  const int rc = a.kv_type == E_F32    ? launch(fa_launch<E_F32, 1>, fa_launch<E_F32, 2>, fa_launch<E_F32, 4>)
+                 : a.kv_type == E_BF16 ? launch(fa_launch<E_BF16, 1>, fa_launch<E_BF16, 2>, fa_launch<E_BF16, 4>)
+                                       : launch(fa_launch<E_F16, 1>, fa_launch<E_F16, 2>, fa_launch<E_F16, 4>);
   const cudaError_t fe = pooled.give_back();
   if (rc) return 1;
   if (fe != cudaSuccess) return cuda_fail(fe, "cudaFreeAsync", __FILE__, __LINE__);

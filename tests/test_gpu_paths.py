@@ -332,6 +332,13 @@ def test_attention_prefill_at_the_edges_of_blocks(native_lib, dtype, s, start, n
         assert float((got[:, h] - want).abs().max()) < (1e-4 if dtype == "bf16" else 4e-6) * float(vh.abs().max())
 
 
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("s,start,nh,nkv", [(64, 0, 2, 1), (65, 0, 2, 1), (128, 5, 4, 2), (300, 0, 2, 1), (260, 130, 6, 3), (100, 60, 40, 8)])
+def test_attention_prefill_of_few_tiles(native_lib, dtype, s, start, nh, nkv):
+    """One to seven tiles: two or four blocks share them, some of which have none, in the last row block or in the first one only."""
+    test_attention_prefill_at_the_edges_of_blocks(native_lib, dtype, s, start, nh, nkv)
+
+
 @pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q4_1", "gguf.q8_0", "gguf.q4_k", "mlx.affine.u4"])
 @pytest.mark.parametrize("m,n,k", [(33, 130, 256), (48, 127, 768), (49, 1000, 2560), (64, 257, 3072), (47, 2049, 1792),
                                    (64, 6000, 1024), (40, 128, 6144), (64, 129, 6400), (65, 1024, 2048), (128, 257, 1536),
