@@ -714,19 +714,37 @@ bool gr_make_plan(const WRef& w, int64_t M, bool swiglu, GrPlan* best) {
   if (!found) return false;
   const void* kernel = gr_kernel(w.enc, best->NM);
   if (ensure_dynamic_smem(kernel, GR_MAX_SMEM)) return false;
-  // Blocks of more rows and fewer K warps where the blocks do not fit the SMs well: eight warps on one SM get through a tile's K
-  // faster alone than beside a second block, and a second round of a few blocks costs as much as a full one. us before / with twice
-  // the rows: Q4_0, one row, 5120 x 4096 (320 blocks for 296 places) 10.1 / 6.9, 4096 x 4096 (256) 6.0 / 5.4, 3072 x 2048 (192)
-  // 4.3 / 3.9; four rows 4096 x 4096 15.5 / 14.5, 10240 x 5120 38 / 32. Beyond eight stages per warp the second block's loads count for
-  // more (4096 x 14336 14.1 / 17.4), with that second round beyond twelve (5120 x 13824 Q8_0, four rows 56 / 60).
+  // Blocks of twice the rows and half the K warps where the blocks do not fit the SMs well. Measured on 2560 to 9216 rows x 512 to 8192
+  // (and 5120 x 13824) of five encodings, weights out of L2 and out of HBM; us with the plan above / with twice the rows.
+  //   More blocks than places: a second round of a few blocks costs as much as a full one (5120 x 4096 Q4_0, 320 blocks for 296
+  //     places, one row 10.0 / 6.8, four rows 26.7 / 18.9), up to twelve stages per warp (5120 x 13824 Q8_0, four rows 56 / 60).
+  //   Two blocks on some SMs: eight warps get through a tile's K faster alone than beside a second block.
+  //     Two and more rows: up to eight stages per warp (4096 x 4096 four rows 15.7 / 14.5). Q4_K, whose decoding needs the warps, with two
+  //       rows only while that makes two tiles per block (4096 x 4096 9.9 / 9.6, 6144 x 4096 12.2 / 12.7).
+  //     One row: up to two stages per warp (3072 x 2048 Q4_0 4.3 / 4.0, 6144 x 1024 4.4 / 4.1; 6144 x 4096 with eight 7.0 / 7.4,
+  //       Q8_0 8.0 / 8.6); up to four where that makes two tiles per block and leaves few SMs without one (4096 x 4096 Q4_0 5.8 / 5.6,
+  //       3584 x 4096 Q8_0 7 % slower) or the encoding is MLX-U4 (4096 x 4096 5.9 / 5.1, 3584 x 4096 4 to 8 % faster); Q4_K never
+  //       (4096 x 4096 6.2 / 6.5).
   const int tile_rows = swiglu ? 8 : 16;
+  const int64_t sms = std::max(1, sm_count());
+  auto alone = [&](int64_t ctas) {  // a block on its own rather than two
+    const int stages = (2 * best->cstages + best->KW - 1) / best->KW;  // of a warp with twice the rows
+    const bool pairs = best->RW == 1;                                  // two tiles per block then
+    if (best->KW < 4 || ctas <= sms) return false;
+    if (best->NM >= 2) return stages <= 8 && (best->NM > 2 || pairs || w.enc != E_Q4_K);
+    if (w.enc == E_Q4_K) return false;
+    return stages <= 2 || (stages <= 4 && pairs && (w.enc == E_MLX_U4 || 10 * ctas >= 17 * sms));
+  };
+  auto tail = [&](int64_t ctas) {  // a second round of a few blocks
+    const int64_t places = best->per_sm * sms;
+    return best->KW >= 2 && ctas > places && 10 * ctas <= 13 * places && 2 * best->cstages <= 12 * best->KW;
+  };
   for (int i = 0;; i++) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&best->per_sm, kernel, best->RW * best->KW * 32, best->smem) != cudaSuccess || best->per_sm < 1)
       best->per_sm = 1;
     best->groups = (N + tile_rows * best->RW - 1) / (tile_rows * best->RW);
-    const int64_t ctas = best->groups * best->CK, places = (int64_t)best->per_sm * std::max(1, sm_count());
-    const bool halves = best->KW >= 4 && ctas > sm_count() && 2 * best->cstages <= 8 * best->KW, spills = best->KW >= 2 && ctas > places && 10 * ctas <= 13 * places && 2 * best->cstages <= 12 * best->KW;
-    if (best->RW * best->KW != 8 || !(i == 0 ? halves || spills : spills)) break;
+    const int64_t ctas = best->groups * best->CK;
+    if (best->RW * best->KW != 8 || !(tail(ctas) || (i == 0 && alone(ctas)))) break;
     GrPlan q = *best;
     q.RW *= 2, q.KW /= 2;
     q.nst = std::min((q.cstages + q.KW - 1) / q.KW, 2);
