@@ -318,16 +318,8 @@ int gc_launch(const GcArgs& a, const CUtensorMap& wmap, const CUtensorMap& xmap,
 
 }  // namespace
 
-// Where the kernel is ahead of gemm_skinny.cu among the products that one takes: more rows than 32 (with up to 32 the activations that
-// every CTA of that kernel reads weigh less: 1024 x 2048 Q4_0, activation pass included, 24 rows 6.6 there and 6.9 us here, 37
-// rows 8.2 and 7.0, 64 rows 9.7 and 7.4; 65 rows, against the kernels behind that one, 13.1 and 7.8, 128 rows 13.5 and 9.8; a
-// second tile of 128 rows is slower than they are), and a K that four CTAs share, or two with a third of the SMs to spare (6144 x 1024, 64
-// rows 12.4 and 8.7; 12288 x 512 in whole tiles 11.6 and 12.9, 8192 x 768 Q8_0 in 128 CTAs 11.5 and 11.8).
 bool gemm_cluster_prefers(const WRef& w, int64_t M, bool swiglu) {
-  GcPlan p;
-  if (M <= 32 || M > GC_MAX_BN || !gemm_stream_takes(w) || w.rows > (1 << 30) || (swiglu && w.rows % 2) || !gc_plan(w, M, swiglu, &p)) return false;
-  if (M > 64) return !swiglu && p.CK >= 2 && w.cols >= 1536 && p.tiles <= 20;
-  return p.CK >= 4 || (p.CK >= 2 && p.upc <= 2 && 3 * p.tiles * p.CK <= 2 * sm_count());
+  return gemm_stream_takes(w) && w.rows <= (1 << 30) && gc_prefers(w.rows, w.cols, gs_words(w.enc), M, swiglu, std::max(1, sm_count()), gc_places);
 }
 
 // Activation rows the kernel's boxes read: x has this many rows allocated (those from M on may hold anything).

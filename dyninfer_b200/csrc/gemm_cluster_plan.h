@@ -65,4 +65,17 @@ bool gc_plan(int64_t rows, int64_t cols, int words, int64_t M, bool swiglu, int6
   return true;
 }
 
+// Where the kernel is ahead of gemm_skinny.cu among the products that one takes: more rows than 32 (with up to 32 the activations that
+// every CTA of that kernel reads weigh less: 1024 x 2048 Q4_0, activation pass included, 24 rows 6.6 there and 6.9 us here, 37
+// rows 8.2 and 7.0, 64 rows 9.7 and 7.4; 65 rows, against the kernels behind that one, 13.1 and 7.8, 128 rows 13.5 and 9.8; a
+// second tile of 128 rows is slower than they are), and a K that four CTAs share, or two with a third of the SMs to spare (6144 x 1024, 64
+// rows 12.4 and 8.7; 12288 x 512 in whole tiles 11.6 and 12.9, 8192 x 768 Q8_0 in 128 CTAs 11.5 and 11.8).
+template <class Places>
+bool gc_prefers(int64_t rows, int64_t cols, int words, int64_t M, bool swiglu, int64_t sms, Places places) {
+  GcPlan p;
+  if (M <= 32 || M > GC_MAX_BN || (swiglu && rows % 2) || !gc_plan(rows, cols, words, M, swiglu, sms, places, &p)) return false;
+  if (M > 64) return !swiglu && p.CK >= 2 && cols >= 1536 && p.tiles <= 20;
+  return p.CK >= 4 || (p.CK >= 2 && p.upc <= 2 && 3 * p.tiles * p.CK <= 2 * sms);
+}
+
 }  // namespace dyn

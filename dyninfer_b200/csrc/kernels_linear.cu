@@ -129,7 +129,8 @@ int launch_linear(const WRef& w, const void* x, int x_type, int64_t m, float* y,
     if (launch_gemv_rows(w, x, x_type, m, nullptr, 0, 0.f, y, residual, false, s, &handled)) return 1;
     if (handled) return 0;
   }
-  // up to 64 rows beyond what the exact few-row kernels take: one activation pass, weights streamed once
+  // beyond what the exact few-row kernels take, one activation pass and one product: up to 64 rows on mma.sync or over a cluster, 65 to
+  // 128 over a cluster only
   if (m > (x_type == E_BF16 ? 8 : 4) && (m > 64 ? gemm_cluster_prefers(w, m, false) : gemm_skinny_prefers(w, m, false))) {
     bool handled = false;
     if (launch_linear_skinny(w, x, x_type, m, y, residual, s, &handled)) return 1;

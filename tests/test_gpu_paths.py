@@ -358,6 +358,33 @@ def test_linear_rows_over_a_cluster(native_lib, oracle, enc, m, n, k):
     assert helpers.rel_err(got, oracle.linear(ow, x, fast=True)) < 4e-4
 
 
+# encoding, activation rows, matrix rows, K, MLX group and type of scales; that the GEMM over a cluster takes them: test_gemm_cluster_plan.py
+CLUSTER_PRODUCTS = [("gguf.q5_k", 65, 1000, 2048, 0, ""), ("gguf.q5_k", 128, 257, 1536, 0, ""), ("gguf.q5_k", 99, 2048, 2560, 0, ""),
+                    ("mlx.affine.u4", 48, 1000, 2048, 32, "bf16"), ("mlx.affine.u4", 64, 257, 1024, 32, "f16"),
+                    ("mlx.affine.u4", 65, 1000, 1792, 32, "f32"), ("mlx.affine.u4", 128, 300, 2304, 64, "bf16"),
+                    ("mlx.affine.u4", 100, 2048, 2048, 128, "f32"), ("mlx.affine.u4", 66, 129, 2816, 256, "f16")]
+
+
+@pytest.mark.parametrize("enc,m,n,k,group,aux", CLUSTER_PRODUCTS)
+def test_linear_encodings_over_a_cluster(native_lib, oracle, enc, m, n, k, group, aux):
+    """Q5_K (65 rows and more only), MLX groups of 32 to 256, scales of every type and rows of an odd multiple of 256. The bound is that of
+    test_linear_rows_over_a_cluster."""
+    from dyninfer_b200 import ops
+    t = synth.random_weight(enc, n, k, m + n, **({"group": group} if group else {}))
+    if group:
+        scales, biases = (synth.bf16_bits_to_f32(t[c]) for c in ("scales", "biases"))
+        if aux == "f16":
+            scales, biases = scales.astype(np.float16), biases.astype(np.float16)
+        if aux == "bf16":
+            scales, biases = t["scales"], t["biases"]
+        args = (enc, n, k, t["packed"], scales, biases, "plain." + aux, group)
+    else:
+        args = (enc, n, k, t["data"])
+    x = np.random.default_rng(m).normal(size=(m, k)).astype(np.float32)
+    got = ops.linear(ops.DeviceWeight(*args), torch.from_numpy(x).cuda()).cpu().numpy()
+    assert helpers.rel_err(got, oracle.linear(oracle.Weight(*args), x, fast=True)) < 4e-4
+
+
 @pytest.mark.parametrize("hidden", [1280, 1536, 2816, 3584, 7168, 1344])
 def test_many_row_norm_widths(native_lib, oracle, tmp_path, hidden):
     """Rows that are multiples of 256 but not of 1024 elements (the last runs of a thread stay empty), and one that is
