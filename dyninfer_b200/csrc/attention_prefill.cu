@@ -3,15 +3,20 @@
 //
 // Same mathematics as the per-row kernel (kernels.rs:310-458: s = (q.k) * 1/sqrt(d), keys beyond the
 // row's position masked, online max / sum merge, out / sum at the end), restructured the usual
-// flash-attention way. One CTA = 128 consecutive rows of one query head = the 128 lanes of tensor memory, a thread = a row:
+// flash-attention way. One CTA = 128 consecutive rows of one query head = the 128 lanes of tensor memory:
 //   * Q lies in tensor memory as (hi, lo) pairs (128 columns). 64-key tiles of K and V arrive as tensor copies.
-//   * Two streams of four warps take the tiles in turn, each with its own running (max, sum, out), so that one's softmax runs
-//     under the other's MMAs. A fifth warp per stream asks for its tiles and issues its MMAs. Per tile: S (64 columns) = Qhi Khi, a second
-//     accumulator for the terms with a lo part; the thread reads its row twice (maximum, then weights), leaves P as (hi, lo)
-//     pairs in place of S; U (128 columns) = P V, with V's tile as an operand that is contiguous along N; the thread folds U into its 128
-//     f32 sums. The second score accumulator uses U's columns, so a stream needs 192, and 512 hold everything.
+//   * Two streams of eight warps take the tiles in turn, each with its own running (max, sum, out), so that one's softmax runs under
+//     the other's MMAs. Two threads share a row: each has half of a tile's keys and half of the output's dims. A ninth warp per stream
+//     (warps 16 and 17) asks for its tiles and issues its MMAs, a tenth (18 and 19) looks for values that are not finite. Per tile: S (64
+//     columns) = Qhi Khi, a second accumulator for the terms with a lo part; a thread reads its half of the row twice (maximum, then
+//     weights) and leaves P as (hi, lo) pairs in place of S; U (128 columns) = P V, with V's tile as an operand that is
+//     contiguous along N; a thread folds its half of U into 64 f32 sums. The second score accumulator uses U's columns, so a
+//     stream needs 192, and 512 hold everything.
 //   * Keys are also dealt over the CTAs of a cluster where there are few (head, row block) pairs (16 heads x 512 rows: 64); all streams'
 //     states meet through shared memory at the end and are merged in a fixed order.
+//   * From 32 rows on. Against the kernels for fewer (attention_decode.cu, f32 caches the slices of kernels_misc.cu), us here / there with
+//     16 heads: bf16 16 rows at 0 6.1 / 5.3, 32 at 0 6.2 / 10.3, 32 at 1000 17.4 / 30.1; f32 32 at 0 9.7 / 7.1, 48 at 0 10.0 / 9.7,
+//     32 at 200 11.8 / 19.3. (Calls of 17 to 31 rows behind a context would gain by a lower line.)
 // On mma.sync (16 rows per warp, 64 per CTA) the MMAs alone kept an SM busy four times as long: 512 rows of 16 heads at 1536, f32
 // cache, 92 us.
 //

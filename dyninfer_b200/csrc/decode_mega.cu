@@ -604,7 +604,7 @@ __device__ __forceinline__ void run_unit(int enc, int aux, int group_shift, cons
 // the A operand with its own block of rows g and g + 8, and the B operand holds that block's activations only in columns 2 t
 // (hi) and 2 t + 1 (lo), so a lane ends up with its own block's sums and applies one scale and bias per eight MMAs. Block by block, all
 // four quarters fetched the same scales and applied them to the same sums, about 200 instructions per 128 weights of 16 rows
-// against 70 now (tile math of a 0.6B token 177 -> 117 us). The accumulator then holds the quarter's share of a row: the
+// against 70 now (tile math of a 0.6B token 177 -> 117 us, with gate and up rows in one tile 95). The accumulator then holds the quarter's share of a row: the
 // quarters are added up when the tile ends. Q4_0, whose scale lies beside its block, gains nothing (its blocks start in the middle
 // of a word).
 __device__ __forceinline__ void run_quad(int aux, int group_shift, const uint8_t* p0, const uint8_t* p1, const uint8_t* a0,

@@ -385,6 +385,26 @@ def test_linear_encodings_over_a_cluster(native_lib, oracle, enc, m, n, k, group
     assert helpers.rel_err(got, oracle.linear(oracle.Weight(*args), x, fast=True)) < 4e-4
 
 
+def test_linear_over_a_cluster_on_two_streams(native_lib, oracle):
+    """Products of plans with 256 and with 512 columns of tensor memory, on two streams at a time (blocks of both kinds are kept off
+    one SM: test_gemm_cluster_plan.py). Each gives the bits that it gives alone."""
+    from dyninfer_b200 import ops
+    from test_gpu_ops import make_pair
+    ws = [make_pair(oracle, "gguf.q4_0", n, 1024, seed=n)[0] for n in (4096, 6144, 1024)]
+    xs = [torch.randn(m, 1024, generator=torch.Generator("cuda").manual_seed(m), device="cuda") for m in (64, 40)]
+    want = [[ops.linear(w, x) for w in ws] for x in xs]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in xs], [[], []]
+    for i in range(30):
+        for j, (stream, x) in enumerate(zip(streams, xs)):
+            with torch.cuda.stream(stream):
+                got[j].append(ops.linear(ws[(i + j) % 3], x))
+    torch.cuda.synchronize()
+    ops.check_device_error()
+    for j in range(2):
+        assert all(torch.equal(y, want[j][(i + j) % 3]) for i, y in enumerate(got[j]))
+
+
 @pytest.mark.parametrize("hidden", [1280, 1536, 2816, 3584, 7168, 1344])
 def test_many_row_norm_widths(native_lib, oracle, tmp_path, hidden):
     """Rows that are multiples of 256 but not of 1024 elements (the last runs of a thread stay empty), and one that is
