@@ -28,8 +28,8 @@
 // term). The tile scales are exact: the keys' multiply the scores, the values' a tile's share of the output.
 // Weight 0 times an entry that is not finite would reach rows that do not see its key. On 2-byte caches a warp per stream, idle
 // otherwise, looks through the values of the tiles on the diagonal while their scores are made, puts zeros in such places and
-// marks the keys; rows that see one add the entry itself at the end (in the softmax warps' loop the same cost 0.5 us per tile of
-// 64 keys; bf16, 16 heads, 128 rows at 0: 11.5 us without, 11.8 with; f16 12.1 and 12.1).
+// marks the keys; where there are any, the idle warps add the entry itself to the states of the rows that see its key. (Code for
+// it in the softmax warps, in their loop or behind it, costs the loop registers: 2 to 7 % of a call.)
 // Every tile's products start from zero and join the running output by a rounded fma, because a tensor-core accumulation
 // truncates.
 #include <algorithm>
@@ -191,16 +191,12 @@ __device__ __forceinline__ uint32_t fa_fma0(uint32_t w, uint32_t c) {
   else asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(0u), "r"(c));
   return r;
 }
-// Adds what is not finite of eight entries to their sums.
+// Adds what is not finite of two entries to their sums.
 template <bool BF>
-__device__ __forceinline__ void fa_add_not_finite8(float* o, const uint4& v) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint32_t m = fa_not_finite2<BF>(w[i]);
-    if (m & 0x8000u) o[2 * i] += BF ? __uint_as_float(w[i] << 16) : f16_bits_to_f32(w[i] & 0xffffu);
-    if (m & 0x80000000u) o[2 * i + 1] += BF ? __uint_as_float(w[i] & 0xffff0000u) : f16_bits_to_f32(w[i] >> 16);
-  }
+__device__ __forceinline__ void fa_add_not_finite2(float* o, uint32_t w) {
+  const uint32_t m = fa_not_finite2<BF>(w);
+  if (m & 0x8000u) o[0] += BF ? __uint_as_float(w << 16) : f16_bits_to_f32(w & 0xffffu);
+  if (m & 0x80000000u) o[1] += BF ? __uint_as_float(w & 0xffff0000u) : f16_bits_to_f32(w >> 16);
 }
 
 // NS CTAs share the keys of a row block (a template: each count's merge, and the loop in front of it, in as few registers as it needs).
@@ -283,6 +279,10 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
   auto cluster_sync = [] {
     if constexpr (NS > 1) asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
     else __syncthreads();
+  };
+  auto any_lost = [&] {  // the same for the whole CTA, behind drained()
+    const uint4 u = s_lost4[0], v = s_lost4[1];
+    return (u.x | u.y | u.z | u.w | v.x | v.y) != 0;
   };
   // row of this thread, and its half of a tile's keys and of the output's dims
   const int row = (warp & 3) * 32 + lane, part = (warp >> 2) & 1;
@@ -445,23 +445,6 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
       }
     }
     drained();
-    if constexpr (!SPLIT) {
-      const uint4 u = s_lost4[0], v = s_lost4[1];
-      if (u.x | u.y | u.z | u.w | v.x | v.y) {  // zeros took the places of what is not finite: rows that see the keys add it now
-#pragma unroll 1
-        for (int t = first; t < ntiles; t += step)
-#pragma unroll 1
-          for (int q = 0; q < 2 && t >= diag0; q++)
-#pragma unroll 1
-            for (unsigned m = s_lost[2 * (t - diag0) + q]; m; m &= m - 1) {
-              const int key = t * FA_SPLIT_TILE + 32 * q + __ffs(m) - 1;
-              if (key > pos) break;
-              const uint4* v8 = reinterpret_cast<const uint4*>(a.vals + (kvh * a.cap + key) * FA_D + part * (FA_D / 2));
-#pragma unroll
-              for (int d = 0; d < FA_D / 2; d += 8) fa_add_not_finite8<BF>(o + d, __ldcg(v8 + d / 8));
-            }
-      }
-    }
     // ---- the streams' states: [stream][row][pitch]
     float* const state = reinterpret_cast<float*>(smem);
     if (mine && row_lo + (row & ~31) < a.rows) {  // (what is read below)
@@ -471,6 +454,7 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
       s_m[stream][row] = m_run, s_l[stream][part][row] = l_run;
     }
     __syncwarp();
+    if (!SPLIT && any_lost()) __syncthreads();  // the other warps correct the states
     cluster_sync();
     {
       constexpr int NP = 2 * NS;
@@ -664,6 +648,22 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
     }
     // (the softmax warps' ends are theirs alone: these warps have given their registers away)
     drained();
+    if (!SPLIT && any_lost()) {
+      // zeros took the places of what is not finite: a thread adds it to its row's states, for the keys that the row sees. (Here, because the same in
+      // the softmax warps costs their loop registers: 2 to 3 % of a call.)
+      __syncthreads();
+      const int r = tid - 512;
+      for (int64_t t = rank; t < ntiles && row_lo + r < a.rows; t += NS)
+        for (int q = 0; q < 2 && t >= diag0; q++)
+          for (unsigned m = s_lost[2 * (t - diag0) + q]; m; m &= m - 1) {
+            const int64_t key = t * FA_SPLIT_TILE + 32 * q + __ffs(m) - 1;
+            if (key > a.base_pos + row_lo + r) break;
+            const uint32_t* const w = reinterpret_cast<const uint32_t*>(a.vals + (kvh * a.cap + key) * FA_D);
+            float* const p = reinterpret_cast<float*>(smem) + ((t / NS & 1) * FA_BR + r) * FA_PITCH;
+#pragma unroll 1
+            for (int d = 0; d < FA_D; d += 2) fa_add_not_finite2<BF>(p + d, __ldcg(w + d / 2));
+          }
+    }
     cluster_sync();
     if constexpr (NS > 1) cluster_sync();
   }
