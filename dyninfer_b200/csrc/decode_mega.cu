@@ -1636,6 +1636,16 @@ static bool can_interleave(const WRef& g, const WRef& u, int I) {
          std::llabs(((u.data - g.data) - 8 * (int64_t)g.row_bytes()) / 16) < (1LL << 31);
 }
 
+// Whether they do. An interleaved tile has eight rows of each, so a CTA's share is a multiple of eight and may be larger than the
+// multiple of four it is otherwise. MLX-U4: for fewer tiles on the busiest CTA (1024 x 3072, 3 for 4: 160 -> 140 us for six layers), with as many
+// only for a K of one slice (512 x 1536, 2 for 2: 124.4 -> 120.7; 2048 x 6144, 6 for 6 with up to 48 rows instead of 44: 326 -> 334).
+static bool interleaves(const WRef& g, const WRef& u, int I, int grid) {
+  if (!can_interleave(g, u, I)) return false;
+  if (g.enc != E_MLX_U4) return true;
+  const int64_t shared = (I / 8 + grid - 1) / grid, apart = 2 * ((4 * ((I / 4 + grid - 1) / grid) + 15) / 16);
+  return shared < apart || (shared == apart && g.cols <= 1024);
+}
+
 int mega_build_program(const MegaBuildLayer* layers, const MegaLayer* full, int nlayers, const WRef& lm_head, int nh,
                        int nkv, int d, int H, int I, int V, int grid, std::vector<uint8_t>* blob, MegaProgLayout* lay) {
   DYN_CHECK(H % 4 == 0 && I % 4 == 0 && (nh * d) % 4 == 0 && (nkv * d) % 4 == 0,
@@ -1663,7 +1673,7 @@ int mega_build_program(const MegaBuildLayer* layers, const MegaLayer* full, int 
       pc.begin_phase();
       pc.add_rows(L.o, nullptr, h0, h1, 0, MEGA_EP_RESID_O);
       pc.begin_phase();
-      if (can_interleave(L.gate, L.up, I))
+      if (interleaves(L.gate, L.up, I, grid))
         pc.add_rows_interleaved(L.gate, L.up, split8(I, cta, grid), split8(I, cta + 1, grid));
       else
         pc.add_rows(L.gate, &L.up, split4(I, cta, grid), split4(I, cta + 1, grid), 0, MEGA_EP_SWIGLU);

@@ -564,6 +564,12 @@ def test_persistent_mlx_widths_and_groups(native_lib, tmp_path, hidden, inter, g
     assert np.abs(got[0] - got[1]).max() <= 1e-4 * np.abs(got[1]).max()
 
 
+@pytest.mark.parametrize("hidden,inter,group", [(2048, 4096, 128), (1536, 4608, 64), (1536, 6144, 32), (512, 1536, 64)])
+def test_persistent_mlx_gate_and_up_by_tiles(native_lib, tmp_path, hidden, inter, group):
+    """As many tiles on the busiest block with gate and up in one as with each in its own: apart for several slices of K, together for one."""
+    test_persistent_mlx_widths_and_groups(native_lib, tmp_path, hidden, inter, group)
+
+
 @pytest.mark.parametrize("enc", ["gguf.q4_0", "gguf.q8_0"])
 @pytest.mark.parametrize("kv", ["bf16", "f16", "f32"])
 def test_few_row_chains_give_the_same_bits_every_time(native_lib, tmp_path, enc, kv):
