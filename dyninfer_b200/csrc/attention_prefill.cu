@@ -664,6 +664,7 @@ attention_prefill_kernel(const FaArgs a, const __grid_constant__ CUtensorMap qma
             for (int d = 0; d < FA_D; d += 2) fa_add_not_finite2<BF>(p + d, __ldcg(w + d / 2));
           }
     }
+    __syncwarp();  // (the rows' loops differ in length)
     cluster_sync();
     if constexpr (NS > 1) cluster_sync();
   }

@@ -34,8 +34,8 @@ WORDS = {"gguf.q4_0": 36, "gguf.q4_1": 40, "gguf.q8_0": 68, "gguf.q4_k": 36, "gg
 
 
 def test_products_that_the_gpu_tests_mean_go_over_a_cluster(tmp_path):
-    """The dispatch's own rule at the sizes of test_linear_rows_over_a_cluster (whose first and third last but one have too little
-    or too much of K) and of test_linear_encodings_over_a_cluster, all of whose products it has to take."""
+    """The dispatch's own rule at the sizes of test_linear_rows_over_a_cluster (of which K = 256 is too little and 6400 too much) and of
+    test_linear_encodings_over_a_cluster, all of whose products it has to take."""
     sizes = [(33, 130, 256), (48, 127, 768), (49, 1000, 2560), (64, 257, 3072), (47, 2049, 1792), (64, 6000, 1024), (40, 128, 6144),
              (64, 129, 6400), (65, 1024, 2048), (128, 257, 1536), (100, 2048, 2048), (127, 1000, 3072)]
     for words in (32, 36, 40, 68):
